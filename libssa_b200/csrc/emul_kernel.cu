@@ -182,7 +182,8 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
             id = p.order[t / p.qv.n_slots];
         }
         const uint32_t L = p.db.lens[id];
-        const uint32_t Lb = (L + 3u) & ~3u;          // pad to the block end
+        // the 8- and 16-bit lanes score to the block end; the scalar 64-bit code ends at the last residue
+        const uint32_t Lb = (W == 64) ? L : (L + 3u) & ~3u;
         const uint8_t * dseq = p.db.codes + p.db.offsets[id];
         const uint32_t Q = p.qv.qlen[slot];
         const uint32_t qpad = p.qv.qpad[slot];
