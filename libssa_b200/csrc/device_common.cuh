@@ -54,6 +54,13 @@ struct PassSink {
     // the 64-bit pass in int64 arithmetic writes its scores here (same index)
     // and SCORE_IN_WIDE into score[]
     int64_t * score64 = nullptr;
+    // the 16x2 Smith-Waterman kernels at the 16- and 64-bit entry: a pair whose
+    // score leaves their range goes to this list, which the lane emulation
+    // scores from the start; nullptr at the 8-bit entry, where a crossing is
+    // the lane's own overflow and goes to next[]
+    PairTask * redo = nullptr;
+    unsigned int * redo_count = nullptr;
+    uint32_t redo_cap = 0;
 };
 
 // score[] marker of a pair whose exact score is in PassSink::score64
@@ -64,6 +71,27 @@ enum ErrorBits : unsigned int {
     ERR_SCRATCH_OVERFLOW = 2u,
     ERR_PIPELINE = 4u,            // a stripe pipeline ran past its step bound
 };
+
+// Appends (slot, id) to a list; an entry past its end raises the error flag.
+__device__ __forceinline__ void append_task( PairTask * list, unsigned int * count, uint32_t cap, uint32_t slot,
+        uint32_t id, int32_t nblocks, unsigned int * error_flags ) {
+    const unsigned q = atomicAdd( count, 1u );
+    if( q < cap )
+        list[q] = PairTask{ slot, id, nblocks, 0 };
+    else
+        atomicOr( error_flags, ERR_REQUEUE_OVERFLOW );
+}
+
+// A sequence whose running maximum reached the pass's limit in block
+// nblocks - 1: the 8-bit lane's overflow, or a pair for the lane emulation.
+__device__ __forceinline__ void report_crossing( const PassSink & s, uint32_t slot, uint32_t id, int32_t nblocks ) {
+    if( s.redo ) {
+        append_task( s.redo, s.redo_count, s.redo_cap, slot, id, 0, s.error_flags );
+        return;
+    }
+    s.score[(uint64_t) slot * s.score_stride + id] = 255;
+    append_task( s.next, s.next_count, s.next_cap, slot, id, nblocks, s.error_flags );
+}
 
 
 // Parameters of the saturating-lane emulation kernel (emul_kernel.cu).
@@ -168,8 +196,9 @@ struct FastParams {
     const uint32_t * chunk_bounds;
     uint64_t n_units;
     unsigned long long * unit_counter;
-    int gap_oe;                   // (int8) (gapO + gapE)
+    int gap_oe;                   // gapO + gapE at the entry width
     int gap_e;
+    int limit;                    // running maximum that ends a sequence: 255, or the 16x2 range (16- and 64-bit entry)
     PassSink sink;
     int4 * scratch;               // per warp and group slot (4 per warp, 8 for the 4-column kernel): scratch_cols entries
     uint32_t scratch_cols;
@@ -210,8 +239,9 @@ struct QPairParams {
     const uint32_t * chunk_bounds;
     uint64_t n_units;
     unsigned long long * unit_counter;
-    int gap_oe;                   // (int8) (gapO + gapE)
+    int gap_oe;                   // gapO + gapE at the entry width
     int gap_e;
+    int limit;                    // Smith-Waterman: as in FastParams
     PassSink sink;
     int4 * scratch;               // per warp and group: scratch_cols column pairs (H, F of two columns)
     uint32_t scratch_cols;
@@ -219,9 +249,7 @@ struct QPairParams {
     int gap_open;
     const uint32_t * qlen;        // per slot
     const uint32_t * qp_lmax;     // per query pair: longest sequence the kernel scores exactly
-    PairTask * redo;              // longer sequences: (slot, id) for the lane emulation
-    unsigned int * redo_count;
-    uint32_t redo_cap;
+    // (longer sequences go to sink.redo for the lane emulation)
 };
 
 // mb: 4 or 5 resident CTAs per SM (register bound of the instantiation)

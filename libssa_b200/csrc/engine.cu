@@ -493,6 +493,7 @@ private:
     void run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
             uint32_t cap, const std::vector<uint32_t> * slots = nullptr, uint32_t seq_lo = 0,
             uint32_t seq_hi = UINT32_MAX );
+    void run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap );
     int32_t * score_sink() { return serving_ ? d_serve_score_.as<int32_t>() : d_score_.as<int32_t>(); }
     void build_profiles( int width, uint32_t n_slots );
     // scores_from_regions: the hits carry no score yet; take it from the
@@ -690,21 +691,61 @@ static bool needs_int64( const SearchRequest & req, uint32_t max_qlen, uint32_t 
 // Needleman-Wunsch at the 16-bit entry: the query-pair kernel scores exactly
 // the sequences short enough that no value can come near the int16 limits
 // (nw_qpair_kernel); it needs non-positive gap costs.
+// The 64-bit entry takes the same kernel where the score table fits int16.
 static bool nw_fast_eligible( const SearchRequest & req ) {
-    if( req.algo != 1 || req.bit_width != 16 || getenv( "SSA_B200_NO_FAST" ) )
+    if( req.algo != 1 || req.bit_width == 8 || getenv( "SSA_B200_NO_FAST" ) )
         return false;
+    for( int k = 0; k < 1024 && req.bit_width == 64; k++ )
+        if( req.matrix[k] != (int16_t) req.matrix[k] )
+            return false;
     return req.gap_open <= 0 && req.gap_extend <= 0;
 }
 
-static bool fast_eligible( const SearchRequest & req ) {
-    if( req.algo != 0 || req.bit_width != 8 )
+// The running maximum at which the 16x2 Smith-Waterman kernels end a
+// sequence, 0 where they do not apply.  8-bit entry: 255, the lane's own
+// overflow.  At 16 and 64 bits the lane saturates far above (65535) or not at
+// all, and the kernels are exact up to where a 16-bit half could leave its
+// range: a cell below the limit plus one score-table entry stays below 0x7c00
+// (the bound of the fp16 maximum, under the integer one of 32767 - bias); the
+// few sequences that reach it are scored by the lane emulation.  Measured on a
+// B200 against the lane emulation of every pair, which carries one cell per
+// 32-bit lane and reads its profile through L1: 24 queries x 20,000 proteins at
+// the 16-bit entry 98.9 -> 18.8 ms a call (entry pass 92 -> 12 ms), one query of
+// 375 x 10,000 at 64 bits 1.51 -> 0.86 ms.
+static int sw_fast_limit( const SearchRequest & req ) {
+    if( req.algo != 0 || getenv( "SSA_B200_NO_FAST" ) )
+        return 0;
+    // the kernels also use gapO + gapE <= gapE (at the entry width) to let the
+    // next row's F depend on Hdiag + V and E only
+    const int goe = req.bit_width == 8 ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
+    if( req.gap_extend > 0 || goe > 0 || goe > req.gap_extend )
+        return 0;
+    if( req.bit_width == 8 )
+        return 255;
+    int64_t most = 0;
+    for( int k = 0; k < 1024; k++ ) {
+        const int64_t v = (int16_t) req.matrix[k];
+        if( req.bit_width == 64 && v != req.matrix[k] )
+            return 0;
+        most = std::max( most, v );
+        // the kernels score a last block's pad columns (code 0), which the
+        // 64-bit code does not have: they must not raise a score
+        if( req.bit_width == 64 && k < 32 && v > 0 )
+            return 0;
+    }
+    return most <= 8192 ? (int) (0x7c00 - 1024 - most) : 0;
+}
+
+static bool fast_eligible( const SearchRequest & req ) { return sw_fast_limit( req ) > 0; }
+
+// The single-query kernels keep the profile in int8.
+static bool fast_single_eligible( const SearchRequest & req ) {
+    if( !fast_eligible( req ) )
         return false;
-    if( getenv( "SSA_B200_NO_FAST" ) )
-        return false;
-    // the kernel also uses gapO + gapE <= gapE (in 8-bit terms) to let the next
-    // row's F depend on Hdiag + V and E only
-    const int goe8 = (int8_t) (req.gap_open + req.gap_extend);
-    return req.gap_extend <= 0 && goe8 <= 0 && goe8 <= req.gap_extend;
+    for( int k = 0; k < 1024 && req.bit_width != 8; k++ )
+        if( (req.bit_width == 16 ? (int16_t) req.matrix[k] : req.matrix[k]) != (int8_t) req.matrix[k] )
+            return false;
+    return true;
 }
 
 struct FastShape {
@@ -890,8 +931,11 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     CUDA_CHECK( cudaMemcpyAsync( d_bounds_.p, bounds.data(), bounds.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
             stream_ ) );
     CUDA_CHECK( cudaMemcpyAsync( d_group_.p, group_of.data(), nq * sizeof(uint16_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     const uint32_t cols_max = ((db_.max_len + 7u) & ~7u) + 8;
+    unsigned * redo_count = d_counts_.as<unsigned>() + 5;
+    if( req.bit_width != 8 )
+        CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
+    CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     size_t class_first = 0;
     for( int ci = 0; ci < 8; ci++ ) {
         const std::vector<uint32_t> & cls = by_r[ci];
@@ -941,8 +985,14 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         p.chunk_bounds = d_bounds_.as<uint32_t>();
         p.n_units = (uint64_t) n_chunks * cls.size();
         p.unit_counter = unit_counter;
-        p.gap_oe = (int8_t) (req.gap_open + req.gap_extend);
+        p.gap_oe = req.bit_width == 8 ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
         p.gap_e = req.gap_extend;
+        p.limit = sw_fast_limit( req );
+        if( req.bit_width != 8 ) {
+            p.sink.redo = d_list_b_.as<PairTask>();
+            p.sink.redo_count = redo_count;
+            p.sink.redo_cap = cap;
+        }
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
         p.sink.next = next;
@@ -961,9 +1011,11 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_class_[ri], 0 ) );
         class_first += cls.size();
     }
+    if( req.bit_width != 8 )
+        run_redo( req, nq, next, next_count, cap );
     if( !fallback.empty() ) {
         const uint64_t n_ne = db_.order_desc.size();
-        run_pass( 0, 8, req, nq, nullptr, (uint64_t) fallback.size() * n_ne, true, next, next_count, cap,
+        run_pass( 0, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_ne, true, next, next_count, cap,
                 d_slots_.as<uint32_t>() + n_shaped, (uint32_t) fallback.size() );
     }
 }
@@ -1061,6 +1113,18 @@ static int choose_qpair_rows( uint32_t Q, uint32_t * passes, int pinned, int buc
     return best_r;
 }
 
+// The pairs that a 16x2 entry pass left out of its range (16- and 64-bit
+// entry): the lane emulation at the entry width.
+void Engine::run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap ) {
+    unsigned n_redo = 0;
+    CUDA_CHECK( cudaMemcpyAsync( &n_redo, d_counts_.as<unsigned>() + 5, sizeof(unsigned), cudaMemcpyDeviceToHost,
+            stream_ ) );
+    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+    n_redo = std::min( n_redo, cap );
+    if( n_redo )
+        run_pass( req.algo, req.bit_width, req, nq, d_list_b_.as<PairTask>(), n_redo, false, next, next_count, cap );
+}
+
 void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
         uint32_t cap, const std::vector<uint32_t> * slots, uint32_t seq_lo, uint32_t seq_hi ) {
     // the sequences order_desc[seq_lo, seq_hi) (all by default)
@@ -1147,8 +1211,10 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     d_qp_lmax_.ensure( qp_lmax.size() * sizeof(uint32_t) );
     CUDA_CHECK( cudaMemcpyAsync( d_qp_lmax_.p, qp_lmax.data(), qp_lmax.size() * sizeof(uint32_t),
             cudaMemcpyHostToDevice, stream_ ) );
+    // pairs outside the kernels' range, for the lane emulation (the 8-bit entry has none)
+    const bool redo = req.bit_width != 8;
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
-    if( nw )
+    if( redo )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
     CUDA_CHECK( cudaMemcpyAsync( d_qp_off_.p, qp_off.data(), qp_off.size() * sizeof(uint64_t), cudaMemcpyHostToDevice,
             stream_ ) );
@@ -1162,7 +1228,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     if( n_qp ) {
         CUDA_CHECK( launch_build_profile_qp( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
                 d_qp_slots_.as<uint32_t>(), n_qp, d_qp_rows_.as<uint32_t>(), d_matrix_.as<int64_t>(),
-                d_qp_prof_.as<uint32_t>(), d_qp_off_.as<uint64_t>(), nw ? 16 : 8, stream_ ) );
+                d_qp_prof_.as<uint32_t>(), d_qp_off_.as<uint64_t>(), req.bit_width == 8 ? 8 : 16, stream_ ) );
         launches_++;
     }
 
@@ -1248,8 +1314,9 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         p.n_units = (uint64_t) n_chunks * cls.size();
         p.unit_counter = unit_counter;
         // the 8-bit Smith-Waterman lanes add the int8 truncation of gapO + gapE
-        p.gap_oe = nw ? req.gap_open + req.gap_extend : (int8_t) (req.gap_open + req.gap_extend);
+        p.gap_oe = req.bit_width != 8 ? req.gap_open + req.gap_extend : (int8_t) (req.gap_open + req.gap_extend);
         p.gap_e = req.gap_extend;
+        p.limit = nw ? 0 : sw_fast_limit( req );
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
         p.sink.next = next;
@@ -1264,9 +1331,11 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         p.gap_open = req.gap_open;
         p.qlen = d_qlen_.as<uint32_t>();
         p.qp_lmax = d_qp_lmax_.as<uint32_t>();
-        p.redo = d_list_b_.as<PairTask>();
-        p.redo_count = redo_count;
-        p.redo_cap = cap;
+        if( redo ) {
+            p.sink.redo = d_list_b_.as<PairTask>();
+            p.sink.redo_count = redo_count;
+            p.sink.redo_cap = cap;
+        }
         if( timing )
             CUDA_CHECK( cudaEventRecord( ev_cls_t_[2 * ri], class_stream_[ri] ) );
         CUDA_CHECK( launch( p, grid, nullptr ) );
@@ -1294,15 +1363,8 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
                     cells / (ms * 1e-3) / 1e9 );
         }
     }
-    if( nw ) {
-        // sequences beyond a pair's exact range: the 16-bit lane emulation
-        unsigned n_redo = 0;
-        CUDA_CHECK( cudaMemcpyAsync( &n_redo, redo_count, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        n_redo = std::min( n_redo, cap );
-        if( n_redo )
-            run_pass( 1, 16, req, nq, d_list_b_.as<PairTask>(), n_redo, false, next, next_count, cap );
-    }
+    if( redo )
+        run_redo( req, nq, next, next_count, cap );
     if( !fallback.empty() ) {
         d_slots_.ensure( fallback.size() * sizeof(uint32_t) );
         CUDA_CHECK( cudaMemcpyAsync( d_slots_.p, fallback.data(), fallback.size() * sizeof(uint32_t),
@@ -1405,10 +1467,11 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
             const uint64_t seg_pairs = (uint64_t) nq * (hi - lo);
             CUDA_CHECK( cudaEventRecord( ev_seg_[0], stream_ ) );
             auto run_entry = [&]() {
-                if( (fast_eligible( req ) && (nq >= 2 || streaming_) && !getenv( "SSA_B200_NO_QPAIR" )) ||
+                if( (fast_eligible( req ) && (nq >= 2 || streaming_ || !fast_single_eligible( req )) &&
+                            !getenv( "SSA_B200_NO_QPAIR" )) ||
                         nw_fast_eligible( req ) )
                     run_qpair_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap, nullptr, lo, hi );
-                else if( fast_eligible( req ) )
+                else if( fast_single_eligible( req ) )
                     run_fast_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap );
                 else
                     run_pass( req.algo, entry, req, nq, nullptr, seg_pairs, true, d_list_a_.as<PairTask>(), cnt + 0,

@@ -43,7 +43,6 @@ namespace ssa {
 
 constexpr uint32_t FAST_BIAS = 1024u;
 constexpr uint32_t FAST_BIAS2 = (FAST_BIAS << 16) | FAST_BIAS;
-constexpr int FAST_THRESHOLD = 255;           // 8-bit lane overflow: running max reaches 255
 
 __device__ __forceinline__ uint32_t prmt( uint32_t a, uint32_t b, uint32_t sel ) {
     uint32_t d;
@@ -95,7 +94,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast_kernel( FastParams p ) {
             warp_in_cta * 32u;
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
-    const uint32_t TH = FAST_BIAS + FAST_THRESHOLD;
+    const uint32_t TH = FAST_BIAS + (uint32_t) p.limit;
     uint64_t loaded_key = ~0ull;
 
     for( ;; ) {
@@ -263,12 +262,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast_kernel( FastParams p ) {
                         p.sink.score[(uint64_t) slot * p.sink.score_stride + idv[h]] = (int32_t) (sv[h] - FAST_BIAS);
                     }
                     else {
-                        p.sink.score[(uint64_t) slot * p.sink.score_stride + idv[h]] = FAST_THRESHOLD;
-                        unsigned q = atomicAdd( p.sink.next_count, 1u );
-                        if( q < p.sink.next_cap )
-                            p.sink.next[q] = PairTask{ slot, idv[h], cross[h] / 4 + 1, 0 };
-                        else
-                            atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                        report_crossing( p.sink, slot, idv[h], cross[h] / 4 + 1 );
                     }
                 }
             }
@@ -323,8 +317,6 @@ cudaError_t launch_sw_fast( int R, const FastParams & p, int grid, cudaStream_t 
 // query (H and F of four columns, 32 bytes per block) goes through the
 // group's scratch row, thread 0 reading it one block ahead.  G (threads per
 // pair) is 4, 8, 16 or 32, so a warp holds up to 8 groups; R is 8, 16 or 24.
-constexpr uint32_t FAST_CROSS_ADD =
-        ((0x8000u - (FAST_BIAS + FAST_THRESHOLD)) << 16) | (0x8000u - (FAST_BIAS + FAST_THRESHOLD));
 
 template <int R>
 __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
@@ -336,6 +328,8 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
     int8_t * slice = sprof + (size_t) warp_in_cta * 32u * p.slice_rows;
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
+    // sets bit 15 of a half exactly when the half is >= FAST_BIAS + limit
+    const uint32_t CROSS_ADD = (0x8000u - (FAST_BIAS + (uint32_t) p.limit)) * 0x10001u;
     uint64_t loaded_key = ~0ull;
 
     for( ;; ) {
@@ -518,7 +512,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
                         out_f[j] = f[j];
                     }
                     // first block at which this thread's maximum reached 255
-                    const uint32_t ge = (smax + FAST_CROSS_ADD) & 0x80008000u;
+                    const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )
                             cross_lo = min( cross_lo, b );
@@ -560,12 +554,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
                         *dst = (int32_t) (sv[h] - FAST_BIAS);
                     }
                     else {
-                        *dst = FAST_THRESHOLD;
-                        unsigned q = atomicAdd( p.sink.next_count, 1u );
-                        if( q < p.sink.next_cap )
-                            p.sink.next[q] = PairTask{ slot, idv[h], cross[h] + 1, 0 };
-                        else
-                            atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                        report_crossing( p.sink, slot, idv[h], cross[h] + 1 );
                     }
                 }
             }

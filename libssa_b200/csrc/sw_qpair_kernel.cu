@@ -39,9 +39,11 @@ namespace ssa {
 
 constexpr uint32_t QP_BIAS = 1024u;
 constexpr uint32_t QP_BIAS2 = (QP_BIAS << 16) | QP_BIAS;
-// adding this per half sets bit 15 exactly when the half is >= 1024 + 255
+// adding this per half sets bit 15 exactly when the half is >= 1024 + limit
 // (halves stay in [0, 32767], so no carry crosses into the other half)
-constexpr uint32_t QP_CROSS_ADD = ((0x8000u - (QP_BIAS + 255u)) << 16) | (0x8000u - (QP_BIAS + 255u));
+__device__ __forceinline__ uint32_t qp_cross_add( int limit ) {
+    return (0x8000u - (QP_BIAS + (uint32_t) limit)) * 0x10001u;
+}
 constexpr int QP_THREADS = QP_THREADS_PER_CTA;
 
 // MB: resident CTAs per SM the register allocation is bounded for (4: up to
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
     const int g = lane / G;                      // group within the warp
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
+    const uint32_t CROSS_ADD = qp_cross_add( p.limit );
     int4 * scratch = p.scratch + ((uint64_t) warp_global * QP_GPW + (uint32_t) g) * p.scratch_cols;
     uint64_t loaded_key = ~0ull;
 
@@ -209,7 +212,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
                     out_h1 = H[R - 1];
                     out_f1 = fb;
                     // first column pair at which this thread's maximum reached 255
-                    const uint32_t ge = (smax + QP_CROSS_ADD) & 0x80008000u;
+                    const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )
                             cross_a = min( cross_a, cp );
@@ -248,12 +251,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
                     }
                     else {
                         // columns 2cp and 2cp + 1 lie in 4-column block cp / 2
-                        *dst = 255;
-                        unsigned q = atomicAdd( p.sink.next_count, 1u );
-                        if( q < p.sink.next_cap )
-                            p.sink.next[q] = PairTask{ slots[h], id, (cross[h] >> 1) + 1, 0 };
-                        else
-                            atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                        report_crossing( p.sink, slots[h], id, (cross[h] >> 1) + 1 );
                     }
                 }
             }
@@ -315,6 +313,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
     const int g = lane / G;
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
+    const uint32_t CROSS_ADD = qp_cross_add( p.limit );
     int4 * scratch = p.scratch + ((uint64_t) warp_global * QP_GPW + (uint32_t) g) * p.scratch_cols;
     uint64_t loaded_key = ~0ull;
 
@@ -497,7 +496,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                         out_f[j] = f[j];
                     }
                     // first block at which this thread's maximum reached 255
-                    const uint32_t ge = (smax + QP_CROSS_ADD) & 0x80008000u;
+                    const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )
                             cross_a = min( cross_a, b );
@@ -539,12 +538,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                         *dst = (int32_t) (sv[h] - QP_BIAS);
                     }
                     else {
-                        *dst = 255;
-                        unsigned q = atomicAdd( p.sink.next_count, 1u );
-                        if( q < p.sink.next_cap )
-                            p.sink.next[q] = PairTask{ slots[h], id, cross[h] + 1, 0 };
-                        else
-                            atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                        report_crossing( p.sink, slots[h], id, cross[h] + 1 );
                     }
                 }
             }
@@ -752,11 +746,8 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
                 for( int h = 0; h < 2; h++ ) {
                     if( slots[h] == 0xffffffffu )
                         continue;
-                    const unsigned q = atomicAdd( p.redo_count, 1u );
-                    if( q < p.redo_cap )
-                        p.redo[q] = PairTask{ slots[h], id, 0, 0 };
-                    else
-                        atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                    append_task( p.sink.redo, p.sink.redo_count, p.sink.redo_cap, slots[h], id, 0,
+                            p.sink.error_flags );
                 }
             }
             const uint32_t ncp = exact ? (((L + 3u) & ~3u) >> 1) : 0u;
@@ -1062,11 +1053,8 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                 for( int h = 0; h < 2; h++ ) {
                     if( slots[h] == 0xffffffffu )
                         continue;
-                    const unsigned q = atomicAdd( p.redo_count, 1u );
-                    if( q < p.redo_cap )
-                        p.redo[q] = PairTask{ slots[h], id, 0, 0 };
-                    else
-                        atomicOr( p.sink.error_flags, ERR_REQUEUE_OVERFLOW );
+                    append_task( p.sink.redo, p.sink.redo_count, p.sink.redo_cap, slots[h], id, 0,
+                            p.sink.error_flags );
                 }
             }
             const uint32_t nb = exact ? (L + 3u) >> 2 : 0u;         // 4-column blocks
