@@ -1695,6 +1695,9 @@ static int64_t max_abs_step( const SearchRequest & req ) {
     return m;
 }
 
+// Least direction memory of one traceback wave (automatic budget).
+constexpr uint64_t TB_MIN_BUDGET = (uint64_t) 256 << 20;
+
 void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>> & out,
         const std::vector<std::pair<uint32_t, uint32_t>> & lists, SearchStats & stats, bool scores_from_regions ) {
     std::vector<TbHit> hits;
@@ -1932,7 +1935,9 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         ops_bytes[h] = (uint64_t) (rg.a_end - rg.a_begin + 1) + (uint64_t) (rg.b_end - rg.b_begin + 1) + 1;
         total_dir += dir_words[h] * sizeof(uint16_t);
     }
-    const uint64_t budget = traceback_budget();
+    // matrices within the smallest automatic budget make one wave whatever the
+    // free memory is: asking the driver for it costs up to milliseconds
+    const uint64_t budget = (!tb_budget_ && total_dir <= TB_MIN_BUDGET) ? TB_MIN_BUDGET : traceback_budget();
     auto region_group = [&]( uint32_t h ) {
         if( fused )
             return tb_group( h_qlen_[hits[h].qslot], db_.len[hits[h].id] );
@@ -2108,8 +2113,7 @@ uint64_t Engine::traceback_budget() {
     CUDA_CHECK( cudaMemGetInfo( &free_b, &total_b ) );
     const uint64_t avail = (uint64_t) free_b + d_tb_dirs_.bytes;
     const uint64_t reserve = std::max<uint64_t>( (uint64_t) 4 << 30, (uint64_t) total_b / 16 );
-    const uint64_t floor = (uint64_t) 256 << 20;
-    return avail > reserve + floor ? avail - reserve : floor;
+    return avail > reserve + TB_MIN_BUDGET ? avail - reserve : TB_MIN_BUDGET;
 }
 
 // ---- long pairs -------------------------------------------------------------------
