@@ -20,41 +20,50 @@
 
 #include <algorithm>
 #include <cstring>
-#include <tuple>
 
 namespace ssa {
 
-// Report order of a list of sequences scheduled on `lanes` channels, where
-// sequence k occupies nb[k] blocks.  Returns indices into the list.
-static void simulate_lanes( int lanes, const std::vector<int32_t> & nb, std::vector<uint32_t> & order ) {
+// When every sequence of a list scheduled on `lanes` channels reports, where
+// sequence k occupies nb[k] blocks: the sequences report in ascending key
+// order.  A sequence enters the channel that frees first, the lowest among
+// equals; key = its last block, then its channel.  The channels are kept as a
+// binary heap of (free block, channel), so a sequence costs log2(lanes) steps.
+static void simulate_lanes( int lanes, const std::vector<int32_t> & nb, std::vector<int64_t> & key ) {
     const size_t n = nb.size();
-    order.clear();
-    if( n == 0 )
-        return;
-    // free time of each lane; a lane that frees at block t takes the next
-    // sequence in lane order among all lanes freeing at t
-    std::vector<int64_t> free_at( (size_t) lanes, 0 );
-    std::vector<std::tuple<int64_t, int, uint32_t>> ends;
-    ends.reserve( n );
+    key.resize( n );
+    int64_t heap[64];                              // free block << 6 | channel
+    if( lanes > 64 )
+        fatal( "Internal error: %d channels.", lanes );
+    for( int c = 0; c < lanes; c++ )
+        heap[c] = c;
     for( size_t k = 0; k < n; k++ ) {
-        int best = 0;
-        for( int c = 1; c < lanes; c++ )
-            if( free_at[c] < free_at[best] )
-                best = c;
-        const int64_t t_end = free_at[best] + nb[k];
-        ends.emplace_back( t_end, best, (uint32_t) k );
-        free_at[best] = t_end;
+        const int64_t v = heap[0] + ((int64_t) nb[k] << 6);
+        key[k] = v;
+        int at = 0;
+        for( int c = 1; c < lanes; c = 2 * at + 1 ) {
+            if( c + 1 < lanes && heap[c + 1] < heap[c] )
+                c++;
+            if( heap[c] >= v )
+                break;
+            heap[at] = heap[c];
+            at = c;
+        }
+        heap[at] = v;
     }
-    std::sort( ends.begin(), ends.end() );
-    order.resize( n );
-    for( size_t k = 0; k < n; k++ )
-        order[k] = std::get<2>( ends[k] );
+}
+
+// The indices of `pick` in report order: by key, then position in the list (a
+// channel that takes a sequence of no blocks reports twice at the same block).
+static void report_order( const std::vector<int64_t> & key, std::vector<uint32_t> & pick ) {
+    std::sort( pick.begin(), pick.end(),
+            [&]( uint32_t x, uint32_t y ) { return key[x] != key[y] ? key[x] < key[y] : x < y; } );
 }
 
 void schedule_ranks( const HostDb & db, size_t chunk_size, int lanes, std::vector<uint32_t> & rank ) {
     rank.assign( db.n_ids, 0 );
     std::vector<uint32_t> ids;
     std::vector<int32_t> nb;
+    std::vector<int64_t> key;
     std::vector<uint32_t> order;
     const uint64_t cs = (uint64_t) chunk_size * db.upi;    // a chunk of records, in units
     for( uint64_t start = 0; start < db.n_ids; start += cs ) {
@@ -67,7 +76,11 @@ void schedule_ranks( const HostDb & db, size_t chunk_size, int lanes, std::vecto
             ids.push_back( (uint32_t) id );
             nb.push_back( (int32_t) ((db.len[id] + 3) / 4) );
         }
-        simulate_lanes( lanes, nb, order );
+        simulate_lanes( lanes, nb, key );
+        order.resize( ids.size() );
+        for( size_t k = 0; k < order.size(); k++ )
+            order[k] = (uint32_t) k;
+        report_order( key, order );
         for( size_t k = 0; k < order.size(); k++ )
             rank[ids[order[k]]] = (uint32_t) k;
     }
@@ -88,8 +101,9 @@ struct MinHeap {
 
     explicit MinHeap( size_t k ) : alloc( k ) { a.reserve( k ); }
 
-    bool full() const { return a.size() >= alloc; }
-    int64_t root() const { return a[0].score; }
+    // the score that an element has to exceed to enter (INT64_MIN: any enters);
+    // it never falls, so an element at or below it can be left out from here on
+    int64_t bar() const { return a.size() < alloc ? INT64_MIN : alloc ? a[0].score : INT64_MAX; }
 
     void add( uint32_t id, int64_t score, uint32_t q = 0 ) {
         if( alloc == 0 )
@@ -148,8 +162,9 @@ void replay_query( const HostDb & db, const SearchRequest & req, const ReplayQue
     BlockMap ovfE{ rq.ovf_entry }, ovf16{ rq.ovf16 };
 
     std::vector<std::pair<uint32_t, uint32_t>> cand;   // (rank, id)
-    std::vector<uint32_t> ids, order, order16, next, list64;
+    std::vector<uint32_t> ids, reports, order16, next, list64;
     std::vector<int32_t> nb;
+    std::vector<int64_t> key, key16;
 
     for( uint64_t start = 0; start < db.n_ids; start += cs ) {
         const uint64_t end = std::min<uint64_t>( db.n_ids, start + cs );
@@ -158,19 +173,17 @@ void replay_query( const HostDb & db, const SearchRequest & req, const ReplayQue
         // src/algo/16/search_16.c:785, src/algo/64/search_64.c:963)
         if( db.nonempty_before[end] == db.nonempty_before[start] )
             break;
-        const bool has_ovf = req.bit_width != 64 && ovfE.lower( (uint32_t) start ) < rq.ovf_entry.size()
-                && rq.ovf_entry[ovfE.lower( (uint32_t) start )].first < end;
+        const int64_t bar = heap.bar();
+        const size_t e0 = ovfE.lower( (uint32_t) start );
+        const bool has_ovf = req.bit_width != 64 && e0 < rq.ovf_entry.size() && rq.ovf_entry[e0].first < end;
         if( !has_ovf ) {
             // every sequence of the chunk reported at the entry pass: the
             // order is the query-independent schedule
-            const bool filter = heap.full();
-            const int64_t r = filter ? heap.root() : 0;
             cand.clear();
             for( uint64_t id = start; id < end; id++ ) {
                 if( db.len[id] == 0 )
                     continue;
-                const int64_t s = rq.score_of( id );
-                if( filter && s <= r )
+                if( bar != INT64_MIN && rq.score_of( (uint32_t) id ) <= bar )
                     continue;
                 cand.emplace_back( req.bit_width == 64 ? (uint32_t) (id - start) : rank_entry[id], (uint32_t) id );
             }
@@ -181,54 +194,73 @@ void replay_query( const HostDb & db, const SearchRequest & req, const ReplayQue
                 heap.add( c.second, rq.score_of( c.second ) );
             continue;
         }
-        // the chunk has overflowing sequences: re-run its schedules
+        // the chunk has overflowing sequences: its counters follow from the
+        // lists alone, its schedules are re-run only when one of its
+        // sequences can enter the heap
+        const size_t e1 = ovfE.lower( (uint32_t) end );
+        const size_t s0 = ovf16.lower( (uint32_t) start ), s1 = ovf16.lower( (uint32_t) end );
+        (req.bit_width == 8 ? counts.overflow8 : counts.overflow16) += e1 - e0;
+        if( req.bit_width == 8 )
+            counts.overflow16 += s1 - s0;
+        bool reported = false, overflowed = false;     // a candidate that reports / overflows at the entry width
+        {
+            size_t at = e0;
+            for( uint64_t id = start; id < end && !overflowed; id++ ) {
+                const bool ovf = at < e1 && rq.ovf_entry[at].first == id;
+                at += ovf;
+                if( db.len[id] == 0 || (bar != INT64_MIN && rq.score_of( (uint32_t) id ) <= bar) )
+                    continue;
+                (ovf ? overflowed : reported) = true;
+            }
+        }
+        if( !reported && !overflowed )
+            continue;
         ids.clear();
         nb.clear();
-        for( uint64_t id = start; id < end; id++ ) {
-            if( db.len[id] == 0 )
-                continue;
-            int32_t b;
-            if( !ovfE.find( (uint32_t) id, b ) )
-                b = (int32_t) ((db.len[id] + 3) / 4);
-            ids.push_back( (uint32_t) id );
-            nb.push_back( b );
-        }
-        simulate_lanes( lanes_entry, nb, order );
+        reports.clear();
         next.clear();
-        const size_t n_entry_before = next.size();
-        for( uint32_t k : order ) {
-            const uint32_t id = ids[k];
-            int32_t b;
-            if( ovfE.find( id, b ) )
-                next.push_back( id );
-            else
-                heap.add( id, rq.score_of( id ) );
-        }
-        if( req.bit_width == 8 )
-            counts.overflow8 += next.size() - n_entry_before;
-        else
-            counts.overflow16 += next.size() - n_entry_before;
-        if( req.bit_width == 8 && !next.empty() ) {
-            nb.clear();
-            for( uint32_t id : next ) {
-                int32_t b;
-                if( !ovf16.find( id, b ) )
-                    b = (int32_t) ((db.len[id] + 3) / 4);
+        {
+            size_t at = e0;
+            for( uint64_t id = start; id < end; id++ ) {
+                const bool ovf = at < e1 && rq.ovf_entry[at].first == id;
+                const int32_t b = ovf ? rq.ovf_entry[at].second : (int32_t) ((db.len[id] + 3) / 4);
+                at += ovf;
+                if( db.len[id] == 0 )
+                    continue;
+                if( ovf )
+                    next.push_back( (uint32_t) ids.size() );
+                else if( bar == INT64_MIN || rq.score_of( (uint32_t) id ) > bar )
+                    reports.push_back( (uint32_t) ids.size() );
+                ids.push_back( (uint32_t) id );
                 nb.push_back( b );
             }
-            simulate_lanes( req.lanes16, nb, order16 );
+        }
+        simulate_lanes( lanes_entry, nb, key );
+        report_order( key, reports );
+        for( uint32_t k : reports )
+            heap.add( ids[k], rq.score_of( ids[k] ) );
+        if( !overflowed )
+            continue;
+        report_order( key, next );
+        for( uint32_t & k : next )
+            k = ids[k];
+        if( req.bit_width == 8 ) {
+            nb.clear();
+            order16.clear();
             list64.clear();
-            for( uint32_t k : order16 ) {
-                const uint32_t id = next[k];
+            for( uint32_t k = 0; k < (uint32_t) next.size(); k++ ) {
                 int32_t b;
-                if( ovf16.find( id, b ) )
-                    list64.push_back( id );
-                else
-                    heap.add( id, rq.score_of( id ) );
+                const bool ovf = s1 > s0 && ovf16.find( next[k], b );
+                (ovf ? list64 : order16).push_back( k );
+                nb.push_back( ovf ? b : (int32_t) ((db.len[next[k]] + 3) / 4) );
             }
-            counts.overflow16 += list64.size();
-            for( uint32_t id : list64 )
-                heap.add( id, rq.score_of( id ) );
+            simulate_lanes( req.lanes16, nb, key16 );
+            report_order( key16, order16 );
+            report_order( key16, list64 );
+            for( uint32_t k : order16 )
+                heap.add( next[k], rq.score_of( next[k] ) );
+            for( uint32_t k : list64 )
+                heap.add( next[k], rq.score_of( next[k] ) );
         }
         else {
             for( uint32_t id : next )
@@ -274,6 +306,7 @@ void replay_frames( const HostDb & db, const SearchRequest & req, const ReplayQu
     auto blocks = [&]( uint32_t u ) { return (int32_t) ((db.len[u] + 3) / 4); };
     std::vector<uint32_t> units, order, ovf_chunk, list64;
     std::vector<int32_t> nb;
+    std::vector<int64_t> key;
     for( uint64_t start = 0; start < db.n_ids; start += cs ) {
         const uint64_t end = std::min<uint64_t>( db.n_ids, start + cs );
         if( db.nonempty_before[end] == db.nonempty_before[start] )
@@ -282,20 +315,40 @@ void replay_frames( const HostDb & db, const SearchRequest & req, const ReplayQu
         for( uint64_t u = start; u < end; u++ )
             if( db.len[u] )
                 units.push_back( (uint32_t) u );
+        // a chunk none of whose pairs can enter the heap leaves it as it is
+        const int64_t bar = heap.bar();
+        bool any = bar == INT64_MIN;
+        for( uint32_t q = 0; q < F && !any; q++ )
+            for( size_t k = 0; k < units.size() && !any; k++ )
+                any = rq[q].score_of( units[k] ) > bar;
         if( req.bit_width == 64 ) {
-            for( uint32_t q = 0; q < F; q++ )
+            for( uint32_t q = 0; q < F && any; q++ )
                 for( uint32_t u : units )
                     heap.add( u, rq[q].score_of( u ), q );
             continue;
         }
+        // the chunk's overflow list: the overflowing units of every query
+        // sequence, in report order (in list order where only its counters count)
         ovf_chunk.clear();
         for( uint32_t q = 0; q < F; q++ ) {
-            nb.clear();
-            for( uint32_t u : units ) {
-                int32_t b;
-                nb.push_back( ovfE[q].find( u, b ) ? b : blocks( u ) );
+            const size_t e0 = ovfE[q].lower( (uint32_t) start ), e1 = ovfE[q].lower( (uint32_t) end );
+            if( !any ) {
+                for( size_t e = e0; e < e1; e++ )
+                    ovf_chunk.push_back( ovfE[q].v[e].first );
+                continue;
             }
-            simulate_lanes( lanes_entry, nb, order );
+            nb.clear();
+            order.clear();
+            size_t at = e0;
+            for( uint32_t k = 0; k < (uint32_t) units.size(); k++ ) {
+                const bool ovf = at < e1 && ovfE[q].v[at].first == units[k];
+                nb.push_back( ovf ? ovfE[q].v[at].second : blocks( units[k] ) );
+                at += ovf;
+                if( ovf || rq[q].score_of( units[k] ) > bar || bar == INT64_MIN )
+                    order.push_back( k );
+            }
+            simulate_lanes( lanes_entry, nb, key );
+            report_order( key, order );
             for( uint32_t k : order ) {
                 const uint32_t u = units[k];
                 int32_t b;
@@ -312,29 +365,37 @@ void replay_frames( const HostDb & db, const SearchRequest & req, const ReplayQu
             list64.clear();
             for( uint32_t q = 0; q < F; q++ ) {
                 // a pair that did not overflow at 8 bits reports at 16 bits too
+                const size_t s0 = ovf16[q].lower( (uint32_t) start );
+                const bool none64 = s0 == ovf16[q].v.size() || ovf16[q].v[s0].first >= end;
+                if( !any && none64 )
+                    continue;
                 nb.clear();
-                for( uint32_t u : ovf_chunk ) {
+                order.clear();
+                for( uint32_t k = 0; k < (uint32_t) ovf_chunk.size(); k++ ) {
                     int32_t b8, b16;
-                    nb.push_back( (ovfE[q].find( u, b8 ) && ovf16[q].find( u, b16 )) ? b16 : blocks( u ) );
+                    const uint32_t u = ovf_chunk[k];
+                    nb.push_back( (!none64 && ovfE[q].find( u, b8 ) && ovf16[q].find( u, b16 )) ? b16 : blocks( u ) );
+                    order.push_back( k );
                 }
-                simulate_lanes( req.lanes16, nb, order );
+                simulate_lanes( req.lanes16, nb, key );
+                report_order( key, order );
                 for( uint32_t k : order ) {
                     const uint32_t u = ovf_chunk[k];
                     int32_t b8, b16;
-                    if( ovfE[q].find( u, b8 ) && ovf16[q].find( u, b16 ) )
+                    if( !none64 && ovfE[q].find( u, b8 ) && ovf16[q].find( u, b16 ) )
                         list64.push_back( u );
                     else
                         heap.add( u, rq[q].score_of( u ), q );
                 }
             }
             counts.overflow16 += list64.size();
-            for( uint32_t q = 0; q < F; q++ )
+            for( uint32_t q = 0; q < F && any; q++ )
                 for( uint32_t u : list64 )
                     heap.add( u, rq[q].score_of( u ), q );
         }
         else {
             counts.overflow16 += ovf_chunk.size();
-            for( uint32_t q = 0; q < F; q++ )
+            for( uint32_t q = 0; q < F && any; q++ )
                 for( uint32_t u : ovf_chunk )
                     heap.add( u, rq[q].score_of( u ), q );
         }
