@@ -122,14 +122,10 @@ struct TbRegion {
     int32_t a_begin, a_end;   // query rows
     int32_t b_begin, b_end;   // database columns
     int32_t fwd_score;        // SW: forward-pass maximum; NW: H(a_end, b_end) from the direction pass
-    // layout of the hit's direction words: words per column (query rows / 8,
-    // rounded up) and the first database column stored
-    int32_t dir_words, dir_col0;
+    int32_t dir_steps;        // wavefront steps per stripe in the hit's direction bytes (columns + 31)
+    int32_t pad_;
     int32_t status;           // 0 ok, 1 no positive cell, 2 reverse pass found nothing
 };
-
-// Query rows per 16-bit direction word (2 bits per cell).
-constexpr int TB_WORD_ROWS = 8;
 
 struct TbParams {
     DbView db;
@@ -138,21 +134,29 @@ struct TbParams {
     const uint32_t * qlen;
     const int64_t * matrix;     // 32x32 [(row << 5) + col]
     int gap_open, gap_extend;
-    const TbHit * hits;
+    const TbHit * hits;         // most stripes first
     uint32_t n_hits;
     TbRegion * regions;
-    int4 * scratch;             // per group of warps on one hit
-    uint32_t scratch_cols;
     int32_t * last_h;           // per hit: forward pass last-row H (query-indexed)
     int32_t * last_e;           // per hit: forward pass last-row vertical gap
     const uint64_t * last_off;  // per hit offset into last_h / last_e
-    uint16_t * dirs;            // per hit direction words
+    // per hit direction bytes, 2 bits per cell: [stripe][wavefront step][lane][R / 4]
+    uint8_t * dirs;
     const uint64_t * dir_off;   // per hit offset into dirs
     char * ops;                 // per hit reversed op string
     const uint64_t * ops_off;
     uint32_t * ops_len;
     unsigned int * error_flags;
-    unsigned long long * hit_counters;   // forward, reverse, directions: next hit to take (start at 0)
+    // the stripes of the pass (stream_stripes.cuh)
+    const uint32_t * cum;       // first ticket of stripe i, i = 0 .. levels
+    uint32_t levels;            // stripes of the hit with the most
+    uint32_t n_tickets;
+    unsigned long long * counter;   // next ticket (0 at the start)
+    uint32_t * progress;        // per ticket (0 at the start)
+    int4 * result;              // per ticket: end or begin cell of the stripes so far
+    int2 * boundary;            // per hit with several stripes: (H, F) per database column
+    const uint64_t * bnd_off;   // per hit offset into boundary
+    int32_t * limit;            // per hit: last column worth computing in the reverse pass
 };
 
 // Kernel launchers.
@@ -169,11 +173,13 @@ cudaError_t preload_emul64();
 cudaError_t launch_build_profile64( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
         const uint32_t * qpad, const uint64_t * prof_off, const int64_t * matrix, int64_t * prof, uint32_t n_slots,
         cudaStream_t st );
-// group: warps per hit, 1, 2 or 4 (scratch: one boundary row per group)
-cudaError_t launch_tb_regions( const TbParams & p, int group, int grid, cudaStream_t st, cudaEvent_t * ev );
-cudaError_t launch_tb_paths( const TbParams & p, int group, int grid, cudaStream_t st, cudaEvent_t * ev );
-cudaError_t launch_tb_fused( const TbParams & p, int group, int grid, cudaStream_t st, cudaEvent_t * ev );
-
+// Traceback passes: R query rows per lane (4 or 8), p8: the score table fits int8.
+cudaError_t launch_tb_forward( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_reverse( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_directions( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
+// forward and directions in one sweep (Smith-Waterman, symmetric score table)
+cudaError_t launch_tb_fwddir( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_walk( const TbParams & p, int R, cudaStream_t st );
 
 // ---- fast Smith-Waterman entry pass (sw_fast_kernel.cu) --------------------
 // Residue code used after a sequence's last 4-column block in the pair layout;

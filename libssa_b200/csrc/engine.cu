@@ -453,14 +453,15 @@ public:
             &d_scratch_fast_[0], &d_scratch_fast_[1], &d_scratch_fast_[2], &d_scratch_fast_[3], &d_scratch_fast_[4],
             &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_qcodes_, &d_qoff_, &d_qlen_, &d_qpad_,
             &d_prof_off_, &d_prof_, &d_matrix_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
-            &d_tb_hits_, &d_tb_regions_, &d_tb_last_, &d_tb_last_off_, &d_tb_dirs_, &d_tb_dir_off_, &d_tb_ops_,
-            &d_tb_ops_off_, &d_tb_ops_len_, &d_qp_prof_, &d_qp_off_, &d_qp_rows_, &d_qp_slots_, &d_qp_units_,
-            &d_serve_score_, &d_qp_lmax_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_, &d_scratch2_, &d_scratch4_,
+            &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_, &d_qp_off_, &d_qp_rows_, &d_qp_slots_, &d_qp_units_,
+            &d_serve_score_, &d_qp_lmax_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_,
             &d_seg_[0], &d_seg_[1], &d_gather_codes_, &d_gather_off_, &d_gather_len_, &d_prof64_, &d_score64_ };
         for( DevBuf * b : bufs )
             b->release();
         h_score_.release();
         h_score64_.release();
+        h_tb_in_.release();
+        h_tb_out_.release();
         h_stage_.release();
         resident_seg_ = -1;
         streaming_ = false;
@@ -545,10 +546,9 @@ private:
     cudaEvent_t ev_seg_[2] = {};     // around one segment's entry pass
     cudaEvent_t ev_tb_[5] = {};   // batch start, entry pass done, cascade done, copies done, traceback
     DevBuf d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_prof_, d_matrix_;
-    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_scratch2_, d_scratch4_;
-    DevBuf d_tb_hits_, d_tb_regions_, d_tb_last_, d_tb_last_off_, d_tb_dirs_, d_tb_dir_off_, d_tb_ops_,
-            d_tb_ops_off_, d_tb_ops_len_;
-    PinnedBuf h_score_;
+    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_;
+    DevBuf d_tb_io_, d_tb_last_, d_tb_dirs_, d_tb_sync_, d_tb_result_, d_tb_bnd_;
+    PinnedBuf h_score_, h_tb_in_, h_tb_out_;
 public:
     // entry-pass shapes of the last search call: kernel, (R, CTAs per SM) for
     // the query-pair kernel or (G, R) for the single-query one, queries or
@@ -1677,16 +1677,6 @@ void Engine::upload_queries( const QueryCodes * queries, uint32_t nq, bool profi
     prof_width_ = -1;
 }
 
-// Warps per hit in the traceback passes (stripe_pipeline.cuh): 4 for at least
-// 4 stripes of query rows and 8M cells, 2 for at least 2 stripes (they run
-// side by side instead of one after the other), else 1.
-static int tb_group( uint32_t rows, uint32_t cols ) {
-    const uint32_t stripes = (rows + 32u * TB_WORD_ROWS - 1) / (32u * TB_WORD_ROWS);
-    if( stripes >= 4 && (uint64_t) rows * cols >= ((uint64_t) 1 << 23) )
-        return 4;
-    return stripes >= 2 ? 2 : 1;
-}
-
 // Largest magnitude of one DP step: a score-table entry or a gap cost.
 static int64_t max_abs_step( const SearchRequest & req ) {
     int64_t m = std::llabs( (int64_t) req.gap_open ) + std::llabs( (int64_t) req.gap_extend );
@@ -1716,30 +1706,11 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     const uint32_t nh = (uint32_t) hits.size();
     if( nh == 0 )
         return;
-    // the hits by warps per hit (4, 2, 1), each class largest first: the
-    // kernels hand hits out in this order
-    {
-        std::vector<uint32_t> perm( nh );
-        for( uint32_t h = 0; h < nh; h++ )
-            perm[h] = h;
-        auto work = [&]( uint32_t h ) { return (uint64_t) h_qlen_[hits[h].qslot] * db_.len[hits[h].id]; };
-        auto group = [&]( uint32_t h ) { return tb_group( h_qlen_[hits[h].qslot], db_.len[hits[h].id] ); };
-        std::stable_sort( perm.begin(), perm.end(), [&]( uint32_t a, uint32_t b ) {
-            return group( a ) != group( b ) ? group( a ) > group( b ) : work( a ) > work( b );
-        } );
-        std::vector<TbHit> hs( nh );
-        std::vector<std::pair<uint32_t, uint32_t>> ws( nh );
-        for( uint32_t h = 0; h < nh; h++ ) {
-            hs[h] = hits[perm[h]];
-            ws[h] = where[perm[h]];
-        }
-        hits.swap( hs );
-        where.swap( ws );
-    }
     // value range guard: every DP value is bounded by (q + d) * max |step|
     const int64_t mabs = max_abs_step( req );
     std::vector<TbRegion> regions( nh );
     std::vector<uint64_t> last_off( nh + 1, 0 );
+    uint64_t stripes128 = 0;
     for( uint32_t h = 0; h < nh; h++ ) {
         const uint32_t A = h_qlen_[hits[h].qslot], B = db_.len[hits[h].id];
         if( (int64_t) (A + B + 4) * (mabs + 1) * 2 > INT32_MAX )
@@ -1754,7 +1725,20 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         }
         regions[h] = rg;
         last_off[h + 1] = last_off[h] + A;
+        stripes128 += (A + 127u) / 128u;
     }
+    // rows per lane: 4 while every stripe of 128 rows can be resident (32 warps
+    // per SM), else 8.  Measured on a B200, sweep with directions at R = 8 and
+    // R = 4: 10 hits of 375 x 380 0.214 and 0.181 ms, 10 of 300 x 33,000 12.8
+    // and 8.8 ms, 960 of 30-1,803 x 20,000 25.1 and 20.0 ms; past the line, 48
+    // pairs of 5,000-30,000 residues 30.6 and 36.4 ms (Needleman-Wunsch).
+    int R = stripes128 <= (uint64_t) sms_ * 32 ? 4 : 8;
+    if( const char * pin = getenv( "SSA_B200_TB_R" ) )   // pins the rows per lane (tests)
+        R = atoi( pin ) == 8 ? 8 : 4;
+    const uint32_t stripe_rows = 32u * (uint32_t) R;
+    bool p8 = true;
+    for( int k = 0; k < 1024; k++ )
+        p8 = p8 && req.matrix[k] == (int8_t) req.matrix[k];
     TbParams p{};
     // the hits as the device sees them: with a streamed database their
     // sequences are gathered into a view of their own and renumbered
@@ -1782,87 +1766,15 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     p.gap_open = req.gap_open;
     p.gap_extend = req.gap_extend;
     p.error_flags = d_counts_.as<unsigned>() + 2;
-    const int grid = sms_ * 2;
-    const uint32_t cols = db_.max_len + 4;
-    constexpr uint32_t stripe_rows = 32 * TB_WORD_ROWS;
-    // boundary rows in global memory: one per group of warps (8, 4 and 2
-    // groups per CTA of 256 threads for groups of 1, 2 and 4)
-    int4 * scratch1 = max_qlen_ > stripe_rows ? (int4 *) d_scratch_.ensure( (size_t) grid * 8 * cols * sizeof(int4) )
-                                              : nullptr;
-    int4 * scratch2 = max_qlen_ > 2 * stripe_rows
-            ? (int4 *) d_scratch2_.ensure( (size_t) grid * 4 * cols * sizeof(int4) ) : nullptr;
-    int4 * scratch4 = max_qlen_ > 4 * stripe_rows
-            ? (int4 *) d_scratch4_.ensure( (size_t) grid * 2 * cols * sizeof(int4) ) : nullptr;
-    unsigned long long * counters = d_counts_.as<unsigned long long>() + 16;   // bytes 128..223
-    // Launches one phase over the hits [0, n) of the current arrays: [0, k4) on
-    // groups of 4 warps, [k4, k2) on groups of 2, [k2, n) on single warps, the
-    // three classes concurrently on three streams.
-    enum { TB_REGIONS, TB_PATHS, TB_FUSED };
-    auto launch_split = [&]( int phase, uint32_t n, uint32_t k4, uint32_t k2, cudaEvent_t * ev ) {
-        const uint32_t lo[3] = { 0, k4, k2 }, hi[3] = { k4, k2, n };
-        const int group[3] = { 4, 2, 1 };
-        int4 * scratch[3] = { scratch4, scratch2, scratch1 };
-        cudaStream_t st[3] = { stream_, class_stream_[0], class_stream_[1] };
-        CUDA_CHECK( cudaMemsetAsync( counters, 0, 12 * sizeof(unsigned long long), stream_ ) );
-        CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
-        bool timed = false;
-        for( int c = 0; c < 3; c++ ) {
-            if( hi[c] <= lo[c] )
-                continue;
-            TbParams q = p;
-            q.n_hits = hi[c] - lo[c];
-            q.scratch = scratch[c];
-            q.scratch_cols = scratch[c] ? cols : 0;
-            q.hit_counters = counters + 4 * c;
-            q.hits = p.hits + lo[c];
-            q.regions = p.regions + lo[c];
-            if( p.last_off )
-                q.last_off = p.last_off + lo[c];
-            if( p.dir_off ) {
-                q.dir_off = p.dir_off + lo[c];
-                q.ops_off = p.ops_off + lo[c];
-                q.ops_len = p.ops_len + lo[c];
-            }
-            if( c > 0 )
-                CUDA_CHECK( cudaStreamWaitEvent( st[c], ev_ready_, 0 ) );
-            // events around the first class that runs (the largest hits)
-            cudaEvent_t * e = timed ? nullptr : ev;
-            timed = timed || ev != nullptr;
-            CUDA_CHECK( phase == TB_REGIONS ? launch_tb_regions( q, group[c], grid, st[c], e )
-                        : phase == TB_PATHS ? launch_tb_paths( q, group[c], grid, st[c], e )
-                                            : launch_tb_fused( q, group[c], grid, st[c], e ) );
-            if( c > 0 ) {
-                CUDA_CHECK( cudaEventRecord( ev_class_[c], st[c] ) );
-                CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_class_[c], 0 ) );
-            }
-            launches_ += (phase == TB_FUSED) ? 3 : 2;
-        }
-    };
-    // class bounds of hits sorted by warps per hit
-    auto class_bounds = [&]( uint32_t n, auto group_of, uint32_t & k4, uint32_t & k2 ) {
-        k4 = 0;
-        while( k4 < n && group_of( k4 ) == 4 )
-            k4++;
-        k2 = k4;
-        while( k2 < n && group_of( k2 ) == 2 )
-            k2++;
-    };
-    const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
-    float t_fwd = 0, t_rev = 0, t_dir = 0, t_walk = 0;
-    auto check_errors = [&]() {
-        unsigned err = 0;
-        CUDA_CHECK( cudaMemcpyAsync( &err, d_counts_.as<unsigned>() + 2, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        if( err )
-            fatal( "Internal error in the GPU traceback (flags 0x%x).", err );
-    };
+    int32_t * last_all = (int32_t *) d_tb_last_.ensure( 2 * last_off[nh] * sizeof(int32_t) + 16 );
+    p.last_h = last_all;
+    p.last_e = last_all + last_off[nh];
 
     // Smith-Waterman with a symmetric score table: the forward region pass and
-    // the direction pass run as one sweep per hit (tb_fwddir_kernel), then the
-    // reverse pass and the walk, wave by wave.  It needs every hit's last
-    // database column past the initial E terms: (B - 1) x gapE < gapO + gapE
-    // with B >= 2, and initial E and F values that are not above zero (gapO <= 0).
+    // the direction pass run as one sweep per hit, then the reverse pass and
+    // the walk.  It needs every hit's last database column past the initial E
+    // terms: (B - 1) x gapE < gapO + gapE with B >= 2, and initial E and F
+    // values that are not above zero (gapO <= 0).
     bool fused = req.algo == 0 && req.gap_extend < 0 && req.gap_open <= 0;
     for( int d = 0; d < 32 && fused; d++ )
         for( int q = 0; q < 32 && fused; q++ )
@@ -1870,177 +1782,151 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     for( uint32_t h = 0; h < nh && fused; h++ )
         fused = db_.len[hits[h].id] >= 2 &&
                 ((int64_t) db_.len[hits[h].id] - 1) * req.gap_extend < (int64_t) req.gap_open + req.gap_extend;
-    int32_t * last_all = nullptr;
-    if( fused ) {
-        last_all = (int32_t *) d_tb_last_.ensure( 2 * last_off[nh] * sizeof(int32_t) + 16 );
-        p.last_h = last_all;
-        p.last_e = last_all + last_off[nh];
-    }
-
-    // ---- region phase (Smith-Waterman): end cell and begin cell of every hit
-    if( req.algo == 0 && !fused ) {
-        p.hits = (const TbHit *) d_tb_hits_.ensure( nh * sizeof(TbHit) );
-        p.n_hits = nh;
-        p.regions = (TbRegion *) d_tb_regions_.ensure( nh * sizeof(TbRegion) );
-        int32_t * last = (int32_t *) d_tb_last_.ensure( 2 * last_off[nh] * sizeof(int32_t) + 16 );
-        p.last_h = last;
-        p.last_e = last + last_off[nh];
-        p.last_off = (const uint64_t *) d_tb_last_off_.ensure( (nh + 1) * sizeof(uint64_t) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.hits, dev_hits.data(), nh * sizeof(TbHit), cudaMemcpyHostToDevice,
-                stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( p.regions, regions.data(), nh * sizeof(TbRegion), cudaMemcpyHostToDevice,
-                stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.last_off, last_off.data(), (nh + 1) * sizeof(uint64_t),
-                cudaMemcpyHostToDevice, stream_ ) );
-        uint32_t k4, k2;
-        class_bounds( nh, [&]( uint32_t h ) { return tb_group( h_qlen_[hits[h].qslot], db_.len[hits[h].id] ); }, k4,
-                k2 );
-        launch_split( TB_REGIONS, nh, k4, k2, timing ? ev_tb_ : nullptr );
-        CUDA_CHECK( cudaMemcpyAsync( regions.data(), p.regions, nh * sizeof(TbRegion), cudaMemcpyDeviceToHost,
-                stream_ ) );
-        check_errors();
-        if( timing ) {
-            CUDA_CHECK( cudaEventElapsedTime( &t_fwd, ev_tb_[0], ev_tb_[1] ) );
-            CUDA_CHECK( cudaEventElapsedTime( &t_rev, ev_tb_[1], ev_tb_[2] ) );
-        }
-        stats.h2d_bytes += nh * (sizeof(TbHit) + sizeof(TbRegion) + sizeof(uint64_t));
-        stats.d2h_bytes += nh * sizeof(TbRegion);
-    }
-
-    // ---- path phase: direction words (2 bits per cell of rows 0..a_end and
-    // columns b_begin..b_end) and the walk, in waves whose direction words fit
-    // the traceback memory
-    std::vector<uint64_t> dir_words( nh, 0 ), ops_bytes( nh, 0 );
+    const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
+    float t_fwd = 0, t_rev = 0, t_dir = 0, t_walk = 0;
     uint64_t total_dir = 0;
-    for( uint32_t h = 0; h < nh; h++ ) {
-        TbRegion & rg = regions[h];
-        if( fused ) {
-            // the whole matrix: every query row and database column
-            const uint32_t A = h_qlen_[hits[h].qslot], B = db_.len[hits[h].id];
-            rg.dir_words = (int32_t) ((A + TB_WORD_ROWS - 1) / TB_WORD_ROWS);
-            rg.dir_col0 = 0;
-            dir_words[h] = (uint64_t) B * (uint64_t) rg.dir_words;
-            ops_bytes[h] = (uint64_t) A + B + 1;
-            total_dir += dir_words[h] * sizeof(uint16_t);
-            continue;
+    size_t n_waves = 0;
+
+    // One wave: the hits of `wave`, most stripes first (rows[h] query rows and
+    // cols[h] database columns each).  All its arrays travel in one copy each
+    // way: hits, regions and offsets down; regions, move counts, error flags
+    // and move strings up.
+    struct Layout {
+        size_t bytes = 0;
+        size_t add( size_t n ) {
+            const size_t at = bytes;
+            bytes += (n + 15) & ~(size_t) 15;
+            return at;
         }
-        if( rg.status == 2 )
-            fatal( "Internal error in align function." );   // reference: src/algo/align.c:131
-        if( rg.status != 0 )
-            continue;
-        // rows 0..a_end and columns b_begin..b_end
-        rg.dir_words = (rg.a_end + TB_WORD_ROWS) / TB_WORD_ROWS;
-        rg.dir_col0 = rg.b_begin;
-        dir_words[h] = (uint64_t) (rg.b_end - rg.b_begin + 1) * (uint64_t) rg.dir_words;
-        ops_bytes[h] = (uint64_t) (rg.a_end - rg.a_begin + 1) + (uint64_t) (rg.b_end - rg.b_begin + 1) + 1;
-        total_dir += dir_words[h] * sizeof(uint16_t);
-    }
-    // matrices within the smallest automatic budget make one wave whatever the
-    // free memory is: asking the driver for it costs up to milliseconds
-    const uint64_t budget = (!tb_budget_ && total_dir <= TB_MIN_BUDGET) ? TB_MIN_BUDGET : traceback_budget();
-    auto region_group = [&]( uint32_t h ) {
-        if( fused )
-            return tb_group( h_qlen_[hits[h].qslot], db_.len[hits[h].id] );
-        const TbRegion & rg = regions[h];
-        return rg.status == 0 ? tb_group( (uint32_t) rg.a_end + 1, (uint32_t) rg.b_end + 1 ) : 1;
     };
-    // waves: consecutive runs of the hits in (more warps per hit first,
-    // largest direction matrix first) order, each run as long as its matrices
-    // fit
-    std::vector<std::vector<uint32_t>> waves;
-    {
-        std::vector<uint32_t> order( nh );
-        for( uint32_t h = 0; h < nh; h++ )
-            order[h] = h;
-        std::stable_sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
-            const int gx = region_group( x ), gy = region_group( y );
-            return gx != gy ? gx > gy : dir_words[x] > dir_words[y];
-        } );
-        uint64_t load = 0;
-        for( uint32_t h : order ) {
-            const uint64_t need = dir_words[h] * sizeof(uint16_t);
-            if( waves.empty() || (load + need > budget && !waves.back().empty()) ) {
-                waves.emplace_back();
-                load = 0;
-            }
-            waves.back().push_back( h );
-            load += need;
-        }
-    }
-    for( const std::vector<uint32_t> & wave : waves ) {
+    auto run_wave = [&]( const std::vector<uint32_t> & wave, const std::vector<uint32_t> & rows,
+            const std::vector<uint32_t> & cols, bool regions_only ) {
         const uint32_t nw = (uint32_t) wave.size();
-        std::vector<TbHit> whits( nw );
-        std::vector<TbRegion> wregs( nw );
-        std::vector<uint64_t> wdir( nw + 1, 0 ), wops( nw + 1, 0 ), wlast( nw, 0 );
-        for( uint32_t k = 0; k < nw; k++ ) {
-            whits[k] = dev_hits[wave[k]];
-            wregs[k] = regions[wave[k]];
-            wdir[k + 1] = wdir[k] + dir_words[wave[k]];
-            wops[k + 1] = wops[k] + ops_bytes[wave[k]];
-            wlast[k] = last_off[wave[k]];
+        const bool paths = !regions_only;
+        const bool reverse = req.algo == 0 && (fused || regions_only);
+        // tickets stripe by stripe: stripe i exists in the first n_i hits
+        std::vector<uint32_t> cum{ 0 };
+        for( uint32_t left = nw, i = 0;; i++ ) {
+            while( left && (uint64_t) i * stripe_rows >= rows[wave[left - 1]] )
+                left--;
+            if( left == 0 )
+                break;
+            cum.push_back( cum.back() + left );
         }
-        if( fused ) {
-            // the fused pass writes each hit's last column into its slice of
-            // the last-row arrays of all hits
-            p.last_off = (const uint64_t *) d_tb_last_off_.ensure( std::max<uint32_t>( 1, nw ) * sizeof(uint64_t) );
-            CUDA_CHECK( cudaMemcpyAsync( (void *) p.last_off, wlast.data(), nw * sizeof(uint64_t),
-                    cudaMemcpyHostToDevice, stream_ ) );
-            stats.h2d_bytes += nw * sizeof(uint64_t);
-        }
-        p.hits = (const TbHit *) d_tb_hits_.ensure( nw * sizeof(TbHit) );
-        p.n_hits = nw;
-        p.regions = (TbRegion *) d_tb_regions_.ensure( nw * sizeof(TbRegion) );
-        p.dirs = (uint16_t *) d_tb_dirs_.ensure( wdir[nw] * sizeof(uint16_t) + 16 );
-        p.dir_off = (const uint64_t *) d_tb_dir_off_.ensure( (nw + 1) * sizeof(uint64_t) );
-        p.ops = (char *) d_tb_ops_.ensure( wops[nw] + 16 );
-        p.ops_off = (const uint64_t *) d_tb_ops_off_.ensure( (nw + 1) * sizeof(uint64_t) );
-        p.ops_len = (uint32_t *) d_tb_ops_len_.ensure( nw * sizeof(uint32_t) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.hits, whits.data(), nw * sizeof(TbHit), cudaMemcpyHostToDevice,
-                stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( p.regions, wregs.data(), nw * sizeof(TbRegion), cudaMemcpyHostToDevice, stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.dir_off, wdir.data(), (nw + 1) * sizeof(uint64_t),
-                cudaMemcpyHostToDevice, stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.ops_off, wops.data(), (nw + 1) * sizeof(uint64_t),
-                cudaMemcpyHostToDevice, stream_ ) );
-        uint32_t k4, k2;
-        class_bounds( nw, [&]( uint32_t k ) { return region_group( wave[k] ); }, k4, k2 );
-        launch_split( fused ? TB_FUSED : TB_PATHS, nw, k4, k2, timing ? ev_tb_ + 2 : nullptr );
-        std::vector<uint32_t> ops_len( nw );
-        std::vector<char> ops( wops[nw] + 1 );
-        CUDA_CHECK( cudaMemcpyAsync( ops_len.data(), p.ops_len, nw * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( ops.data(), p.ops, wops[nw], cudaMemcpyDeviceToHost, stream_ ) );
-        if( fused || (scores_from_regions && req.algo == 1) ) {
-            CUDA_CHECK( cudaMemcpyAsync( wregs.data(), p.regions, nw * sizeof(TbRegion), cudaMemcpyDeviceToHost,
-                    stream_ ) );
-            stats.d2h_bytes += nw * sizeof(TbRegion);
-        }
-        check_errors();
-        if( fused ) {
-            // the regions the fused and reverse passes found
-            for( uint32_t k = 0; k < nw; k++ ) {
-                if( wregs[k].status == 2 )
-                    fatal( "Internal error in align function." );   // reference: src/algo/align.c:131
-                regions[wave[k]] = wregs[k];
-            }
-        }
-        else if( scores_from_regions && req.algo == 1 ) {
-            for( uint32_t k = 0; k < nw; k++ )
-                regions[wave[k]].fwd_score = wregs[k].fwd_score;
-        }
-        if( timing ) {
-            float a = 0, b = 0;
-            CUDA_CHECK( cudaEventElapsedTime( &a, ev_tb_[2], ev_tb_[3] ) );
-            CUDA_CHECK( cudaEventElapsedTime( &b, ev_tb_[3], ev_tb_[4] ) );
-            t_dir += a;
-            t_walk += b;
-        }
-        stats.h2d_bytes += nw * (sizeof(TbHit) + sizeof(TbRegion) + 2 * sizeof(uint64_t));
-        stats.d2h_bytes += nw * sizeof(uint32_t) + wops[nw];
+        uint64_t dir_bytes = 0, bnd_cols = 0, ops_bytes = 0;
+        Layout in, res;
+        const size_t o_hits = in.add( nw * sizeof(TbHit) ), o_last = in.add( nw * sizeof(uint64_t) ),
+                o_dir = in.add( nw * sizeof(uint64_t) ), o_ops = in.add( (nw + 1) * sizeof(uint64_t) ),
+                o_bnd = in.add( nw * sizeof(uint64_t) ), o_cum = in.add( cum.size() * sizeof(uint32_t) ),
+                o_reg = in.add( nw * sizeof(TbRegion) );
+        uint8_t * hin = (uint8_t *) h_tb_in_.ensure( in.bytes );
         for( uint32_t k = 0; k < nw; k++ ) {
             const uint32_t h = wave[k];
+            const uint64_t stripes = (rows[h] + stripe_rows - 1) / stripe_rows;
+            TbRegion rg = regions[h];
+            rg.dir_steps = (int32_t) cols[h] + 31;
+            ((TbHit *) (hin + o_hits))[k] = dev_hits[h];
+            ((TbRegion *) (hin + o_reg))[k] = rg;
+            ((uint64_t *) (hin + o_last))[k] = last_off[h];
+            ((uint64_t *) (hin + o_dir))[k] = dir_bytes;
+            ((uint64_t *) (hin + o_ops))[k] = ops_bytes;
+            ((uint64_t *) (hin + o_bnd))[k] = bnd_cols;
+            if( paths ) {
+                dir_bytes += stripes * ((uint64_t) cols[h] + 31) * (32 * R / 4);
+                ops_bytes += (uint64_t) rows[h] + cols[h] + 1;
+            }
+            if( stripes > 1 )
+                bnd_cols += cols[h];
+        }
+        ((uint64_t *) (hin + o_ops))[nw] = ops_bytes;
+        memcpy( hin + o_cum, cum.data(), cum.size() * sizeof(uint32_t) );
+        const uint32_t n_tickets = cum.back();
+        // device side: inputs (regions last, updated in place), then the
+        // passes' results in the order they are copied back
+        const size_t r_reg = res.add( nw * sizeof(TbRegion) ), r_len = res.add( nw * sizeof(uint32_t) ),
+                r_ops = res.add( paths ? ops_bytes : 0 );
+        uint8_t * din = (uint8_t *) d_tb_io_.ensure( in.bytes + res.bytes );
+        uint8_t * dout = din + o_reg;            // the regions of the inputs are the first results
+        uint8_t * hout = (uint8_t *) h_tb_out_.ensure( res.bytes + sizeof(unsigned) );
+        // progress of both sweeps, ticket counters and column limits: cleared
+        // by one memset (the limits to a large positive number)
+        Layout sy;
+        const size_t s_prog = sy.add( (size_t) n_tickets * 2 * sizeof(uint32_t) ),
+                s_cnt = sy.add( 2 * sizeof(unsigned long long) );
+        const size_t s_zero = sy.bytes;
+        const size_t s_lim = sy.add( nw * sizeof(int32_t) );
+        uint8_t * dsy = (uint8_t *) d_tb_sync_.ensure( sy.bytes );
+        p.hits = (const TbHit *) (din + o_hits);
+        p.n_hits = nw;
+        p.last_off = (const uint64_t *) (din + o_last);
+        p.dir_off = (const uint64_t *) (din + o_dir);
+        p.ops_off = (const uint64_t *) (din + o_ops);
+        p.bnd_off = (const uint64_t *) (din + o_bnd);
+        p.cum = (const uint32_t *) (din + o_cum);
+        p.regions = (TbRegion *) (dout + r_reg);
+        p.ops_len = (uint32_t *) (dout + r_len);
+        p.ops = (char *) (dout + r_ops);
+        p.levels = (uint32_t) cum.size() - 1;
+        p.n_tickets = n_tickets;
+        p.result = (int4 *) d_tb_result_.ensure( std::max<size_t>( 16, (size_t) n_tickets * sizeof(int4) ) );
+        p.boundary = (int2 *) d_tb_bnd_.ensure( bnd_cols * sizeof(int2) + 16 );
+        p.limit = (int32_t *) (dsy + s_lim);
+        if( paths )
+            p.dirs = (uint8_t *) d_tb_dirs_.ensure( dir_bytes + 16 );
+        CUDA_CHECK( cudaMemcpyAsync( din, hin, in.bytes, cudaMemcpyHostToDevice, stream_ ) );
+        CUDA_CHECK( cudaMemsetAsync( dsy, 0, s_zero, stream_ ) );
+        if( reverse )
+            CUDA_CHECK( cudaMemsetAsync( dsy + s_lim, 0x7f, nw * sizeof(int32_t), stream_ ) );
+        auto sweep = [&]( int k ) {
+            p.progress = (uint32_t *) (dsy + s_prog) + (size_t) k * n_tickets;
+            p.counter = (unsigned long long *) (dsy + s_cnt) + k;
+            launches_++;
+        };
+        if( timing )
+            CUDA_CHECK( cudaEventRecord( ev_tb_[0], stream_ ) );
+        sweep( 0 );
+        CUDA_CHECK( regions_only ? launch_tb_forward( p, R, p8, sms_, stream_ )
+                    : fused ? launch_tb_fwddir( p, R, p8, sms_, stream_ )
+                            : launch_tb_directions( p, R, p8, sms_, stream_ ) );
+        if( timing )
+            CUDA_CHECK( cudaEventRecord( ev_tb_[1], stream_ ) );
+        if( reverse ) {
+            sweep( 1 );
+            CUDA_CHECK( launch_tb_reverse( p, R, p8, sms_, stream_ ) );
+        }
+        if( paths ) {
+            launches_++;
+            CUDA_CHECK( launch_tb_walk( p, R, stream_ ) );
+        }
+        if( timing )
+            CUDA_CHECK( cudaEventRecord( ev_tb_[2], stream_ ) );
+        CUDA_CHECK( cudaMemcpyAsync( hout, dout, res.bytes, cudaMemcpyDeviceToHost, stream_ ) );
+        CUDA_CHECK( cudaMemcpyAsync( hout + res.bytes, p.error_flags, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                stream_ ) );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+        unsigned err = 0;
+        memcpy( &err, hout + res.bytes, sizeof err );
+        if( err )
+            fatal( "Internal error in the GPU traceback (flags 0x%x).", err );
+        stats.h2d_bytes += in.bytes;
+        stats.d2h_bytes += res.bytes;
+        total_dir += dir_bytes;
+        n_waves++;
+        if( timing ) {
+            float x = 0, y = 0;
+            CUDA_CHECK( cudaEventElapsedTime( &x, ev_tb_[0], ev_tb_[1] ) );
+            CUDA_CHECK( cudaEventElapsedTime( &y, ev_tb_[1], ev_tb_[2] ) );
+            (regions_only ? t_fwd : t_dir) += x;
+            (regions_only ? t_rev : t_walk) += y;
+        }
+        for( uint32_t k = 0; k < nw; k++ ) {
+            const uint32_t h = wave[k];
+            const TbRegion & rg = regions[h] = ((const TbRegion *) (hout + r_reg))[k];
+            if( rg.status == 2 )
+                fatal( "Internal error in align function." );   // reference: src/algo/align.c:131
+            if( regions_only )
+                continue;
             Hit & hit = out[where[h].first][where[h].second];
-            const TbRegion & rg = regions[h];
             hit.has_cigar = true;
             if( scores_from_regions )
                 hit.score = rg.fwd_score;
@@ -2056,11 +1942,10 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
             hit.d_end = (uint32_t) rg.b_end;
             // run-length encode the moves in alignment order; counts of 1 are
             // omitted (reference: src/algo/cigar.c:221-263)
-            const char * mv = ops.data() + wops[k];
-            uint32_t n = (uint32_t) std::min<uint64_t>( ops_len[k], wops[k + 1] - wops[k] );
+            const uint64_t * off = (const uint64_t *) (hin + o_ops);
+            const char * mv = (const char *) (hout + r_ops) + off[k];
+            uint32_t i = (uint32_t) std::min<uint64_t>( ((const uint32_t *) (hout + r_len))[k], off[k + 1] - off[k] );
             std::string cig;
-            uint32_t i = n;
-            char buf[24];
             while( i > 0 ) {
                 const char op = mv[i - 1];
                 uint32_t run = 0;
@@ -2068,19 +1953,67 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
                     run++;
                     i--;
                 }
-                if( run > 1 ) {
-                    snprintf( buf, sizeof(buf), "%u", run );
-                    cig += buf;
-                }
+                if( run > 1 )
+                    cig += std::to_string( run );
                 cig += op;
             }
             hit.cigar = std::move( cig );
         }
+    };
+    // Waves: runs of the hits in (most stripes first, most columns first) order
+    // whose direction bytes and boundary rows fit the traceback memory.
+    auto run_waves = [&]( const std::vector<uint32_t> & rows, const std::vector<uint32_t> & cols, bool regions_only ) {
+        std::vector<uint32_t> order( nh );
+        for( uint32_t h = 0; h < nh; h++ )
+            order[h] = h;
+        auto stripes = [&]( uint32_t h ) { return (rows[h] + stripe_rows - 1) / stripe_rows; };
+        std::stable_sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
+            return stripes( x ) != stripes( y ) ? stripes( x ) > stripes( y ) : cols[x] > cols[y];
+        } );
+        auto need = [&]( uint32_t h ) {
+            return (regions_only ? 0 : (uint64_t) stripes( h ) * (cols[h] + 31) * (32 * R / 4)) +
+                    (stripes( h ) > 1 ? cols[h] * sizeof(int2) : 0);
+        };
+        uint64_t total = 0;
+        for( uint32_t h = 0; h < nh; h++ )
+            total += need( h );
+        // matrices within the smallest automatic budget make one wave whatever
+        // the free memory is: asking the driver for it costs up to milliseconds
+        const uint64_t budget = (!tb_budget_ && total <= TB_MIN_BUDGET) ? TB_MIN_BUDGET : traceback_budget();
+        std::vector<uint32_t> wave;
+        uint64_t load = 0;
+        for( uint32_t h : order ) {
+            if( !wave.empty() && load + need( h ) > budget ) {
+                run_wave( wave, rows, cols, regions_only );
+                wave.clear();
+                load = 0;
+            }
+            wave.push_back( h );
+            load += need( h );
+        }
+        run_wave( wave, rows, cols, regions_only );
+    };
+    std::vector<uint32_t> rows( nh ), cols( nh );
+    for( uint32_t h = 0; h < nh; h++ ) {
+        rows[h] = h_qlen_[hits[h].qslot];
+        cols[h] = db_.len[hits[h].id];
     }
+    if( req.algo == 0 && !fused ) {
+        // the end and begin cell of every hit, then rows 0 .. a_end and columns
+        // 0 .. b_end of the direction matrix
+        run_waves( rows, cols, true );
+        for( uint32_t h = 0; h < nh; h++ ) {
+            rows[h] = regions[h].status == 0 ? (uint32_t) regions[h].a_end + 1 : 1;
+            cols[h] = regions[h].status == 0 ? (uint32_t) regions[h].b_end + 1 : 1;
+        }
+    }
+    run_waves( rows, cols, false );
     // a very large direction buffer (long pairs) is not kept for later calls,
     // whose scores, lists and database segments need the device memory
     if( d_tb_dirs_.bytes > ((uint64_t) 8 << 30) )
         d_tb_dirs_.release();
+    if( d_tb_bnd_.bytes > ((uint64_t) 1 << 30) )
+        d_tb_bnd_.release();
     if( timing ) {
         uint64_t max_cells = 0;
         uint32_t max_a = 0, max_b = 0;
@@ -2095,11 +2028,11 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         if( fused )
             fprintf( stderr, "[ssa timing] traceback %u hits: forward with directions %.3f ms, reverse and walk "
                     "%.3f ms in %zu wave(s) (%.3f GB of directions); largest hit %u x %u\n", nh, t_dir, t_walk,
-                    waves.size(), total_dir * 1e-9, max_a, max_b );
+                    n_waves, total_dir * 1e-9, max_a, max_b );
         else
             fprintf( stderr, "[ssa timing] traceback %u hits: forward %.3f ms, reverse %.3f ms, directions %.3f ms, "
                     "walk %.3f ms in %zu wave(s) (%.3f GB of directions); largest hit %u x %u\n", nh, t_fwd, t_rev,
-                    t_dir, t_walk, waves.size(), total_dir * 1e-9, max_a, max_b );
+                    t_dir, t_walk, n_waves, total_dir * 1e-9, max_a, max_b );
     }
 }
 
@@ -2427,6 +2360,8 @@ void Engine::align_hits( const SearchRequest & req, const std::vector<QueryCodes
     serve_layout_ = false;
     d_matrix_.ensure( 1024 * sizeof(int64_t) );
     CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
+    d_counts_.ensure( 32 * sizeof(unsigned long long) );
+    CUDA_CHECK( cudaMemsetAsync( d_counts_.p, 0, 32 * sizeof(unsigned long long), stream_ ) );
     const uint32_t nq = (uint32_t) queries.size();
     const uint32_t batch = 65535;
     for( uint32_t b0 = 0; b0 < nq; b0 += batch ) {
