@@ -65,6 +65,8 @@ struct PassSink {
 
 // score[] marker of a pair whose exact score is in PassSink::score64
 constexpr int32_t SCORE_IN_WIDE = INT32_MIN;
+// score[] marker of a pair that the lane emulation re-queued to the next width
+constexpr int32_t SCORE_REQUEUED = INT32_MIN + 1;
 
 enum ErrorBits : unsigned int {
     ERR_REQUEUE_OVERFLOW = 1u,
@@ -205,6 +207,7 @@ struct FastParams {
     int gap_oe;                   // gapO + gapE at the entry width
     int gap_e;
     int limit;                    // running maximum that ends a sequence: 255, or the 16x2 range (16- and 64-bit entry)
+    uint32_t pair_skip;           // leading pairs that another kernel scores
     PassSink sink;
     int4 * scratch;               // per warp and group slot (4 per warp, 8 for the 4-column kernel): scratch_cols entries
     uint32_t scratch_cols;
@@ -220,6 +223,37 @@ cudaError_t launch_sw_fast4( int R, const FastParams & p, int grid, cudaStream_t
 cudaError_t launch_build_profile8( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
         const uint32_t * slots, uint32_t n, const uint32_t * rows_of, const int64_t * matrix, int8_t * prof,
         const uint64_t * prof_off, cudaStream_t st );
+
+// ---- chosen Smith-Waterman pairs on streamed stripes (sw_stream_kernel.cu) ---
+struct SwStreamItem {
+    uint32_t slot;                // query
+    uint32_t id_a, id_b;          // two sequences (B = 0xffffffff when absent)
+    uint32_t pad_;
+};
+
+struct SwStreamParams {
+    DbView db;
+    const uint8_t * qcodes;
+    const uint64_t * qoff;
+    const uint32_t * qlen;
+    const int64_t * matrix;       // 32 x 32, [database code][query code], entries within int8
+    int gap_oe, gap_e;
+    int limit;                    // as in FastParams
+    const SwStreamItem * items;   // most stripes first
+    const uint64_t * bnd_off;     // per item offset into boundary
+    const uint32_t * cum;         // first ticket of stripe i, i = 0 .. levels
+    uint32_t levels, n_tickets;
+    unsigned long long * counter; // next ticket (0 at the start)
+    uint32_t * progress;          // per ticket (0 at the start)
+    uint32_t * result;            // per ticket: maximum of the stripes so far
+    int32_t * cross;              // 8-bit entry: per item and sequence, first block that reached the limit (large at
+                                  // the start); nullptr otherwise
+    int4 * boundary;              // per item with several stripes: two words per block of four columns
+    PassSink sink;                // score; next (8-bit entry) or redo
+};
+
+// R: query rows per lane (4 or 8)
+cudaError_t launch_sw_stream( int R, const SwStreamParams & p, int sms, cudaStream_t st );
 
 // ---- query-pair Smith-Waterman entry pass (sw_qpair_kernel.cu) -------------
 // Two queries of similar length share each 32-bit register (low half query A,
@@ -248,6 +282,7 @@ struct QPairParams {
     int gap_oe;                   // gapO + gapE at the entry width
     int gap_e;
     int limit;                    // Smith-Waterman: as in FastParams
+    const uint32_t * qp_skip;     // per query pair: leading sequences that another kernel scores (nullptr: none)
     PassSink sink;
     int4 * scratch;               // per warp and group: scratch_cols column pairs (H, F of two columns)
     uint32_t scratch_cols;
@@ -256,6 +291,7 @@ struct QPairParams {
     const uint32_t * qlen;        // per slot
     const uint32_t * qp_lmax;     // per query pair: longest sequence the kernel scores exactly
     // (longer sequences go to sink.redo for the lane emulation)
+    bool marked_only;             // score only the pairs that hold SCORE_REQUEUED
 };
 
 // mb: 4 or 5 resident CTAs per SM (register bound of the instantiation)

@@ -199,6 +199,11 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
         int first_ovf = -1;
         V nw_score = 0;
 
+        // Columns worth computing: once the rows so far overflow in a block, the
+        // lane's report is that block or an earlier one, so this pass ends
+        // there and the next ones go no further (an 8-bit Needleman-Wunsch
+        // search of 100 rows and more overflows in the first blocks).
+        uint32_t cols = Lb;
         for( uint32_t pass = 0; pass < passes; pass++ ) {
             const bool final_pass = (pass + 1 == passes);
             const int64_t row0 = (int64_t) pass * EMUL_ROWS + lane * R;
@@ -225,16 +230,27 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
 
             V out_h = 0, out_f = 0, out_a = 0, out_b = 0;
             Col pf = BoundaryCol<V>::make( 0, 0, 0, 0 );
-            if( pass > 0 && (uint32_t) lane < p.scratch_cols && (uint32_t) lane < Lb )
+            if( pass > 0 && (uint32_t) lane < p.scratch_cols && (uint32_t) lane < cols )
                 pf = scratch[lane];
-            const uint32_t steps = Lb + 31;
-            for( uint32_t s = 0; s < steps; s++ ) {
+            // lane 31: the rows so far
+            s_run = SW ? SW_ZERO : (V) 0;
+            blk_min = 0;
+            blk_max = 0;
+            first_ovf = -1;
+            for( uint32_t s = 0; s < cols + 31; s++ ) {
+                if( W != 64 && (s & 7u) == 0 && s >= 32 ) {
+                    const int b = __shfl_sync( 0xffffffffu, first_ovf, 31 );
+                    if( b >= 0 ) {
+                        cols = min( cols, 4u * (uint32_t) b + 4u );
+                        break;
+                    }
+                }
                 if( pass > 0 && (s & 31u) == 0 ) {
                     __syncwarp();
                     tile[lane] = pf;
                     __syncwarp();
                     const uint32_t col = s + 32u + (uint32_t) lane;
-                    if( col < p.scratch_cols && col < Lb )
+                    if( col < p.scratch_cols && col < cols )
                         pf = scratch[col];
                 }
                 V up_h = __shfl_up_sync( 0xffffffffu, out_h, 1 );
@@ -242,7 +258,7 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
                 V up_a = __shfl_up_sync( 0xffffffffu, out_a, 1 );
                 V up_b = __shfl_up_sync( 0xffffffffu, out_b, 1 );
                 const int64_t c = (int64_t) s - lane;
-                if( c < 0 || c >= (int64_t) Lb )
+                if( c < 0 || c >= (int64_t) cols )
                     continue;
                 if( lane == 0 ) {
                     if( pass == 0 ) {
@@ -332,7 +348,7 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
                         else
                             atomicOr( p.sink.error_flags, ERR_SCRATCH_OVERFLOW );
                     }
-                    else if( first_ovf < 0 ) {
+                    if( W != 64 ? first_ovf < 0 : final_pass ) {
                         if constexpr( SW ) {
                             s_run = max( s_run, out_a );
                             if( (c & 3) == 3 && W != 64 && s_run == (V) Width<W>::MAX )
@@ -350,6 +366,11 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
                         }
                     }
                 }
+            }
+            if constexpr( W != 64 ) {
+                const int b = __shfl_sync( 0xffffffffu, first_ovf, 31 );
+                if( b >= 0 )
+                    cols = min( cols, 4u * (uint32_t) b + 4u );
             }
             __syncwarp();
         }
@@ -378,7 +399,8 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
                     p.sink.score[at] = SCORE_IN_WIDE;
             }
             else {
-                p.sink.score[at] = score;
+                // a re-queued pair is marked until the next width scores it
+                p.sink.score[at] = (W == 64 || ok) ? (int32_t) score : SCORE_REQUEUED;
             }
             if( !ok ) {
                 unsigned k = atomicAdd( p.sink.next_count, 1u );

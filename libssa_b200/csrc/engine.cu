@@ -454,13 +454,14 @@ public:
             &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_qcodes_, &d_qoff_, &d_qlen_, &d_qpad_,
             &d_prof_off_, &d_prof_, &d_matrix_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
             &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_, &d_qp_off_, &d_qp_rows_, &d_qp_slots_, &d_qp_units_,
-            &d_serve_score_, &d_qp_lmax_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_,
+            &d_serve_score_, &d_qp_lmax_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_, &d_list_c_, &d_sw_in_,
             &d_seg_[0], &d_seg_[1], &d_gather_codes_, &d_gather_off_, &d_gather_len_, &d_prof64_, &d_score64_ };
         for( DevBuf * b : bufs )
             b->release();
         h_score_.release();
         h_score64_.release();
         h_tb_in_.release();
+        h_sw_in_.release();
         h_tb_out_.release();
         h_stage_.release();
         resident_seg_ = -1;
@@ -491,10 +492,18 @@ private:
             uint64_t n_tasks, bool implicit, PairTask * next, unsigned * next_count, uint32_t next_cap,
             const uint32_t * slot_list = nullptr, uint32_t n_sub = 0, uint32_t order_lo = 0 );
     void run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap );
+    // marked: the 16-bit pass of the cascade, only the pairs that the 8-bit entry re-queued (Needleman-Wunsch)
     void run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
-            uint32_t cap, const std::vector<uint32_t> * slots = nullptr, uint32_t seq_lo = 0,
-            uint32_t seq_hi = UINT32_MAX );
-    void run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap );
+            uint32_t cap, PairTask * redo_list, const std::vector<uint32_t> * slots = nullptr, uint32_t seq_lo = 0,
+            uint32_t seq_hi = UINT32_MAX, bool marked = false );
+    void run_sw_stream( const SearchRequest & req, const std::vector<PairTask> & tasks, PairTask * redo_list );
+    // The passes after the entry width: list A holds n_a pairs that it re-queued.
+    // Leaves their scores, and the lists on the host (appended).
+    void run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, uint32_t cap,
+            std::vector<PairTask> & list_entry, std::vector<PairTask> & list_16, const std::vector<uint32_t> * slots,
+            uint32_t lo, uint32_t hi );
+    void run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap,
+            const PairTask * redo_list );
     int32_t * score_sink() { return serving_ ? d_serve_score_.as<int32_t>() : d_score_.as<int32_t>(); }
     void build_profiles( int width, uint32_t n_slots );
     // scores_from_regions: the hits carry no score yet; take it from the
@@ -546,9 +555,9 @@ private:
     cudaEvent_t ev_seg_[2] = {};     // around one segment's entry pass
     cudaEvent_t ev_tb_[5] = {};   // batch start, entry pass done, cascade done, copies done, traceback
     DevBuf d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_prof_, d_matrix_;
-    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_;
+    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_in_;
     DevBuf d_tb_io_, d_tb_last_, d_tb_dirs_, d_tb_sync_, d_tb_result_, d_tb_bnd_;
-    PinnedBuf h_score_, h_tb_in_, h_tb_out_;
+    PinnedBuf h_score_, h_tb_in_, h_tb_out_, h_sw_in_;
 public:
     // entry-pass shapes of the last search call: kernel, (R, CTAs per SM) for
     // the query-pair kernel or (G, R) for the single-query one, queries or
@@ -1012,7 +1021,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         class_first += cls.size();
     }
     if( req.bit_width != 8 )
-        run_redo( req, nq, next, next_count, cap );
+        run_redo( req, nq, next, next_count, cap, d_list_b_.as<PairTask>() );
     if( !fallback.empty() ) {
         const uint64_t n_ne = db_.order_desc.size();
         run_pass( 0, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_ne, true, next, next_count, cap,
@@ -1115,18 +1124,20 @@ static int choose_qpair_rows( uint32_t Q, uint32_t * passes, int pinned, int buc
 
 // The pairs that a 16x2 entry pass left out of its range (16- and 64-bit
 // entry): the lane emulation at the entry width.
-void Engine::run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap ) {
+void Engine::run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap,
+        const PairTask * redo_list ) {
     unsigned n_redo = 0;
     CUDA_CHECK( cudaMemcpyAsync( &n_redo, d_counts_.as<unsigned>() + 5, sizeof(unsigned), cudaMemcpyDeviceToHost,
             stream_ ) );
     CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
     n_redo = std::min( n_redo, cap );
     if( n_redo )
-        run_pass( req.algo, req.bit_width, req, nq, d_list_b_.as<PairTask>(), n_redo, false, next, next_count, cap );
+        run_pass( req.algo, req.bit_width, req, nq, redo_list, n_redo, false, next, next_count, cap );
 }
 
 void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
-        uint32_t cap, const std::vector<uint32_t> * slots, uint32_t seq_lo, uint32_t seq_hi ) {
+        uint32_t cap, PairTask * redo_list, const std::vector<uint32_t> * slots, uint32_t seq_lo, uint32_t seq_hi,
+        bool marked ) {
     // the sequences order_desc[seq_lo, seq_hi) (all by default)
     const uint32_t n_all = (uint32_t) db_.order_desc.size();
     const uint32_t lo = std::min( seq_lo, n_all ), hi = std::min( seq_hi, n_all );
@@ -1331,8 +1342,9 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         p.gap_open = req.gap_open;
         p.qlen = d_qlen_.as<uint32_t>();
         p.qp_lmax = d_qp_lmax_.as<uint32_t>();
+        p.marked_only = marked;
         if( redo ) {
-            p.sink.redo = d_list_b_.as<PairTask>();
+            p.sink.redo = redo_list;
             p.sink.redo_count = redo_count;
             p.sink.redo_cap = cap;
         }
@@ -1364,13 +1376,157 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         }
     }
     if( redo )
-        run_redo( req, nq, next, next_count, cap );
+        run_redo( req, nq, next, next_count, cap, redo_list );
     if( !fallback.empty() ) {
         d_slots_.ensure( fallback.size() * sizeof(uint32_t) );
         CUDA_CHECK( cudaMemcpyAsync( d_slots_.p, fallback.data(), fallback.size() * sizeof(uint32_t),
                 cudaMemcpyHostToDevice, stream_ ) );
         run_pass( req.algo, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_seq, true, next,
                 next_count, cap, d_slots_.as<uint32_t>(), (uint32_t) fallback.size(), lo );
+    }
+}
+
+// The 16-bit Smith-Waterman scores of `tasks`, two sequences of a query per
+// register (sw_stream_kernel.cu): the tasks of a query, longest first, in pairs.
+void Engine::run_sw_stream( const SearchRequest & req, const std::vector<PairTask> & tasks, PairTask * redo_list ) {
+    std::vector<uint32_t> order( tasks.size() );
+    for( uint32_t k = 0; k < (uint32_t) tasks.size(); k++ )
+        order[k] = k;
+    // queries with the most rows first (their pairs have the most stripes)
+    std::sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
+        const PairTask & a = tasks[x];
+        const PairTask & b = tasks[y];
+        if( a.qslot != b.qslot )
+            return h_qlen_[a.qslot] != h_qlen_[b.qslot] ? h_qlen_[a.qslot] > h_qlen_[b.qslot] : a.qslot < b.qslot;
+        return db_.len[a.id] != db_.len[b.id] ? db_.len[a.id] > db_.len[b.id] : a.id < b.id;
+    } );
+    uint64_t stripes128 = 0;
+    std::vector<SwStreamItem> items;
+    for( size_t k = 0; k < order.size(); ) {
+        const PairTask & a = tasks[order[k]];
+        const bool two = k + 1 < order.size() && tasks[order[k + 1]].qslot == a.qslot;
+        items.push_back( SwStreamItem{ a.qslot, a.id, two ? tasks[order[k + 1]].id : 0xffffffffu, 0 } );
+        stripes128 += (h_qlen_[a.qslot] + 127u) / 128u;
+        k += two ? 2 : 1;
+    }
+    // rows per lane: 4 while every stripe of 128 rows can be resident (24 warps per SM)
+    const int R = stripes128 <= (uint64_t) sms_ * 24 ? 4 : 8;
+    const uint32_t rows = 32u * (uint32_t) R;
+    const uint32_t ni = (uint32_t) items.size();
+    // launches of as many items as 1 GB of boundary rows holds
+    for( uint32_t i0 = 0; i0 < ni; ) {
+        std::vector<uint64_t> bnd;
+        uint64_t words = 0;
+        uint32_t i1 = i0;
+        for( ; i1 < ni; i1++ ) {
+            const SwStreamItem & t = items[i1];
+            const uint64_t w = h_qlen_[t.slot] > rows ? 2ull * ((db_.len[t.id_a] + 3u) / 4u) : 0;   // A is the longer
+            if( i1 > i0 && (words + w) * sizeof(int4) > ((uint64_t) 1 << 30) )
+                break;
+            bnd.push_back( words );
+            words += w;
+        }
+        const uint32_t n = i1 - i0;
+        std::vector<uint32_t> cum{ 0 };
+        for( uint32_t left = n, i = 0;; i++ ) {
+            while( left && (uint64_t) i * rows >= h_qlen_[items[i0 + left - 1].slot] )
+                left--;
+            if( left == 0 )
+                break;
+            cum.push_back( cum.back() + left );
+        }
+        const size_t b_items = n * sizeof(SwStreamItem), b_bnd = (n * sizeof(uint64_t) + 15) & ~(size_t) 15,
+                b_cum = cum.size() * sizeof(uint32_t);
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the staging buffer is free
+        uint8_t * h = (uint8_t *) h_sw_in_.ensure( b_items + b_bnd + b_cum );
+        memcpy( h, items.data() + i0, b_items );
+        memcpy( h + b_items, bnd.data(), n * sizeof(uint64_t) );
+        memcpy( h + b_items + b_bnd, cum.data(), b_cum );
+        uint8_t * d = (uint8_t *) d_sw_in_.ensure( b_items + b_bnd + b_cum );
+        CUDA_CHECK( cudaMemcpyAsync( d, h, b_items + b_bnd + b_cum, cudaMemcpyHostToDevice, stream_ ) );
+        const uint32_t nt = cum.back();
+        // ticket counter, then progress and results
+        uint8_t * sy = (uint8_t *) d_tb_sync_.ensure( 16 + (size_t) nt * 2 * sizeof(uint32_t) );
+        CUDA_CHECK( cudaMemsetAsync( sy, 0, 16 + (size_t) nt * sizeof(uint32_t), stream_ ) );
+        SwStreamParams p{};
+        p.db = db_view();
+        p.qcodes = d_qcodes_.as<uint8_t>();
+        p.qoff = d_qoff_.as<uint64_t>();
+        p.qlen = d_qlen_.as<uint32_t>();
+        p.matrix = d_matrix_.as<int64_t>();
+        p.gap_oe = req.gap_open + req.gap_extend;
+        p.gap_e = req.gap_extend;
+        p.limit = sw_fast_limit( req );
+        p.items = (const SwStreamItem *) d;
+        p.bnd_off = (const uint64_t *) (d + b_items);
+        p.cum = (const uint32_t *) (d + b_items + b_bnd);
+        p.levels = (uint32_t) cum.size() - 1;
+        p.n_tickets = nt;
+        p.counter = (unsigned long long *) sy;
+        p.progress = (uint32_t *) (sy + 16);
+        p.result = p.progress + nt;
+        p.boundary = (int4 *) d_tb_bnd_.ensure( words * sizeof(int4) + 16 );
+        p.sink.score = score_sink();
+        p.sink.score_stride = db_.n_ids;
+        p.sink.error_flags = d_counts_.as<unsigned>() + 2;
+        p.sink.redo = redo_list;
+        p.sink.redo_count = d_counts_.as<unsigned>() + 5;
+        p.sink.redo_cap = (uint32_t) tasks.size();
+        CUDA_CHECK( launch_sw_stream( R, p, sms_, stream_ ) );
+        launches_++;
+        i0 = i1;
+    }
+}
+
+void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, uint32_t cap,
+        std::vector<PairTask> & list_entry, std::vector<PairTask> & list_16, const std::vector<uint32_t> * slots,
+        uint32_t lo, uint32_t hi ) {
+    unsigned * cnt = d_counts_.as<unsigned>();
+    PairTask * list_a = d_list_a_.as<PairTask>();
+    PairTask * list_b = d_list_b_.as<PairTask>();
+    const size_t first = list_entry.size();
+    list_entry.resize( first + n_a );
+    CUDA_CHECK( cudaMemcpyAsync( list_entry.data() + first, list_a, n_a * sizeof(PairTask), cudaMemcpyDeviceToHost,
+            stream_ ) );
+    if( req.bit_width != 8 ) {
+        run_pass( req.algo, 64, req, nq, list_a, n_a, false, nullptr, cnt + 3, 0 );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the host list
+        return;
+    }
+    // the 16-bit pass: the 16x2 kernels where they are exact, and the lane
+    // emulation for the pairs that leave their range
+    SearchRequest r16 = req;
+    r16.bit_width = 16;
+    const bool queries_fit = max_qlen_ <= FAST_MAX_ROWS;
+    const uint64_t searched = (uint64_t) (slots ? slots->size() : nq) * (hi - lo);
+    if( fast_single_eligible( r16 ) ) {
+        PairTask * redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
+        CUDA_CHECK( cudaMemsetAsync( cnt + 5, 0, sizeof(unsigned), stream_ ) );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+        run_sw_stream( r16, std::vector<PairTask>( list_entry.begin() + first, list_entry.end() ), redo );
+        run_redo( r16, nq, list_b, cnt + 1, cap, redo );
+    }
+    else if( nw_fast_eligible( r16 ) && queries_fit && n_a >= searched / 4 ) {
+        // most pairs overflowed: the query-pair kernel over all of them, which
+        // scores the marked ones.  It computes a pair an order of magnitude
+        // faster than the emulation of the list, so it wins from a quarter on.
+        PairTask * redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
+        run_qpair_entry( r16, nq, list_b, cnt + 1, std::min( cap, n_a ), redo, slots, lo, hi, true );
+    }
+    else {
+        run_pass( req.algo, 16, req, nq, list_a, n_a, false, list_b, cnt + 1, cap );
+    }
+    unsigned n_b = 0;
+    CUDA_CHECK( cudaMemcpyAsync( &n_b, cnt + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
+    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+    n_b = std::min( n_b, cap );
+    if( n_b ) {
+        const size_t at = list_16.size();
+        list_16.resize( at + n_b );
+        run_pass( req.algo, 64, req, nq, list_b, n_b, false, nullptr, cnt + 3, 0 );
+        CUDA_CHECK( cudaMemcpyAsync( list_16.data() + at, list_b, n_b * sizeof(PairTask), cudaMemcpyDeviceToHost,
+                stream_ ) );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
     }
 }
 
@@ -1452,7 +1608,6 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         CUDA_CHECK( cudaEventRecord( ev_phase_[0], stream_ ) );
         const int entry = req.bit_width;
         std::vector<PairTask> list_entry, list_16;   // host copies for the replay
-        uint64_t n_a = 0, n_b = 0;
         float entry_ms = 0;     // the entry passes of all segments
         // a resident database is one segment; a streamed one runs the entry pass
         // and the cascade of each segment while it is on the device
@@ -1470,7 +1625,8 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
                 if( (fast_eligible( req ) && (nq >= 2 || streaming_ || !fast_single_eligible( req )) &&
                             !getenv( "SSA_B200_NO_QPAIR" )) ||
                         nw_fast_eligible( req ) )
-                    run_qpair_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap, nullptr, lo, hi );
+                    run_qpair_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), nullptr,
+                            lo, hi );
                 else if( fast_single_eligible( req ) )
                     run_fast_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap );
                 else
@@ -1478,6 +1634,7 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
                             cap, nullptr, 0, lo );
             };
             run_entry();
+            uint32_t n_req = 0;     // pairs the entry pass re-queued
             for( ;; ) {
                 // counts of the entry list and the NW redo list (their atomic
                 // counters count every append, kept or not) and the error flags
@@ -1485,8 +1642,10 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
                 CUDA_CHECK( cudaMemcpyAsync( c, cnt, sizeof c, cudaMemcpyDeviceToHost, stream_ ) );
                 CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
                 const uint64_t need = std::max<uint64_t>( c[0], c[5] );
-                if( need <= cap && !(c[2] & ERR_REQUEUE_OVERFLOW) )
+                if( need <= cap && !(c[2] & ERR_REQUEUE_OVERFLOW) ) {
+                    n_req = c[0];
                     break;
+                }
                 cap = (uint32_t) std::min<uint64_t>( all_pairs, std::max<uint64_t>( need, 2ull * cap ) );
                 d_list_a_.ensure( (size_t) cap * sizeof(PairTask) );
                 d_list_b_.ensure( (size_t) cap * sizeof(PairTask) );
@@ -1498,38 +1657,14 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
             float seg_ms = 0;
             CUDA_CHECK( cudaEventElapsedTime( &seg_ms, ev_seg_[0], ev_seg_[1] ) );
             entry_ms += seg_ms;
-            if( entry == 64 )
+            if( entry == 64 || n_req == 0 )
                 continue;
-            unsigned sa = 0, sb = 0;
-            CUDA_CHECK( cudaMemcpyAsync( &sa, cnt + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-            CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-            sa = std::min( sa, cap );
-            if( sa == 0 )
-                continue;
-            const int w2 = (entry == 8) ? 16 : 64;
-            PairTask * nx = (w2 == 16) ? d_list_b_.as<PairTask>() : nullptr;
-            run_pass( req.algo, w2, req, nq, d_list_a_.as<PairTask>(), sa, false, nx, cnt + 1, cap );
-            if( w2 == 16 ) {
-                CUDA_CHECK( cudaMemcpyAsync( &sb, cnt + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-                CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-                sb = std::min( sb, cap );
-                if( sb )
-                    run_pass( req.algo, 64, req, nq, d_list_b_.as<PairTask>(), sb, false, nullptr, cnt + 3, 0 );
-            }
-            list_entry.resize( n_a + sa );
-            CUDA_CHECK( cudaMemcpyAsync( list_entry.data() + n_a, d_list_a_.p, sa * sizeof(PairTask),
-                    cudaMemcpyDeviceToHost, stream_ ) );
-            if( sb ) {
-                list_16.resize( n_b + sb );
-                CUDA_CHECK( cudaMemcpyAsync( list_16.data() + n_b, d_list_b_.p, sb * sizeof(PairTask),
-                        cudaMemcpyDeviceToHost, stream_ ) );
-            }
-            n_a += sa;
-            n_b += sb;
+            run_cascade( req, nq, n_req, cap, list_entry, list_16, nullptr, lo, hi );
             if( streaming_ )
                 CUDA_CHECK( cudaStreamSynchronize( stream_ ) );   // the lists are reused by the next segment
         }
         CUDA_CHECK( cudaEventRecord( ev_phase_[2], stream_ ) );
+        const uint64_t n_a = list_entry.size(), n_b = list_16.size();
         stats.d2h_bytes += score_bytes + (n_a + n_b) * sizeof(PairTask);
         int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
         if( score_bytes )
@@ -2283,37 +2418,20 @@ void Engine::shard_scores( const SearchRequest & req, const std::vector<QueryCod
         const int entry = req.bit_width;
         CUDA_CHECK( cudaEventRecord( ev_seg_[0], stream_ ) );
         if( fast_eligible( req ) || nw_fast_eligible( req ) )
-            run_qpair_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap, nullptr, 0, (uint32_t) n_sh );
+            run_qpair_entry( req, nq, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), nullptr, 0,
+                    (uint32_t) n_sh );
         else
             run_pass( req.algo, entry, req, nq, nullptr, (uint64_t) nq * n_sh, true, d_list_a_.as<PairTask>(),
                     cnt + 0, cap );
         CUDA_CHECK( cudaEventRecord( ev_seg_[1], stream_ ) );
         std::vector<PairTask> list_entry, list_16;
-        unsigned sa = 0, sb = 0;
+        unsigned sa = 0;
         if( entry != 64 ) {
             CUDA_CHECK( cudaMemcpyAsync( &sa, cnt + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
             CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
             sa = std::min( sa, cap );
-            if( sa ) {
-                const int w2 = (entry == 8) ? 16 : 64;
-                PairTask * nx = (w2 == 16) ? d_list_b_.as<PairTask>() : nullptr;
-                run_pass( req.algo, w2, req, nq, d_list_a_.as<PairTask>(), sa, false, nx, cnt + 1, cap );
-                if( w2 == 16 ) {
-                    CUDA_CHECK( cudaMemcpyAsync( &sb, cnt + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-                    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-                    sb = std::min( sb, cap );
-                    if( sb )
-                        run_pass( req.algo, 64, req, nq, d_list_b_.as<PairTask>(), sb, false, nullptr, cnt + 3, 0 );
-                }
-                list_entry.resize( sa );
-                CUDA_CHECK( cudaMemcpyAsync( list_entry.data(), d_list_a_.p, sa * sizeof(PairTask),
-                        cudaMemcpyDeviceToHost, stream_ ) );
-                if( sb ) {
-                    list_16.resize( sb );
-                    CUDA_CHECK( cudaMemcpyAsync( list_16.data(), d_list_b_.p, sb * sizeof(PairTask),
-                            cudaMemcpyDeviceToHost, stream_ ) );
-                }
-            }
+            if( sa )
+                run_cascade( req, nq, sa, cap, list_entry, list_16, nullptr, 0, (uint32_t) n_sh );
         }
         int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
         CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
@@ -2330,7 +2448,7 @@ void Engine::shard_scores( const SearchRequest & req, const std::vector<QueryCod
         float ms = 0;
         CUDA_CHECK( cudaEventElapsedTime( &ms, ev_seg_[0], ev_seg_[1] ) );
         stats.entry_seconds += ms * 1e-3;
-        stats.d2h_bytes += score_bytes + (sa + sb) * sizeof(PairTask);
+        stats.d2h_bytes += score_bytes + (list_entry.size() + list_16.size()) * sizeof(PairTask);
         for( uint32_t q = 0; q < nq; q++ ) {
             const uint64_t row = (uint64_t) (b0 + q) * width;
             ReplayQuery rq;
@@ -2486,7 +2604,8 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
     const int entry = req.bit_width;
     CUDA_CHECK( cudaEventRecord( ev_phase_[0], stream_ ) );
     if( fast_eligible( req ) || nw_fast_eligible( req ) ) {
-        run_qpair_entry( req, serve_slots_, d_list_a_.as<PairTask>(), cnt + 0, cap, &active, seq_lo, seq_hi );
+        run_qpair_entry( req, serve_slots_, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), &active,
+                seq_lo, seq_hi );
     }
     else {
         d_slots_.ensure( active.size() * sizeof(uint32_t) );
@@ -2496,32 +2615,13 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
                 d_slots_.as<uint32_t>(), (uint32_t) active.size(), seq_lo );
     }
     CUDA_CHECK( cudaEventRecord( ev_phase_[1], stream_ ) );
-    unsigned n_a = 0, n_b = 0;
+    unsigned n_a = 0;
     if( entry != 64 ) {
         CUDA_CHECK( cudaMemcpyAsync( &n_a, cnt + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
         CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
         n_a = std::min( n_a, cap );
-        if( n_a ) {
-            const int w2 = (entry == 8) ? 16 : 64;
-            PairTask * nx = (w2 == 16) ? d_list_b_.as<PairTask>() : nullptr;
-            run_pass( req.algo, w2, req, serve_slots_, d_list_a_.as<PairTask>(), n_a, false, nx, cnt + 1, cap );
-            if( w2 == 16 ) {
-                CUDA_CHECK( cudaMemcpyAsync( &n_b, cnt + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-                CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-                n_b = std::min( n_b, cap );
-                if( n_b )
-                    run_pass( req.algo, 64, req, serve_slots_, d_list_b_.as<PairTask>(), n_b, false, nullptr, cnt + 3,
-                            0 );
-            }
-            ovf_entry.resize( n_a );
-            CUDA_CHECK( cudaMemcpyAsync( ovf_entry.data(), d_list_a_.p, n_a * sizeof(PairTask),
-                    cudaMemcpyDeviceToHost, stream_ ) );
-            if( n_b ) {
-                ovf16.resize( n_b );
-                CUDA_CHECK( cudaMemcpyAsync( ovf16.data(), d_list_b_.p, n_b * sizeof(PairTask),
-                        cudaMemcpyDeviceToHost, stream_ ) );
-            }
-        }
+        if( n_a )
+            run_cascade( req, serve_slots_, n_a, cap, ovf_entry, ovf16, &active, seq_lo, seq_hi );
     }
     unsigned err = 0;
     CUDA_CHECK( cudaMemcpyAsync( &err, cnt + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
@@ -2535,8 +2635,8 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
     CUDA_CHECK( cudaEventElapsedTime( &ms[1], ev_phase_[1], ev_phase_[2] ) );
     stats.entry_seconds += ms[0] * 1e-3;
     stats.kernel_seconds += (ms[0] + ms[1]) * 1e-3;
-    stats.overflow8 += n_a;
-    stats.overflow16 += n_b;
+    stats.overflow8 += ovf_entry.size();
+    stats.overflow16 += ovf16.size();
 }
 
 void Engine::serve_finish( const SearchRequest & req, const std::vector<uint32_t> & done,

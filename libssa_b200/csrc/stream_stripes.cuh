@@ -19,7 +19,7 @@
 //     order also keeps few stripes of many alignments in flight rather than all
 //     of one, whose last ones would wait for the whole pipeline to fill.
 //   * The boundary row is updated in place: stripe i reads column c before it
-//     writes it (it writes 31 columns behind its own reads), stripe i + 1 reads
+//     writes it (it writes 31 columns behind its own reads); stripe i + 1 reads
 //     it after stripe i published it.
 //   * A wait has an iteration limit, after which it sets ERR_PIPELINE, and every
 //     other wait sees the flag and gives up too; the stripe below takes what
@@ -38,10 +38,12 @@ constexpr uint32_t STREAM_DONE = 0x80000000u;         // progress word: the stri
 constexpr uint32_t STREAM_WAIT_LIMIT = 1u << 24;      // polls of 100 ns and more each
 
 // Shared memory of one warp: the rows entering and leaving the stripe in the
-// current 32 columns, and the residues.
+// current chunk of steps, one word per lane.  A column of a row is 32 / CHUNK
+// words: CHUNK = 32 with int2 words (H and F of one column), CHUNK = 16 with
+// int4 words (two per block of four columns).
+template <class Word>
 struct StreamStage {
-    int2 in[32], out[32];
-    uint8_t residues[64];
+    Word in[32], out[32];
 };
 
 __device__ __forceinline__ uint32_t load_acquire( const uint32_t * p ) {
@@ -78,58 +80,66 @@ __device__ __forceinline__ uint32_t stream_wait( const uint32_t * progress, uint
     return v;
 }
 
-// One stripe's place among the alignment's.
+// One stripe's place among the alignment's.  "Columns" are whatever one
+// wavefront step advances by (the 16x2 kernels: blocks of four columns).
+template <class Word>
 struct StreamStripe {
     uint32_t cols;                 // database columns
-    int2 * row;                    // the alignment's boundary row
+    Word * row;                    // the alignment's boundary row
     const uint32_t * above;        // progress of the stripe above, nullptr: the first stripe
     uint32_t * mine;               // this stripe's progress
-    const int32_t * limit;         // last column worth computing, shrinking while the stripes run; nullptr: none
     bool last;                     // no stripe below
     unsigned * error_flags;
 };
 
-// Sweeps one stripe.  column( s, edge, cols ) computes wavefront step s: edge
-// says that some lane may be on a column outside 0 .. cols - 1, or on the
-// last one.  Lane 0 finds the row above column s in st.in[s & 31], lane 31
-// leaves the row below column s - 31 in st.out[s & 31].  Returns the columns
-// swept; the caller publishes the end with stream_end().
-template <class Column>
-__device__ __forceinline__ uint32_t stream_columns( const StreamStripe & sp, StreamStage & st, ResidueRing & rr,
-        int lane, Column && column ) {
+__device__ __forceinline__ int2 zero_word( const int2 * ) { return make_int2( 0, 0 ); }
+__device__ __forceinline__ int4 zero_word( const int4 * ) { return make_int4( 0, 0, 0, 0 ); }
+
+// No column limit.
+struct StreamAll {
+    static constexpr bool NONE = true;
+    __device__ int32_t operator()() const { return 0; }
+};
+
+// Sweeps one stripe.  limit() reads the last column worth computing, which may
+// shrink while the stripes run (lane 0's value counts).  refill( s0 ) runs before the steps s0 .. s0 + CHUNK - 1,
+// column( s, edge, cols ) computes wavefront step s: edge says that some lane
+// may be on a column outside 0 .. cols - 1, or on the last one.  Lane 0 finds
+// the row above column s in st.in (word s % CHUNK, or the words from there),
+// lane 31 leaves the row below column s - 31 in the same place of st.out.
+// Returns the columns swept; the caller publishes the end with stream_end().
+template <int CHUNK, class Word, class Limit, class Refill, class Column>
+__device__ __forceinline__ uint32_t stream_columns( const StreamStripe<Word> & sp, StreamStage<Word> & st, int lane,
+        const Limit & limit, Refill && refill, Column && column ) {
+    constexpr uint32_t WPC = 32 / CHUNK;       // words per column
     uint32_t cols = sp.cols;
     uint32_t avail = 0;            // columns of the row above known to be written
-    bool have = false;             // pf holds the next 32 columns of it
-    int2 pf = make_int2( 0, 0 );
-    rr.start( lane );
-    for( uint32_t s0 = 0;; s0 += 32 ) {
-        if( sp.limit ) {
-            int32_t lim = 0;
-            if( lane == 0 )
-                lim = *(volatile const int32_t *) sp.limit;
-            lim = __shfl_sync( 0xffffffffu, lim, 0 );
-            cols = min( cols, (uint32_t) lim + 1u );
-        }
+    bool have = false;             // pf holds the next chunk of it
+    Word pf = zero_word( (const Word *) nullptr );
+    for( uint32_t s0 = 0;; s0 += CHUNK ) {
+        if constexpr( !Limit::NONE )
+            cols = min( cols, (uint32_t) __shfl_sync( 0xffffffffu, lane == 0 ? limit() : 0, 0 ) + 1u );
         if( sp.above && s0 < cols ) {
             if( !have ) {
-                const uint32_t need = min( s0 + 32u, cols );
+                const uint32_t need = min( s0 + (uint32_t) CHUNK, cols );
                 if( avail < need ) {
                     const uint32_t v = stream_wait( sp.above, need, lane, sp.error_flags );
                     avail = v & ~STREAM_DONE;
                     if( avail < need )             // the stripe above has ended there
                         cols = min( cols, avail );
                 }
-                if( s0 + (uint32_t) lane < cols )
-                    pf = __ldcg( sp.row + s0 + lane );
+                if( s0 * WPC + (uint32_t) lane < cols * WPC )
+                    pf = __ldcg( sp.row + (uint64_t) s0 * WPC + lane );
             }
             __syncwarp();
             st.in[lane] = pf;
             __syncwarp();
-            // the next 32 columns now if they are there, so that their load is
-            // not on the critical path; else after a wait at the next turn
+            // the next chunk now if it is there, so that its load is not on
+            // the critical path; else after a wait at the next turn
             have = false;
-            if( s0 + 32u < cols ) {
-                const uint32_t need = min( s0 + 64u, cols );
+            const uint32_t s2 = s0 + (uint32_t) CHUNK;
+            if( s2 < cols ) {
+                const uint32_t need = min( s2 + (uint32_t) CHUNK, cols );
                 if( avail < need ) {
                     uint32_t v = 0;
                     if( lane == 0 )
@@ -139,8 +149,8 @@ __device__ __forceinline__ uint32_t stream_columns( const StreamStripe & sp, Str
                     avail = max( avail, v & ~STREAM_DONE );
                 }
                 if( avail >= need ) {
-                    if( s0 + 32u + (uint32_t) lane < cols )
-                        pf = __ldcg( sp.row + s0 + 32 + lane );
+                    if( s2 * WPC + (uint32_t) lane < cols * WPC )
+                        pf = __ldcg( sp.row + (uint64_t) s2 * WPC + lane );
                     have = true;
                 }
             }
@@ -148,8 +158,8 @@ __device__ __forceinline__ uint32_t stream_columns( const StreamStripe & sp, Str
         const uint32_t steps = cols + 31u;
         if( cols == 0 || s0 >= steps )
             break;
-        rr.step( s0, lane );
-        const uint32_t s1 = min( s0 + 32u, steps );
+        refill( s0 );
+        const uint32_t s1 = min( s0 + (uint32_t) CHUNK, steps );
         if( s0 >= 31u && s1 < cols ) {
             for( uint32_t s = s0; s < s1; s++ )
                 column( s, false, cols );
@@ -160,9 +170,9 @@ __device__ __forceinline__ uint32_t stream_columns( const StreamStripe & sp, Str
         }
         if( !sp.last ) {
             __syncwarp();
-            const int32_t c = (int32_t) s0 - 31 + lane;
+            const int32_t c = (int32_t) s0 - 31 + lane / (int) WPC;
             if( c >= 0 && c < (int32_t) s1 - 31 )
-                __stcg( sp.row + c, st.out[lane] );
+                __stcg( sp.row + (uint64_t) c * WPC + lane % WPC, st.out[lane] );
             __syncwarp();
             if( lane == 0 && s1 > 31u )
                 store_release( sp.mine, s1 - 31u );
@@ -175,7 +185,8 @@ __device__ __forceinline__ uint32_t stream_columns( const StreamStripe & sp, Str
 
 // The stripe has ended after `cols` columns; whatever the warp wrote before is
 // visible to a warp that sees this.
-__device__ __forceinline__ void stream_end( const StreamStripe & sp, uint32_t cols, int lane ) {
+template <class Word>
+__device__ __forceinline__ void stream_end( const StreamStripe<Word> & sp, uint32_t cols, int lane ) {
     __syncwarp();
     if( lane == 0 && !sp.last )
         store_release( sp.mine, STREAM_DONE | cols );

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast_kernel( FastParams p ) {
             break;
         const uint32_t slot = p.unit_slots[u % p.n_class];
         const uint32_t chunk = (uint32_t) (u / p.n_class);
-        const uint32_t pair_begin = p.chunk_bounds[chunk], pair_end = p.chunk_bounds[chunk + 1];
+        const uint32_t pair_begin = max( p.chunk_bounds[chunk], p.pair_skip ), pair_end = p.chunk_bounds[chunk + 1];
         const int G = (int) p.slot_group[slot];
         const uint32_t GR = (uint32_t) (G * R);
         const uint32_t rows = p.slot_rows[slot];
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
             break;
         const uint32_t slot = p.unit_slots[u % p.n_class];
         const uint32_t chunk = (uint32_t) (u / p.n_class);
-        const uint32_t pair_begin = p.chunk_bounds[chunk], pair_end = p.chunk_bounds[chunk + 1];
+        const uint32_t pair_begin = max( p.chunk_bounds[chunk], p.pair_skip ), pair_end = p.chunk_bounds[chunk + 1];
         const int G = (int) p.slot_group[slot];
         const uint32_t GR = (uint32_t) (G * R);
         const uint32_t rows = p.slot_rows[slot];

@@ -157,6 +157,14 @@ __device__ __forceinline__ Cell warp_best( Cell c ) {
     return c;
 }
 
+// The reverse pass's limit: the first column that holds a candidate so far.
+template <bool REVERSE>
+struct ColumnLimit {
+    static constexpr bool NONE = !REVERSE;
+    const int32_t * p;
+    __device__ int32_t operator()() const { return *(volatile const int32_t *) p; }
+};
+
 enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR };
 
 // ---------------------------------------------------------------------------
@@ -199,7 +207,8 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
     constexpr int ROWS = 32 * R;
     constexpr bool DIRS = PHASE == TB_DIRECTIONS || PHASE == TB_FWDDIR;
     constexpr bool ENDS = PHASE == TB_FORWARD || PHASE == TB_FWDDIR;       // looks for the end cell
-    __shared__ StreamStage stages[TB_WARPS];
+    __shared__ StreamStage<int2> stages[TB_WARPS];
+    __shared__ uint8_t residues[TB_WARPS][64];
     __shared__ int32_t smat[1024];
     __shared__ __align__( 16 ) uint32_t tables[P8 ? TB_WARPS : 1][P8 ? 32 * 32 * (R / 4) : 1];
     const int lane = threadIdx.x & 31;
@@ -212,7 +221,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         smat[i] = (int32_t) (DIRS ? p.matrix[(d << 5) + q] : p.matrix[(q << 5) + d]);
     }
     __syncthreads();
-    StreamStage & st = stages[warp];
+    StreamStage<int2> & st = stages[warp];
 
     for( ;; ) {
         const uint32_t ticket = next_hit( p.counter, lane );
@@ -239,15 +248,14 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             continue;                                   // the reverse pass may need fewer rows than the query has
         const uint8_t * a = p.qcodes + p.qoff[hit.qslot];
 
-        StreamStripe sp;
+        StreamStripe<int2> sp;
         sp.cols = B;
         sp.row = p.boundary + p.bnd_off[h];
         sp.above = stripe ? p.progress + pred : nullptr;
         sp.mine = p.progress + ticket;
-        sp.limit = PHASE == TB_REVERSE ? p.limit + h : nullptr;
         sp.last = (stripe + 1u) * (uint32_t) ROWS >= A;
         sp.error_flags = p.error_flags;
-        ResidueRing rr{ st.residues, 0, p.db.codes + p.db.offsets[hit.id], (int32_t) B,
+        ResidueRing rr{ residues[warp], 0, p.db.codes + p.db.offsets[hit.id], (int32_t) B,
             PHASE == TB_REVERSE ? rg.b_end : -1 };
 
         TbLane<R, P8> t;
@@ -413,7 +421,10 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             if( lane == 31 )
                 st.out[s & 31u] = make_int2( t.out_h, t.out_f );
         };
-        const uint32_t swept = stream_columns( sp, st, rr, lane, column );
+        rr.start( lane );
+        const ColumnLimit<PHASE == TB_REVERSE> limit{ p.limit + h };
+        const uint32_t swept = stream_columns<32>( sp, st, lane, limit, [&]( uint32_t s0 ) { rr.step( s0, lane ); },
+                column );
         if constexpr( PHASE != TB_DIRECTIONS ) {
             // this stripe's cell against that of the stripes above (theirs is
             // final once the stripe above has ended)
