@@ -134,6 +134,8 @@ public:
             CUDA_CHECK( cudaEventCreate( &ev_cls_t_[2 * i] ) );
             CUDA_CHECK( cudaEventCreate( &ev_cls_t_[2 * i + 1] ) );
         }
+        CUDA_CHECK( cudaStreamCreateWithFlags( &long_stream_, cudaStreamNonBlocking ) );
+        CUDA_CHECK( cudaEventCreateWithFlags( &ev_long_, cudaEventDisableTiming ) );
         device_ = dev;
         ready_ = true;
     }
@@ -454,7 +456,7 @@ public:
             &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_qcodes_, &d_qoff_, &d_qlen_, &d_qpad_,
             &d_prof_off_, &d_prof_, &d_matrix_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
             &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_, &d_qp_off_, &d_qp_rows_, &d_qp_slots_, &d_qp_units_,
-            &d_serve_score_, &d_qp_lmax_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_, &d_list_c_, &d_sw_in_,
+            &d_serve_score_, &d_qp_lmax_, &d_qp_skip_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_, &d_list_c_, &d_sw_in_, &d_sw_sync_, &d_sw_bnd_,
             &d_seg_[0], &d_seg_[1], &d_gather_codes_, &d_gather_off_, &d_gather_len_, &d_prof64_, &d_score64_ };
         for( DevBuf * b : bufs )
             b->release();
@@ -496,7 +498,8 @@ private:
     void run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
             uint32_t cap, PairTask * redo_list, const std::vector<uint32_t> * slots = nullptr, uint32_t seq_lo = 0,
             uint32_t seq_hi = UINT32_MAX, bool marked = false );
-    void run_sw_stream( const SearchRequest & req, const std::vector<PairTask> & tasks, PairTask * redo_list );
+    void run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
+            cudaStream_t st );
     // The passes after the entry width: list A holds n_a pairs that it re-queued.
     // Leaves their scores, and the lists on the host (appended).
     void run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, uint32_t cap,
@@ -540,7 +543,7 @@ private:
     DevBuf d_prof8_, d_prof8_off_, d_rows_, d_slots_;
     DevBuf d_scratch_fast_[8];      // per class of the single-query pass
     DevBuf d_bounds_, d_group_;
-    DevBuf d_qp_prof_, d_qp_off_, d_qp_rows_, d_qp_slots_, d_qp_units_, d_qp_lmax_;
+    DevBuf d_qp_prof_, d_qp_off_, d_qp_rows_, d_qp_slots_, d_qp_units_, d_qp_lmax_, d_qp_skip_;
     // serving: fixed query slots and their own score rows
     DevBuf d_serve_score_;
     bool serving_ = false;           // passes write d_serve_score_
@@ -550,12 +553,14 @@ private:
     cudaStream_t class_stream_[4] = { nullptr, nullptr, nullptr, nullptr };
     cudaEvent_t ev_class_[4] = { nullptr, nullptr, nullptr, nullptr };
     cudaEvent_t ev_cls_t_[8] = {};   // per class start / end, timed (SSA_B200_TIMING)
+    cudaStream_t long_stream_ = nullptr;      // an entry pass's longest pairs
+    cudaEvent_t ev_long_ = nullptr;
     cudaEvent_t ev_ready_ = nullptr;
     cudaEvent_t ev_phase_[6] = {};
     cudaEvent_t ev_seg_[2] = {};     // around one segment's entry pass
     cudaEvent_t ev_tb_[5] = {};   // batch start, entry pass done, cascade done, copies done, traceback
     DevBuf d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_prof_, d_matrix_;
-    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_in_;
+    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_in_, d_sw_sync_, d_sw_bnd_;
     DevBuf d_tb_io_, d_tb_last_, d_tb_dirs_, d_tb_sync_, d_tb_result_, d_tb_bnd_;
     PinnedBuf h_score_, h_tb_in_, h_tb_out_, h_sw_in_;
 public:
@@ -830,6 +835,15 @@ static FastShape choose_shape( uint32_t Q, double mean_len, int bucket ) {
     return best;
 }
 
+// Steps above which an entry pass gives a pair to the streamed stripes: every
+// resident group's share of the pass, at least 256 (about 0.1 ms, below which
+// the extra launch costs what it saves).  SSA_B200_STREAM_SHARE pins it (tests).
+static uint64_t stream_share( uint64_t share ) {
+    if( const char * pin = getenv( "SSA_B200_STREAM_SHARE" ) )
+        return strtoull( pin, nullptr, 10 );
+    return std::max<uint64_t>( share, 256 );
+}
+
 void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
         uint32_t cap ) {
     const uint32_t n_pairs = (uint32_t) db_.pair_cols.size();
@@ -944,7 +958,36 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
     if( req.bit_width != 8 )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
+    // the longest pairs on streamed stripes, as in run_qpair_entry: those that
+    // take more steps than every resident group's share of the pass
+    uint32_t pair_skip = 0;
+    std::vector<SwStreamItem> items;
+    if( nq == 1 && n_shaped == 1 && !getenv( "SSA_B200_NO_STREAM" ) ) {
+        const uint64_t groups = (uint64_t) sms_ * 16 * (32u / (uint32_t) shape[0].G);
+        const uint64_t P = (uint64_t) shape[0].P;
+        const uint64_t share = stream_share( P * (total_cols / 4u) / groups );
+        if( 2 * P * (db_.pair_cols[0] / 4u) > 3 * share )
+            while( pair_skip < n_pairs && P * (db_.pair_cols[pair_skip] / 4u) > share ) {
+                items.push_back( SwStreamItem{ 0, db_.pair_a[pair_skip], db_.pair_b[pair_skip], 0 } );
+                pair_skip++;
+            }
+    }
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
+    if( pair_skip ) {
+        PassSink lists{};
+        lists.next = next;
+        lists.next_count = next_count;
+        lists.next_cap = cap;
+        if( req.bit_width != 8 ) {
+            lists.redo = d_list_b_.as<PairTask>();
+            lists.redo_count = redo_count;
+            lists.redo_cap = cap;
+        }
+        CUDA_CHECK( cudaStreamWaitEvent( long_stream_, ev_ready_, 0 ) );
+        run_sw_stream( req, items, lists, long_stream_ );
+        CUDA_CHECK( cudaEventRecord( ev_long_, long_stream_ ) );
+        CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_long_, 0 ) );
+    }
     size_t class_first = 0;
     for( int ci = 0; ci < 8; ci++ ) {
         const std::vector<uint32_t> & cls = by_r[ci];
@@ -997,6 +1040,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         p.gap_oe = req.bit_width == 8 ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
         p.gap_e = req.gap_extend;
         p.limit = sw_fast_limit( req );
+        p.pair_skip = pair_skip;
         if( req.bit_width != 8 ) {
             p.sink.redo = d_list_b_.as<PairTask>();
             p.sink.redo_count = redo_count;
@@ -1274,6 +1318,69 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     uint64_t seg_residues = 0;
     for( uint32_t i = lo; i < hi; i++ )
         seg_residues += db_.len[db_.order_desc[i]];
+    // The longest sequences against the longest queries on streamed stripes.  A
+    // group of 4 threads takes passes x blocks steps for a pair, one after the
+    // other; the whole call takes `share` steps of every resident group.  Pairs
+    // of more steps than that would still run when the rest is done.  Measured on
+    // a B200: a server's 32 requests against 100,000 proteins, whose first wave
+    // holds the longest sequences, 108 -> 96 ms; one query of 300 x 200,000
+    // with 1% of 8,000-35,000 residues (run_fast_entry) entry pass 28.5 -> 5.9
+    // ms, half of it because both sequences of a pair overflow early and end
+    // it.  Where no pair takes half as long again as the
+    // share, the entry kernel keeps them all (it needs fewer instructions per
+    // cell: four chains of 20-28 rows against 4 or 8).
+    std::vector<uint32_t> qp_skip( std::max<uint32_t>( 1, n_qp ), 0 );
+    std::vector<SwStreamItem> items;
+    if( !nw && fast_single_eligible( req ) && !getenv( "SSA_B200_NO_STREAM" ) ) {
+        auto passes_of = [&]( uint32_t i, int R ) { return (uint64_t) qp_rows[i] / (uint64_t) (QP_G * R); };
+        auto blocks_of = [&]( uint32_t i ) { return (uint64_t) (db_.len[db_.order_desc[lo + i]] + 3u) / 4u; };
+        uint64_t steps = 0, longest = 0;
+        for( int ri = 0; ri < 4; ri++ )
+            for( uint32_t i : by_r[ri] ) {
+                steps += passes_of( i, 4 * (ri + 4) ) * (total_cols / 4u);
+                longest = std::max( longest, passes_of( i, 4 * (ri + 4) ) * blocks_of( 0 ) );
+            }
+        const uint64_t share = stream_share( steps / ((uint64_t) sms_ * 16 * QP_GPW) );
+        if( 2 * longest > 3 * share )
+            for( int ri = 0; ri < 4; ri++ )
+                for( uint32_t i : by_r[ri] ) {
+                    const uint64_t P = passes_of( i, 4 * (ri + 4) );
+                    uint32_t a = 0, b = n_seq;          // sequences of more than share / P blocks come first
+                    while( a < b ) {
+                        const uint32_t mid = (a + b) / 2;
+                        if( P * blocks_of( mid ) > share )
+                            a = mid + 1;
+                        else
+                            b = mid;
+                    }
+                    qp_skip[i] = std::min( n_seq, (a + 1u) & ~1u );
+                    for( int h = 0; h < 2; h++ ) {
+                        const uint32_t slot = qp_slots[2 * i + h];
+                        for( uint32_t k = 0; k < qp_skip[i] && slot != 0xffffffffu; k += 2 )
+                            items.push_back( SwStreamItem{ slot, db_.order_desc[lo + k],
+                                    k + 1 < qp_skip[i] ? db_.order_desc[lo + k + 1] : 0xffffffffu, 0 } );
+                    }
+                }
+    }
+    if( !items.empty() ) {
+        d_qp_skip_.ensure( qp_skip.size() * sizeof(uint32_t) );
+        CUDA_CHECK( cudaMemcpyAsync( d_qp_skip_.p, qp_skip.data(), qp_skip.size() * sizeof(uint32_t),
+                cudaMemcpyHostToDevice, stream_ ) );
+        CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
+        PassSink lists{};
+        lists.next = next;
+        lists.next_count = next_count;
+        lists.next_cap = cap;
+        if( redo ) {
+            lists.redo = redo_list;
+            lists.redo_count = redo_count;
+            lists.redo_cap = cap;
+        }
+        CUDA_CHECK( cudaStreamWaitEvent( long_stream_, ev_ready_, 0 ) );
+        run_sw_stream( req, items, lists, long_stream_ );
+        CUDA_CHECK( cudaEventRecord( ev_long_, long_stream_ ) );
+        CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_long_, 0 ) );
+    }
     // classes launched heaviest first (most rows per thread: the longest
     // queries), so that the last class to finish is the lightest
     size_t class_start[4] = { 0, 0, 0, 0 };
@@ -1343,6 +1450,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         p.qlen = d_qlen_.as<uint32_t>();
         p.qp_lmax = d_qp_lmax_.as<uint32_t>();
         p.marked_only = marked;
+        p.qp_skip = items.empty() ? nullptr : d_qp_skip_.as<uint32_t>();
         if( redo ) {
             p.sink.redo = redo_list;
             p.sink.redo_count = redo_count;
@@ -1386,33 +1494,23 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     }
 }
 
-// The 16-bit Smith-Waterman scores of `tasks`, two sequences of a query per
-// register (sw_stream_kernel.cu): the tasks of a query, longest first, in pairs.
-void Engine::run_sw_stream( const SearchRequest & req, const std::vector<PairTask> & tasks, PairTask * redo_list ) {
-    std::vector<uint32_t> order( tasks.size() );
-    for( uint32_t k = 0; k < (uint32_t) tasks.size(); k++ )
-        order[k] = k;
-    // queries with the most rows first (their pairs have the most stripes)
-    std::sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
-        const PairTask & a = tasks[x];
-        const PairTask & b = tasks[y];
-        if( a.qslot != b.qslot )
-            return h_qlen_[a.qslot] != h_qlen_[b.qslot] ? h_qlen_[a.qslot] > h_qlen_[b.qslot] : a.qslot < b.qslot;
-        return db_.len[a.id] != db_.len[b.id] ? db_.len[a.id] > db_.len[b.id] : a.id < b.id;
+// Smith-Waterman scores of `items` at the request's width (two sequences of a
+// query per register, sw_stream_kernel.cu) on stream st; lists: where the pairs
+// that the kernel does not report go.
+void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
+        cudaStream_t st ) {
+    // queries with the most rows first: their items have the most stripes
+    std::stable_sort( items.begin(), items.end(), [&]( const SwStreamItem & x, const SwStreamItem & y ) {
+        return h_qlen_[x.slot] > h_qlen_[y.slot];
     } );
     uint64_t stripes128 = 0;
-    std::vector<SwStreamItem> items;
-    for( size_t k = 0; k < order.size(); ) {
-        const PairTask & a = tasks[order[k]];
-        const bool two = k + 1 < order.size() && tasks[order[k + 1]].qslot == a.qslot;
-        items.push_back( SwStreamItem{ a.qslot, a.id, two ? tasks[order[k + 1]].id : 0xffffffffu, 0 } );
-        stripes128 += (h_qlen_[a.qslot] + 127u) / 128u;
-        k += two ? 2 : 1;
-    }
+    for( const SwStreamItem & t : items )
+        stripes128 += (h_qlen_[t.slot] + 127u) / 128u;
     // rows per lane: 4 while every stripe of 128 rows can be resident (24 warps per SM)
     const int R = stripes128 <= (uint64_t) sms_ * 24 ? 4 : 8;
     const uint32_t rows = 32u * (uint32_t) R;
     const uint32_t ni = (uint32_t) items.size();
+    const bool blocks = req.bit_width == 8;
     // launches of as many items as 1 GB of boundary rows holds
     for( uint32_t i0 = 0; i0 < ni; ) {
         std::vector<uint64_t> bnd;
@@ -1437,24 +1535,26 @@ void Engine::run_sw_stream( const SearchRequest & req, const std::vector<PairTas
         }
         const size_t b_items = n * sizeof(SwStreamItem), b_bnd = (n * sizeof(uint64_t) + 15) & ~(size_t) 15,
                 b_cum = cum.size() * sizeof(uint32_t);
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the staging buffer is free
+        if( i0 )
+            CUDA_CHECK( cudaStreamSynchronize( st ) );      // the buffers of the launch before are free
         uint8_t * h = (uint8_t *) h_sw_in_.ensure( b_items + b_bnd + b_cum );
         memcpy( h, items.data() + i0, b_items );
         memcpy( h + b_items, bnd.data(), n * sizeof(uint64_t) );
         memcpy( h + b_items + b_bnd, cum.data(), b_cum );
         uint8_t * d = (uint8_t *) d_sw_in_.ensure( b_items + b_bnd + b_cum );
-        CUDA_CHECK( cudaMemcpyAsync( d, h, b_items + b_bnd + b_cum, cudaMemcpyHostToDevice, stream_ ) );
+        CUDA_CHECK( cudaMemcpyAsync( d, h, b_items + b_bnd + b_cum, cudaMemcpyHostToDevice, st ) );
         const uint32_t nt = cum.back();
-        // ticket counter, then progress and results
-        uint8_t * sy = (uint8_t *) d_tb_sync_.ensure( 16 + (size_t) nt * 2 * sizeof(uint32_t) );
-        CUDA_CHECK( cudaMemsetAsync( sy, 0, 16 + (size_t) nt * sizeof(uint32_t), stream_ ) );
+        // ticket counter, progress, results, and per sequence its first crossing
+        const size_t b_zero = 16 + (size_t) nt * sizeof(uint32_t), b_cross = blocks ? n * 2 * sizeof(int32_t) : 0;
+        uint8_t * sy = (uint8_t *) d_sw_sync_.ensure( b_zero + (size_t) nt * sizeof(uint32_t) + b_cross );
+        CUDA_CHECK( cudaMemsetAsync( sy, 0, b_zero, st ) );
         SwStreamParams p{};
         p.db = db_view();
         p.qcodes = d_qcodes_.as<uint8_t>();
         p.qoff = d_qoff_.as<uint64_t>();
         p.qlen = d_qlen_.as<uint32_t>();
         p.matrix = d_matrix_.as<int64_t>();
-        p.gap_oe = req.gap_open + req.gap_extend;
+        p.gap_oe = blocks ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
         p.gap_e = req.gap_extend;
         p.limit = sw_fast_limit( req );
         p.items = (const SwStreamItem *) d;
@@ -1465,14 +1565,16 @@ void Engine::run_sw_stream( const SearchRequest & req, const std::vector<PairTas
         p.counter = (unsigned long long *) sy;
         p.progress = (uint32_t *) (sy + 16);
         p.result = p.progress + nt;
-        p.boundary = (int4 *) d_tb_bnd_.ensure( words * sizeof(int4) + 16 );
+        if( blocks ) {
+            p.cross = (int32_t *) (p.result + nt);
+            CUDA_CHECK( cudaMemsetAsync( p.cross, 0x7f, b_cross, st ) );
+        }
+        p.boundary = (int4 *) d_sw_bnd_.ensure( words * sizeof(int4) + 16 );
+        p.sink = lists;
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
         p.sink.error_flags = d_counts_.as<unsigned>() + 2;
-        p.sink.redo = redo_list;
-        p.sink.redo_count = d_counts_.as<unsigned>() + 5;
-        p.sink.redo_cap = (uint32_t) tasks.size();
-        CUDA_CHECK( launch_sw_stream( R, p, sms_, stream_ ) );
+        CUDA_CHECK( launch_sw_stream( R, p, sms_, st ) );
         launches_++;
         i0 = i1;
     }
@@ -1502,8 +1604,25 @@ void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, 
     if( fast_single_eligible( r16 ) ) {
         PairTask * redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
         CUDA_CHECK( cudaMemsetAsync( cnt + 5, 0, sizeof(unsigned), stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        run_sw_stream( r16, std::vector<PairTask>( list_entry.begin() + first, list_entry.end() ), redo );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the host list
+        // the re-queued sequences of a query, longest first, in pairs
+        std::vector<PairTask> tasks( list_entry.begin() + first, list_entry.end() );
+        std::sort( tasks.begin(), tasks.end(), [&]( const PairTask & a, const PairTask & b ) {
+            if( a.qslot != b.qslot )
+                return a.qslot < b.qslot;
+            return db_.len[a.id] != db_.len[b.id] ? db_.len[a.id] > db_.len[b.id] : a.id < b.id;
+        } );
+        std::vector<SwStreamItem> items;
+        for( size_t k = 0; k < tasks.size(); ) {
+            const bool two = k + 1 < tasks.size() && tasks[k + 1].qslot == tasks[k].qslot;
+            items.push_back( SwStreamItem{ tasks[k].qslot, tasks[k].id, two ? tasks[k + 1].id : 0xffffffffu, 0 } );
+            k += two ? 2 : 1;
+        }
+        PassSink lists{};
+        lists.redo = redo;
+        lists.redo_count = cnt + 5;
+        lists.redo_cap = n_a;
+        run_sw_stream( r16, items, lists, stream_ );
         run_redo( r16, nq, list_b, cnt + 1, cap, redo );
     }
     else if( nw_fast_eligible( r16 ) && queries_fit && n_a >= searched / 4 ) {

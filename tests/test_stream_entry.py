@@ -1,0 +1,32 @@
+"""An entry pass's longest pairs on streamed stripes, with the share above
+which a pair goes there pinned from "all" to "the few longest": scores,
+overflow blocks (through the tie order and the counters) and CIGARs against
+the oracle, one query and batches, at every width."""
+import numpy as np
+import pytest
+
+from libssa_b200 import workloads as W
+from test_wide_entry import _check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("share", [0, 40, 400])
+@pytest.mark.parametrize("width", [8, 16, 64])
+def test_longest_pairs(built_library, monkeypatch, width, share):
+    monkeypatch.setenv("SSA_B200_STREAM_SHARE", str(share))
+    rng = np.random.default_rng(31 + share)
+    queries = [W.random_residues(rng, n, W.AA20) for n in (30, 128, 129, 260, 700)]
+    records = [W.random_residues(rng, int(n), W.AA20) for n in rng.integers(1, 700, 60)]
+    # overflows at the start, in the middle and at the end of long records, in
+    # one sequence of a register pair or both, and lengths around the blocks
+    for q in queries[1:]:
+        for n, at in ((900, 0), (901, 400), (902, 700), (903, 901 - len(q)), (2050, 1500), (2051, None)):
+            r = W.random_residues(rng, max(n, len(q)), W.AA20)
+            if at is not None:
+                at = max(0, min(at, len(r) - len(q)))
+                r[at:at + len(q)] = W.mutate(rng, q, W.AA20, 0.05, 0.0, (1, 1))
+            records.append(r)
+    records += [np.tile(queries[3], 12), np.zeros(0, np.uint8)]
+    _check(dict(algo="sw", width=width, align=1, hits=16, gap=(-11, -1), chunk=25, simd=2,
+                records=[r.tobytes() for r in records], queries=[q.tobytes() for q in queries]))
