@@ -183,6 +183,25 @@ cudaError_t launch_tb_directions( const TbParams & p, int R, bool p8, int sms, c
 cudaError_t launch_tb_fwddir( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
 cudaError_t launch_tb_walk( const TbParams & p, int R, cudaStream_t st );
 
+// Dynamic shared memory limit and resident blocks per SM of a kernel, asked of
+// the driver once per kernel and size (the engine's one device; its launches
+// are serialised by the engine's lock).
+struct LaunchShape {
+    size_t smem = (size_t) -1;
+    int blocks = 0;
+    template <class Kernel>
+    cudaError_t set( Kernel kernel, int threads, size_t bytes ) {
+        if( smem == bytes )
+            return cudaSuccess;
+        cudaError_t e = cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes );
+        if( e == cudaSuccess )
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor( &blocks, kernel, threads, bytes );
+        if( e == cudaSuccess )
+            smem = bytes;
+        return e;
+    }
+};
+
 // ---- fast Smith-Waterman entry pass (sw_fast_kernel.cu) --------------------
 // Residue code used after a sequence's last 4-column block in the pair layout;
 // its profile row is -128, so it never changes a Smith-Waterman maximum.

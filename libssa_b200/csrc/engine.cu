@@ -93,6 +93,70 @@ struct PinnedBuf {
     }
 };
 
+// A device array inside a buffer that something else owns.
+struct DevView {
+    void * p = nullptr;
+    template <class T>
+    T * as() const {
+        return (T *) p;
+    }
+};
+
+// The small arrays of one call on their way to the device: gathered in pinned
+// memory and sent in one copy.  (A copy from pageable memory costs the host
+// several microseconds, and a call has a dozen of them.)
+class Stager {
+public:
+    // A new call: the device has finished the one before.
+    void begin() {
+        used_ = sent_ = 0;
+        for( auto & o : old_ ) {
+            o.first.release();
+            o.second.release();
+        }
+        old_.clear();
+    }
+    // Copies n elements of data; returns where they will be on the device.
+    template <class T>
+    T * add( const T * data, size_t n, cudaStream_t st ) {
+        const size_t bytes = (n * sizeof(T) + 15) & ~(size_t) 15;
+        if( used_ + bytes > h_.bytes || !h_.p ) {
+            // arrays added before stay where they are until the next call
+            send( st );
+            const size_t want = std::max<size_t>( { 2 * h_.bytes, 2 * bytes, (size_t) 1 << 16 } );
+            if( h_.p )
+                old_.emplace_back( h_, d_ );
+            h_ = PinnedBuf();
+            d_ = DevBuf();
+            h_.ensure( want );
+            d_.ensure( want );
+            used_ = sent_ = 0;
+        }
+        const size_t at = used_;
+        if( n )
+            memcpy( (char *) h_.p + at, data, n * sizeof(T) );
+        used_ += bytes;
+        return (T *) ((char *) d_.p + at);
+    }
+    void send( cudaStream_t st ) {
+        if( used_ > sent_ )
+            CUDA_CHECK( cudaMemcpyAsync( (char *) d_.p + sent_, (char *) h_.p + sent_, used_ - sent_,
+                    cudaMemcpyHostToDevice, st ) );
+        sent_ = used_;
+    }
+    void release() {
+        begin();
+        h_.release();
+        d_.release();
+    }
+
+private:
+    PinnedBuf h_;
+    DevBuf d_;
+    size_t used_ = 0, sent_ = 0;
+    std::vector<std::pair<PinnedBuf, DevBuf>> old_;
+};
+
 class Engine {
 public:
     static Engine & get() {
@@ -451,19 +515,19 @@ public:
 
     void shutdown() {
         DevBuf * bufs[] = { &d_codes_, &d_off_, &d_len_, &d_order_, &d_pair_res_, &d_pair_off_, &d_pair_cols_,
-            &d_pair_ids_, &d_prof8_, &d_prof8_off_, &d_rows_, &d_slots_, &d_bounds_, &d_group_,
+            &d_pair_ids_, &d_prof8_,
             &d_scratch_fast_[0], &d_scratch_fast_[1], &d_scratch_fast_[2], &d_scratch_fast_[3], &d_scratch_fast_[4],
-            &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_qcodes_, &d_qoff_, &d_qlen_, &d_qpad_,
-            &d_prof_off_, &d_prof_, &d_matrix_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
-            &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_, &d_qp_off_, &d_qp_rows_, &d_qp_slots_, &d_qp_units_,
-            &d_serve_score_, &d_qp_lmax_, &d_qp_skip_, &d_pair_slot_, &d_pair_unit_, &d_pair_score_, &d_list_c_, &d_sw_in_, &d_sw_sync_, &d_sw_bnd_,
+            &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_serve_block_, &d_prof_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
+            &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_,
+            &d_serve_score_, &d_pair_score_, &d_list_c_, &d_sw_sync_, &d_sw_bnd_,
             &d_seg_[0], &d_seg_[1], &d_gather_codes_, &d_gather_off_, &d_gather_len_, &d_prof64_, &d_score64_ };
         for( DevBuf * b : bufs )
             b->release();
+        stage_.release();
+        h_counts_.release();
         h_score_.release();
         h_score64_.release();
         h_tb_in_.release();
-        h_sw_in_.release();
         h_tb_out_.release();
         h_stage_.release();
         resident_seg_ = -1;
@@ -515,7 +579,8 @@ private:
             const std::vector<std::pair<uint32_t, uint32_t>> & lists, SearchStats & stats,
             bool scores_from_regions = false );
     uint64_t traceback_budget();
-    void upload_queries( const QueryCodes * queries, uint32_t nq, bool profiles, SearchStats & stats );
+    void upload_queries( const SearchRequest & req, const QueryCodes * queries, uint32_t nq, bool profiles,
+            SearchStats & stats );
 
     bool ready_ = false;
     int device_ = 0;
@@ -540,10 +605,9 @@ private:
     // device buffers
     DevBuf d_codes_, d_off_, d_len_, d_order_;
     DevBuf d_pair_res_, d_pair_off_, d_pair_cols_, d_pair_ids_;
-    DevBuf d_prof8_, d_prof8_off_, d_rows_, d_slots_;
+    DevBuf d_prof8_;
     DevBuf d_scratch_fast_[8];      // per class of the single-query pass
-    DevBuf d_bounds_, d_group_;
-    DevBuf d_qp_prof_, d_qp_off_, d_qp_rows_, d_qp_slots_, d_qp_units_, d_qp_lmax_, d_qp_skip_;
+    DevBuf d_qp_prof_;
     // serving: fixed query slots and their own score rows
     DevBuf d_serve_score_;
     bool serving_ = false;           // passes write d_serve_score_
@@ -559,10 +623,14 @@ private:
     cudaEvent_t ev_phase_[6] = {};
     cudaEvent_t ev_seg_[2] = {};     // around one segment's entry pass
     cudaEvent_t ev_tb_[5] = {};   // batch start, entry pass done, cascade done, copies done, traceback
-    DevBuf d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_prof_, d_matrix_;
-    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_in_, d_sw_sync_, d_sw_bnd_;
+    // the current queries and score table: in the stager, or the server's own block
+    DevView d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_matrix_;
+    DevBuf d_prof_, d_serve_block_;
+    Stager stage_;
+    PinnedBuf h_counts_;
+    DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_sync_, d_sw_bnd_;
     DevBuf d_tb_io_, d_tb_last_, d_tb_dirs_, d_tb_sync_, d_tb_result_, d_tb_bnd_;
-    PinnedBuf h_score_, h_tb_in_, h_tb_out_, h_sw_in_;
+    PinnedBuf h_score_, h_tb_in_, h_tb_out_;
 public:
     // entry-pass shapes of the last search call: kernel, (R, CTAs per SM) for
     // the query-pair kernel or (G, R) for the single-query one, queries or
@@ -580,7 +648,7 @@ private:
     PinnedBuf h_score64_;
     bool wide_ = false;
     int prof64_width_ = -1;
-    DevBuf d_pair_slot_, d_pair_unit_, d_pair_score_;
+    DevBuf d_pair_score_;
     uint64_t tb_budget_ = 0;         // traceback direction memory per wave (0 = automatic)
     // streaming: the database does not fit its device memory budget; segments
     // of consecutive positions of the length order take turns on the device
@@ -639,6 +707,7 @@ void Engine::run_pass( int algo, int width, const SearchRequest & req, uint32_t 
         const uint32_t * slot_list, uint32_t n_sub, uint32_t order_lo ) {
     if( n_tasks == 0 )
         return;
+    stage_.send( stream_ );
     build_profiles( width, n_slots );
     EmulParams p;
     p.db = db_view();
@@ -896,21 +965,9 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     for( uint32_t s : fallback )
         slots.push_back( s );
     d_prof8_.ensure( total + 16 );
-    d_prof8_off_.ensure( nq * sizeof(uint64_t) );
-    d_rows_.ensure( nq * sizeof(uint32_t) );
-    d_slots_.ensure( std::max<size_t>( 1, slots.size() ) * sizeof(uint32_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_prof8_off_.p, prof_off.data(), nq * sizeof(uint64_t), cudaMemcpyHostToDevice,
-            stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_rows_.p, rows_of.data(), nq * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_slots_.p, slots.data(), slots.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-            stream_ ) );
-    if( n_shaped ) {
-        CUDA_CHECK( launch_build_profile8( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
-                d_slots_.as<uint32_t>(), (uint32_t) n_shaped, d_rows_.as<uint32_t>(), d_matrix_.as<int64_t>(),
-                d_prof8_.as<int8_t>(), d_prof8_off_.as<uint64_t>(), stream_ ) );
-        launches_++;
-    }
-
+    const uint64_t * dev_prof_off = stage_.add( prof_off.data(), nq, stream_ );
+    const uint32_t * dev_rows = stage_.add( rows_of.data(), nq, stream_ );
+    const uint32_t * dev_slots = stage_.add( slots.data(), slots.size(), stream_ );
     // work units: ranges of length-sorted pairs holding about equal numbers
     // of columns, the longest first; every query of a class gets every range.
     // A warp takes one unit at a time and runs its pairs 32 / G at a time, so
@@ -949,11 +1006,15 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     for( uint32_t s = 0; s < nq; s++ )
         if( shape[s].G )
             group_of[s] = (uint16_t) shape[s].G;
-    d_bounds_.ensure( bounds.size() * sizeof(uint32_t) );
-    d_group_.ensure( nq * sizeof(uint16_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_bounds_.p, bounds.data(), bounds.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-            stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_group_.p, group_of.data(), nq * sizeof(uint16_t), cudaMemcpyHostToDevice, stream_ ) );
+    const uint32_t * dev_bounds = stage_.add( bounds.data(), bounds.size(), stream_ );
+    const uint16_t * dev_group = stage_.add( group_of.data(), nq, stream_ );
+    stage_.send( stream_ );
+    if( n_shaped ) {
+        CUDA_CHECK( launch_build_profile8( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
+                dev_slots, (uint32_t) n_shaped, dev_rows, d_matrix_.as<int64_t>(),
+                d_prof8_.as<int8_t>(), dev_prof_off, stream_ ) );
+        launches_++;
+    }
     const uint32_t cols_max = ((db_.max_len + 7u) & ~7u) + 8;
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
     if( req.bit_width != 8 )
@@ -1029,12 +1090,12 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         p.pair_cols = d_pair_cols_.as<uint32_t>();
         p.pair_ids = d_pair_ids_.as<uint2>();
         p.prof8 = d_prof8_.as<int8_t>();
-        p.prof8_off = d_prof8_off_.as<uint64_t>();
-        p.slot_group = d_group_.as<uint16_t>();
-        p.slot_rows = d_rows_.as<uint32_t>();
-        p.unit_slots = d_slots_.as<uint32_t>() + class_first;
+        p.prof8_off = dev_prof_off;
+        p.slot_group = dev_group;
+        p.slot_rows = dev_rows;
+        p.unit_slots = dev_slots + class_first;
         p.n_class = (uint32_t) cls.size();
-        p.chunk_bounds = d_bounds_.as<uint32_t>();
+        p.chunk_bounds = dev_bounds;
         p.n_units = (uint64_t) n_chunks * cls.size();
         p.unit_counter = unit_counter;
         p.gap_oe = req.bit_width == 8 ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
@@ -1069,7 +1130,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     if( !fallback.empty() ) {
         const uint64_t n_ne = db_.order_desc.size();
         run_pass( 0, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_ne, true, next, next_count, cap,
-                d_slots_.as<uint32_t>() + n_shaped, (uint32_t) fallback.size() );
+                dev_slots + n_shaped, (uint32_t) fallback.size() );
     }
 }
 
@@ -1259,34 +1320,16 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         units.insert( units.end(), v.begin(), v.end() );
     }
     d_qp_prof_.ensure( std::max<uint64_t>( total, 4 ) * sizeof(uint32_t) );
-    d_qp_off_.ensure( qp_off.size() * sizeof(uint64_t) );
-    d_qp_rows_.ensure( qp_rows.size() * sizeof(uint32_t) );
-    d_qp_slots_.ensure( qp_slots.size() * sizeof(uint32_t) );
-    d_qp_units_.ensure( std::max<size_t>( 1, units.size() ) * sizeof(uint32_t) );
-    d_qp_lmax_.ensure( qp_lmax.size() * sizeof(uint32_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qp_lmax_.p, qp_lmax.data(), qp_lmax.size() * sizeof(uint32_t),
-            cudaMemcpyHostToDevice, stream_ ) );
+    const uint64_t * dev_off = stage_.add( qp_off.data(), qp_off.size(), stream_ );
+    const uint32_t * dev_rows = stage_.add( qp_rows.data(), qp_rows.size(), stream_ );
+    const uint32_t * dev_qslots = stage_.add( qp_slots.data(), qp_slots.size(), stream_ );
+    const uint32_t * dev_units = stage_.add( units.data(), units.size(), stream_ );
+    const uint32_t * dev_lmax = stage_.add( qp_lmax.data(), qp_lmax.size(), stream_ );
     // pairs outside the kernels' range, for the lane emulation (the 8-bit entry has none)
     const bool redo = req.bit_width != 8;
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
     if( redo )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qp_off_.p, qp_off.data(), qp_off.size() * sizeof(uint64_t), cudaMemcpyHostToDevice,
-            stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qp_rows_.p, qp_rows.data(), qp_rows.size() * sizeof(uint32_t),
-            cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qp_slots_.p, qp_slots.data(), qp_slots.size() * sizeof(uint32_t),
-            cudaMemcpyHostToDevice, stream_ ) );
-    if( !units.empty() )
-        CUDA_CHECK( cudaMemcpyAsync( d_qp_units_.p, units.data(), units.size() * sizeof(uint32_t),
-                cudaMemcpyHostToDevice, stream_ ) );
-    if( n_qp ) {
-        CUDA_CHECK( launch_build_profile_qp( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
-                d_qp_slots_.as<uint32_t>(), n_qp, d_qp_rows_.as<uint32_t>(), d_matrix_.as<int64_t>(),
-                d_qp_prof_.as<uint32_t>(), d_qp_off_.as<uint64_t>(), req.bit_width == 8 ? 8 : 16, stream_ ) );
-        launches_++;
-    }
-
     // work units: ranges of length-sorted sequences (multiples of QP_GPW)
     // holding about equal numbers of columns, the longest first; every pair of
     // a class gets every range.  A warp takes one unit at a time.
@@ -1309,9 +1352,14 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
             bounds.push_back( n_seq );
     }
     const uint32_t n_chunks = (uint32_t) bounds.size() - 1;
-    d_bounds_.ensure( bounds.size() * sizeof(uint32_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_bounds_.p, bounds.data(), bounds.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-            stream_ ) );
+    const uint32_t * dev_bounds = stage_.add( bounds.data(), bounds.size(), stream_ );
+    stage_.send( stream_ );
+    if( n_qp ) {
+        CUDA_CHECK( launch_build_profile_qp( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
+                dev_qslots, n_qp, dev_rows, d_matrix_.as<int64_t>(),
+                d_qp_prof_.as<uint32_t>(), dev_off, req.bit_width == 8 ? 8 : 16, stream_ ) );
+        launches_++;
+    }
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     const uint32_t scratch_cols = (((db_.max_len + 3u) & ~3u) >> 1) + 2u;
     const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
@@ -1329,6 +1377,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     // it.  Where no pair takes half as long again as the
     // share, the entry kernel keeps them all (it needs fewer instructions per
     // cell: four chains of 20-28 rows against 4 or 8).
+    const uint32_t * dev_skip = nullptr;
     std::vector<uint32_t> qp_skip( std::max<uint32_t>( 1, n_qp ), 0 );
     std::vector<SwStreamItem> items;
     if( !nw && fast_single_eligible( req ) && !getenv( "SSA_B200_NO_STREAM" ) ) {
@@ -1363,9 +1412,8 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
                 }
     }
     if( !items.empty() ) {
-        d_qp_skip_.ensure( qp_skip.size() * sizeof(uint32_t) );
-        CUDA_CHECK( cudaMemcpyAsync( d_qp_skip_.p, qp_skip.data(), qp_skip.size() * sizeof(uint32_t),
-                cudaMemcpyHostToDevice, stream_ ) );
+        dev_skip = stage_.add( qp_skip.data(), qp_skip.size(), stream_ );
+        stage_.send( stream_ );
         CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
         PassSink lists{};
         lists.next = next;
@@ -1422,13 +1470,13 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         p.db = db_view();
         p.order = d_order_.as<uint32_t>() + lo;
         p.prof = d_qp_prof_.as<uint32_t>();
-        p.prof_off = d_qp_off_.as<uint64_t>();
-        p.qp_slots = d_qp_slots_.as<uint32_t>();
-        p.qp_rows = d_qp_rows_.as<uint32_t>();
-        p.unit_pairs = d_qp_units_.as<uint32_t>() + class_first;
+        p.prof_off = dev_off;
+        p.qp_slots = dev_qslots;
+        p.qp_rows = dev_rows;
+        p.unit_pairs = dev_units + class_first;
         p.n_class = (uint32_t) cls.size();
         p.n_chunks = n_chunks;
-        p.chunk_bounds = d_bounds_.as<uint32_t>();
+        p.chunk_bounds = dev_bounds;
         p.n_units = (uint64_t) n_chunks * cls.size();
         p.unit_counter = unit_counter;
         // the 8-bit Smith-Waterman lanes add the int8 truncation of gapO + gapE
@@ -1448,9 +1496,9 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         }
         p.gap_open = req.gap_open;
         p.qlen = d_qlen_.as<uint32_t>();
-        p.qp_lmax = d_qp_lmax_.as<uint32_t>();
+        p.qp_lmax = dev_lmax;
         p.marked_only = marked;
-        p.qp_skip = items.empty() ? nullptr : d_qp_skip_.as<uint32_t>();
+        p.qp_skip = dev_skip;
         if( redo ) {
             p.sink.redo = redo_list;
             p.sink.redo_count = redo_count;
@@ -1486,11 +1534,9 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     if( redo )
         run_redo( req, nq, next, next_count, cap, redo_list );
     if( !fallback.empty() ) {
-        d_slots_.ensure( fallback.size() * sizeof(uint32_t) );
-        CUDA_CHECK( cudaMemcpyAsync( d_slots_.p, fallback.data(), fallback.size() * sizeof(uint32_t),
-                cudaMemcpyHostToDevice, stream_ ) );
+        const uint32_t * dev_slots = stage_.add( fallback.data(), fallback.size(), stream_ );
         run_pass( req.algo, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_seq, true, next,
-                next_count, cap, d_slots_.as<uint32_t>(), (uint32_t) fallback.size(), lo );
+                next_count, cap, dev_slots, (uint32_t) fallback.size(), lo );
     }
 }
 
@@ -1533,16 +1579,10 @@ void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem>
                 break;
             cum.push_back( cum.back() + left );
         }
-        const size_t b_items = n * sizeof(SwStreamItem), b_bnd = (n * sizeof(uint64_t) + 15) & ~(size_t) 15,
-                b_cum = cum.size() * sizeof(uint32_t);
-        if( i0 )
-            CUDA_CHECK( cudaStreamSynchronize( st ) );      // the buffers of the launch before are free
-        uint8_t * h = (uint8_t *) h_sw_in_.ensure( b_items + b_bnd + b_cum );
-        memcpy( h, items.data() + i0, b_items );
-        memcpy( h + b_items, bnd.data(), n * sizeof(uint64_t) );
-        memcpy( h + b_items + b_bnd, cum.data(), b_cum );
-        uint8_t * d = (uint8_t *) d_sw_in_.ensure( b_items + b_bnd + b_cum );
-        CUDA_CHECK( cudaMemcpyAsync( d, h, b_items + b_bnd + b_cum, cudaMemcpyHostToDevice, st ) );
+        const SwStreamItem * dev_items = stage_.add( items.data() + i0, n, st );
+        const uint64_t * dev_bnd = stage_.add( bnd.data(), n, st );
+        const uint32_t * dev_cum = stage_.add( cum.data(), cum.size(), st );
+        stage_.send( st );
         const uint32_t nt = cum.back();
         // ticket counter, progress, results, and per sequence its first crossing
         const size_t b_zero = 16 + (size_t) nt * sizeof(uint32_t), b_cross = blocks ? n * 2 * sizeof(int32_t) : 0;
@@ -1557,9 +1597,9 @@ void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem>
         p.gap_oe = blocks ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
         p.gap_e = req.gap_extend;
         p.limit = sw_fast_limit( req );
-        p.items = (const SwStreamItem *) d;
-        p.bnd_off = (const uint64_t *) (d + b_items);
-        p.cum = (const uint32_t *) (d + b_items + b_bnd);
+        p.items = dev_items;
+        p.bnd_off = dev_bnd;
+        p.cum = dev_cum;
         p.levels = (uint32_t) cum.size() - 1;
         p.n_tickets = nt;
         p.counter = (unsigned long long *) sy;
@@ -1671,9 +1711,6 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         return;
     const uint64_t n_ne = db.order_desc.size();
 
-    // matrix on the device
-    d_matrix_.ensure( 1024 * sizeof(int64_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
 
     // the 64-bit pass in int64 arithmetic when the values can leave the int32 range
     {
@@ -1698,7 +1735,8 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         const size_t b0 = gstart[g0];
         const uint32_t nq = (uint32_t) (gstart[g1] - b0);
         // ---- upload queries
-        upload_queries( queries.data() + b0, nq, true, stats );
+        stage_.begin();
+        upload_queries( req, queries.data() + b0, nq, true, stats );
         for( uint32_t q = 0; q < nq; q++ )
             stats.cells += (uint64_t) h_qlen_[q] * db.residues;
 
@@ -1727,6 +1765,10 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         CUDA_CHECK( cudaEventRecord( ev_phase_[0], stream_ ) );
         const int entry = req.bit_width;
         std::vector<PairTask> list_entry, list_16;   // host copies for the replay
+        // few scores come back with the entry pass's counts: they are final when
+        // nothing was re-queued, and the call then waits for the device once
+        int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
+        const bool early = !streaming_ && !wide_ && score_bytes && score_bytes <= ((size_t) 1 << 20);
         float entry_ms = 0;     // the entry passes of all segments
         // a resident database is one segment; a streamed one runs the entry pass
         // and the cascade of each segment while it is on the device
@@ -1757,8 +1799,10 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
             for( ;; ) {
                 // counts of the entry list and the NW redo list (their atomic
                 // counters count every append, kept or not) and the error flags
-                unsigned c[6] = {};
-                CUDA_CHECK( cudaMemcpyAsync( c, cnt, sizeof c, cudaMemcpyDeviceToHost, stream_ ) );
+                unsigned * c = (unsigned *) h_counts_.ensure( 6 * sizeof(unsigned) );
+                CUDA_CHECK( cudaMemcpyAsync( c, cnt, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
+                if( early )
+                    CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
                 CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
                 const uint64_t need = std::max<uint64_t>( c[0], c[5] );
                 if( need <= cap && !(c[2] & ERR_REQUEUE_OVERFLOW) ) {
@@ -1785,8 +1829,8 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         CUDA_CHECK( cudaEventRecord( ev_phase_[2], stream_ ) );
         const uint64_t n_a = list_entry.size(), n_b = list_16.size();
         stats.d2h_bytes += score_bytes + (n_a + n_b) * sizeof(PairTask);
-        int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
-        if( score_bytes )
+        const bool have_scores = early && n_a == 0;
+        if( score_bytes && !have_scores )
             CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
         int64_t * hs64 = nullptr;
         if( wide_ && score_bytes ) {
@@ -1794,12 +1838,14 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
             CUDA_CHECK( cudaMemcpyAsync( hs64, d_score64_.p, 2 * score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
             stats.d2h_bytes += 2 * score_bytes;
         }
-        unsigned err = 0;
-        CUDA_CHECK( cudaMemcpyAsync( &err, cnt + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
+        unsigned * err = (unsigned *) h_counts_.p + 2;
+        if( !have_scores )
+            CUDA_CHECK( cudaMemcpyAsync( err, cnt + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
         CUDA_CHECK( cudaEventRecord( ev_phase_[3], stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        if( err )
-            fatal( "Internal error in the GPU search (flags 0x%x).", err );
+        if( !have_scores )
+            CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+        if( *err )
+            fatal( "Internal error in the GPU search (flags 0x%x).", *err );
         const auto t_replay0 = std::chrono::steady_clock::now();
 
         // ---- host replay, one query (group of query sequences) per worker
@@ -1894,7 +1940,8 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
 
 // Query codes of one batch to the device (slot s = queries[s]); profiles: also
 // size the int32 profile buffer of the lane emulation.
-void Engine::upload_queries( const QueryCodes * queries, uint32_t nq, bool profiles, SearchStats & stats ) {
+void Engine::upload_queries( const SearchRequest & req, const QueryCodes * queries, uint32_t nq, bool profiles,
+        SearchStats & stats ) {
     h_qoff_.assign( nq, 0 );
     h_qlen_.assign( nq, 0 );
     h_qpad_.assign( nq, 0 );
@@ -1914,20 +1961,16 @@ void Engine::upload_queries( const QueryCodes * queries, uint32_t nq, bool profi
     std::vector<uint8_t> hq( qtotal + 16, 0 );
     for( uint32_t s = 0; s < nq; s++ )
         memcpy( hq.data() + h_qoff_[s], queries[s].codes, queries[s].len );
-    d_qcodes_.ensure( hq.size() );
-    d_qoff_.ensure( nq * sizeof(uint64_t) );
-    d_qlen_.ensure( nq * sizeof(uint32_t) );
-    d_qpad_.ensure( nq * sizeof(uint32_t) );
-    d_prof_off_.ensure( nq * sizeof(uint64_t) );
     if( profiles )
         d_prof_.ensure( ptotal * sizeof(int32_t) );
     stats.h2d_bytes += hq.size() + nq * (2 * sizeof(uint64_t) + 2 * sizeof(uint32_t));
-    CUDA_CHECK( cudaMemcpyAsync( d_qcodes_.p, hq.data(), hq.size(), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qoff_.p, h_qoff_.data(), nq * sizeof(uint64_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qlen_.p, h_qlen_.data(), nq * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qpad_.p, h_qpad_.data(), nq * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_prof_off_.p, h_prof_off_.data(), nq * sizeof(uint64_t), cudaMemcpyHostToDevice,
-            stream_ ) );
+    // sent with the arrays of the pass that reads them
+    d_matrix_.p = stage_.add( req.matrix, 1024, stream_ );
+    d_qcodes_.p = stage_.add( hq.data(), hq.size(), stream_ );
+    d_qoff_.p = stage_.add( h_qoff_.data(), nq, stream_ );
+    d_prof_off_.p = stage_.add( h_prof_off_.data(), nq, stream_ );
+    d_qlen_.p = stage_.add( h_qlen_.data(), nq, stream_ );
+    d_qpad_.p = stage_.add( h_qpad_.data(), nq, stream_ );
     prof_width_ = -1;
 }
 
@@ -2019,7 +2062,6 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     p.matrix = d_matrix_.as<int64_t>();
     p.gap_open = req.gap_open;
     p.gap_extend = req.gap_extend;
-    p.error_flags = d_counts_.as<unsigned>() + 2;
     int32_t * last_all = (int32_t *) d_tb_last_.ensure( 2 * last_off[nh] * sizeof(int32_t) + 16 );
     p.last_h = last_all;
     p.last_e = last_all + last_off[nh];
@@ -2072,8 +2114,9 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         const size_t o_hits = in.add( nw * sizeof(TbHit) ), o_last = in.add( nw * sizeof(uint64_t) ),
                 o_dir = in.add( nw * sizeof(uint64_t) ), o_ops = in.add( (nw + 1) * sizeof(uint64_t) ),
                 o_bnd = in.add( nw * sizeof(uint64_t) ), o_cum = in.add( cum.size() * sizeof(uint32_t) ),
-                o_reg = in.add( nw * sizeof(TbRegion) );
+                o_reg = in.add( nw * sizeof(TbRegion) ), o_err = in.add( sizeof(unsigned) );
         uint8_t * hin = (uint8_t *) h_tb_in_.ensure( in.bytes );
+        memset( hin + o_err, 0, sizeof(unsigned) );
         for( uint32_t k = 0; k < nw; k++ ) {
             const uint32_t h = wave[k];
             const uint64_t stripes = (rows[h] + stripe_rows - 1) / stripe_rows;
@@ -2095,13 +2138,14 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         ((uint64_t *) (hin + o_ops))[nw] = ops_bytes;
         memcpy( hin + o_cum, cum.data(), cum.size() * sizeof(uint32_t) );
         const uint32_t n_tickets = cum.back();
-        // device side: inputs (regions last, updated in place), then the
-        // passes' results in the order they are copied back
-        const size_t r_reg = res.add( nw * sizeof(TbRegion) ), r_len = res.add( nw * sizeof(uint32_t) ),
-                r_ops = res.add( paths ? ops_bytes : 0 );
+        // device side: inputs (regions and error flags last, updated in place),
+        // then the passes' results in the order they are copied back
+        const size_t r_reg = res.add( nw * sizeof(TbRegion) ), r_err = res.add( sizeof(unsigned) ),
+                r_len = res.add( nw * sizeof(uint32_t) ), r_ops = res.add( paths ? ops_bytes : 0 );
         uint8_t * din = (uint8_t *) d_tb_io_.ensure( in.bytes + res.bytes );
-        uint8_t * dout = din + o_reg;            // the regions of the inputs are the first results
-        uint8_t * hout = (uint8_t *) h_tb_out_.ensure( res.bytes + sizeof(unsigned) );
+        uint8_t * dout = din + o_reg;            // the regions and flags of the inputs are the first results
+        uint8_t * hout = (uint8_t *) h_tb_out_.ensure( res.bytes );
+        p.error_flags = (unsigned *) (dout + r_err);
         // progress of both sweeps, ticket counters and column limits: cleared
         // by one memset (the limits to a large positive number)
         Layout sy;
@@ -2127,6 +2171,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         p.limit = (int32_t *) (dsy + s_lim);
         if( paths )
             p.dirs = (uint8_t *) d_tb_dirs_.ensure( dir_bytes + 16 );
+        stage_.send( stream_ );
         CUDA_CHECK( cudaMemcpyAsync( din, hin, in.bytes, cudaMemcpyHostToDevice, stream_ ) );
         CUDA_CHECK( cudaMemsetAsync( dsy, 0, s_zero, stream_ ) );
         if( reverse )
@@ -2155,11 +2200,9 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         if( timing )
             CUDA_CHECK( cudaEventRecord( ev_tb_[2], stream_ ) );
         CUDA_CHECK( cudaMemcpyAsync( hout, dout, res.bytes, cudaMemcpyDeviceToHost, stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( hout + res.bytes, p.error_flags, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                stream_ ) );
         CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
         unsigned err = 0;
-        memcpy( &err, hout + res.bytes, sizeof err );
+        memcpy( &err, hout + r_err, sizeof err );
         if( err )
             fatal( "Internal error in the GPU traceback (flags 0x%x).", err );
         stats.h2d_bytes += in.bytes;
@@ -2340,9 +2383,9 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
     } );
     const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
     CUDA_CHECK( cudaEventRecord( ev0_, stream_ ) );
-    d_matrix_.ensure( 1024 * sizeof(int64_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
-    upload_queries( queries.data(), n, false, stats );
+    stage_.begin();
+    upload_queries( req, queries.data(), n, false, stats );
+    stage_.send( stream_ );
     d_counts_.ensure( 32 * sizeof(unsigned long long) );
     CUDA_CHECK( cudaMemsetAsync( d_counts_.p, 0, 32 * sizeof(unsigned long long), stream_ ) );
     const uint32_t nw = (uint32_t) work.size();
@@ -2391,8 +2434,9 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
         p.qcodes = d_qcodes_.as<uint8_t>();
         p.qoff = d_qoff_.as<uint64_t>();
         p.qlen = d_qlen_.as<uint32_t>();
-        p.pair_slot = (const uint32_t *) d_pair_slot_.ensure( nw * sizeof(uint32_t) );
-        p.pair_unit = (const uint32_t *) d_pair_unit_.ensure( nw * sizeof(uint32_t) );
+        p.pair_slot = stage_.add( hs.data(), nw, stream_ );
+        p.pair_unit = stage_.add( hu.data(), nw, stream_ );
+        stage_.send( stream_ );
         p.n_pairs = nw;
         p.matrix = d_matrix_.as<int64_t>();
         p.gap_open = req.gap_open;
@@ -2407,10 +2451,6 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
             p.scratch_cols = max_b;
             p.scratch = (int4 *) d_scratch_.ensure( (size_t) grid * (PAIR_THREADS / (32 * PAIR_W)) * max_b * sizeof(int4) );
         }
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.pair_slot, hs.data(), nw * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( (void *) p.pair_unit, hu.data(), nw * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                stream_ ) );
         stats.h2d_bytes += 2 * nw * sizeof(uint32_t);
         CUDA_CHECK( cudaEventRecord( ev_phase_[0], stream_ ) );
         CUDA_CHECK( launch_pair_score( req.algo, p, grid, stream_, nullptr ) );
@@ -2503,8 +2543,6 @@ void Engine::shard_scores( const SearchRequest & req, const std::vector<QueryCod
             qmax = std::max( qmax, q.len );
         wide_ = needs_int64( req, qmax, db.max_len );
     }
-    d_matrix_.ensure( 1024 * sizeof(int64_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
     std::vector<uint32_t> full_order;
     full_order.swap( db_.order_desc );
     db_.order_desc = shard;
@@ -2516,7 +2554,8 @@ void Engine::shard_scores( const SearchRequest & req, const std::vector<QueryCod
             pair_budget / std::max<uint64_t>( 1, db.n_ids ) ) );
     for( uint32_t b0 = 0; b0 < nq_all && n_sh; b0 += batch ) {
         const uint32_t nq = std::min( batch, nq_all - b0 );
-        upload_queries( queries.data() + b0, nq, true, stats );
+        stage_.begin();
+        upload_queries( req, queries.data() + b0, nq, true, stats );
         for( uint32_t q = 0; q < nq; q++ ) {
             uint64_t res = 0;
             for( uint32_t id : shard )
@@ -2595,15 +2634,13 @@ void Engine::align_hits( const SearchRequest & req, const std::vector<QueryCodes
     database();
     serving_ = false;
     serve_layout_ = false;
-    d_matrix_.ensure( 1024 * sizeof(int64_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
-    d_counts_.ensure( 32 * sizeof(unsigned long long) );
-    CUDA_CHECK( cudaMemsetAsync( d_counts_.p, 0, 32 * sizeof(unsigned long long), stream_ ) );
     const uint32_t nq = (uint32_t) queries.size();
     const uint32_t batch = 65535;
     for( uint32_t b0 = 0; b0 < nq; b0 += batch ) {
         const uint32_t n = std::min( batch, nq - b0 );
-        upload_queries( queries.data() + b0, n, false, stats );
+        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+        stage_.begin();
+        upload_queries( req, queries.data() + b0, n, false, stats );
         std::vector<std::pair<uint32_t, uint32_t>> lists;
         for( uint32_t q = 0; q < n; q++ )
             lists.emplace_back( b0 + q, q );
@@ -2614,8 +2651,6 @@ void Engine::align_hits( const SearchRequest & req, const std::vector<QueryCodes
 
 void Engine::serve_restore( const SearchRequest & req ) {
     const uint32_t S = serve_slots_;
-    d_matrix_.ensure( 1024 * sizeof(int64_t) );
-    CUDA_CHECK( cudaMemcpyAsync( d_matrix_.p, req.matrix, 1024 * sizeof(int64_t), cudaMemcpyHostToDevice, stream_ ) );
     h_qoff_.assign( S, 0 );
     h_qlen_.assign( S, 0 );
     h_qpad_.assign( S, 256 );
@@ -2627,18 +2662,26 @@ void Engine::serve_restore( const SearchRequest & req ) {
         h_qpad_[s] = std::max<uint32_t>( 256, (len + 255u) & ~255u );
         h_prof_off_[s] = (uint64_t) s * 32 * SERVE_MAX_QUERY;
     }
-    d_qcodes_.ensure( (size_t) S * SERVE_QSTRIDE + 16 );
-    d_qoff_.ensure( S * sizeof(uint64_t) );
-    d_qlen_.ensure( S * sizeof(uint32_t) );
-    d_qpad_.ensure( S * sizeof(uint32_t) );
-    d_prof_off_.ensure( S * sizeof(uint64_t) );
+    // one block: score table, offsets, lengths, codes
+    const size_t at_qoff = 1024 * sizeof(int64_t), at_poff = at_qoff + S * sizeof(uint64_t),
+            at_len = at_poff + S * sizeof(uint64_t), at_pad = at_len + S * sizeof(uint32_t),
+            at_codes = (at_pad + S * sizeof(uint32_t) + 15) & ~(size_t) 15;
+    char * block = (char *) d_serve_block_.ensure( at_codes + (size_t) S * SERVE_QSTRIDE + 16 );
+    d_matrix_.p = block;
+    d_qoff_.p = block + at_qoff;
+    d_prof_off_.p = block + at_poff;
+    d_qlen_.p = block + at_len;
+    d_qpad_.p = block + at_pad;
+    d_qcodes_.p = block + at_codes;
     d_prof_.ensure( (size_t) S * 32 * SERVE_MAX_QUERY * sizeof(int32_t) );
     d_counts_.ensure( 32 * sizeof(unsigned long long) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qoff_.p, h_qoff_.data(), S * sizeof(uint64_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qlen_.p, h_qlen_.data(), S * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qpad_.p, h_qpad_.data(), S * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_prof_off_.p, h_prof_off_.data(), S * sizeof(uint64_t), cudaMemcpyHostToDevice,
-            stream_ ) );
+    std::vector<char> head( at_codes, 0 );
+    memcpy( head.data(), req.matrix, 1024 * sizeof(int64_t) );
+    memcpy( head.data() + at_qoff, h_qoff_.data(), S * sizeof(uint64_t) );
+    memcpy( head.data() + at_poff, h_prof_off_.data(), S * sizeof(uint64_t) );
+    memcpy( head.data() + at_len, h_qlen_.data(), S * sizeof(uint32_t) );
+    memcpy( head.data() + at_pad, h_qpad_.data(), S * sizeof(uint32_t) );
+    CUDA_CHECK( cudaMemcpyAsync( block, head.data(), head.size(), cudaMemcpyHostToDevice, stream_ ) );
     for( uint32_t s = 0; s < S; s++ )
         if( !serve_codes_[s].empty() )
             CUDA_CHECK( cudaMemcpyAsync( d_qcodes_.as<uint8_t>() + h_qoff_[s], serve_codes_[s].data(),
@@ -2703,6 +2746,7 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
         return;
     if( !serve_layout_ )
         serve_restore( req );
+    stage_.begin();
     serving_ = true;
     wide_ = false;                 // the server's settings were checked at serve_open
     const uint32_t n_seg = seq_hi - seq_lo;
@@ -2727,11 +2771,9 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
                 seq_lo, seq_hi );
     }
     else {
-        d_slots_.ensure( active.size() * sizeof(uint32_t) );
-        CUDA_CHECK( cudaMemcpyAsync( d_slots_.p, active.data(), active.size() * sizeof(uint32_t),
-                cudaMemcpyHostToDevice, stream_ ) );
+        const uint32_t * dev_slots = stage_.add( active.data(), active.size(), stream_ );
         run_pass( req.algo, entry, req, serve_slots_, nullptr, n_pairs, true, d_list_a_.as<PairTask>(), cnt + 0, cap,
-                d_slots_.as<uint32_t>(), (uint32_t) active.size(), seq_lo );
+                dev_slots, (uint32_t) active.size(), seq_lo );
     }
     CUDA_CHECK( cudaEventRecord( ev_phase_[1], stream_ ) );
     unsigned n_a = 0;

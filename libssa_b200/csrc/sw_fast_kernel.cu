@@ -273,11 +273,14 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast_kernel( FastParams p ) {
 // grid == 0: report the resident CTAs per SM in *blocks_per_sm without launching.
 template <int R>
 static cudaError_t launch_one( const FastParams & p, int grid, size_t smem, cudaStream_t st, int * blocks_per_sm ) {
-    cudaError_t e = cudaFuncSetAttribute( sw_fast_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( sw_fast_kernel<R>, FAST_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, sw_fast_kernel<R>, FAST_THREADS, smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     sw_fast_kernel<R><<<grid, FAST_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }
@@ -564,11 +567,14 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
 
 template <int R>
 static cudaError_t launch_four( const FastParams & p, int grid, size_t smem, cudaStream_t st, int * blocks_per_sm ) {
-    cudaError_t e = cudaFuncSetAttribute( sw_fast4_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( sw_fast4_kernel<R>, FAST_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, sw_fast4_kernel<R>, FAST_THREADS, smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     sw_fast4_kernel<R><<<grid, FAST_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }

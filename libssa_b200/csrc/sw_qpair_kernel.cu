@@ -552,13 +552,14 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
 template <int R, int MB, bool HM, int G = QP_G>
 static cudaError_t launch_qp4_one( const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm ) {
     const size_t smem = (size_t) (QP_THREADS / 32) * QP_CODES * G * R * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute( sw_qpair4_kernel<R, MB, HM, G>,
-            cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( sw_qpair4_kernel<R, MB, HM, G>, QP_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, sw_qpair4_kernel<R, MB, HM, G>,
-                QP_THREADS, smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     sw_qpair4_kernel<R, MB, HM, G><<<grid, QP_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }
@@ -593,13 +594,14 @@ cudaError_t launch_sw_qpair4( int R, int mb, bool hmax, bool g8, const QPairPara
 template <int R, int MB>
 static cudaError_t launch_qp_one( const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm ) {
     const size_t smem = (size_t) (QP_THREADS / 32) * QP_CODES * QP_G * R * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute( sw_qpair_kernel<R, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( sw_qpair_kernel<R, MB>, QP_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, sw_qpair_kernel<R, MB>, QP_THREADS,
-                smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     sw_qpair_kernel<R, MB><<<grid, QP_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }
@@ -888,12 +890,14 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
 template <int R>
 static cudaError_t launch_nw_one( const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm ) {
     const size_t smem = (size_t) (QP_THREADS / 32) * QP_CODES * QP_G * R * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute( nw_qpair_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( nw_qpair_kernel<R>, QP_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, nw_qpair_kernel<R>, QP_THREADS, smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     nw_qpair_kernel<R><<<grid, QP_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }
@@ -1232,12 +1236,14 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
 template <int R>
 static cudaError_t launch_nw4_one( const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm ) {
     const size_t smem = nw4_smem_bytes<R>();
-    cudaError_t e = cudaFuncSetAttribute( nw_qpair4_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            (int) smem );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( nw_qpair4_kernel<R>, QP_THREADS, smem );
     if( e != cudaSuccess )
         return e;
-    if( grid == 0 )
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( blocks_per_sm, nw_qpair4_kernel<R>, QP_THREADS, smem );
+    if( grid == 0 ) {
+        *blocks_per_sm = shape.blocks;
+        return cudaSuccess;
+    }
     nw_qpair4_kernel<R><<<grid, QP_THREADS, smem, st>>>( p );
     return cudaGetLastError();
 }

@@ -275,12 +275,11 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
 
 template <int R, bool BLOCKS>
 static cudaError_t launch_stream( const SwStreamParams & p, int sms, cudaStream_t st ) {
-    int per_sm = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, sw_stream_kernel<R, BLOCKS>,
-            STREAM_THREADS, 0 );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( sw_stream_kernel<R, BLOCKS>, STREAM_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
-    const uint32_t grid = min( (p.n_tickets + STREAM_WARPS - 1) / STREAM_WARPS, (uint32_t) (sms * max( 1, per_sm )) );
+    const uint32_t grid = min( (p.n_tickets + STREAM_WARPS - 1) / STREAM_WARPS, (uint32_t) (sms * max( 1, shape.blocks )) );
     if( grid )
         sw_stream_kernel<R, BLOCKS><<<grid, STREAM_THREADS, 0, st>>>( p );
     return cudaGetLastError();

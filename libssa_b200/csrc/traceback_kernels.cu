@@ -559,13 +559,12 @@ cudaError_t launch_tb_walk( const TbParams & p, int R, cudaStream_t st ) {
 
 template <int PHASE, int R, bool P8>
 static cudaError_t launch_stripes( const TbParams & p, int sms, cudaStream_t st ) {
-    int per_sm = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, tb_stripes_kernel<PHASE, R, P8>,
-            TB_THREADS, 0 );
+    static LaunchShape shape;
+    const cudaError_t e = shape.set( tb_stripes_kernel<PHASE, R, P8>, TB_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
     const uint32_t want = (p.n_tickets + TB_WARPS - 1) / TB_WARPS;
-    const uint32_t grid = min( want, (uint32_t) (sms * max( 1, per_sm )) );
+    const uint32_t grid = min( want, (uint32_t) (sms * max( 1, shape.blocks )) );
     if( grid )
         tb_stripes_kernel<PHASE, R, P8><<<grid, TB_THREADS, 0, st>>>( p );
     return cudaGetLastError();
