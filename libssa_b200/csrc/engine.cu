@@ -905,12 +905,16 @@ static FastShape choose_shape( uint32_t Q, double mean_len, int bucket ) {
 }
 
 // Steps above which an entry pass gives a pair to the streamed stripes: every
-// resident group's share of the pass, at least 256 (about 0.1 ms, below which
-// the extra launch costs what it saves).  SSA_B200_STREAM_SHARE pins it (tests).
+// resident group's share of the pass, at least 64.  Entry pass on a B200 with
+// the line at none / 256 / 64 steps: 4 queries of 200 x 500 proteins 1.51 / 0.62
+// / 0.27 ms, one of 1,000 x 3,000 1.11 / 0.71 / 0.56, one of 128 x 2,000 0.37 /
+// 0.25 / 0.24, 8 of 300 x 3,000 5.0 / 1.5 / 1.6; below the share the streamed
+// kernel loses to the entry kernel (32 x 20,000, share 7,350: 16.7 ms, at 800
+// 19.7).  SSA_B200_STREAM_SHARE pins the line (tests).
 static uint64_t stream_share( uint64_t share ) {
     if( const char * pin = getenv( "SSA_B200_STREAM_SHARE" ) )
         return strtoull( pin, nullptr, 10 );
-    return std::max<uint64_t>( share, 256 );
+    return std::max<uint64_t>( share, 64 );
 }
 
 void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
