@@ -84,6 +84,12 @@ __device__ __forceinline__ void append_task( PairTask * list, unsigned int * cou
         atomicOr( error_flags, ERR_REQUEUE_OVERFLOW );
 }
 
+// Whether a pass scores a pair: all of them, or those that the 8-bit entry
+// re-queued.
+__device__ __forceinline__ bool pair_wanted( const PassSink & s, bool marked_only, uint32_t slot, uint32_t id ) {
+    return !marked_only || s.score[(uint64_t) slot * s.score_stride + id] == SCORE_REQUEUED;
+}
+
 // A sequence whose running maximum reached the pass's limit in block
 // nblocks - 1: the 8-bit lane's overflow, or a pair for the lane emulation.
 __device__ __forceinline__ void report_crossing( const PassSink & s, uint32_t slot, uint32_t id, int32_t nblocks ) {
@@ -243,7 +249,7 @@ cudaError_t launch_build_profile8( const uint8_t * qcodes, const uint64_t * qoff
         const uint32_t * slots, uint32_t n, const uint32_t * rows_of, const int64_t * matrix, int8_t * prof,
         const uint64_t * prof_off, cudaStream_t st );
 
-// ---- chosen Smith-Waterman pairs on streamed stripes (sw_stream_kernel.cu) ---
+// ---- chosen pairs on streamed stripes (sw_stream_kernel.cu) ------------------
 struct SwStreamItem {
     uint32_t slot;                // query
     uint32_t id_a, id_b;          // two sequences (B = 0xffffffff when absent)
@@ -269,10 +275,14 @@ struct SwStreamParams {
                                   // the start); nullptr otherwise
     int4 * boundary;              // per item with several stripes: two words per block of four columns
     PassSink sink;                // score; next (8-bit entry) or redo
+    // Needleman-Wunsch
+    int gap_open;
+    bool marked_only;             // as in QPairParams
 };
 
-// R: query rows per lane (4 or 8)
+// R: query rows per lane (4 or 8; Needleman-Wunsch: 4)
 cudaError_t launch_sw_stream( int R, const SwStreamParams & p, int sms, cudaStream_t st );
+cudaError_t launch_nw_stream( const SwStreamParams & p, int sms, cudaStream_t st );
 
 // ---- query-pair Smith-Waterman entry pass (sw_qpair_kernel.cu) -------------
 // Two queries of similar length share each 32-bit register (low half query A,
@@ -301,7 +311,7 @@ struct QPairParams {
     int gap_oe;                   // gapO + gapE at the entry width
     int gap_e;
     int limit;                    // Smith-Waterman: as in FastParams
-    const uint32_t * qp_skip;     // per query pair: leading sequences that another kernel scores (nullptr: none)
+    const uint2 * qp_skip;        // per query pair: range [x, y) of the sequences that another kernel scores
     PassSink sink;
     int4 * scratch;               // per warp and group: scratch_cols column pairs (H, F of two columns)
     uint32_t scratch_cols;

@@ -562,8 +562,8 @@ private:
     void run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
             uint32_t cap, PairTask * redo_list, const std::vector<uint32_t> * slots = nullptr, uint32_t seq_lo = 0,
             uint32_t seq_hi = UINT32_MAX, bool marked = false );
-    void run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
-            cudaStream_t st );
+    void run_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
+            cudaStream_t st, bool marked = false );
     // The passes after the entry width: list A holds n_a pairs that it re-queued.
     // Leaves their scores, and the lists on the host (appended).
     void run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, uint32_t cap,
@@ -1027,7 +1027,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     // take more steps than every resident group's share of the pass
     uint32_t pair_skip = 0;
     std::vector<SwStreamItem> items;
-    if( nq == 1 && n_shaped == 1 && !getenv( "SSA_B200_NO_STREAM" ) ) {
+    if( nq == 1 && n_shaped == 1 && (!pin_g || getenv( "SSA_B200_STREAM_SHARE" )) ) {
         const uint64_t groups = (uint64_t) sms_ * 16 * (32u / (uint32_t) shape[0].G);
         const uint64_t P = (uint64_t) shape[0].P;
         const uint64_t share = stream_share( P * (total_cols / 4u) / groups );
@@ -1049,7 +1049,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
             lists.redo_cap = cap;
         }
         CUDA_CHECK( cudaStreamWaitEvent( long_stream_, ev_ready_, 0 ) );
-        run_sw_stream( req, items, lists, long_stream_ );
+        run_stream( req, items, lists, long_stream_ );
         CUDA_CHECK( cudaEventRecord( ev_long_, long_stream_ ) );
         CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_long_, 0 ) );
     }
@@ -1302,13 +1302,17 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     // changes a value by at most m, and a path has at most rows + L + 4 steps
     // and two gap openings
     std::vector<uint32_t> qp_lmax( std::max<uint32_t>( 1, n_qp ), 0 );
+    int64_t nw_step = std::max<int64_t>( 1, std::llabs( (int64_t) req.gap_extend ) );
+    const int64_t nw_budget = 30000 - 2 * std::llabs( (int64_t) req.gap_open );
+    bool nw_table8 = true;       // the scores at the pass width fit int8
     if( nw ) {
-        int64_t m = std::max<int64_t>( 1, std::llabs( (int64_t) req.gap_extend ) );
-        for( int c = 0; c < 1024; c++ )
-            m = std::max<int64_t>( m, std::llabs( (int64_t) (int16_t) req.matrix[c] ) );
-        const int64_t budget = 30000 - 2 * std::llabs( (int64_t) req.gap_open );
+        for( int c = 0; c < 1024; c++ ) {
+            const int64_t v = (int16_t) req.matrix[c];
+            nw_step = std::max<int64_t>( nw_step, std::llabs( v ) );
+            nw_table8 = nw_table8 && v == (int8_t) v;
+        }
         for( uint32_t i = 0; i < n_qp; i++ ) {
-            const int64_t l = budget / m - (int64_t) qp_rows[i] - 4;
+            const int64_t l = nw_budget / nw_step - (int64_t) qp_rows[i] - 4;
             qp_lmax[i] = (uint32_t) std::max<int64_t>( 0, l );
         }
     }
@@ -1380,45 +1384,69 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     // ms, half of it because both sequences of a pair overflow early and end
     // it.  Where no pair takes half as long again as the
     // share, the entry kernel keeps them all (it needs fewer instructions per
-    // cell: four chains of 20-28 rows against 4 or 8).
-    const uint32_t * dev_skip = nullptr;
-    std::vector<uint32_t> qp_skip( std::max<uint32_t>( 1, n_qp ), 0 );
+    // cell: four chains of 20-28 rows against 4 or 8).  A Needleman-Wunsch query
+    // without a partner goes there whole in calls of less than 2,048 steps per
+    // group: the entry kernel computes an empty half for it, and its longest
+    // pairs take most of such a call (one of 250 x 20,000 proteins, 280 steps,
+    // 1.97 -> 1.00 ms; 500 x 50,000 reads, 2,640 steps, 6.8 and 6.6; 300 x
+    // 200,000, 2,800 steps, 9.3 and 14.2).  Batches: 4 of 200 x 500 1.31 -> 0.31
+    // ms, 8 of 300 x 3,000 7.3 -> 5.0, 64 reads x 20,000 unchanged.
+    constexpr uint64_t NW_STREAM_SHARE = 2048;
+    const bool table8 = nw ? nw_table8 : fast_single_eligible( req );
+    const bool pinned = pin || pin_mb || pin_c || pin_h || pin_g8;      // a pinned shape keeps the entry kernel
+    std::vector<uint2> qp_skip( std::max<uint32_t>( 1, n_qp ), make_uint2( 0, 0 ) );
     std::vector<SwStreamItem> items;
-    if( !nw && fast_single_eligible( req ) && !getenv( "SSA_B200_NO_STREAM" ) ) {
+    if( table8 && (!pinned || getenv( "SSA_B200_STREAM_SHARE" )) ) {
         auto passes_of = [&]( uint32_t i, int R ) { return (uint64_t) qp_rows[i] / (uint64_t) (QP_G * R); };
-        auto blocks_of = [&]( uint32_t i ) { return (uint64_t) (db_.len[db_.order_desc[lo + i]] + 3u) / 4u; };
+        auto len_of = [&]( uint32_t i ) { return db_.len[db_.order_desc[lo + i]]; };
+        // the first sequence from k on that satisfies `past` (monotonic: the lengths descend)
+        auto first = [&]( uint32_t k, auto past ) {
+            uint32_t a = k, b = n_seq;
+            while( a < b ) {
+                const uint32_t mid = (a + b) / 2;
+                if( past( mid ) )
+                    b = mid;
+                else
+                    a = mid + 1;
+            }
+            return a;
+        };
         uint64_t steps = 0, longest = 0;
         for( int ri = 0; ri < 4; ri++ )
             for( uint32_t i : by_r[ri] ) {
                 steps += passes_of( i, 4 * (ri + 4) ) * (total_cols / 4u);
-                longest = std::max( longest, passes_of( i, 4 * (ri + 4) ) * blocks_of( 0 ) );
+                longest = std::max<uint64_t>( longest, passes_of( i, 4 * (ri + 4) ) * ((len_of( 0 ) + 3u) / 4u) );
             }
         const uint64_t share = stream_share( steps / ((uint64_t) sms_ * 16 * QP_GPW) );
-        if( 2 * longest > 3 * share )
-            for( int ri = 0; ri < 4; ri++ )
-                for( uint32_t i : by_r[ri] ) {
-                    const uint64_t P = passes_of( i, 4 * (ri + 4) );
-                    uint32_t a = 0, b = n_seq;          // sequences of more than share / P blocks come first
-                    while( a < b ) {
-                        const uint32_t mid = (a + b) / 2;
-                        if( P * blocks_of( mid ) > share )
-                            a = mid + 1;
-                        else
-                            b = mid;
-                    }
-                    qp_skip[i] = std::min( n_seq, (a + 1u) & ~1u );
-                    for( int h = 0; h < 2; h++ ) {
-                        const uint32_t slot = qp_slots[2 * i + h];
-                        for( uint32_t k = 0; k < qp_skip[i] && slot != 0xffffffffu; k += 2 )
-                            items.push_back( SwStreamItem{ slot, db_.order_desc[lo + k],
-                                    k + 1 < qp_skip[i] ? db_.order_desc[lo + k + 1] : 0xffffffffu, 0 } );
-                    }
+        for( int ri = 0; ri < 4; ri++ )
+            for( uint32_t i : by_r[ri] ) {
+                const uint64_t P = passes_of( i, 4 * (ri + 4) );
+                const bool single = qp_slots[2 * i + 1] == 0xffffffffu;
+                const uint32_t Q = h_qlen_[qp_slots[2 * i]];
+                // Needleman-Wunsch: within the exact range for stripes of 128
+                // rows (the entry kernel sends the longer ones to the redo list)
+                const int64_t most = nw ? nw_budget / nw_step - (int64_t) ((Q + 127u) & ~127u) - 4 : INT64_MAX;
+                const uint32_t from = first( 0, [&]( uint32_t k ) { return (int64_t) len_of( k ) <= most; } );
+                uint32_t to = from;
+                if( nw && single && share < NW_STREAM_SHARE )
+                    to = n_seq;
+                else if( 2 * longest > 3 * share )
+                    to = first( from, [&]( uint32_t k ) { return P * ((len_of( k ) + 3u) / 4u) <= share; } );
+                if( to < n_seq && ((to - from) & 1u) )
+                    to++;
+                qp_skip[i] = make_uint2( from, to );
+                for( int h = 0; h < 2; h++ ) {
+                    const uint32_t slot = qp_slots[2 * i + h];
+                    for( uint32_t k = from; k < to && slot != 0xffffffffu; k += 2 )
+                        items.push_back( SwStreamItem{ slot, db_.order_desc[lo + k],
+                                k + 1 < to ? db_.order_desc[lo + k + 1] : 0xffffffffu, 0 } );
                 }
+            }
     }
+    const uint2 * dev_skip = stage_.add( qp_skip.data(), qp_skip.size(), stream_ );
+    stage_.send( stream_ );
+    CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     if( !items.empty() ) {
-        dev_skip = stage_.add( qp_skip.data(), qp_skip.size(), stream_ );
-        stage_.send( stream_ );
-        CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
         PassSink lists{};
         lists.next = next;
         lists.next_count = next_count;
@@ -1429,12 +1457,13 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
             lists.redo_cap = cap;
         }
         CUDA_CHECK( cudaStreamWaitEvent( long_stream_, ev_ready_, 0 ) );
-        run_sw_stream( req, items, lists, long_stream_ );
+        run_stream( req, items, lists, long_stream_, marked );
         CUDA_CHECK( cudaEventRecord( ev_long_, long_stream_ ) );
         CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_long_, 0 ) );
     }
     // classes launched heaviest first (most rows per thread: the longest
     // queries), so that the last class to finish is the lightest
+    bool launched[4] = { false, false, false, false };
     size_t class_start[4] = { 0, 0, 0, 0 };
     for( int ri = 1; ri < 4; ri++ )
         class_start[ri] = class_start[ri - 1] + by_r[ri - 1].size();
@@ -1442,8 +1471,12 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         const int ri = 3 - k;
         const size_t class_first = class_start[ri];
         const std::vector<uint32_t> & cls = by_r[ri];
-        if( cls.empty() )
+        bool work = false;       // sequences that the streamed stripes leave
+        for( uint32_t i : cls )
+            work = work || qp_skip[i].y - qp_skip[i].x < n_seq;
+        if( !work )
             continue;
+        launched[ri] = true;
         const int R = 4 * (ri + 4);
         // Needleman-Wunsch: 4 columns per step unless SSA_B200_QP_C=2 pins the
         // 2-column kernel (4 resident CTAs per SM either way)
@@ -1519,7 +1552,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     }
     if( timing ) {
         for( int ri = 0; ri < 4; ri++ ) {
-            if( by_r[ri].empty() )
+            if( !launched[ri] )
                 continue;
             float ms = 0;
             CUDA_CHECK( cudaEventSynchronize( ev_cls_t_[2 * ri + 1] ) );
@@ -1544,11 +1577,12 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     }
 }
 
-// Smith-Waterman scores of `items` at the request's width (two sequences of a
+// Scores of `items` at the request's width (two sequences of a
 // query per register, sw_stream_kernel.cu) on stream st; lists: where the pairs
 // that the kernel does not report go.
-void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
-        cudaStream_t st ) {
+void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & items, const PassSink & lists,
+        cudaStream_t st, bool marked ) {
+    const bool nw = req.algo == 1;
     // queries with the most rows first: their items have the most stripes
     std::stable_sort( items.begin(), items.end(), [&]( const SwStreamItem & x, const SwStreamItem & y ) {
         return h_qlen_[x.slot] > h_qlen_[y.slot];
@@ -1557,10 +1591,10 @@ void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem>
     for( const SwStreamItem & t : items )
         stripes128 += (h_qlen_[t.slot] + 127u) / 128u;
     // rows per lane: 4 while every stripe of 128 rows can be resident (24 warps per SM)
-    const int R = stripes128 <= (uint64_t) sms_ * 24 ? 4 : 8;
+    const int R = nw || stripes128 <= (uint64_t) sms_ * 24 ? 4 : 8;
     const uint32_t rows = 32u * (uint32_t) R;
     const uint32_t ni = (uint32_t) items.size();
-    const bool blocks = req.bit_width == 8;
+    const bool blocks = req.bit_width == 8;       // Smith-Waterman 8-bit entry
     // launches of as many items as 1 GB of boundary rows holds
     for( uint32_t i0 = 0; i0 < ni; ) {
         std::vector<uint64_t> bnd;
@@ -1600,7 +1634,9 @@ void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem>
         p.matrix = d_matrix_.as<int64_t>();
         p.gap_oe = blocks ? (int8_t) (req.gap_open + req.gap_extend) : req.gap_open + req.gap_extend;
         p.gap_e = req.gap_extend;
-        p.limit = sw_fast_limit( req );
+        p.limit = nw ? 0 : sw_fast_limit( req );
+        p.gap_open = req.gap_open;
+        p.marked_only = marked;
         p.items = dev_items;
         p.bnd_off = dev_bnd;
         p.cum = dev_cum;
@@ -1618,7 +1654,7 @@ void Engine::run_sw_stream( const SearchRequest & req, std::vector<SwStreamItem>
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
         p.sink.error_flags = d_counts_.as<unsigned>() + 2;
-        CUDA_CHECK( launch_sw_stream( R, p, sms_, st ) );
+        CUDA_CHECK( nw ? launch_nw_stream( p, sms_, st ) : launch_sw_stream( R, p, sms_, st ) );
         launches_++;
         i0 = i1;
     }
@@ -1666,7 +1702,7 @@ void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, 
         lists.redo = redo;
         lists.redo_count = cnt + 5;
         lists.redo_cap = n_a;
-        run_sw_stream( r16, items, lists, stream_ );
+        run_stream( r16, items, lists, stream_ );
         run_redo( r16, nq, list_b, cnt + 1, cap, redo );
     }
     else if( nw_fast_eligible( r16 ) && queries_fit && n_a >= searched / 4 ) {

@@ -74,16 +74,18 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
             break;
         const uint32_t qp = p.unit_pairs[u / p.n_chunks];
         const uint32_t chunk = (uint32_t) (u % p.n_chunks);
-        const uint32_t seq_begin = max( p.chunk_bounds[chunk], p.qp_skip ? p.qp_skip[qp] : 0u );
-        const uint32_t seq_end = p.chunk_bounds[chunk + 1];
+        const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
+        const uint2 skip = p.qp_skip[qp];
         const uint32_t rows = p.qp_rows[qp];
         const uint32_t passes = rows / GR;
         const uint32_t * prof = p.prof + p.prof_off[qp];
         const uint32_t slot_a = p.qp_slots[2 * qp], slot_b = p.qp_slots[2 * qp + 1];
 
         for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) QP_GPW ) {
+            if( b0 >= skip.x && b0 + (uint32_t) QP_GPW <= skip.y )
+                continue;
             const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end;
+            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const uint32_t ncp = ((L + 3u) & ~3u) >> 1;          // column pairs up to the block end
@@ -327,16 +329,18 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
             break;
         const uint32_t qp = p.unit_pairs[u / p.n_chunks];
         const uint32_t chunk = (uint32_t) (u % p.n_chunks);
-        const uint32_t seq_begin = max( p.chunk_bounds[chunk], p.qp_skip ? p.qp_skip[qp] : 0u );
-        const uint32_t seq_end = p.chunk_bounds[chunk + 1];
+        const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
+        const uint2 skip = p.qp_skip[qp];
         const uint32_t rows = p.qp_rows[qp];
         const uint32_t passes = rows / GR;
         const uint32_t * prof = p.prof + p.prof_off[qp];
         const uint32_t slot_a = p.qp_slots[2 * qp], slot_b = p.qp_slots[2 * qp + 1];
 
         for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) GPW ) {
+            if( b0 >= skip.x && b0 + (uint32_t) GPW <= skip.y )
+                continue;
             const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end;
+            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const uint32_t nb = (L + 3u) >> 2;                    // 4-column blocks
@@ -645,12 +649,6 @@ __device__ __forceinline__ uint32_t nw_pack( int32_t v ) {
     return u | (u << 16);
 }
 
-// Whether the pass scores a pair: all of them, or those that the 8-bit entry
-// re-queued.
-__device__ __forceinline__ bool nw_wanted( const QPairParams & p, uint32_t slot, uint32_t id ) {
-    return !p.marked_only || p.sink.score[(uint64_t) slot * p.sink.score_stride + id] == SCORE_REQUEUED;
-}
-
 // one step's rows: column c (cell A, row r) interleaved with column c + 1
 // (cell B, row r - 1); CAPTURE records H at the queries' last rows when one
 // of the two columns is the sequence's last
@@ -736,6 +734,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
         const uint32_t qp = p.unit_pairs[u / p.n_chunks];
         const uint32_t chunk = (uint32_t) (u % p.n_chunks);
         const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
+        const uint2 skip = p.qp_skip[qp];
         const uint32_t rows = p.qp_rows[qp];
         const uint32_t passes = rows / GR;
         const uint32_t * prof = p.prof + p.prof_off[qp];
@@ -745,8 +744,10 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
         const uint32_t lmax = p.qp_lmax[qp];
 
         for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) QP_GPW ) {
+            if( b0 >= skip.x && b0 + (uint32_t) QP_GPW <= skip.y )
+                continue;
             const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end;
+            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const bool exact = valid && L <= lmax;
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
                 // beyond the guarded range: the lane emulation scores it
                 const uint32_t slots[2] = { slot_a, slot_b };
                 for( int h = 0; h < 2; h++ ) {
-                    if( slots[h] == 0xffffffffu || !nw_wanted( p, slots[h], id ) )
+                    if( slots[h] == 0xffffffffu || !pair_wanted( p.sink, p.marked_only, slots[h], id ) )
                         continue;
                     append_task( p.sink.redo, p.sink.redo_count, p.sink.redo_cap, slots[h], id, 0,
                             p.sink.error_flags );
@@ -876,10 +877,10 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
                 cap_b = max( cap_b, __shfl_xor_sync( 0xffffffffu, cap_b, o, G ) );
             }
             if( exact && k == 0 ) {
-                if( nw_wanted( p, slot_a, id ) )
+                if( pair_wanted( p.sink, p.marked_only, slot_a, id ) )
                     p.sink.score[(uint64_t) slot_a * p.sink.score_stride + id] =
                             (int32_t) (cap_a & 0xffffu) - (int32_t) NWQ_BIAS;
-                if( slot_b != 0xffffffffu && nw_wanted( p, slot_b, id ) )
+                if( slot_b != 0xffffffffu && pair_wanted( p.sink, p.marked_only, slot_b, id ) )
                     p.sink.score[(uint64_t) slot_b * p.sink.score_stride + id] =
                             (int32_t) (cap_b >> 16) - (int32_t) NWQ_BIAS;
             }
@@ -1046,6 +1047,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
         const uint32_t qp = p.unit_pairs[u / p.n_chunks];
         const uint32_t chunk = (uint32_t) (u % p.n_chunks);
         const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
+        const uint2 skip = p.qp_skip[qp];
         const uint32_t rows = p.qp_rows[qp];
         const uint32_t passes = rows / GR;
         const uint32_t * prof = p.prof + p.prof_off[qp];
@@ -1055,8 +1057,10 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
         const uint32_t lmax = p.qp_lmax[qp];
 
         for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) QP_GPW ) {
+            if( b0 >= skip.x && b0 + (uint32_t) QP_GPW <= skip.y )
+                continue;
             const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end;
+            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const bool exact = valid && L <= lmax;
@@ -1064,7 +1068,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                 // beyond the guarded range: the lane emulation scores it
                 const uint32_t slots[2] = { slot_a, slot_b };
                 for( int h = 0; h < 2; h++ ) {
-                    if( slots[h] == 0xffffffffu || !nw_wanted( p, slots[h], id ) )
+                    if( slots[h] == 0xffffffffu || !pair_wanted( p.sink, p.marked_only, slots[h], id ) )
                         continue;
                     append_task( p.sink.redo, p.sink.redo_count, p.sink.redo_cap, slots[h], id, 0,
                             p.sink.error_flags );
@@ -1222,10 +1226,10 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                 cap_b = max( cap_b, __shfl_xor_sync( 0xffffffffu, cap_b, o, G ) );
             }
             if( exact && k == 0 ) {
-                if( nw_wanted( p, slot_a, id ) )
+                if( pair_wanted( p.sink, p.marked_only, slot_a, id ) )
                     p.sink.score[(uint64_t) slot_a * p.sink.score_stride + id] =
                             (int32_t) (cap_a & 0xffffu) - (int32_t) NWQ_BIAS;
-                if( slot_b != 0xffffffffu && nw_wanted( p, slot_b, id ) )
+                if( slot_b != 0xffffffffu && pair_wanted( p.sink, p.marked_only, slot_b, id ) )
                     p.sink.score[(uint64_t) slot_b * p.sink.score_stride + id] =
                             (int32_t) (cap_b >> 16) - (int32_t) NWQ_BIAS;
             }

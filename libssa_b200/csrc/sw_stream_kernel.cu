@@ -1,5 +1,5 @@
-// sw_stream_kernel.cu -- Smith-Waterman scores of chosen (query, sequence)
-// pairs, two sequences of one query per register, on streamed stripes.
+// sw_stream_kernel.cu -- scores of chosen (query, sequence) pairs, two sequences
+// of one query per register, on streamed stripes.
 //
 // For the pairs that would outlast everything else in a call.  The kernels of
 // the entry pass give a sequence to 4 to 32 threads, which pass over it once
@@ -54,7 +54,16 @@ struct CrossLimit {
     }
 };
 
-template <int R, bool BLOCKS>
+// NW: Needleman-Wunsch as in nw_qpair4_kernel (exact unsigned 16x2 values with a
+// bias of 32768, for sequences up to the host's length limit; the score is H of
+// the query's last row in the sequence's last column).
+constexpr uint32_t STREAM_NW_BIAS = 32768u;
+
+__device__ __forceinline__ uint32_t stream_nw_pack( int32_t v ) {
+    return ((uint32_t) (v + (int32_t) STREAM_NW_BIAS) & 0xffffu) * 0x10001u;
+}
+
+template <int R, bool BLOCKS, bool NW>
 __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_kernel( SwStreamParams p ) {
     constexpr int C = 4;
     constexpr int WORDS = R / 4;
@@ -72,8 +81,10 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
     const uint32_t GOE32 = (uint32_t) (p.gap_oe * 65536 + p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
     // sets bit 15 of a half exactly when the half is >= STREAM_BIAS + limit
+    const int gO = p.gap_open, gE = p.gap_e;
     const uint32_t CROSS_ADD = (0x8000u - (STREAM_BIAS + (uint32_t) p.limit)) * 0x10001u;
 
+    uint64_t loaded_key = ~0ull;
     for( ;; ) {
         const uint32_t ticket = next_hit( p.counter, lane );
         if( ticket >= p.n_tickets )
@@ -98,10 +109,14 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
         sp.last = (stripe + 1u) * (uint32_t) ROWS >= Q;
         sp.error_flags = p.sink.error_flags;
 
-        // the lane's rows: int8 scores of every code, -128 past the query and
-        // for the pad code
+        // the lane's rows: int8 scores of every code; past the query and for the
+        // pad code -128 (never raises a maximum), or 0 (Needleman-Wunsch: never
+        // reaches the score, and keeps every value in range)
+        constexpr int PAST = NW ? 0 : -128;
         const int32_t row0 = (int32_t) (stripe * (uint32_t) ROWS) + lane * R;
-        {
+        const uint64_t key = ((uint64_t) item.slot << 32) | stripe;
+        if( key != loaded_key ) {                   // the same for the next ticket of this stripe of the query
+            loaded_key = key;
             int code[R];
 #pragma unroll
             for( int r = 0; r < R; r++ )
@@ -113,7 +128,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
 #pragma unroll
                     for( int b = 0; b < 4; b++ ) {
                         const int c = code[4 * w + b];
-                        const int m = (c >= 0 && d != (int) FAST_PAD_CODE) ? smat[(d << 5) + c] : -128;
+                        const int m = (c >= 0 && d != (int) FAST_PAD_CODE) ? smat[(d << 5) + c] : PAST;
                         v |= ((uint32_t) m & 0xffu) << (8 * b);
                     }
                     table[d * 32 * WORDS + w] = v;
@@ -123,10 +138,17 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
         uint32_t H[R], E[R];
 #pragma unroll
         for( int r = 0; r < R; r++ ) {
-            H[r] = STREAM_BIAS2;
-            E[r] = STREAM_BIAS2;
+            // the reference's column before the first: H(i, -1), E(i, -1)
+            H[r] = NW ? stream_nw_pack( gO + (row0 + r + 1) * gE ) : STREAM_BIAS2;
+            E[r] = NW ? stream_nw_pack( 2 * gO + (row0 + r + 2) * gE ) : STREAM_BIAS2;
         }
-        uint32_t diag = STREAM_BIAS2, smax = STREAM_BIAS2, seen = 0;
+        uint32_t diag = NW ? stream_nw_pack( row0 ? gO + row0 * gE : 0 ) : STREAM_BIAS2, smax = STREAM_BIAS2, seen = 0;
+        // Needleman-Wunsch: the lane of the query's last row, where it is in the
+        // lane, and the last column of each sequence
+        const int q_last = (int) Q - 1 - row0;
+        const bool owner = NW && sp.last && q_last >= 0 && q_last < R;
+        const int32_t la = (int32_t) p.db.lens[item.id_a] - 1, lb = two ? (int32_t) p.db.lens[item.id_b] - 1 : -1;
+        uint32_t cap_a = 0, cap_b = 0;
         int32_t * cross = BLOCKS ? p.cross + 2 * it : nullptr;
         uint32_t out_h[C], out_f[C];
 #pragma unroll
@@ -160,8 +182,9 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
                 if( stripe == 0 ) {
 #pragma unroll
                     for( int j = 0; j < C; j++ ) {
-                        up_h[j] = STREAM_BIAS2;
-                        up_f[j] = STREAM_BIAS2;
+                        // H(-1, c) and F entering row 0
+                        up_h[j] = NW ? stream_nw_pack( gO + (4 * b + j + 1) * gE ) : STREAM_BIAS2;
+                        up_f[j] = NW ? stream_nw_pack( 2 * gO + (4 * b + j + 2) * gE ) : STREAM_BIAS2;
                     }
                 }
                 else {
@@ -202,13 +225,22 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
                     const uint32_t v = (r & 3) == 0 ? pair_score<0>( x, y ) : (r & 3) == 1 ? pair_score<1>( x, y )
                             : (r & 3) == 2 ? pair_score<2>( x, y ) : pair_score<3>( x, y );
                     const uint32_t hd = r == 0 ? (j == 0 ? diag : up_h[j - 1]) : (j == 0 ? H[r - 1] : hv[j - 1][r - 1]);
-                    const uint32_t t = __vimax3_s16x2( E[r], f[j], STREAM_BIAS2 );
-                    const uint32_t h = __viaddmax_s16x2( hd, v, t );
-                    const uint32_t hg = h + GOE32;                      // no borrow: h >= bias
-                    f[j] = __viaddmax_s16x2( f[j], GE2, hg );
-                    E[r] = __viaddmax_s16x2( E[r], GE2, hg );
+                    uint32_t h;
+                    if constexpr( NW ) {
+                        h = __viaddmax_u16x2( hd, v, __vmaxu2( E[r], f[j] ) );
+                        const uint32_t hg = h + GOE32;                  // one carry out of the low half
+                        f[j] = __viaddmax_u16x2( f[j], GE2, hg );
+                        E[r] = __viaddmax_u16x2( E[r], GE2, hg );
+                    }
+                    else {
+                        const uint32_t t = __vimax3_s16x2( E[r], f[j], STREAM_BIAS2 );
+                        h = __viaddmax_s16x2( hd, v, t );
+                        const uint32_t hg = h + GOE32;                  // no borrow: h >= bias
+                        f[j] = __viaddmax_s16x2( f[j], GE2, hg );
+                        E[r] = __viaddmax_s16x2( E[r], GE2, hg );
+                    }
                     hv[j][r] = h;
-                    if( j & 1 )
+                    if( !NW && (j & 1) )
                         smax = __vimax3_s16x2( smax, hv[j - 1][r], h );
                     if( j == C - 1 )
                         H[r] = h;
@@ -219,6 +251,19 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
             for( int j = 0; j < C; j++ ) {
                 out_h[j] = hv[j][R - 1];
                 out_f[j] = f[j];
+            }
+            if constexpr( NW ) {
+                if( owner && (b == la >> 2 || b == lb >> 2) ) {
+#pragma unroll
+                    for( int j = 0; j < C; j++ )
+#pragma unroll
+                        for( int r = 0; r < R; r++ ) {
+                            if( r == q_last && 4 * b + j == la )
+                                cap_a = hv[j][r];
+                            if( r == q_last && 4 * b + j == lb )
+                                cap_b = hv[j][r];
+                        }
+                }
             }
             if constexpr( BLOCKS ) {
                 // first block in which this lane's maximum reached the limit
@@ -239,6 +284,17 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
         };
         const CrossLimit<BLOCKS> limit{ cross, two };
         const uint32_t swept = stream_columns<16>( sp, st, lane, limit, []( uint32_t ) {}, column );
+        if constexpr( NW ) {
+            if( owner ) {
+                const uint64_t row = (uint64_t) item.slot * p.sink.score_stride;
+                if( pair_wanted( p.sink, p.marked_only, item.slot, item.id_a ) )
+                    p.sink.score[row + item.id_a] = (int32_t) (cap_a & 0xffffu) - (int32_t) STREAM_NW_BIAS;
+                if( two && pair_wanted( p.sink, p.marked_only, item.slot, item.id_b ) )
+                    p.sink.score[row + item.id_b] = (int32_t) (cap_b >> 16) - (int32_t) STREAM_NW_BIAS;
+            }
+            stream_end( sp, swept, lane );
+            continue;
+        }
         // the pair's maximum goes down the stripes; a half that reached the
         // limit anywhere holds a value at or above it
 #pragma unroll
@@ -273,22 +329,26 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
     }
 }
 
-template <int R, bool BLOCKS>
+template <int R, bool BLOCKS, bool NW>
 static cudaError_t launch_stream( const SwStreamParams & p, int sms, cudaStream_t st ) {
     static LaunchShape shape;
-    const cudaError_t e = shape.set( sw_stream_kernel<R, BLOCKS>, STREAM_THREADS, 0 );
+    const cudaError_t e = shape.set( sw_stream_kernel<R, BLOCKS, NW>, STREAM_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
     const uint32_t grid = min( (p.n_tickets + STREAM_WARPS - 1) / STREAM_WARPS, (uint32_t) (sms * max( 1, shape.blocks )) );
     if( grid )
-        sw_stream_kernel<R, BLOCKS><<<grid, STREAM_THREADS, 0, st>>>( p );
+        sw_stream_kernel<R, BLOCKS, NW><<<grid, STREAM_THREADS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
 cudaError_t launch_sw_stream( int R, const SwStreamParams & p, int sms, cudaStream_t st ) {
     if( p.cross )
-        return R == 4 ? launch_stream<4, true>( p, sms, st ) : launch_stream<8, true>( p, sms, st );
-    return R == 4 ? launch_stream<4, false>( p, sms, st ) : launch_stream<8, false>( p, sms, st );
+        return R == 4 ? launch_stream<4, true, false>( p, sms, st ) : launch_stream<8, true, false>( p, sms, st );
+    return R == 4 ? launch_stream<4, false, false>( p, sms, st ) : launch_stream<8, false, false>( p, sms, st );
+}
+
+cudaError_t launch_nw_stream( const SwStreamParams & p, int sms, cudaStream_t st ) {
+    return launch_stream<4, false, true>( p, sms, st );
 }
 
 }  // namespace ssa

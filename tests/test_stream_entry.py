@@ -30,3 +30,21 @@ def test_longest_pairs(built_library, monkeypatch, width, share):
     records += [np.tile(queries[3], 12), np.zeros(0, np.uint8)]
     _check(dict(algo="sw", width=width, align=1, hits=16, gap=(-11, -1), chunk=25, simd=2,
                 records=[r.tobytes() for r in records], queries=[q.tobytes() for q in queries]))
+
+
+@pytest.mark.parametrize("share", [None, 0, 40])
+@pytest.mark.parametrize("width", [8, 16, 64])
+def test_needleman_wunsch_pairs(built_library, monkeypatch, width, share):
+    """Needleman-Wunsch on the streamed stripes: a query without a partner
+    whole, batches from "all" to "the longest"; records around the blocks, one
+    register half ending long before the other, and records past the exact
+    16-bit range, which go to the lane emulation."""
+    if share is not None:
+        monkeypatch.setenv("SSA_B200_STREAM_SHARE", str(share))
+    rng = np.random.default_rng(41 + width)
+    queries = [W.random_residues(rng, n, W.AA20) for n in (1, 30, 127, 128, 129, 300)]
+    records = [W.random_residues(rng, int(n), W.AA20) for n in rng.integers(1, 600, 50)]
+    records += [W.random_residues(rng, n, W.AA20) for n in (1, 2, 3, 4, 5, 61, 62, 63, 64, 65, 66, 1500, 2600, 9000)]
+    records += [W.mutate(rng, q, W.AA20, 0.1, 0.03, (1, 5)) for q in queries for _ in range(3)]
+    _check(dict(algo="nw", width=width, align=1, hits=14, gap=(-11, -1), chunk=25, simd=2,
+                records=[r.tobytes() for r in records], queries=[q.tobytes() for q in queries]))
