@@ -295,7 +295,7 @@ constexpr int QP_THREADS_PER_CTA = 128;
 struct QPairParams {
     DbView db;
     const uint32_t * order;       // non-empty IDs, longest first
-    const uint32_t * prof;        // per query pair: QP_CODES x rows words (16x2: A low, B high)
+    const uint32_t * prof;        // per query pair: profile words (16x2: A low, B high), launch_build_profile_qp
     const uint64_t * prof_off;    // per query pair, in words
     const uint32_t * qp_slots;    // per query pair: slot A, slot B (0xffffffff when absent)
     const uint32_t * qp_rows;     // per query pair: profile rows (passes x QP_G x R)
@@ -334,10 +334,11 @@ cudaError_t launch_nw_qpair( int R, const QPairParams & p, int grid, cudaStream_
 // the same pass with one 4-column block per step (four dependency chains per thread)
 cudaError_t launch_nw_qpair4( int R, const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm );
 // width 8: (int8) scores, -128 past a query (Smith-Waterman 8-bit entry);
-// width 16: (int16) scores, 0 past a query (Needleman-Wunsch 16-bit entry)
+// width 16: (int16) scores, 0 past a query; lane_rows: per query pair the layout,
+// 0 or the rows per lane of the 4-column kernels
 cudaError_t launch_build_profile_qp( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
-        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const int64_t * matrix, uint32_t * prof,
-        const uint64_t * prof_off, int width, cudaStream_t st );
+        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const uint32_t * lane_rows,
+        const int64_t * matrix, uint32_t * prof, const uint64_t * prof_off, int width, cudaStream_t st );
 
 // ---- long pairs (pair_kernel.cu) ---------------------------------------------
 // A group of PAIR_W warps scores one (query, database sequence) pair exactly in

@@ -1316,11 +1316,20 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
             qp_lmax[i] = (uint32_t) std::max<int64_t>( 0, l );
         }
     }
-    // profiles: QP_CODES x rows words per pair (16-byte aligned: rows % 16 == 0)
+    // Needleman-Wunsch: 4 columns per step unless SSA_B200_QP_C=2 pins the
+    // 2-column kernel (4 resident CTAs per SM either way)
+    QpVariant variant[4];
+    for( int ri = 0; ri < 4; ri++ )
+        variant[ri] = nw ? QpVariant{ 4, pinned_c == 2 ? 2 : 4, false, false, 0 }
+                         : qpair_variant( bucket, 4 * (ri + 4), pinned_mb, pinned_c, pinned_h, pinned_g8 );
+    // profiles (16-byte aligned: rows % 16 == 0): QP_CODES x rows words per
+    // pair, twice that in the layout of the 4-column kernels with 4 threads
+    std::vector<uint32_t> lane_rows( std::max<uint32_t>( 1, n_qp ), 0 );
     for( int ri = 0; ri < 4; ri++ )
         for( uint32_t i : by_r[ri] ) {
             qp_off[i] = total;
-            total += (uint64_t) QP_CODES * qp_rows[i];
+            lane_rows[i] = variant[ri].cols == 2 ? 0 : variant[ri].g8 ? 12 : 4 * (ri + 4);
+            total += (uint64_t) QP_CODES * qp_rows[i] * (lane_rows[i] && !variant[ri].g8 ? 2 : 1);
         }
     std::vector<uint32_t> units;                  // pairs grouped by class, longest first
     for( auto & v : by_r ) {
@@ -1330,6 +1339,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     d_qp_prof_.ensure( std::max<uint64_t>( total, 4 ) * sizeof(uint32_t) );
     const uint64_t * dev_off = stage_.add( qp_off.data(), qp_off.size(), stream_ );
     const uint32_t * dev_rows = stage_.add( qp_rows.data(), qp_rows.size(), stream_ );
+    const uint32_t * dev_lane_rows = stage_.add( lane_rows.data(), lane_rows.size(), stream_ );
     const uint32_t * dev_qslots = stage_.add( qp_slots.data(), qp_slots.size(), stream_ );
     const uint32_t * dev_units = stage_.add( units.data(), units.size(), stream_ );
     const uint32_t * dev_lmax = stage_.add( qp_lmax.data(), qp_lmax.size(), stream_ );
@@ -1338,12 +1348,14 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
     if( redo )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
-    // work units: ranges of length-sorted sequences (multiples of QP_GPW)
-    // holding about equal numbers of columns, the longest first; every pair of
-    // a class gets every range.  A warp takes one unit at a time.
+    // work units: ranges of length-sorted sequences (multiples of what a CTA
+    // holds side by side) with about equal numbers of columns, the longest
+    // first; every pair of a class gets every range.  A CTA takes one unit at a
+    // time (a warp, in the 2-column kernels).
     uint64_t total_cols = 0;
     for( uint32_t i = lo; i < hi; i++ )
         total_cols += (db_.len[db_.order_desc[i]] + 3u) & ~3u;
+    constexpr uint32_t CTA_SEQS = QP_THREADS_PER_CTA / QP_G;
     const uint64_t want_units = (uint64_t) sms_ * 16 * 24;
     const uint64_t target = std::max<uint64_t>( 1, total_cols * std::max<uint32_t>( 1, n_qp ) / want_units );
     std::vector<uint32_t> bounds{ 0 };
@@ -1351,7 +1363,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         uint64_t acc = 0;
         for( uint32_t i = 0; i < n_seq; i++ ) {
             acc += (db_.len[db_.order_desc[lo + i]] + 3u) & ~3u;
-            if( acc >= target && (i + 1) % QP_GPW == 0 ) {
+            if( acc >= target && (i + 1) % CTA_SEQS == 0 ) {
                 bounds.push_back( i + 1 );
                 acc = 0;
             }
@@ -1364,7 +1376,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     stage_.send( stream_ );
     if( n_qp ) {
         CUDA_CHECK( launch_build_profile_qp( d_qcodes_.as<uint8_t>(), d_qoff_.as<uint64_t>(), d_qlen_.as<uint32_t>(),
-                dev_qslots, n_qp, dev_rows, d_matrix_.as<int64_t>(),
+                dev_qslots, n_qp, dev_rows, dev_lane_rows, d_matrix_.as<int64_t>(),
                 d_qp_prof_.as<uint32_t>(), dev_off, req.bit_width == 8 ? 8 : 16, stream_ ) );
         launches_++;
     }
@@ -1478,10 +1490,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
             continue;
         launched[ri] = true;
         const int R = 4 * (ri + 4);
-        // Needleman-Wunsch: 4 columns per step unless SSA_B200_QP_C=2 pins the
-        // 2-column kernel (4 resident CTAs per SM either way)
-        const QpVariant var = nw ? QpVariant{ 4, pinned_c == 2 ? 2 : 4, false, false, 0 }
-                                 : qpair_variant( bucket, R, pinned_mb, pinned_c, pinned_h, pinned_g8 );
+        const QpVariant var = variant[ri];
         const int mb = var.mb;
         auto launch = [&]( const QPairParams & pp, int grid, int * per ) {
             if( nw )

@@ -301,46 +301,167 @@ __device__ __forceinline__ uint32_t hmax_bits( uint32_t a, uint32_t b ) {
 // G: threads per database sequence (4, or 8 with R = 12: one group per
 // quarter-warp, whose rows 12k fall into 8 distinct shared-memory bank groups,
 // so the 128-bit profile loads are conflict-free; a pass still holds 96 rows).
+// The profile slice of a pass is shared by the CTA's four warps, which work on
+// 32 sequences of one unit side by side (they are sorted by length, so the warps
+// stay close).  It lies in shared memory as
+// [code][group of four rows][lane % 8][4 words]: the eight lanes of a quarter
+// warp, whose 128-bit loads are served together, always hit eight different
+// bank groups, whatever their residue codes (with 4 threads per sequence the
+// profile holds each row twice, for the two sequences of a quarter warp).  The
+// profile has that layout in global memory too, so a slice is one contiguous
+// block that one thread fetches with a bulk copy, two slices ahead of its use
+// (SlicePipe).  Measured on a B200 against a slice per warp, loaded by the warp
+// before each pass and read with 2-way conflicts on half of the accesses
+// (entry pass): 32 queries x 20,000 proteins 16.8 -> 15.5 ms, 24 at 16 bits 12.4
+// -> 11.8, 64 Needleman-Wunsch reads x 20,000 56.1 -> 54.7, 96 x 200,000 697 ->
+// 691 (6.5 TCUPS of computed cells; the 4.5 ALU instructions per cell pair alone
+// reach 7.1 at this occupancy); R = 16, which every access of a group hit the
+// same banks for, 30 -> 20.6 ps per pair, pass and column of 200,000 sequences.
+//
+// Slices of one unit in use order: use i lies in buffer i % 2 and completes its
+// mbarrier's phase i / 2.
+struct SlicePipe {
+    uint32_t * buf;          // two slices
+    uint64_t * full;         // two mbarriers
+    uint32_t * readers;      // warps done with each buffer's use
+    uint32_t words;          // of a slice
+    unsigned * error_flags;
+    uint32_t use;            // uses before the current one
+
+    __device__ static uint32_t smem( const void * p ) { return (uint32_t) __cvta_generic_to_shared( p ); }
+    __device__ void init() {
+        use = 0;
+        if( threadIdx.x == 0 ) {
+            readers[0] = readers[1] = 0;
+            for( int b = 0; b < 2; b++ )
+                asm volatile( "mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"( smem( full + b ) ) : "memory" );
+            asm volatile( "fence.proxy.async.shared::cta;" ::: "memory" );
+        }
+        __syncthreads();
+    }
+    // one thread, when no thread reads buffer (use + ahead) % 2 any more
+    __device__ void fetch( uint32_t ahead, const uint32_t * src ) {
+        const uint32_t b = (use + ahead) & 1u, bytes = words * (uint32_t) sizeof(uint32_t);
+        asm volatile( "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"( smem( full + b ) ), "r"( bytes )
+                : "memory" );
+        asm volatile( "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                smem( buf + (size_t) b * words ) ), "l"( src ), "r"( bytes ), "r"( smem( full + b ) ) : "memory" );
+    }
+    // A warp is done with the current use; the last of the four fetches the use
+    // after the next (src, nullptr: none) into the buffer it frees.  No warp
+    // waits for another here, so they may be up to a pass apart.
+    __device__ void next( int lane, const uint32_t * src ) {
+        if( lane == 0 ) {
+            __threadfence_block();
+            if( atomicAdd( readers + (use & 1u), 1u ) == (uint32_t) (QP_THREADS / 32 - 1) ) {
+                readers[use & 1u] = 0;
+                __threadfence_block();
+                if( src )
+                    fetch( 2, src );
+            }
+        }
+        use++;
+    }
+    // the current use's slice; a copy that never lands raises the error flag
+    __device__ const uint32_t * wait() {
+        const uint32_t b = use & 1u, parity = (use >> 1) & 1u;
+        for( uint32_t n = 0;; n++ ) {
+            uint32_t ok;
+            asm volatile( "{\n\t.reg .pred p;\n\t"
+                          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                          "selp.u32 %0, 1, 0, p;\n\t}"
+                          : "=r"( ok )
+                          : "r"( smem( full + b ) ), "r"( parity )
+                          : "memory" );
+            if( ok )
+                break;
+            if( n >= (1u << 22) ) {
+                atomicOr( error_flags, ERR_PIPELINE );
+                break;
+            }
+        }
+        return buf + (size_t) b * words;
+    }
+};
+
+// The CTA's next work unit: the query pair, its passes, and its sequences less
+// those at either end that another kernel scores.
+struct QpUnit {
+    uint32_t qp, passes, seq_begin, seq_end, rounds;
+    uint2 skip;
+    __device__ bool take( const QPairParams & p, unsigned long long * shared_unit, uint32_t pass_rows,
+            uint32_t per_round ) {
+        __syncthreads();             // every thread has read the last unit, and is done with its slices
+        if( threadIdx.x == 0 )
+            *shared_unit = atomicAdd( p.unit_counter, 1ull );
+        __syncthreads();
+        const unsigned long long u = *shared_unit;
+        if( u >= p.n_units )
+            return false;
+        qp = p.unit_pairs[u / p.n_chunks];
+        const uint32_t chunk = (uint32_t) (u % p.n_chunks);
+        seq_begin = p.chunk_bounds[chunk];
+        seq_end = p.chunk_bounds[chunk + 1];
+        skip = p.qp_skip[qp];
+        if( skip.x <= seq_begin )
+            seq_begin = max( seq_begin, min( skip.y, seq_end ) );
+        if( skip.y >= seq_end )
+            seq_end = max( seq_begin, min( skip.x, seq_end ) );
+        passes = p.qp_rows[qp] / pass_rows;
+        rounds = (seq_end - seq_begin + per_round - 1u) / per_round;
+        return true;
+    }
+    __device__ bool valid( uint32_t idx ) const { return idx < seq_end && (idx < skip.x || idx >= skip.y); }
+    // uses of slices: every pass of every round, or the one slice of a single pass
+    __device__ uint32_t uses() const { return passes == 1u ? min( rounds, 1u ) : rounds * passes; }
+};
+
+// shared memory of the 4-column kernels: two slices
+template <int R>
+constexpr uint32_t qp4_slice_words() {
+    return (uint32_t) QP_CODES * (R / 4) * 32u;
+}
+
 template <int R, int MB, bool HM, int G = QP_G>
 __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParams p ) {
     static_assert( G == 4 || G == 8, "4 or 8 threads per sequence" );
     constexpr int GPW = 32 / G;                  // sequences per warp
     constexpr int C = 4;
     constexpr uint32_t GR = (uint32_t) (G * R);
-    extern __shared__ __align__( 16 ) uint32_t qsm[];
+    constexpr uint32_t WORDS = qp4_slice_words<R>();
+    constexpr uint32_t PER_ROUND = (uint32_t) (QP_THREADS / G);
+    extern __shared__ __align__( 128 ) uint32_t qsm[];
+    __shared__ uint64_t full[2];
+    __shared__ uint32_t readers[2];
+    __shared__ unsigned long long shared_unit;
     const int lane = threadIdx.x & 31;
     const uint32_t warp_in_cta = threadIdx.x >> 5;
     const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t * slice = qsm + warp_in_cta * (QP_CODES * GR);
     const int k = lane & (G - 1);
     const int g = lane / G;
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
     const uint32_t CROSS_ADD = qp_cross_add( p.limit );
     int4 * scratch = p.scratch + ((uint64_t) warp_global * QP_GPW + (uint32_t) g) * p.scratch_cols;
-    uint64_t loaded_key = ~0ull;
+    SlicePipe pipe{ qsm, full, readers, WORDS, p.sink.error_flags, 0 };
+    pipe.init();
+    QpUnit unit;
 
-    for( ;; ) {
-        unsigned long long u = 0;
-        if( lane == 0 )
-            u = atomicAdd( p.unit_counter, 1ull );
-        u = __shfl_sync( 0xffffffffu, u, 0 );
-        if( u >= p.n_units )
-            break;
-        const uint32_t qp = p.unit_pairs[u / p.n_chunks];
-        const uint32_t chunk = (uint32_t) (u % p.n_chunks);
-        const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
-        const uint2 skip = p.qp_skip[qp];
-        const uint32_t rows = p.qp_rows[qp];
-        const uint32_t passes = rows / GR;
-        const uint32_t * prof = p.prof + p.prof_off[qp];
-        const uint32_t slot_a = p.qp_slots[2 * qp], slot_b = p.qp_slots[2 * qp + 1];
+    while( unit.take( p, &shared_unit, GR, PER_ROUND ) ) {
+        const uint32_t passes = unit.passes, n_use = unit.uses();
+        const uint32_t * prof = p.prof + p.prof_off[unit.qp];
+        const uint32_t slot_a = p.qp_slots[2 * unit.qp], slot_b = p.qp_slots[2 * unit.qp + 1];
+        if( threadIdx.x == 0 ) {
+            if( n_use > 0 )
+                pipe.fetch( 0, prof );
+            if( n_use > 1 )
+                pipe.fetch( 1, prof + WORDS );
+        }
+        uint32_t done = 0;                       // uses of this unit
 
-        for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) GPW ) {
-            if( b0 >= skip.x && b0 + (uint32_t) GPW <= skip.y )
-                continue;
-            const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
+        for( uint32_t round = 0; round < unit.rounds; round++ ) {
+            const uint32_t idx = unit.seq_begin + round * PER_ROUND + warp_in_cta * (uint32_t) GPW + (uint32_t) g;
+            const bool valid = unit.valid( idx );
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const uint32_t nb = (L + 3u) >> 2;                    // 4-column blocks
@@ -352,19 +473,8 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
 
             for( uint32_t pass = 0; pass < passes; pass++ ) {
                 const bool last_pass = (pass + 1 == passes);
-                const uint64_t key = ((uint64_t) qp << 24) | pass;
-                if( key != loaded_key ) {
-                    __syncwarp();
-                    constexpr uint32_t per_code = GR / 4u;
-                    const uint4 * src = reinterpret_cast<const uint4 *>( prof + (size_t) pass * GR );
-                    uint4 * dst = reinterpret_cast<uint4 *>( slice );
-                    for( uint32_t i = (uint32_t) lane; i < QP_CODES * per_code; i += 32u ) {
-                        const uint32_t code = i / per_code, w = i % per_code;
-                        dst[i] = src[(size_t) code * (rows / 4u) + w];
-                    }
-                    loaded_key = key;
-                    __syncwarp();
-                }
+                // this lane's column of the slice
+                const uint32_t * slice = pipe.wait() + 4 * (lane & 7);
                 uint32_t H[R], E[R];
 #pragma unroll
                 for( int r = 0; r < R; r++ ) {
@@ -440,7 +550,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                     const uint32_t * pc[C];
 #pragma unroll
                     for( int j = 0; j < C; j++ )
-                        pc[j] = slice + ((w >> (8 * j)) & 0xffu) * GR + (uint32_t) (k * R);
+                        pc[j] = slice + ((w >> (8 * j)) & 0xffu) * (uint32_t) (8 * R);
                     uint4 x[C];
                     uint32_t f[C];
                     // hv[j][r]: H of chain j (column c + j) at row r; only the
@@ -458,7 +568,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                             if( r < 0 || r >= R )
                                 continue;
                             if( (r & 3) == 0 )
-                                x[j] = *reinterpret_cast<const uint4 *>( pc[j] + r );
+                                x[j] = *reinterpret_cast<const uint4 *>( pc[j] + 8 * r );
                             const uint32_t v = (r & 3) == 0 ? x[j].x : (r & 3) == 1 ? x[j].y
                                     : (r & 3) == 2 ? x[j].z : x[j].w;
                             uint32_t hd;
@@ -524,6 +634,10 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                 }
                 best = __vmaxs2( best, smax );
                 __syncwarp();
+                if( passes > 1u ) {
+                    pipe.next( lane, done + 2u < n_use ? prof + (size_t) ((done + 2u) % passes) * WORDS : nullptr );
+                    done++;
+                }
             }
 #pragma unroll
             for( int o = 1; o < G; o <<= 1 ) {
@@ -549,13 +663,15 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                 }
             }
         }
+        if( passes == 1u && n_use )
+            pipe.use++;
     }
 }
 
 // grid == 0: report the resident CTAs per SM in *blocks_per_sm without launching.
 template <int R, int MB, bool HM, int G = QP_G>
 static cudaError_t launch_qp4_one( const QPairParams & p, int grid, cudaStream_t st, int * blocks_per_sm ) {
-    const size_t smem = (size_t) (QP_THREADS / 32) * QP_CODES * G * R * sizeof(uint32_t);
+    const size_t smem = 2 * qp4_slice_words<R>() * sizeof(uint32_t);
     static LaunchShape shape;
     const cudaError_t e = shape.set( sw_qpair4_kernel<R, MB, HM, G>, QP_THREADS, smem );
     if( e != cudaSuccess )
@@ -951,7 +1067,7 @@ __device__ __forceinline__ void nw4_block( uint32_t (&H)[R], uint32_t (&E)[R], c
             if( r < 0 || r >= R )
                 continue;
             if( (r & 3) == 0 )
-                x[j] = *reinterpret_cast<const uint4 *>( pc[j] + r );
+                x[j] = *reinterpret_cast<const uint4 *>( pc[j] + 8 * r );
             const uint32_t v = (r & 3) == 0 ? x[j].x : (r & 3) == 1 ? x[j].y : (r & 3) == 2 ? x[j].z : x[j].w;
             uint32_t hd;
             if( r == 0 )
@@ -1004,12 +1120,11 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile( "cp.async.wait_group %0;" ::"n"( N ) : "memory" );
 }
 
-// shared memory of nw_qpair4_kernel: the warps' profile slices, then the
-// groups' boundary rings
+// shared memory of nw_qpair4_kernel: two profile slices, then the groups'
+// boundary rings
 template <int R>
 constexpr size_t nw4_smem_bytes() {
-    return (size_t) (QP_THREADS / 32) * QP_CODES * QP_G * R * sizeof(uint32_t) +
-            (size_t) (QP_THREADS / QP_G) * NW4_SLOTS * 2 * sizeof(int4);
+    return 2 * qp4_slice_words<R>() * sizeof(uint32_t) + (size_t) (QP_THREADS / QP_G) * NW4_SLOTS * 2 * sizeof(int4);
 }
 
 template <int R>
@@ -1017,50 +1132,49 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
     constexpr int G = QP_G;
     constexpr int C = 4;
     constexpr uint32_t GR = (uint32_t) (G * R);
-    extern __shared__ __align__( 16 ) uint32_t qsm[];
+    constexpr uint32_t WORDS = qp4_slice_words<R>();
+    constexpr uint32_t PER_ROUND = (uint32_t) (QP_THREADS / G);
+    extern __shared__ __align__( 128 ) uint32_t qsm[];
+    __shared__ uint64_t full[2];
+    __shared__ uint32_t readers[2];
+    __shared__ unsigned long long shared_unit;
     const int lane = threadIdx.x & 31;
     const uint32_t warp_in_cta = threadIdx.x >> 5;
     const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t * slice = qsm + warp_in_cta * (QP_CODES * GR);
     const int k = lane & (G - 1);
     const int g = lane / G;
     const int gO = p.gap_open, gE = p.gap_e;
     const uint32_t GOE32 = (uint32_t) ((int32_t) p.gap_oe * 65536 + (int32_t) p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) gE << 16) | (uint16_t) (int16_t) gE;
     int4 * scratch = p.scratch + ((uint64_t) warp_global * QP_GPW + (uint32_t) g) * p.scratch_cols;
-    // this group's boundary ring, after all warps' profile slices
-    int4 * ring = reinterpret_cast<int4 *>( qsm + (QP_THREADS / 32) * (QP_CODES * GR) ) +
-            (size_t) (threadIdx.x / G) * (NW4_SLOTS * 2);
-    uint64_t loaded_key = ~0ull;
+    // this group's boundary ring, after the two profile slices
+    int4 * ring = reinterpret_cast<int4 *>( qsm + 2 * WORDS ) + (size_t) (threadIdx.x / G) * (NW4_SLOTS * 2);
+    SlicePipe pipe{ qsm, full, readers, WORDS, p.sink.error_flags, 0 };
+    pipe.init();
+    QpUnit unit;
     auto left_h = [&]( int32_t i ) { return gO + (i + 1) * gE; };           // H(i, -1)
     auto left_e = [&]( int32_t i ) { return 2 * gO + (i + 2) * gE; };       // E entering column 0
     auto top_h = [&]( int32_t j ) { return j < 0 ? 0 : gO + (j + 1) * gE; };   // H(-1, j)
     auto top_f = [&]( int32_t c ) { return 2 * gO + (c + 2) * gE; };        // F entering row 0
 
-    for( ;; ) {
-        unsigned long long u = 0;
-        if( lane == 0 )
-            u = atomicAdd( p.unit_counter, 1ull );
-        u = __shfl_sync( 0xffffffffu, u, 0 );
-        if( u >= p.n_units )
-            break;
-        const uint32_t qp = p.unit_pairs[u / p.n_chunks];
-        const uint32_t chunk = (uint32_t) (u % p.n_chunks);
-        const uint32_t seq_begin = p.chunk_bounds[chunk], seq_end = p.chunk_bounds[chunk + 1];
-        const uint2 skip = p.qp_skip[qp];
-        const uint32_t rows = p.qp_rows[qp];
-        const uint32_t passes = rows / GR;
-        const uint32_t * prof = p.prof + p.prof_off[qp];
-        const uint32_t slot_a = p.qp_slots[2 * qp], slot_b = p.qp_slots[2 * qp + 1];
+    while( unit.take( p, &shared_unit, GR, PER_ROUND ) ) {
+        const uint32_t passes = unit.passes, n_use = unit.uses();
+        const uint32_t * prof = p.prof + p.prof_off[unit.qp];
+        const uint32_t slot_a = p.qp_slots[2 * unit.qp], slot_b = p.qp_slots[2 * unit.qp + 1];
         const int32_t qa_last = (int32_t) p.qlen[slot_a] - 1;
         const int32_t qb_last = (slot_b == 0xffffffffu) ? -1 : (int32_t) p.qlen[slot_b] - 1;
-        const uint32_t lmax = p.qp_lmax[qp];
+        const uint32_t lmax = p.qp_lmax[unit.qp];
+        if( threadIdx.x == 0 ) {
+            if( n_use > 0 )
+                pipe.fetch( 0, prof );
+            if( n_use > 1 )
+                pipe.fetch( 1, prof + WORDS );
+        }
+        uint32_t done = 0;                       // uses of this unit
 
-        for( uint32_t b0 = seq_begin; b0 < seq_end; b0 += (uint32_t) QP_GPW ) {
-            if( b0 >= skip.x && b0 + (uint32_t) QP_GPW <= skip.y )
-                continue;
-            const uint32_t idx = b0 + (uint32_t) g;
-            const bool valid = idx < seq_end && (idx < skip.x || idx >= skip.y);
+        for( uint32_t round = 0; round < unit.rounds; round++ ) {
+            const uint32_t idx = unit.seq_begin + round * PER_ROUND + warp_in_cta * (uint32_t) QP_GPW + (uint32_t) g;
+            const bool valid = unit.valid( idx );
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const bool exact = valid && L <= lmax;
@@ -1076,8 +1190,6 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
             }
             const uint32_t nb = exact ? (L + 3u) >> 2 : 0u;         // 4-column blocks
             const uint32_t max_nb = __reduce_max_sync( 0xffffffffu, nb );
-            if( max_nb == 0 )
-                continue;
             const uint8_t * res = p.db.codes + (valid ? p.db.offsets[id] : 0ull);
             const int32_t last_col = (int32_t) L - 1;
             const int32_t cap_blk = last_col >> 2;
@@ -1086,19 +1198,8 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
 
             for( uint32_t pass = 0; pass < passes; pass++ ) {
                 const bool last_pass = (pass + 1 == passes);
-                const uint64_t key = ((uint64_t) qp << 24) | pass;
-                if( key != loaded_key ) {
-                    __syncwarp();
-                    constexpr uint32_t per_code = GR / 4u;
-                    const uint4 * src = reinterpret_cast<const uint4 *>( prof + (size_t) pass * GR );
-                    uint4 * dst = reinterpret_cast<uint4 *>( slice );
-                    for( uint32_t i = (uint32_t) lane; i < QP_CODES * per_code; i += 32u ) {
-                        const uint32_t code = i / per_code, w = i % per_code;
-                        dst[i] = src[(size_t) code * (rows / 4u) + w];
-                    }
-                    loaded_key = key;
-                    __syncwarp();
-                }
+                // this lane's column of the slice
+                const uint32_t * slice = pipe.wait() + 4 * (lane & 7);
                 const int32_t row0 = (int32_t) (pass * GR) + k * R;
                 const int ra = qa_last - row0, rb = qb_last - row0;
                 // does this thread hold a query's last row in this pass?
@@ -1188,7 +1289,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                     const uint32_t * pc[C];
 #pragma unroll
                     for( int j = 0; j < C; j++ )
-                        pc[j] = slice + ((w >> (8 * j)) & 0xffu) * GR + (uint32_t) (k * R);
+                        pc[j] = slice + ((w >> (8 * j)) & 0xffu) * (uint32_t) (8 * R);
                     uint32_t f[C];
 #pragma unroll
                     for( int j = 0; j < C; j++ )
@@ -1218,6 +1319,10 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                 if( reads_boundary )
                     cp_async_wait<0>();
                 __syncwarp();
+                if( passes > 1u ) {
+                    pipe.next( lane, done + 2u < n_use ? prof + (size_t) ((done + 2u) % passes) * WORDS : nullptr );
+                    done++;
+                }
             }
             // the threads holding the last rows report (values are > 0 with the bias)
 #pragma unroll
@@ -1234,6 +1339,8 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
                             (int32_t) (cap_b >> 16) - (int32_t) NWQ_BIAS;
             }
         }
+        if( passes == 1u && n_use )
+            pipe.use++;
     }
 }
 
@@ -1267,25 +1374,41 @@ cudaError_t launch_nw_qpair4( int R, const QPairParams & p, int grid, cudaStream
     }
 }
 
-// prof[qp][code][row] = (A's score, B's score) as a 16x2 word at the entry
-// width; rows past a query, and the absent query of an odd batch, score -128
-// (8-bit Smith-Waterman: never raises a maximum) or 0 (16-bit
-// Needleman-Wunsch: rows below a query do not feed back into it).
+// (A's score, B's score) of every code and row as 16x2 words at the entry width;
+// rows past a query, and the absent query of an odd batch, score -128 (8-bit
+// Smith-Waterman: never raises a maximum) or 0 (16-bit entry: rows below a query
+// do not feed back into it).  lane_rows 0: prof[qp][code][row], for the 2-column
+// kernels; else prof[qp][pass][code][group of 4 rows][lane % 8][4], for the
+// 4-column kernels with lane_rows rows per lane (SlicePipe), where the group's
+// threads are lane % 4, or lane % 8 for lane_rows 12.
 __global__ void build_profile_qp_kernel( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
-        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const int64_t * matrix, uint32_t * prof,
-        const uint64_t * prof_off, int width ) {
+        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const uint32_t * lane_rows,
+        const int64_t * matrix, uint32_t * prof, const uint64_t * prof_off, int width ) {
     const uint32_t qp = blockIdx.y;
     if( qp >= n_qp )
         return;
-    const uint32_t rows = qp_rows[qp];
+    const uint32_t rows = qp_rows[qp], R = lane_rows[qp], G = R == 12u ? 8u : (uint32_t) QP_G;
     const uint32_t sa = qp_slots[2 * qp], sb = qp_slots[2 * qp + 1];
     const uint32_t La = qlen[sa], Lb = (sb == 0xffffffffu) ? 0u : qlen[sb];
     const uint8_t * qa = qcodes + qoff[sa];
     const uint8_t * qb = (sb == 0xffffffffu) ? qa : qcodes + qoff[sb];
     uint32_t * out = prof + prof_off[qp];
-    for( uint64_t x = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; x < (uint64_t) QP_CODES * rows;
+    const uint64_t n = (uint64_t) QP_CODES * rows * (R ? 8u / G : 1u);
+    for( uint64_t x = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; x < n;
             x += (uint64_t) gridDim.x * blockDim.x ) {
-        const uint32_t code = (uint32_t) (x / rows), row = (uint32_t) (x % rows);
+        uint32_t code, row;
+        if( R == 0 ) {
+            code = (uint32_t) (x / rows);
+            row = (uint32_t) (x % rows);
+        }
+        else {
+            const uint32_t i = (uint32_t) x & 3u, l = ((uint32_t) x >> 2) & 7u;
+            const uint64_t y = x >> 5;                      // (pass, code, group of rows)
+            const uint32_t r4 = (uint32_t) (y % (R / 4u));
+            const uint64_t z = y / (R / 4u);
+            code = (uint32_t) (z % QP_CODES);
+            row = (uint32_t) (z / QP_CODES) * G * R + (l % G) * R + 4u * r4 + i;
+        }
         const int32_t pad = (width == 8) ? -128 : 0;
         int32_t a = pad, b = pad;
         if( row < La ) {
@@ -1301,12 +1424,12 @@ __global__ void build_profile_qp_kernel( const uint8_t * qcodes, const uint64_t 
 }
 
 cudaError_t launch_build_profile_qp( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
-        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const int64_t * matrix, uint32_t * prof,
-        const uint64_t * prof_off, int width, cudaStream_t st ) {
+        const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const uint32_t * lane_rows,
+        const int64_t * matrix, uint32_t * prof, const uint64_t * prof_off, int width, cudaStream_t st ) {
     if( n_qp == 0 )
         return cudaSuccess;
     dim3 grid( 16, n_qp );
-    build_profile_qp_kernel<<<grid, 256, 0, st>>>( qcodes, qoff, qlen, qp_slots, n_qp, qp_rows, matrix, prof,
+    build_profile_qp_kernel<<<grid, 256, 0, st>>>( qcodes, qoff, qlen, qp_slots, n_qp, qp_rows, lane_rows, matrix, prof,
             prof_off, width );
     return cudaGetLastError();
 }
