@@ -32,10 +32,10 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-I" + INCLUDE, "-I" + CSRC]
 
 CU_SOURCES = ["engine.cu", "emul_kernel.cu", "traceback_kernels.cu", "diag_kernels.cu", "sw_fast_kernel.cu",
-              "noalloc.cu", "sw_qpair_kernel.cu", "pair_kernel.cu",
+              "noalloc.cu", "sw_qpair_kernel.cu",
               "sw_stream_kernel.cu"]
 CPP_SOURCES = ["api.cpp", "replay.cpp", "tuning.cpp"]
-HEADERS = ["device_common.cuh", "wavefront.cuh", "stripe_pipeline.cuh", "stream_stripes.cuh", "ssa_internal.h", "builtin_matrices.inc"]
+HEADERS = ["device_common.cuh", "wavefront.cuh", "stream_stripes.cuh", "ssa_internal.h", "builtin_matrices.inc"]
 
 LIB = os.path.join(OUT, "libssa.so")
 PLUGIN = os.path.join(OUT, "libsdb_b200.so")

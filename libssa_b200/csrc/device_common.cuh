@@ -130,7 +130,7 @@ struct TbRegion {
     int32_t a_begin, a_end;   // query rows
     int32_t b_begin, b_end;   // database columns
     int32_t fwd_score;        // SW: forward-pass maximum; NW: H(a_end, b_end) from the direction pass
-    int32_t dir_steps;        // wavefront steps per stripe in the hit's direction bytes (columns + 31)
+    int32_t dir_steps;        // wavefront steps per stripe in the hit's direction words (blocks of 4 columns + 31)
     int32_t pad_;
     int32_t status;           // 0 ok, 1 no positive cell, 2 reverse pass found nothing
 };
@@ -148,8 +148,8 @@ struct TbParams {
     int32_t * last_h;           // per hit: forward pass last-row H (query-indexed)
     int32_t * last_e;           // per hit: forward pass last-row vertical gap
     const uint64_t * last_off;  // per hit offset into last_h / last_e
-    // per hit direction bytes, 2 bits per cell: [stripe][wavefront step][lane][R / 4]
-    uint8_t * dirs;
+    // per hit direction words, 2 bits per cell: [stripe][wavefront step][lane], a word per 4 rows x 4 columns
+    uint32_t * dirs;
     const uint64_t * dir_off;   // per hit offset into dirs
     char * ops;                 // per hit reversed op string
     const uint64_t * ops_off;
@@ -162,9 +162,9 @@ struct TbParams {
     unsigned long long * counter;   // next ticket (0 at the start)
     uint32_t * progress;        // per ticket (0 at the start)
     int4 * result;              // per ticket: end or begin cell of the stripes so far
-    int2 * boundary;            // per hit with several stripes: (H, F) per database column
+    int4 * boundary;            // per hit with several stripes: (H, F) per database column, two words per block of 4
     const uint64_t * bnd_off;   // per hit offset into boundary
-    int32_t * limit;            // per hit: last column worth computing in the reverse pass
+    int32_t * limit;            // per hit: last block worth computing in the reverse pass
 };
 
 // Kernel launchers.
@@ -181,13 +181,16 @@ cudaError_t preload_emul64();
 cudaError_t launch_build_profile64( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
         const uint32_t * qpad, const uint64_t * prof_off, const int64_t * matrix, int64_t * prof, uint32_t n_slots,
         cudaStream_t st );
-// Traceback passes: R query rows per lane (4 or 8), p8: the score table fits int8.
-cudaError_t launch_tb_forward( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
-cudaError_t launch_tb_reverse( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
-cudaError_t launch_tb_directions( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
+// Traceback passes.  p8: the score table fits int8.
+constexpr int TB_ROWS_PER_LANE = 4;
+cudaError_t launch_tb_forward( const TbParams & p, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_reverse( const TbParams & p, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_directions( const TbParams & p, bool nw, bool p8, int sms, cudaStream_t st );
+// scores alone (into the regions' fwd_score)
+cudaError_t launch_tb_scores( const TbParams & p, bool nw, bool p8, int sms, cudaStream_t st );
 // forward and directions in one sweep (Smith-Waterman, symmetric score table)
-cudaError_t launch_tb_fwddir( const TbParams & p, int R, bool p8, int sms, cudaStream_t st );
-cudaError_t launch_tb_walk( const TbParams & p, int R, cudaStream_t st );
+cudaError_t launch_tb_fwddir( const TbParams & p, bool p8, int sms, cudaStream_t st );
+cudaError_t launch_tb_walk( const TbParams & p, cudaStream_t st );
 
 // Dynamic shared memory limit and resident blocks per SM of a kernel, asked of
 // the driver once per kernel and size (the engine's one device; its launches
@@ -339,31 +342,5 @@ cudaError_t launch_nw_qpair4( int R, const QPairParams & p, int grid, cudaStream
 cudaError_t launch_build_profile_qp( const uint8_t * qcodes, const uint64_t * qoff, const uint32_t * qlen,
         const uint32_t * qp_slots, uint32_t n_qp, const uint32_t * qp_rows, const uint32_t * lane_rows,
         const int64_t * matrix, uint32_t * prof, const uint64_t * prof_off, int width, cudaStream_t st );
-
-// ---- long pairs (pair_kernel.cu) ---------------------------------------------
-// A group of PAIR_W warps scores one (query, database sequence) pair exactly in
-// int32: lane k of a warp owns PAIR_R query rows of a stripe of 32 x PAIR_R rows.
-constexpr int PAIR_R = 16;
-constexpr int PAIR_W = 4;
-constexpr int PAIR_THREADS = 256;
-
-struct PairScoreParams {
-    DbView db;
-    const uint8_t * qcodes;       // per query slot: codes at qoff[slot]
-    const uint64_t * qoff;
-    const uint32_t * qlen;
-    const uint32_t * pair_slot;   // per pair, in work order (largest first): query slot
-    const uint32_t * pair_unit;   // per pair: database unit
-    uint32_t n_pairs;
-    const int64_t * matrix;       // 32 x 32, [database code][query code]
-    int gap_open, gap_extend;
-    int32_t * score;              // per pair, in work order
-    int4 * scratch;               // per group of PAIR_W warps: scratch_cols boundary columns (H, F)
-    uint32_t scratch_cols;
-    unsigned long long * counter;
-    unsigned * error_flags;
-};
-
-cudaError_t launch_pair_score( int algo, const PairScoreParams & p, int grid, cudaStream_t st, int * blocks_per_sm );
 
 }  // namespace ssa

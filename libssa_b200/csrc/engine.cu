@@ -519,7 +519,7 @@ public:
             &d_scratch_fast_[0], &d_scratch_fast_[1], &d_scratch_fast_[2], &d_scratch_fast_[3], &d_scratch_fast_[4],
             &d_scratch_fast_[5], &d_scratch_fast_[6], &d_scratch_fast_[7], &d_serve_block_, &d_prof_, &d_score_, &d_list_a_, &d_list_b_, &d_counts_, &d_scratch_,
             &d_tb_io_, &d_tb_last_, &d_tb_dirs_, &d_tb_sync_, &d_tb_result_, &d_tb_bnd_, &d_qp_prof_,
-            &d_serve_score_, &d_pair_score_, &d_list_c_, &d_sw_sync_, &d_sw_bnd_,
+            &d_serve_score_, &d_list_c_, &d_sw_sync_, &d_sw_bnd_,
             &d_seg_[0], &d_seg_[1], &d_gather_codes_, &d_gather_off_, &d_gather_len_, &d_prof64_, &d_score64_ };
         for( DevBuf * b : bufs )
             b->release();
@@ -574,10 +574,11 @@ private:
     int32_t * score_sink() { return serving_ ? d_serve_score_.as<int32_t>() : d_score_.as<int32_t>(); }
     void build_profiles( int width, uint32_t n_slots );
     // scores_from_regions: the hits carry no score yet; take it from the
-    // forward pass (SW, symmetric table) or the direction pass (NW)
+    // forward pass (SW, symmetric table) or the direction pass (NW);
+    // scores_only: score the hits' pairs exactly, no alignment
     void traceback( const SearchRequest & req, std::vector<std::vector<Hit>> & out,
             const std::vector<std::pair<uint32_t, uint32_t>> & lists, SearchStats & stats,
-            bool scores_from_regions = false );
+            bool scores_from_regions = false, bool scores_only = false );
     uint64_t traceback_budget();
     void upload_queries( const SearchRequest & req, const QueryCodes * queries, uint32_t nq, bool profiles,
             SearchStats & stats );
@@ -648,7 +649,6 @@ private:
     PinnedBuf h_score64_;
     bool wide_ = false;
     int prof64_width_ = -1;
-    DevBuf d_pair_score_;
     uint64_t tb_budget_ = 0;         // traceback direction memory per wave (0 = automatic)
     // streaming: the database does not fit its device memory budget; segments
     // of consecutive positions of the length order take turns on the device
@@ -2035,7 +2035,8 @@ static int64_t max_abs_step( const SearchRequest & req ) {
 constexpr uint64_t TB_MIN_BUDGET = (uint64_t) 256 << 20;
 
 void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>> & out,
-        const std::vector<std::pair<uint32_t, uint32_t>> & lists, SearchStats & stats, bool scores_from_regions ) {
+        const std::vector<std::pair<uint32_t, uint32_t>> & lists, SearchStats & stats, bool scores_from_regions,
+        bool scores_only ) {
     std::vector<TbHit> hits;
     std::vector<std::pair<uint32_t, uint32_t>> where;   // (list index, hit index)
     for( const auto & l : lists ) {
@@ -2056,7 +2057,6 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     const int64_t mabs = max_abs_step( req );
     std::vector<TbRegion> regions( nh );
     std::vector<uint64_t> last_off( nh + 1, 0 );
-    uint64_t stripes128 = 0;
     for( uint32_t h = 0; h < nh; h++ ) {
         const uint32_t A = h_qlen_[hits[h].qslot], B = db_.len[hits[h].id];
         if( (int64_t) (A + B + 4) * (mabs + 1) * 2 > INT32_MAX )
@@ -2071,17 +2071,8 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         }
         regions[h] = rg;
         last_off[h + 1] = last_off[h] + A;
-        stripes128 += (A + 127u) / 128u;
     }
-    // rows per lane: 4 while every stripe of 128 rows can be resident (32 warps
-    // per SM), else 8.  Measured on a B200, sweep with directions at R = 8 and
-    // R = 4: 10 hits of 375 x 380 0.214 and 0.181 ms, 10 of 300 x 33,000 12.8
-    // and 8.8 ms, 960 of 30-1,803 x 20,000 25.1 and 20.0 ms; past the line, 48
-    // pairs of 5,000-30,000 residues 30.6 and 36.4 ms (Needleman-Wunsch).
-    int R = stripes128 <= (uint64_t) sms_ * 32 ? 4 : 8;
-    if( const char * pin = getenv( "SSA_B200_TB_R" ) )   // pins the rows per lane (tests)
-        R = atoi( pin ) == 8 ? 8 : 4;
-    const uint32_t stripe_rows = 32u * (uint32_t) R;
+    constexpr uint32_t stripe_rows = 32u * TB_ROWS_PER_LANE;
     bool p8 = true;
     for( int k = 0; k < 1024; k++ )
         p8 = p8 && req.matrix[k] == (int8_t) req.matrix[k];
@@ -2144,11 +2135,12 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
             return at;
         }
     };
+    enum Mode { REGIONS, PATHS, SCORES };
     auto run_wave = [&]( const std::vector<uint32_t> & wave, const std::vector<uint32_t> & rows,
-            const std::vector<uint32_t> & cols, bool regions_only ) {
+            const std::vector<uint32_t> & cols, Mode mode ) {
         const uint32_t nw = (uint32_t) wave.size();
-        const bool paths = !regions_only;
-        const bool reverse = req.algo == 0 && (fused || regions_only);
+        const bool paths = mode == PATHS;
+        const bool reverse = req.algo == 0 && (mode == REGIONS || (fused && paths));
         // tickets stripe by stripe: stripe i exists in the first n_i hits
         std::vector<uint32_t> cum{ 0 };
         for( uint32_t left = nw, i = 0;; i++ ) {
@@ -2158,7 +2150,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
                 break;
             cum.push_back( cum.back() + left );
         }
-        uint64_t dir_bytes = 0, bnd_cols = 0, ops_bytes = 0;
+        uint64_t dir_words = 0, bnd_words = 0, ops_bytes = 0;
         Layout in, res;
         const size_t o_hits = in.add( nw * sizeof(TbHit) ), o_last = in.add( nw * sizeof(uint64_t) ),
                 o_dir = in.add( nw * sizeof(uint64_t) ), o_ops = in.add( (nw + 1) * sizeof(uint64_t) ),
@@ -2170,19 +2162,19 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
             const uint32_t h = wave[k];
             const uint64_t stripes = (rows[h] + stripe_rows - 1) / stripe_rows;
             TbRegion rg = regions[h];
-            rg.dir_steps = (int32_t) cols[h] + 31;
+            rg.dir_steps = (int32_t) ((cols[h] + 3u) / 4u) + 31;
             ((TbHit *) (hin + o_hits))[k] = dev_hits[h];
             ((TbRegion *) (hin + o_reg))[k] = rg;
             ((uint64_t *) (hin + o_last))[k] = last_off[h];
-            ((uint64_t *) (hin + o_dir))[k] = dir_bytes;
+            ((uint64_t *) (hin + o_dir))[k] = dir_words;
             ((uint64_t *) (hin + o_ops))[k] = ops_bytes;
-            ((uint64_t *) (hin + o_bnd))[k] = bnd_cols;
+            ((uint64_t *) (hin + o_bnd))[k] = bnd_words;
             if( paths ) {
-                dir_bytes += stripes * ((uint64_t) cols[h] + 31) * (32 * R / 4);
+                dir_words += stripes * (uint64_t) rg.dir_steps * 32;
                 ops_bytes += (uint64_t) rows[h] + cols[h] + 1;
             }
             if( stripes > 1 )
-                bnd_cols += cols[h];
+                bnd_words += 2ull * ((cols[h] + 3u) / 4u);
         }
         ((uint64_t *) (hin + o_ops))[nw] = ops_bytes;
         memcpy( hin + o_cum, cum.data(), cum.size() * sizeof(uint32_t) );
@@ -2216,10 +2208,10 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         p.levels = (uint32_t) cum.size() - 1;
         p.n_tickets = n_tickets;
         p.result = (int4 *) d_tb_result_.ensure( std::max<size_t>( 16, (size_t) n_tickets * sizeof(int4) ) );
-        p.boundary = (int2 *) d_tb_bnd_.ensure( bnd_cols * sizeof(int2) + 16 );
+        p.boundary = (int4 *) d_tb_bnd_.ensure( bnd_words * sizeof(int4) + 16 );
         p.limit = (int32_t *) (dsy + s_lim);
         if( paths )
-            p.dirs = (uint8_t *) d_tb_dirs_.ensure( dir_bytes + 16 );
+            p.dirs = (uint32_t *) d_tb_dirs_.ensure( dir_words * sizeof(uint32_t) + 16 );
         stage_.send( stream_ );
         CUDA_CHECK( cudaMemcpyAsync( din, hin, in.bytes, cudaMemcpyHostToDevice, stream_ ) );
         CUDA_CHECK( cudaMemsetAsync( dsy, 0, s_zero, stream_ ) );
@@ -2233,18 +2225,19 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         if( timing )
             CUDA_CHECK( cudaEventRecord( ev_tb_[0], stream_ ) );
         sweep( 0 );
-        CUDA_CHECK( regions_only ? launch_tb_forward( p, R, p8, sms_, stream_ )
-                    : fused ? launch_tb_fwddir( p, R, p8, sms_, stream_ )
-                            : launch_tb_directions( p, R, p8, sms_, stream_ ) );
+        CUDA_CHECK( mode == SCORES ? launch_tb_scores( p, req.algo == 1, p8, sms_, stream_ )
+                    : mode == REGIONS ? launch_tb_forward( p, p8, sms_, stream_ )
+                    : fused ? launch_tb_fwddir( p, p8, sms_, stream_ )
+                            : launch_tb_directions( p, req.algo == 1, p8, sms_, stream_ ) );
         if( timing )
             CUDA_CHECK( cudaEventRecord( ev_tb_[1], stream_ ) );
         if( reverse ) {
             sweep( 1 );
-            CUDA_CHECK( launch_tb_reverse( p, R, p8, sms_, stream_ ) );
+            CUDA_CHECK( launch_tb_reverse( p, p8, sms_, stream_ ) );
         }
         if( paths ) {
             launches_++;
-            CUDA_CHECK( launch_tb_walk( p, R, stream_ ) );
+            CUDA_CHECK( launch_tb_walk( p, stream_ ) );
         }
         if( timing )
             CUDA_CHECK( cudaEventRecord( ev_tb_[2], stream_ ) );
@@ -2256,21 +2249,23 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
             fatal( "Internal error in the GPU traceback (flags 0x%x).", err );
         stats.h2d_bytes += in.bytes;
         stats.d2h_bytes += res.bytes;
-        total_dir += dir_bytes;
+        total_dir += dir_words * sizeof(uint32_t);
         n_waves++;
         if( timing ) {
             float x = 0, y = 0;
             CUDA_CHECK( cudaEventElapsedTime( &x, ev_tb_[0], ev_tb_[1] ) );
             CUDA_CHECK( cudaEventElapsedTime( &y, ev_tb_[1], ev_tb_[2] ) );
-            (regions_only ? t_fwd : t_dir) += x;
-            (regions_only ? t_rev : t_walk) += y;
+            (paths ? t_dir : t_fwd) += x;
+            (paths ? t_walk : t_rev) += y;
         }
         for( uint32_t k = 0; k < nw; k++ ) {
             const uint32_t h = wave[k];
             const TbRegion & rg = regions[h] = ((const TbRegion *) (hout + r_reg))[k];
             if( rg.status == 2 )
                 fatal( "Internal error in align function." );   // reference: src/algo/align.c:131
-            if( regions_only )
+            if( mode == SCORES )
+                out[where[h].first][where[h].second].score = rg.fwd_score;
+            if( !paths )
                 continue;
             Hit & hit = out[where[h].first][where[h].second];
             hit.has_cigar = true;
@@ -2308,7 +2303,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     };
     // Waves: runs of the hits in (most stripes first, most columns first) order
     // whose direction bytes and boundary rows fit the traceback memory.
-    auto run_waves = [&]( const std::vector<uint32_t> & rows, const std::vector<uint32_t> & cols, bool regions_only ) {
+    auto run_waves = [&]( const std::vector<uint32_t> & rows, const std::vector<uint32_t> & cols, Mode mode ) {
         std::vector<uint32_t> order( nh );
         for( uint32_t h = 0; h < nh; h++ )
             order[h] = h;
@@ -2317,8 +2312,9 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
             return stripes( x ) != stripes( y ) ? stripes( x ) > stripes( y ) : cols[x] > cols[y];
         } );
         auto need = [&]( uint32_t h ) {
-            return (regions_only ? 0 : (uint64_t) stripes( h ) * (cols[h] + 31) * (32 * R / 4)) +
-                    (stripes( h ) > 1 ? cols[h] * sizeof(int2) : 0);
+            const uint64_t blocks = (cols[h] + 3u) / 4u;
+            return (mode == PATHS ? (uint64_t) stripes( h ) * (blocks + 31) * 32 * sizeof(uint32_t) : 0) +
+                    (stripes( h ) > 1 ? 2 * blocks * sizeof(int4) : 0);
         };
         uint64_t total = 0;
         for( uint32_t h = 0; h < nh; h++ )
@@ -2330,30 +2326,30 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         uint64_t load = 0;
         for( uint32_t h : order ) {
             if( !wave.empty() && load + need( h ) > budget ) {
-                run_wave( wave, rows, cols, regions_only );
+                run_wave( wave, rows, cols, mode );
                 wave.clear();
                 load = 0;
             }
             wave.push_back( h );
             load += need( h );
         }
-        run_wave( wave, rows, cols, regions_only );
+        run_wave( wave, rows, cols, mode );
     };
     std::vector<uint32_t> rows( nh ), cols( nh );
     for( uint32_t h = 0; h < nh; h++ ) {
         rows[h] = h_qlen_[hits[h].qslot];
         cols[h] = db_.len[hits[h].id];
     }
-    if( req.algo == 0 && !fused ) {
+    if( req.algo == 0 && !fused && !scores_only ) {
         // the end and begin cell of every hit, then rows 0 .. a_end and columns
         // 0 .. b_end of the direction matrix
-        run_waves( rows, cols, true );
+        run_waves( rows, cols, REGIONS );
         for( uint32_t h = 0; h < nh; h++ ) {
             rows[h] = regions[h].status == 0 ? (uint32_t) regions[h].a_end + 1 : 1;
             cols[h] = regions[h].status == 0 ? (uint32_t) regions[h].b_end + 1 : 1;
         }
     }
-    run_waves( rows, cols, false );
+    run_waves( rows, cols, scores_only ? SCORES : PATHS );
     // a very large direction buffer (long pairs) is not kept for later calls,
     // whose scores, lists and database segments need the device memory
     if( d_tb_dirs_.bytes > ((uint64_t) 8 << 30) )
@@ -2398,8 +2394,8 @@ uint64_t Engine::traceback_budget() {
 // ---- long pairs -------------------------------------------------------------------
 // Query i against database unit units[i] alone: what sw_align / nw_align return
 // for the query against a database holding only that sequence (one hit, or
-// none for an empty sequence).  One warp scores each pair exactly
-// (pair_kernel.cu); the hits then go through the traceback like a search's.
+// none for an empty sequence).  The traceback's sweep scores each pair exactly;
+// the hits then go through the traceback like a search's.
 void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCodes> & queries,
         const std::vector<uint32_t> & units, std::vector<std::vector<Hit>> & out, SearchStats & stats ) {
     const HostDb & db = database();
@@ -2447,87 +2443,23 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
         for( int q = 0; q < 32; q++ )
             symmetric = symmetric && req.matrix[(d << 5) + q] == req.matrix[(q << 5) + d];
     const bool scores_in_traceback = req.align_type == COMPUTE_ALIGNMENT && (req.algo == 1 || symmetric);
-    if( nw && scores_in_traceback ) {
-        for( uint32_t k = 0; k < nw; k++ ) {
-            const uint32_t i = work[k];
-            Hit h;
-            h.unit = units[i];
-            h.id = units[i] / db.upi;
-            out[i].push_back( h );
-        }
+    for( uint32_t k = 0; k < nw; k++ ) {
+        const uint32_t i = work[k];
+        Hit h;
+        h.unit = units[i];
+        h.id = units[i] / db.upi;
+        out[i].push_back( h );
     }
-    else if( nw ) {
-        std::vector<uint32_t> hs( nw ), hu( nw );
-        for( uint32_t k = 0; k < nw; k++ ) {
-            hs[k] = work[k];
-            hu[k] = units[work[k]];
-        }
-        PairScoreParams p{};
-        if( streaming_ ) {
-            // the pairs' sequences gathered into a view of their own
-            std::vector<uint32_t> ids;
-            std::unordered_map<uint32_t, uint32_t> index;
-            for( uint32_t & u : hu ) {
-                auto it = index.find( u );
-                if( it == index.end() ) {
-                    it = index.emplace( u, (uint32_t) ids.size() ).first;
-                    ids.push_back( u );
-                }
-                u = it->second;
-            }
-            p.db = gather_view( ids, stats );
-        }
-        else {
-            p.db = db_view();
-        }
-        p.qcodes = d_qcodes_.as<uint8_t>();
-        p.qoff = d_qoff_.as<uint64_t>();
-        p.qlen = d_qlen_.as<uint32_t>();
-        p.pair_slot = stage_.add( hs.data(), nw, stream_ );
-        p.pair_unit = stage_.add( hu.data(), nw, stream_ );
-        stage_.send( stream_ );
-        p.n_pairs = nw;
-        p.matrix = d_matrix_.as<int64_t>();
-        p.gap_open = req.gap_open;
-        p.gap_extend = req.gap_extend;
-        p.score = (int32_t *) d_pair_score_.ensure( nw * sizeof(int32_t) );
-        p.counter = d_counts_.as<unsigned long long>() + 15;      // bytes 120..127
-        p.error_flags = d_counts_.as<unsigned>() + 2;
-        int per_sm = 0;
-        CUDA_CHECK( launch_pair_score( req.algo, p, 0, stream_, &per_sm ) );
-        const int grid = sms_ * std::max( 1, per_sm );
-        if( max_a > (uint32_t) (32 * PAIR_R) ) {
-            p.scratch_cols = max_b;
-            p.scratch = (int4 *) d_scratch_.ensure( (size_t) grid * (PAIR_THREADS / (32 * PAIR_W)) * max_b * sizeof(int4) );
-        }
-        stats.h2d_bytes += 2 * nw * sizeof(uint32_t);
-        CUDA_CHECK( cudaEventRecord( ev_phase_[0], stream_ ) );
-        CUDA_CHECK( launch_pair_score( req.algo, p, grid, stream_, nullptr ) );
-        launches_++;
-        CUDA_CHECK( cudaEventRecord( ev_phase_[1], stream_ ) );
-        std::vector<int32_t> sc( nw );
-        unsigned err = 0;
-        CUDA_CHECK( cudaMemcpyAsync( sc.data(), p.score, nw * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_ ) );
-        CUDA_CHECK( cudaMemcpyAsync( &err, p.error_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        if( err )
-            fatal( "Internal error in the GPU pair scores (flags 0x%x).", err );
-        stats.d2h_bytes += nw * sizeof(int32_t);
-        float ms = 0;
-        CUDA_CHECK( cudaEventElapsedTime( &ms, ev_phase_[0], ev_phase_[1] ) );
-        stats.entry_seconds += ms * 1e-3;
-        stats.kernel_seconds += ms * 1e-3;
-        if( timing )
-            fprintf( stderr, "[ssa timing] pair scores: %u pairs, %.3f ms\n", nw, ms );
-        for( uint32_t k = 0; k < nw; k++ ) {
-            const uint32_t i = work[k];
-            Hit h;
-            h.score = sc[k];
-            h.unit = units[i];
-            h.id = units[i] / db.upi;
-            h.q_index = 0;
-            out[i].push_back( h );
-        }
+    if( nw && !scores_in_traceback ) {
+        std::vector<std::pair<uint32_t, uint32_t>> lists;
+        for( uint32_t i = 0; i < n; i++ )
+            if( !out[i].empty() )
+                lists.emplace_back( i, i );
+        const auto t0 = std::chrono::steady_clock::now();
+        traceback( req, out, lists, stats, false, true );
+        const double seconds = std::chrono::duration<double>( std::chrono::steady_clock::now() - t0 ).count();
+        stats.entry_seconds += seconds;
+        stats.kernel_seconds += seconds;
     }
     if( req.align_type == COMPUTE_ALIGNMENT && nw ) {
         std::vector<std::pair<uint32_t, uint32_t>> lists;

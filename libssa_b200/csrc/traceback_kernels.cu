@@ -16,24 +16,32 @@
 //   4. the walk from the end cell with the priority I > D > M.
 //
 // Each pass is a wavefront on warps: lane k owns R query rows of a stripe of
-// 32 x R, database columns stream through the warp, the bottom row of a lane
-// goes to the next lane by shuffle, and the stripes of a hit follow one
-// another on different warps through the hit's boundary row
+// 32 x R, database columns stream through the warp in blocks of four, the bottom
+// row of a lane goes to the next lane by shuffle, and the stripes of a hit
+// follow one another on different warps through the hit's boundary row
 // (stream_stripes.cuh).  All arithmetic is exact (int32, with the host
-// guaranteeing the range), matching the reference's int64 code.
+// guaranteeing the range), matching the reference's int64 code.  The same sweep
+// without directions scores pairs of a query and one chosen sequence
+// (ssa_align_pairs): for a database of one sequence every entry width of the
+// reference reports the exact score.
 //
 // What bounds it: the integer ALU pipe (16 lanes per clock per SM
 // sub-partition) when many hits fill the GPU, the latency of one warp's steps
-// (columns + 64 x stripes of them per hit) when few do.  So R is 4 while all
-// stripes of 128 rows of a call can be resident at once (half the work per
-// step of R = 8, twice the warps), and 8 past that, where the fixed cost of a
-// step is spread over more cells.  Measured on a B200 against groups of 1, 2 or
-// 4 warps of one CTA per hit, whose stripes waited at a group barrier every 32
-// steps (one call each): 48 pairs of 5,000-30,000 residues, SW 780 -> 53 ms and
-// NW 470 -> 35 ms; 10 hits of 300 x 33,000 20.5 -> 9.3 ms; 320 hits of 30-1,355
-// rows 4.7 -> 1.3 ms; 4,096 long pairs, SW and NW, 6.4 -> 3.9 s.  A lane's scores of a column are one (two at
-// R = 8) shared-memory word of int8 entries, added to the diagonal by dp4a
-// (off the ALU pipe); tables past int8 are read entry by entry.
+// (blocks + 48 x stripes of them per hit) when few do.  A step interleaves the
+// four columns of a block row by row (cell (it - j, j) in iteration `it`): four
+// independent dependency chains where one column at a time has one, and the
+// step's fixed work (shuffles, residues, boundary, stores) once per 4 R cells.
+// R is 4: 8 rows per lane measured the same where hits fill the GPU (48 long
+// pairs 32 and 30 ms) and up to 1.7 times longer where they do not (half the
+// warps, twice the work per step).  A lane's scores of a column are one
+// shared-memory word of int8 entries, added to the diagonal by dp4a (off the ALU
+// pipe); tables past int8 are read entry by entry.
+//
+// Measured on a B200 (one call each): groups of 1, 2 or 4 warps of one CTA per
+// hit with a group barrier every 32 steps / streamed stripes, one column per
+// step / four columns per step: 48 pairs of 5,000-30,000 residues, SW 780 / 53 /
+// 42 ms and NW 470 / 35 / 24 ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 ms;
+// 320 hits of 30-1,355 rows 4.7 / 1.3 / 1.1 ms.
 #include "device_common.cuh"
 #include "stream_stripes.cuh"
 
@@ -41,20 +49,20 @@
 
 namespace ssa {
 
+constexpr int R = TB_ROWS_PER_LANE;                   // query rows per lane
 constexpr int TB_THREADS = 128;
 constexpr int TB_WARPS = TB_THREADS / 32;
 
 // What the stripe bodies share: the lane's rows and their scores.
-template <int R, bool P8>
+template <bool P8>
 struct TbLane {
-    static constexpr int WORDS = R / 4;
-    uint32_t * table;              // P8: the warp's scores, [code][lane][WORDS] words of four int8 entries
+    uint32_t * table;              // P8: the warp's scores, a word of four int8 entries per code and lane
     const int32_t * smat;          // the score table, [database code][query code]
     int lane;
     int32_t gO, gE, gOE;
     int qa[P8 ? 1 : R];            // !P8: query codes of the rows (0 past the end)
     int32_t H[R], E[R];
-    int32_t diag, out_h, out_f, row0;
+    int32_t diag, row0;
     int nvalid;                    // rows of this lane inside the query
 
     // rows first, first + step, ... of the codes `a`
@@ -66,17 +74,13 @@ struct TbLane {
         if constexpr( P8 ) {
             // every lane reads back its own entries only
             for( int d = 0; d < 32; d++ ) {
+                uint32_t v = 0;
 #pragma unroll
-                for( int w = 0; w < WORDS; w++ ) {
-                    uint32_t v = 0;
-#pragma unroll
-                    for( int b = 0; b < 4; b++ ) {
-                        const int r = 4 * w + b;
-                        const int32_t m = (r < nvalid) ? smat[(d << 5) + code[r]] : -128;
-                        v |= ((uint32_t) m & 0xffu) << (8 * b);
-                    }
-                    table[(d * 32 + lane) * WORDS + w] = v;
+                for( int r = 0; r < R; r++ ) {
+                    const int32_t m = (r < nvalid) ? smat[(d << 5) + code[r]] : -128;
+                    v |= ((uint32_t) m & 0xffu) << (8 * r);
                 }
+                table[d * 32 + lane] = v;
             }
         }
         else {
@@ -86,55 +90,31 @@ struct TbLane {
         }
     }
     struct Column {
-        uint32_t w[WORDS];
+        uint32_t w;
         const int32_t * m;
     };
     __device__ __forceinline__ Column scores( int d ) const {
-        Column c;
-        if constexpr( P8 ) {
-            if constexpr( WORDS == 2 ) {
-                const uint2 v = *reinterpret_cast<const uint2 *>( table + (d * 32 + lane) * 2 );
-                c.w[0] = v.x;
-                c.w[1] = v.y;
-            }
-            else {
-                c.w[0] = table[d * 32 + lane];
-            }
-            c.m = nullptr;
-        }
-        else {
-            c.m = smat + (d << 5);
-        }
-        return c;
+        if constexpr( P8 )
+            return Column{ table[d * 32 + lane], nullptr };
+        else
+            return Column{ 0, smat + (d << 5) };
     }
     // hd + score of row r in column c
     __device__ __forceinline__ int32_t add_score( const Column & c, int r, int32_t hd ) const {
         if constexpr( P8 )
-            return __dp4a( (int) c.w[r / 4], 1 << (8 * (r % 4)), hd );
+            return __dp4a( (int) c.w, 1 << (8 * r), hd );
         else
             return hd + c.m[qa[r]];
     }
 };
 
 // Largest of the lane's new cells.
-template <int R>
 __device__ __forceinline__ int32_t column_max( const int32_t (&x)[R] ) {
     int32_t m = x[0];
 #pragma unroll
     for( int r = 1; r + 1 < R; r += 2 )
         m = __vimax3_s32( m, x[r], x[r + 1] );
     return max( m, x[R - 1] );
-}
-
-// One wavefront step's direction flags of a lane: 2 bits per row, bit 1 =
-// insertion (LEFT | EXT_LEFT, takes priority), bit 0 = deletion (UP | EXT_UP).
-// A step's 32 lanes are contiguous: one transaction of 32 (R = 4) or 64 bytes.
-template <int R>
-__device__ __forceinline__ void store_flags( uint8_t * dir, uint32_t s, int lane, uint32_t flags ) {
-    if constexpr( R == 8 )
-        reinterpret_cast<uint16_t *>( dir )[(uint64_t) s * 32 + lane] = (uint16_t) flags;
-    else
-        dir[(uint64_t) s * 32 + lane] = (uint8_t) flags;
 }
 
 // The best end cell (value desc, database index asc, query index asc) or
@@ -157,7 +137,7 @@ __device__ __forceinline__ Cell warp_best( Cell c ) {
     return c;
 }
 
-// The reverse pass's limit: the first column that holds a candidate so far.
+// The reverse pass's limit: the first block that holds a candidate so far.
 template <bool REVERSE>
 struct ColumnLimit {
     static constexpr bool NONE = !REVERSE;
@@ -165,7 +145,7 @@ struct ColumnLimit {
     __device__ int32_t operator()() const { return *(volatile const int32_t *) p; }
 };
 
-enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR };
+enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR, TB_NW_DIRECTIONS, TB_SCORE, TB_NW_SCORE };
 
 // ---------------------------------------------------------------------------
 // The stripes of one pass over the hits.
@@ -184,9 +164,13 @@ enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR };
 //    column holding a candidate cannot change it, so that column is the hit's
 //    limit.
 //
-// TB_DIRECTIONS, the direction pass (reference: src/algo/cigar.c:48-198).
-//    Query rows on lanes, database columns streamed, exactly the reference
-//    orientation, rows 0 .. a_end and columns 0 .. b_end.
+// TB_DIRECTIONS and TB_NW_DIRECTIONS, the direction pass (reference:
+//    src/algo/cigar.c:48-198).  Query rows on lanes, database columns streamed,
+//    exactly the reference orientation, rows 0 .. a_end and columns 0 .. b_end.
+//
+// TB_SCORE and TB_NW_SCORE, the same recurrence without directions: the
+//    largest cell, or H of the last row and column
+//    (src/algo/64/smith_waterman_63.c:32-98, needleman_wunsch_64.c:32-98).
 //
 // TB_FWDDIR, both in one sweep of the whole matrix (Smith-Waterman, symmetric
 //    score table).  The direction pass's recurrence (reference:
@@ -202,15 +186,19 @@ enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR };
 //    where (B - 1) x gapE < gapO + gapE, so neither pass's initial term can be
 //    the maximum there.
 // ---------------------------------------------------------------------------
-template <int PHASE, int R, bool P8>
+template <int PHASE, bool P8>
 __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) {
     constexpr int ROWS = 32 * R;
-    constexpr bool DIRS = PHASE == TB_DIRECTIONS || PHASE == TB_FWDDIR;
+    constexpr int C = 4;
+    constexpr bool NW = PHASE == TB_NW_DIRECTIONS || PHASE == TB_NW_SCORE;
+    constexpr bool DIRS = PHASE == TB_DIRECTIONS || PHASE == TB_FWDDIR || PHASE == TB_NW_DIRECTIONS;
     constexpr bool ENDS = PHASE == TB_FORWARD || PHASE == TB_FWDDIR;       // looks for the end cell
-    __shared__ StreamStage<int2> stages[TB_WARPS];
-    __shared__ uint8_t residues[TB_WARPS][64];
+    constexpr bool MATRIX = ENDS || PHASE == TB_SCORE || PHASE == TB_NW_SCORE;     // every row and column
+    constexpr bool MAXIMUM = ENDS || PHASE == TB_SCORE;
+    constexpr bool REVERSE = PHASE == TB_REVERSE;
+    __shared__ StreamStage<int4> stages[TB_WARPS];
     __shared__ int32_t smat[1024];
-    __shared__ __align__( 16 ) uint32_t tables[P8 ? TB_WARPS : 1][P8 ? 32 * 32 * (R / 4) : 1];
+    __shared__ uint32_t tables[P8 ? TB_WARPS : 1][P8 ? 32 * 32 : 1];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     // laid out [database code][query code], so that the lanes of a warp (other
@@ -218,10 +206,10 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
     // matrix[query][db]
     for( int i = threadIdx.x; i < 1024; i += TB_THREADS ) {
         const int d = i >> 5, q = i & 31;
-        smat[i] = (int32_t) (DIRS ? p.matrix[(d << 5) + q] : p.matrix[(q << 5) + d]);
+        smat[i] = (int32_t) (PHASE == TB_FORWARD || REVERSE ? p.matrix[(q << 5) + d] : p.matrix[(d << 5) + q]);
     }
     __syncthreads();
-    StreamStage<int2> & st = stages[warp];
+    StreamStage<int4> & st = stages[warp];
 
     for( ;; ) {
         const uint32_t ticket = next_hit( p.counter, lane );
@@ -232,11 +220,10 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         const uint32_t pred = stripe ? p.cum[stripe - 1] + h : 0u;
         const TbHit hit = p.hits[h];
         const TbRegion rg = p.regions[h];
-        if( PHASE != TB_FORWARD && PHASE != TB_FWDDIR && rg.status != 0 )
+        if( !MATRIX && rg.status != 0 )
             continue;                                   // every stripe of the hit
-        const bool nw = hit.algo == 1;
         uint32_t A, B;
-        if constexpr( ENDS ) {
+        if constexpr( MATRIX ) {
             A = p.qlen[hit.qslot];
             B = p.db.lens[hit.id];
         }
@@ -247,18 +234,17 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         if( stripe * (uint32_t) ROWS >= A )
             continue;                                   // the reverse pass may need fewer rows than the query has
         const uint8_t * a = p.qcodes + p.qoff[hit.qslot];
+        const uint32_t nb = (B + 3u) >> 2;              // blocks of four columns
 
-        StreamStripe<int2> sp;
-        sp.cols = B;
+        StreamStripe<int4> sp;
+        sp.cols = nb;
         sp.row = p.boundary + p.bnd_off[h];
         sp.above = stripe ? p.progress + pred : nullptr;
         sp.mine = p.progress + ticket;
         sp.last = (stripe + 1u) * (uint32_t) ROWS >= A;
         sp.error_flags = p.error_flags;
-        ResidueRing rr{ residues[warp], 0, p.db.codes + p.db.offsets[hit.id], (int32_t) B,
-            PHASE == TB_REVERSE ? rg.b_end : -1 };
 
-        TbLane<R, P8> t;
+        TbLane<P8> t;
         t.table = tables[P8 ? warp : 0];
         t.smat = smat;
         t.lane = lane;
@@ -267,17 +253,14 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         t.gOE = p.gap_open + p.gap_extend;
         t.row0 = (int32_t) (stripe * (uint32_t) ROWS) + lane * R;
         t.nvalid = max( 0, min( R, (int) A - t.row0 ) );
-        t.out_h = 0;
-        t.out_f = 0;
-        t.diag = 0;
         const int32_t gO = t.gO, gE = t.gE, gOE = t.gOE, row0 = t.row0;
         int32_t * lh = nullptr;
         int32_t * le = nullptr;
-        if( ENDS || PHASE == TB_REVERSE ) {
+        if( ENDS || REVERSE ) {
             lh = p.last_h + p.last_off[h];
             le = p.last_e + p.last_off[h];
         }
-        if constexpr( PHASE == TB_REVERSE )
+        if constexpr( REVERSE )
             t.load_rows( a, (int64_t) rg.a_end - row0, -1 );
         else
             t.load_rows( a, row0, 1 );
@@ -287,7 +270,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 t.H[r] = 0;                             // HH[j] = 0
                 t.E[r] = gO + gE;                       // max(EE = gapO, HH + gapO) + gapE at row 0
             }
-            else if constexpr( PHASE == TB_REVERSE ) {
+            else if constexpr( REVERSE ) {
                 const int32_t j = rg.a_end - (row0 + r);    // query index
                 int32_t hh = -1, ee = -1;
                 if( r < t.nvalid && j > rg.b_end ) {
@@ -298,134 +281,200 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 t.E[r] = max( ee, hh + gO ) + gE;       // EE(b_end, j)
             }
             else {
+                // the reference's column before the first: H(i, -1), E(i, -1)
                 const int32_t i = row0 + r;
-                t.H[r] = nw ? gO + (i + 1) * gE : 0;
-                t.E[r] = nw ? 2 * gO + (i + 2) * gE : 0;
+                t.H[r] = NW ? gO + (i + 1) * gE : 0;
+                t.E[r] = NW ? 2 * gO + (i + 2) * gE : 0;
             }
         }
         // the diagonal of the lane's first row at column 0
-        if constexpr( PHASE == TB_REVERSE ) {
+        t.diag = 0;
+        if constexpr( REVERSE ) {
             // HH(b_end + 1, j + 1), or 0 for the end cell itself
             const int32_t jprev = rg.a_end - (row0 - 1);
             t.diag = (row0 == 0) ? 0 : ((jprev > rg.b_end && t.nvalid > 0) ? lh[jprev] : -1);
         }
-        else if constexpr( PHASE == TB_DIRECTIONS ) {
-            t.diag = (nw && row0 > 0) ? gO + row0 * gE : 0;
+        else if constexpr( NW ) {
+            t.diag = row0 > 0 ? gO + row0 * gE : 0;
         }
         // end cell: this lane's first maximum; begin cell: its first candidate (i = column, j = row)
         Cell best{ 0, INT_MAX, INT_MAX };
-        uint8_t * dir = nullptr;
+        uint32_t * dir = nullptr;
         if constexpr( DIRS )
-            dir = p.dirs + p.dir_off[h] + (uint64_t) stripe * ((uint64_t) B + 31) * (32 * R / 4);
+            dir = p.dirs + p.dir_off[h] + (uint64_t) stripe * ((uint64_t) nb + 31) * 32;
+        int32_t out_h[C] = {}, out_f[C] = {};
 
-        auto column = [&]( const uint32_t s, const bool edge, const uint32_t cols ) {
-            int32_t up_h = __shfl_up_sync( 0xffffffffu, t.out_h, 1 );
-            int32_t up_f = __shfl_up_sync( 0xffffffffu, t.out_f, 1 );
-            const int32_t c = (int32_t) s - lane;
-            if( edge && (c < 0 || c >= (int32_t) cols) )
+        // Residue words, two steps ahead of use: block b of the forward
+        // direction is word b.  The reverse pass reads columns b_end - 4b down
+        // to b_end - 4b - 3, which lie in the word of the last of them and the
+        // word after it (the previous block's).
+        const uint32_t * res = reinterpret_cast<const uint32_t *>( p.db.codes + p.db.offsets[hit.id] );
+        auto fetch = [&]( int32_t b ) -> uint32_t {
+            const int32_t w = REVERSE ? (rg.b_end - 4 * b - 3) >> 2 : b;
+            return (uint32_t) w < nb ? __ldg( res + w ) : 0u;
+        };
+        uint32_t before = REVERSE ? fetch( -lane - 1 ) : 0u, w0 = fetch( -lane ), w1 = fetch( 1 - lane );
+        const int32_t last_block = (int32_t) nb - 1, last_chain = (int32_t) (B - 1u) & 3;
+
+        auto block = [&]( const uint32_t s, const bool edge, const uint32_t blocks ) {
+            int32_t up_h[C], up_f[C];
+#pragma unroll
+            for( int j = 0; j < C; j++ ) {
+                up_h[j] = __shfl_up_sync( 0xffffffffu, out_h[j], 1 );
+                up_f[j] = __shfl_up_sync( 0xffffffffu, out_f[j], 1 );
+            }
+            const int32_t b = (int32_t) s - lane;
+            uint32_t word = w0;
+            if constexpr( REVERSE ) {
+                word = __byte_perm( __funnelshift_r( w0, before, 8u * ((uint32_t) (rg.b_end - 3) & 3u) ), 0, 0x0123 );
+                before = w0;
+            }
+            w0 = w1;
+            w1 = fetch( b + 2 );
+            if( edge && (b < 0 || b >= (int32_t) blocks) )
                 return;
             if( lane == 0 ) {
                 if( stripe == 0 ) {
-                    if constexpr( PHASE == TB_FORWARD ) {
-                        up_h = 0;
-                        up_f = gO + gE;                 // f starts at gapO: max(gapO, 0 + gapO) + gapE
-                    }
-                    else if constexpr( PHASE == TB_REVERSE ) {
-                        up_h = -1;                      // h starts at -1 per row; f = max(-1, h + gapO) + gapE
-                        up_f = max( -1, -1 + gO ) + gE;
-                    }
-                    else {
-                        // H(-1, c) is the next column's row-0 diagonal
-                        up_h = nw ? gO + (c + 1) * gE : 0;
-                        up_f = nw ? 2 * gO + (c + 2) * gE : 0;
+#pragma unroll
+                    for( int j = 0; j < C; j++ ) {
+                        if constexpr( PHASE == TB_FORWARD ) {
+                            up_h[j] = 0;
+                            up_f[j] = gO + gE;              // f starts at gapO: max(gapO, 0 + gapO) + gapE
+                        }
+                        else if constexpr( REVERSE ) {
+                            up_h[j] = -1;                   // h starts at -1 per row; f = max(-1, h + gapO) + gapE
+                            up_f[j] = max( -1, -1 + gO ) + gE;
+                        }
+                        else {
+                            // H(-1, c) (the next column's diagonal) and F entering row 0
+                            const int32_t c = 4 * b + j;
+                            up_h[j] = NW ? gO + (c + 1) * gE : 0;
+                            up_f[j] = NW ? 2 * gO + (c + 2) * gE : 0;
+                        }
                     }
                 }
                 else {
-                    const int2 v = st.in[s & 31u];
-                    up_h = v.x;
-                    up_f = v.y;
+                    const int4 x = st.in[2 * (s & 15u)], y = st.in[2 * (s & 15u) + 1];
+                    up_h[0] = x.x;
+                    up_f[0] = x.y;
+                    up_h[1] = x.z;
+                    up_f[1] = x.w;
+                    up_h[2] = y.x;
+                    up_f[2] = y.y;
+                    up_h[3] = y.z;
+                    up_f[3] = y.w;
                 }
             }
-            const auto sc = t.scores( rr.get( s, lane ) );
-            int32_t f = up_f, hd = t.diag;
-            int32_t x[R];
+            typename TbLane<P8>::Column sc[C];
+            int32_t f[C], hv[C][R];
+            // 2 bits per cell (bit 1 = insertion, LEFT | EXT_LEFT, takes priority;
+            // bit 0 = deletion, UP | EXT_UP), a byte per column
             uint32_t flags = 0;
-            const bool last_col = ENDS && edge && c == (int32_t) B - 1;
 #pragma unroll
-            for( int r = 0; r < R; r++ ) {
-                const int32_t e = t.E[r];
-                const int32_t x0 = t.add_score( sc, r, hd );
-                hd = t.H[r];
-                if constexpr( DIRS ) {
-                    // flags as in the reference (strict compares in its
-                    // order): each max also yields the negation of one
-                    bool no_up, no_left, no_ext_up, no_ext_left;
-                    const int32_t m1 = __vibmax_s32( x0, f, &no_up );       // UP: f > x0
-                    const int32_t xr = __vibmax_s32( m1, e, &no_left );     // LEFT: e > max(x0, f)
-                    x[r] = (PHASE == TB_DIRECTIONS && nw) ? xr : max( xr, 0 );
-                    const int32_t y = x[r] + gOE;
-                    f = __vibmax_s32( y, f + gE, &no_ext_up );               // EXT_UP: f + gapE > y
-                    t.E[r] = __vibmax_s32( y, e + gE, &no_ext_left );        // EXT_LEFT: e + gapE > y
-                    // rows past the query's end get flags too; the walk never reads them
-                    if( !(no_left && no_ext_left) )
-                        flags |= 2u << (2 * r);
-                    if( !(no_up && no_ext_up) )
-                        flags |= 1u << (2 * r);
-                }
-                else {
-                    x[r] = PHASE == TB_FORWARD ? __vimax3_s32( max( x0, 0 ), f, e ) : __vimax3_s32( x0, f, e );
-                    const int32_t y = x[r] + gOE;
-                    f = __viaddmax_s32( f, gE, y );
-                    t.E[r] = __viaddmax_s32( e, gE, y );
-                }
-                t.H[r] = x[r];
-                if( last_col && r < t.nvalid ) {
-                    lh[row0 + r] = x[r];
-                    le[row0 + r] = e;
+            for( int j = 0; j < C; j++ ) {
+                sc[j] = t.scores( (int) ((word >> (8 * j)) & 0xffu) );
+                f[j] = up_f[j];
+            }
+            const bool last_col = ENDS && edge && b == last_block;
+            // chain j is column j of the block; H[r] keeps the column before the
+            // block until chain 3 overwrites it, E[r] passes from chain to chain
+#pragma unroll
+            for( int it = 0; it < R + C - 1; it++ ) {
+#pragma unroll
+                for( int j = 0; j < C; j++ ) {
+                    const int r = it - j;
+                    if( r < 0 || r >= R )
+                        continue;
+                    const int32_t e = t.E[r];
+                    const int32_t hd = r == 0 ? (j == 0 ? t.diag : up_h[j - 1]) : (j == 0 ? t.H[r - 1] : hv[j - 1][r - 1]);
+                    const int32_t x0 = t.add_score( sc[j], r, hd );
+                    int32_t x;
+                    if constexpr( DIRS ) {
+                        // flags as in the reference (strict compares in its
+                        // order): each max also yields the negation of one
+                        bool no_up, no_left, no_ext_up, no_ext_left;
+                        const int32_t m1 = __vibmax_s32( x0, f[j], &no_up );       // UP: f > x0
+                        const int32_t xr = __vibmax_s32( m1, e, &no_left );        // LEFT: e > max(x0, f)
+                        x = NW ? xr : max( xr, 0 );
+                        const int32_t y = x + gOE;
+                        f[j] = __vibmax_s32( y, f[j] + gE, &no_ext_up );            // EXT_UP: f + gapE > y
+                        t.E[r] = __vibmax_s32( y, e + gE, &no_ext_left );           // EXT_LEFT: e + gapE > y
+                        // rows past the query's end get flags too; the walk never reads them
+                        if( !(no_left && no_ext_left) )
+                            flags |= 2u << (8 * j + 2 * r);
+                        if( !(no_up && no_ext_up) )
+                            flags |= 1u << (8 * j + 2 * r);
+                    }
+                    else {
+                        x = PHASE == TB_FORWARD || PHASE == TB_SCORE ? __vimax3_s32( max( x0, 0 ), f[j], e )
+                                                                     : __vimax3_s32( x0, f[j], e );
+                        const int32_t y = x + gOE;
+                        f[j] = __viaddmax_s32( f[j], gE, y );
+                        t.E[r] = __viaddmax_s32( e, gE, y );
+                    }
+                    hv[j][r] = x;
+                    if( last_col && j == last_chain && r < t.nvalid ) {
+                        lh[row0 + r] = x;
+                        le[row0 + r] = e;
+                    }
+                    if( j == C - 1 )
+                        t.H[r] = x;
                 }
             }
             if constexpr( DIRS )
-                store_flags<R>( dir, s, lane, flags );
-            if constexpr( ENDS ) {
+                dir[(uint64_t) s * 32 + lane] = flags;     // one transaction of 128 bytes per step
+            if constexpr( MAXIMUM || REVERSE ) {
                 // the lane visits its cells in (column, row) order: its first
-                // maximum wins with a strict compare, and rarely is there one
-                if( column_max<R>( x ) > best.v ) {
+                // maximum (its first candidate) counts, and rarely is there one
+                int32_t most = column_max( hv[0] );
 #pragma unroll
-                    for( int r = 0; r < R; r++ )
-                        if( r < t.nvalid && x[r] > best.v )
-                            best = Cell{ x[r], c, row0 + r };
+                for( int j = 1; j < C; j++ )
+                    most = max( most, column_max( hv[j] ) );
+                if( MAXIMUM && most > best.v ) {
+#pragma unroll
+                    for( int j = 0; j < C; j++ )
+#pragma unroll
+                        for( int r = 0; r < R; r++ )
+                            if( r < t.nvalid && 4 * b + j < (int32_t) B && hv[j][r] > best.v )
+                                best = Cell{ hv[j][r], 4 * b + j, row0 + r };
                 }
-            }
-            if constexpr( PHASE == TB_REVERSE ) {
-                if( column_max<R>( x ) >= rg.fwd_score && best.i == INT_MAX ) {
+                if( REVERSE && most >= rg.fwd_score && best.i == INT_MAX ) {
 #pragma unroll
-                    for( int r = R - 1; r >= 0; r-- )
-                        if( r < t.nvalid && x[r] >= rg.fwd_score )
-                            best = Cell{ 0, c, row0 + r };
+                    for( int j = 0; j < C; j++ )
+#pragma unroll
+                        for( int r = 0; r < R; r++ )
+                            if( r < t.nvalid && 4 * b + j < (int32_t) B && hv[j][r] >= rg.fwd_score &&
+                                    best.i == INT_MAX )
+                                best = Cell{ 0, 4 * b + j, row0 + r };
                     if( best.i != INT_MAX )
-                        atomicMin( p.limit + h, c );
+                        atomicMin( p.limit + h, b );
                 }
             }
-            if constexpr( PHASE == TB_DIRECTIONS ) {
-                if( nw && edge && c == (int32_t) B - 1 ) {
+            if constexpr( NW ) {
+                if( edge && sp.last && b == last_block ) {
                     // the global score: the last cell of the full matrix
 #pragma unroll
-                    for( int r = 0; r < R; r++ )
-                        if( row0 + r == (int32_t) A - 1 )
-                            p.regions[h].fwd_score = x[r];
+                    for( int j = 0; j < C; j++ )
+#pragma unroll
+                        for( int r = 0; r < R; r++ )
+                            if( j == last_chain && row0 + r == (int32_t) A - 1 )
+                                p.regions[h].fwd_score = hv[j][r];
                 }
             }
-            t.diag = up_h;
-            t.out_h = x[R - 1];
-            t.out_f = f;
-            if( lane == 31 )
-                st.out[s & 31u] = make_int2( t.out_h, t.out_f );
+            t.diag = up_h[C - 1];
+#pragma unroll
+            for( int j = 0; j < C; j++ ) {
+                out_h[j] = hv[j][R - 1];
+                out_f[j] = f[j];
+            }
+            if( lane == 31 ) {
+                st.out[2 * (s & 15u)] = make_int4( out_h[0], out_f[0], out_h[1], out_f[1] );
+                st.out[2 * (s & 15u) + 1] = make_int4( out_h[2], out_f[2], out_h[3], out_f[3] );
+            }
         };
-        rr.start( lane );
-        const ColumnLimit<PHASE == TB_REVERSE> limit{ p.limit + h };
-        const uint32_t swept = stream_columns<32>( sp, st, lane, limit, [&]( uint32_t s0 ) { rr.step( s0, lane ); },
-                column );
-        if constexpr( PHASE != TB_DIRECTIONS ) {
+        const ColumnLimit<REVERSE> limit{ p.limit + h };
+        const uint32_t swept = stream_columns<16>( sp, st, lane, limit, []( uint32_t ) {}, block );
+        if constexpr( MAXIMUM || REVERSE ) {
             // this stripe's cell against that of the stripes above (theirs is
             // final once the stripe above has ended)
             best = warp_best( best );
@@ -440,7 +489,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 if( !sp.last ) {
                     __stcg( p.result + ticket, make_int4( best.v, best.i, best.j, 0 ) );
                 }
-                else if constexpr( ENDS ) {
+                else if constexpr( MAXIMUM ) {
                     TbRegion out = rg;                  // the host set the rest of the region; keep it
                     out.fwd_score = best.v;
                     out.a_end = best.j;
@@ -470,19 +519,22 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
 // ---------------------------------------------------------------------------
 // 4. Walk (reference: src/algo/cigar.c:300-334): one warp per hit writes the
 //    moves in traceback order (end to begin); the host run-length encodes.
-//    Each step reads the direction word of the current cell, which the
+//    Each step reads the direction bits of the current cell, which the
 //    previous step chose, so a walk that reads HBM or L2 word by word waits a
-//    memory round trip per move.  In 32 moves the path stays within 32 rows
-//    and 32 columns of its current cell (every move leaves the row or the
-//    column or both by one), so the warp loads that window (32 columns, at
-//    most 9 bytes of 4 rows each) into shared memory with one load round,
-//    lane 0 walks up to 32 moves from it, and the warp loads the next window.
+//    memory round trip per move.  In 64 moves the path stays within 64 rows
+//    and 64 columns of its current cell (every move leaves the row or the
+//    column or both by one), so the warp loads that window (at most 17 x 17
+//    words of 4 x 4 cells, ten loads per lane in flight together) into shared
+//    memory, lane 0 walks up to 64 moves from it, and the warp loads the next
+//    window.  Paths of 20,000 moves, 48 hits: 4.6 -> 2.3 ms against windows of 32 moves.
 // ---------------------------------------------------------------------------
 constexpr int TB_WALK_WARPS = 4;                 // hits per CTA
-constexpr int TB_WALK_GROUPS = 32 / 4 + 1;       // bytes of four rows that a 32-row window spans
+constexpr int TB_WALK_MOVES = 64;
+constexpr int TB_WALK_WORDS = TB_WALK_MOVES / 4 + 1;     // words that a window spans in either direction
 
-__global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams p, int R ) {
-    __shared__ uint8_t win[TB_WALK_WARPS][32][TB_WALK_GROUPS + 3];
+__global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams p ) {
+    constexpr int ROWS = 32 * R, W = TB_WALK_WORDS;
+    __shared__ uint32_t win[TB_WALK_WARPS][W * W];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const uint32_t h = blockIdx.x * TB_WALK_WARPS + (uint32_t) wib;
@@ -494,35 +546,37 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
             p.ops_len[h] = 0;
         return;
     }
-    const uint8_t * dir = p.dirs + p.dir_off[h];
+    const uint32_t * dir = p.dirs + p.dir_off[h];
     char * out = p.ops + p.ops_off[h];
     const uint64_t cap = p.ops_off[h + 1] - p.ops_off[h];
     const int32_t a_begin = rg.a_begin, b_begin = rg.b_begin;
-    const int stripe_rows = 32 * R, lane_bytes = R / 4;
-    const uint64_t stripe_bytes = (uint64_t) rg.dir_steps * 32 * lane_bytes;
+    const uint64_t stripe_words = (uint64_t) rg.dir_steps * 32;
     int32_t i = rg.a_end, j = rg.b_end;
     uint64_t n = 0;
     while( i >= a_begin && j >= b_begin && i >= 0 && j >= 0 ) {
-        // the window: columns j - 31 .. j, groups of four rows that hold i - 31 .. i
-        const int32_t g0 = max( i - 31, 0 ) / 4;
-        const int32_t jc = j - lane;
+        // the window: word (y, x) holds rows 4 (i / 4 - y) .. + 3 of columns 4 (j / 4 - x) .. + 3
+        const int32_t i4 = i / 4, j4 = j / 4;
+        uint32_t v[(W * W + 31) / 32];
 #pragma unroll
-        for( int k = 0; k < TB_WALK_GROUPS; k++ ) {
-            const int32_t row = 4 * (g0 + k);
-            uint8_t v = 0;
-            if( jc >= b_begin && row <= i ) {
-                const int32_t in_stripe = row % stripe_rows;
-                const int32_t owner = in_stripe / R;           // the row's lane, at step jc + owner
-                v = dir[(uint64_t) (row / stripe_rows) * stripe_bytes +
-                        ((uint64_t) (jc + owner) * 32 + owner) * lane_bytes + (in_stripe % R) / 4];
+        for( int k = 0; k < (W * W + 31) / 32; k++ ) {
+            const int t = lane + 32 * k;
+            const int32_t row = 4 * (i4 - t / W), blk = j4 - t % W;
+            v[k] = 0;
+            if( t < W * W && row >= 0 && blk >= 0 ) {
+                const int32_t owner = (row % ROWS) / R;        // the rows' lane, at step blk + owner
+                v[k] = dir[(uint64_t) (row / ROWS) * stripe_words +
+                        (uint64_t) (blk + owner) * 32 + owner];
             }
-            win[wib][lane][k] = v;
         }
         __syncwarp();
+#pragma unroll
+        for( int k = 0; k < (W * W + 31) / 32; k++ )
+            if( lane + 32 * k < W * W )
+                win[wib][lane + 32 * k] = v[k];
+        __syncwarp();
         if( lane == 0 ) {
-            const int32_t j0 = j;
-            for( int m = 0; m < 32 && i >= a_begin && j >= b_begin && i >= 0 && j >= 0; m++ ) {
-                const uint32_t op = ((uint32_t) win[wib][j0 - j][i / 4 - g0] >> (2 * (i % 4))) & 3u;
+            for( int m = 0; m < TB_WALK_MOVES && i >= a_begin && j >= b_begin && i >= 0 && j >= 0; m++ ) {
+                const uint32_t op = (win[wib][(i4 - i / 4) * W + (j4 - j / 4)] >> (8 * (j % 4) + 2 * (i % 4))) & 3u;
                 char ch;
                 if( op & 2u ) {
                     j--;
@@ -545,52 +599,53 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
         i = __shfl_sync( 0xffffffffu, i, 0 );
         j = __shfl_sync( 0xffffffffu, j, 0 );
         n = __shfl_sync( 0xffffffffu, n, 0 );
-        __syncwarp();
     }
     if( lane == 0 )
         p.ops_len[h] = (uint32_t) n;
 }
 
-cudaError_t launch_tb_walk( const TbParams & p, int R, cudaStream_t st ) {
+cudaError_t launch_tb_walk( const TbParams & p, cudaStream_t st ) {
     if( p.n_hits )
-        tb_walk_kernel<<<(p.n_hits + TB_WALK_WARPS - 1) / TB_WALK_WARPS, 32 * TB_WALK_WARPS, 0, st>>>( p, R );
+        tb_walk_kernel<<<(p.n_hits + TB_WALK_WARPS - 1) / TB_WALK_WARPS, 32 * TB_WALK_WARPS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
-template <int PHASE, int R, bool P8>
+template <int PHASE, bool P8>
 static cudaError_t launch_stripes( const TbParams & p, int sms, cudaStream_t st ) {
     static LaunchShape shape;
-    const cudaError_t e = shape.set( tb_stripes_kernel<PHASE, R, P8>, TB_THREADS, 0 );
+    const cudaError_t e = shape.set( tb_stripes_kernel<PHASE, P8>, TB_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
     const uint32_t want = (p.n_tickets + TB_WARPS - 1) / TB_WARPS;
     const uint32_t grid = min( want, (uint32_t) (sms * max( 1, shape.blocks )) );
     if( grid )
-        tb_stripes_kernel<PHASE, R, P8><<<grid, TB_THREADS, 0, st>>>( p );
+        tb_stripes_kernel<PHASE, P8><<<grid, TB_THREADS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
 template <int PHASE>
-static cudaError_t launch_phase( const TbParams & p, int R, bool p8, int sms, cudaStream_t st ) {
-    if( R == 4 )
-        return p8 ? launch_stripes<PHASE, 4, true>( p, sms, st ) : launch_stripes<PHASE, 4, false>( p, sms, st );
-    return p8 ? launch_stripes<PHASE, 8, true>( p, sms, st ) : launch_stripes<PHASE, 8, false>( p, sms, st );
+static cudaError_t launch_phase( const TbParams & p, bool p8, int sms, cudaStream_t st ) {
+    return p8 ? launch_stripes<PHASE, true>( p, sms, st ) : launch_stripes<PHASE, false>( p, sms, st );
 }
 
-cudaError_t launch_tb_forward( const TbParams & p, int R, bool p8, int sms, cudaStream_t st ) {
-    return launch_phase<TB_FORWARD>( p, R, p8, sms, st );
+cudaError_t launch_tb_forward( const TbParams & p, bool p8, int sms, cudaStream_t st ) {
+    return launch_phase<TB_FORWARD>( p, p8, sms, st );
 }
 
-cudaError_t launch_tb_reverse( const TbParams & p, int R, bool p8, int sms, cudaStream_t st ) {
-    return launch_phase<TB_REVERSE>( p, R, p8, sms, st );
+cudaError_t launch_tb_reverse( const TbParams & p, bool p8, int sms, cudaStream_t st ) {
+    return launch_phase<TB_REVERSE>( p, p8, sms, st );
 }
 
-cudaError_t launch_tb_directions( const TbParams & p, int R, bool p8, int sms, cudaStream_t st ) {
-    return launch_phase<TB_DIRECTIONS>( p, R, p8, sms, st );
+cudaError_t launch_tb_directions( const TbParams & p, bool nw, bool p8, int sms, cudaStream_t st ) {
+    return nw ? launch_phase<TB_NW_DIRECTIONS>( p, p8, sms, st ) : launch_phase<TB_DIRECTIONS>( p, p8, sms, st );
 }
 
-cudaError_t launch_tb_fwddir( const TbParams & p, int R, bool p8, int sms, cudaStream_t st ) {
-    return launch_phase<TB_FWDDIR>( p, R, p8, sms, st );
+cudaError_t launch_tb_fwddir( const TbParams & p, bool p8, int sms, cudaStream_t st ) {
+    return launch_phase<TB_FWDDIR>( p, p8, sms, st );
+}
+
+cudaError_t launch_tb_scores( const TbParams & p, bool nw, bool p8, int sms, cudaStream_t st ) {
+    return nw ? launch_phase<TB_NW_SCORE>( p, p8, sms, st ) : launch_phase<TB_SCORE>( p, p8, sms, st );
 }
 
 }  // namespace ssa

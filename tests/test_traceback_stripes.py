@@ -1,12 +1,12 @@
-"""Traceback passes on streamed stripes, 4 and 8 rows per lane: queries around
-the stripe edges (128 and 256 rows), columns around the 32-column chunks, score
+"""Traceback passes on streamed stripes: queries around the stripe edges (128 and
+256 rows), columns around the 4-column blocks and 16-block chunks, score
 tables inside and past int8, symmetric and not, against the oracle: scores,
 order, CIGARs and coordinates."""
 import numpy as np
 import pytest
 
 import oracle
-from helpers import product_search, product_setup
+from helpers import matrix_table, product_search, product_setup
 from libssa_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -24,13 +24,11 @@ def _matrix_text(scale: int, symmetric: bool, rng) -> str:
                                               for i in range(20)]) + "\n"
 
 
-@pytest.mark.parametrize("rows", [4, 8])
 @pytest.mark.parametrize("algo,scale,symmetric", [("sw", 1, True), ("sw", 40, True), ("sw", 1, False), ("nw", 1, True),
                                                   ("nw", 40, False)])
-def test_stripe_edges(built_library, monkeypatch, rows, algo, scale, symmetric):
+def test_stripe_edges(built_library, algo, scale, symmetric):
     import libssa_b200 as L
-    monkeypatch.setenv("SSA_B200_TB_R", str(rows))
-    rng = np.random.default_rng(100 * scale + rows)
+    rng = np.random.default_rng(100 * scale + 4)
     text = _matrix_text(scale, symmetric, rng)
     table = oracle.parse_matrix(text)
     gap = (-11 * scale if scale == 1 else -120, -1 * scale)
@@ -49,3 +47,25 @@ def test_stripe_edges(built_library, monkeypatch, rows, algo, scale, symmetric):
         res, _ = oracle.search(cfg, oracle.map_codes(q.decode(), False, True), db)
         exp = [(h.id, h.score, h.cigar, h.q_start, h.q_end, h.d_start, h.d_end) for h in res]
         assert got[qi] == exp, (qi, len(q))
+
+
+@pytest.mark.parametrize("algo", ["sw", "nw"])
+def test_pair_scores(built_library, algo):
+    """Scores of pairs without alignments on the same sweep."""
+    import libssa_b200 as L
+    rng = np.random.default_rng(7)
+    records = [W.random_residues(rng, n, W.AA20) for n in (1, 2, 3, 4, 5, 63, 64, 65, 127, 130, 700, 2500)]
+    queries = [W.mutate(rng, np.tile(r, 2), W.AA20, 0.2, 0.05, (1, 4)) for r in records]
+    queries = [q if len(q) else records[5] for q in queries]
+    product_setup(1, ("builtin", "blosum62"), (-11, -1), 1000, 2, records=[r.tobytes() for r in records])
+    qs = [L.init_sequence_fasta(L.READ_FROM_STRING, q.tobytes().decode()) for q in queries]
+    got = L.align_pairs(L.SSA_SMITH_WATERMAN if algo == "sw" else L.SSA_NEEDLEMAN_WUNSCH, qs, list(range(len(qs))), 16,
+                        L.COMPUTE_SCORE)
+    for q in qs:
+        L.free_sequence(q)
+    for i, (q, r) in enumerate(zip(queries, records)):
+        cfg = oracle.SearchConfig(algo=algo, bit_width=64, align_type=0, hitcount=1, chunk_size=1000, gap_open=-11,
+                                  gap_extend=-1, lanes8=32, lanes16=16, matrix=matrix_table(("builtin", "blosum62")))
+        res, _ = oracle.search(cfg, oracle.map_codes(q.tobytes().decode(), False, True),
+                               [oracle.map_codes(r.tobytes().decode(), False, False)])
+        assert [h.score for h in got[i]] == [h.score for h in res], (i, len(q), len(r))
