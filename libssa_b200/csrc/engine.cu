@@ -569,8 +569,10 @@ private:
     void run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, uint32_t cap,
             std::vector<PairTask> & list_entry, std::vector<PairTask> & list_16, const std::vector<uint32_t> * slots,
             uint32_t lo, uint32_t hi );
-    void run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap,
-            const PairTask * redo_list );
+    static constexpr size_t LIST_HEAD = 1024;
+    const unsigned * read_counts( bool head, void * scores_to = nullptr, size_t score_bytes = 0 );
+    const unsigned * run_redo( const SearchRequest & req, uint32_t nq, const unsigned * c, PairTask * next,
+            unsigned * next_count, uint32_t cap, const PairTask * redo_list, uint32_t redo_cap );
     int32_t * score_sink() { return serving_ ? d_serve_score_.as<int32_t>() : d_score_.as<int32_t>(); }
     void build_profiles( int width, uint32_t n_slots );
     // scores_from_regions: the hits carry no score yet; take it from the
@@ -615,6 +617,7 @@ private:
     bool serve_layout_ = false;      // the query buffers hold the serving slots
     uint32_t serve_slots_ = 0;
     std::vector<std::vector<uint8_t>> serve_codes_;   // per slot, to restore the layout after a search
+    std::vector<uint32_t> serve_new_;                 // slots whose query the device does not have yet
     cudaStream_t class_stream_[4] = { nullptr, nullptr, nullptr, nullptr };
     cudaEvent_t ev_class_[4] = { nullptr, nullptr, nullptr, nullptr };
     cudaEvent_t ev_cls_t_[8] = {};   // per class start / end, timed (SSA_B200_TIMING)
@@ -1129,8 +1132,6 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         CUDA_CHECK( cudaStreamWaitEvent( stream_, ev_class_[ri], 0 ) );
         class_first += cls.size();
     }
-    if( req.bit_width != 8 )
-        run_redo( req, nq, next, next_count, cap, d_list_b_.as<PairTask>() );
     if( !fallback.empty() ) {
         const uint64_t n_ne = db_.order_desc.size();
         run_pass( 0, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_ne, true, next, next_count, cap,
@@ -1231,17 +1232,32 @@ static int choose_qpair_rows( uint32_t Q, uint32_t * passes, int pinned, int buc
     return best_r;
 }
 
-// The pairs that a 16x2 entry pass left out of its range (16- and 64-bit
-// entry): the lane emulation at the entry width.
-void Engine::run_redo( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count, uint32_t cap,
-        const PairTask * redo_list ) {
-    unsigned n_redo = 0;
-    CUDA_CHECK( cudaMemcpyAsync( &n_redo, d_counts_.as<unsigned>() + 5, sizeof(unsigned), cudaMemcpyDeviceToHost,
-            stream_ ) );
+// The counters of a pass on the host: [0] re-queued pairs, [1] those of the
+// 16-bit pass, [2] error flags, [5] pairs for the lane emulation.  head: also
+// the first entries of list A, which are all of them in most calls, and
+// (scores_to) that many bytes of scores.  One wait for all.
+const unsigned * Engine::read_counts( bool head, void * scores_to, size_t score_bytes ) {
+    unsigned * c = (unsigned *) h_counts_.ensure( 64 + LIST_HEAD * sizeof(PairTask) );
+    CUDA_CHECK( cudaMemcpyAsync( c, d_counts_.p, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
+    if( head )
+        CUDA_CHECK( cudaMemcpyAsync( (char *) c + 64, d_list_a_.p,
+                std::min<size_t>( d_list_a_.bytes, LIST_HEAD * sizeof(PairTask) ), cudaMemcpyDeviceToHost, stream_ ) );
+    if( scores_to )
+        CUDA_CHECK( cudaMemcpyAsync( scores_to, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
     CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-    n_redo = std::min( n_redo, cap );
-    if( n_redo )
-        run_pass( req.algo, req.bit_width, req, nq, redo_list, n_redo, false, next, next_count, cap );
+    return c;
+}
+
+// The pairs that the 16x2 kernels left out of their range (16- and 64-bit
+// passes), by the lane emulation.  c: the pass's counters; returns them as they
+// are afterwards.
+const unsigned * Engine::run_redo( const SearchRequest & req, uint32_t nq, const unsigned * c, PairTask * next,
+        unsigned * next_count, uint32_t cap, const PairTask * redo_list, uint32_t redo_cap ) {
+    const uint32_t n_redo = std::min( c[5], redo_cap );
+    if( req.bit_width == 8 || n_redo == 0 )
+        return c;
+    run_pass( req.algo, req.bit_width, req, nq, redo_list, n_redo, false, next, next_count, cap );
+    return read_counts( true );
 }
 
 void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
@@ -1577,8 +1593,6 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
                     cells / (ms * 1e-3) / 1e9 );
         }
     }
-    if( redo )
-        run_redo( req, nq, next, next_count, cap, redo_list );
     if( !fallback.empty() ) {
         const uint32_t * dev_slots = stage_.add( fallback.data(), fallback.size(), stream_ );
         run_pass( req.algo, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_seq, true, next,
@@ -1677,8 +1691,11 @@ void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, 
     PairTask * list_b = d_list_b_.as<PairTask>();
     const size_t first = list_entry.size();
     list_entry.resize( first + n_a );
-    CUDA_CHECK( cudaMemcpyAsync( list_entry.data() + first, list_a, n_a * sizeof(PairTask), cudaMemcpyDeviceToHost,
-            stream_ ) );
+    if( n_a <= LIST_HEAD )              // came with the counters
+        memcpy( list_entry.data() + first, (const char *) h_counts_.p + 64, n_a * sizeof(PairTask) );
+    else
+        CUDA_CHECK( cudaMemcpyAsync( list_entry.data() + first, list_a, n_a * sizeof(PairTask), cudaMemcpyDeviceToHost,
+                stream_ ) );
     if( req.bit_width != 8 ) {
         run_pass( req.algo, 64, req, nq, list_a, n_a, false, nullptr, cnt + 3, 0 );
         CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the host list
@@ -1690,10 +1707,12 @@ void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, 
     r16.bit_width = 16;
     const bool queries_fit = max_qlen_ <= FAST_MAX_ROWS;
     const uint64_t searched = (uint64_t) (slots ? slots->size() : nq) * (hi - lo);
+    PairTask * redo = nullptr;
     if( fast_single_eligible( r16 ) ) {
-        PairTask * redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
+        redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
         CUDA_CHECK( cudaMemsetAsync( cnt + 5, 0, sizeof(unsigned), stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );     // the host list
+        if( n_a > LIST_HEAD )
+            CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
         // the re-queued sequences of a query, longest first, in pairs
         std::vector<PairTask> tasks( list_entry.begin() + first, list_entry.end() );
         std::sort( tasks.begin(), tasks.end(), [&]( const PairTask & a, const PairTask & b ) {
@@ -1712,22 +1731,21 @@ void Engine::run_cascade( const SearchRequest & req, uint32_t nq, uint32_t n_a, 
         lists.redo_count = cnt + 5;
         lists.redo_cap = n_a;
         run_stream( r16, items, lists, stream_ );
-        run_redo( r16, nq, list_b, cnt + 1, cap, redo );
     }
     else if( nw_fast_eligible( r16 ) && queries_fit && n_a >= searched / 4 ) {
         // most pairs overflowed: the query-pair kernel over all of them, which
         // scores the marked ones.  It computes a pair an order of magnitude
         // faster than the emulation of the list, so it wins from a quarter on.
-        PairTask * redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
+        redo = (PairTask *) d_list_c_.ensure( (size_t) n_a * sizeof(PairTask) );
         run_qpair_entry( r16, nq, list_b, cnt + 1, std::min( cap, n_a ), redo, slots, lo, hi, true );
     }
     else {
         run_pass( req.algo, 16, req, nq, list_a, n_a, false, list_b, cnt + 1, cap );
     }
-    unsigned n_b = 0;
-    CUDA_CHECK( cudaMemcpyAsync( &n_b, cnt + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-    n_b = std::min( n_b, cap );
+    const unsigned * c = read_counts( false );
+    if( redo )
+        c = run_redo( r16, nq, c, list_b, cnt + 1, cap, redo, n_a );
+    const uint32_t n_b = std::min( c[1], cap );
     if( n_b ) {
         const size_t at = list_16.size();
         list_16.resize( at + n_b );
@@ -1818,6 +1836,7 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         // nothing was re-queued, and the call then waits for the device once
         int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
         const bool early = !streaming_ && !wide_ && score_bytes && score_bytes <= ((size_t) 1 << 20);
+        bool redone = false;    // scores written after the entry pass's
         float entry_ms = 0;     // the entry passes of all segments
         // a resident database is one segment; a streamed one runs the entry pass
         // and the cascade of each segment while it is on the device
@@ -1846,13 +1865,13 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
             run_entry();
             uint32_t n_req = 0;     // pairs the entry pass re-queued
             for( ;; ) {
-                // counts of the entry list and the NW redo list (their atomic
-                // counters count every append, kept or not) and the error flags
-                unsigned * c = (unsigned *) h_counts_.ensure( 6 * sizeof(unsigned) );
-                CUDA_CHECK( cudaMemcpyAsync( c, cnt, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-                if( early )
-                    CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
-                CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+                // the counters of the entry list and the redo list count every
+                // append, kept or not
+                const unsigned * c = read_counts( true, early ? hs : nullptr, score_bytes );
+                if( std::max( c[0], c[5] ) <= cap && !(c[2] & ERR_REQUEUE_OVERFLOW) && c[5] ) {
+                    c = run_redo( req, nq, c, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), cap );
+                    redone = true;
+                }
                 const uint64_t need = std::max<uint64_t>( c[0], c[5] );
                 if( need <= cap && !(c[2] & ERR_REQUEUE_OVERFLOW) ) {
                     n_req = c[0];
@@ -1878,7 +1897,7 @@ void Engine::search( const SearchRequest & req, const std::vector<QueryCodes> & 
         CUDA_CHECK( cudaEventRecord( ev_phase_[2], stream_ ) );
         const uint64_t n_a = list_entry.size(), n_b = list_16.size();
         stats.d2h_bytes += score_bytes + (n_a + n_b) * sizeof(PairTask);
-        const bool have_scores = early && n_a == 0;
+        const bool have_scores = early && n_a == 0 && !redone;
         if( score_bytes && !have_scores )
             CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
         int64_t * hs64 = nullptr;
@@ -2564,14 +2583,10 @@ void Engine::shard_scores( const SearchRequest & req, const std::vector<QueryCod
                     cnt + 0, cap );
         CUDA_CHECK( cudaEventRecord( ev_seg_[1], stream_ ) );
         std::vector<PairTask> list_entry, list_16;
-        unsigned sa = 0;
-        if( entry != 64 ) {
-            CUDA_CHECK( cudaMemcpyAsync( &sa, cnt + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-            CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-            sa = std::min( sa, cap );
-            if( sa )
-                run_cascade( req, nq, sa, cap, list_entry, list_16, nullptr, 0, (uint32_t) n_sh );
-        }
+        const unsigned * c = read_counts( true );
+        c = run_redo( req, nq, c, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), cap );
+        if( entry != 64 && std::min( c[0], cap ) )
+            run_cascade( req, nq, std::min( c[0], cap ), cap, list_entry, list_16, nullptr, 0, (uint32_t) n_sh );
         int32_t * hs = (int32_t *) h_score_.ensure( std::max<size_t>( score_bytes, 4 ) );
         CUDA_CHECK( cudaMemcpyAsync( hs, d_score_.p, score_bytes, cudaMemcpyDeviceToHost, stream_ ) );
         int64_t * hs64 = nullptr;
@@ -2670,6 +2685,7 @@ void Engine::serve_restore( const SearchRequest & req ) {
     CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
     prof_width_ = -1;
     serve_layout_ = true;
+    serve_new_.clear();
 }
 
 std::vector<uint32_t> Engine::serve_open( const SearchRequest & req, uint32_t slots, uint32_t segments ) {
@@ -2709,13 +2725,7 @@ void Engine::serve_load( uint32_t slot, const uint8_t * codes, uint32_t len ) {
         return;     // restored before the next wave
     h_qlen_[slot] = len;
     h_qpad_[slot] = std::max<uint32_t>( 256, (len + 255u) & ~255u );
-    CUDA_CHECK( cudaMemcpyAsync( d_qcodes_.as<uint8_t>() + h_qoff_[slot], codes, len, cudaMemcpyHostToDevice,
-            stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qlen_.as<uint32_t>() + slot, &h_qlen_[slot], sizeof(uint32_t),
-            cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaMemcpyAsync( d_qpad_.as<uint32_t>() + slot, &h_qpad_[slot], sizeof(uint32_t),
-            cudaMemcpyHostToDevice, stream_ ) );
-    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+    serve_new_.push_back( slot );       // sent with the next wave
     prof_width_ = -1;
 }
 
@@ -2728,6 +2738,23 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
     if( !serve_layout_ )
         serve_restore( req );
     stage_.begin();
+    // the queries admitted since the last wave
+    if( !serve_new_.empty() ) {
+        for( uint32_t slot : serve_new_ ) {
+            const uint8_t * codes = stage_.add( serve_codes_[slot].data(), serve_codes_[slot].size(), stream_ );
+            stage_.send( stream_ );
+            CUDA_CHECK( cudaMemcpyAsync( d_qcodes_.as<uint8_t>() + h_qoff_[slot], codes, serve_codes_[slot].size(),
+                    cudaMemcpyDeviceToDevice, stream_ ) );
+        }
+        const uint32_t * len = stage_.add( h_qlen_.data(), h_qlen_.size(), stream_ );
+        const uint32_t * pad = stage_.add( h_qpad_.data(), h_qpad_.size(), stream_ );
+        stage_.send( stream_ );
+        CUDA_CHECK( cudaMemcpyAsync( d_qlen_.p, len, h_qlen_.size() * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                stream_ ) );
+        CUDA_CHECK( cudaMemcpyAsync( d_qpad_.p, pad, h_qpad_.size() * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                stream_ ) );
+        serve_new_.clear();
+    }
     serving_ = true;
     wide_ = false;                 // the server's settings were checked at serve_open
     const uint32_t n_seg = seq_hi - seq_lo;
@@ -2757,18 +2784,12 @@ void Engine::serve_wave( const SearchRequest & req, const std::vector<uint32_t> 
                 dev_slots, (uint32_t) active.size(), seq_lo );
     }
     CUDA_CHECK( cudaEventRecord( ev_phase_[1], stream_ ) );
-    unsigned n_a = 0;
-    if( entry != 64 ) {
-        CUDA_CHECK( cudaMemcpyAsync( &n_a, cnt + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
-        CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
-        n_a = std::min( n_a, cap );
-        if( n_a )
-            run_cascade( req, serve_slots_, n_a, cap, ovf_entry, ovf16, &active, seq_lo, seq_hi );
-    }
-    unsigned err = 0;
-    CUDA_CHECK( cudaMemcpyAsync( &err, cnt + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_ ) );
+    const unsigned * c = read_counts( true );
+    c = run_redo( req, serve_slots_, c, d_list_a_.as<PairTask>(), cnt + 0, cap, d_list_b_.as<PairTask>(), cap );
+    if( entry != 64 && std::min( c[0], cap ) )
+        run_cascade( req, serve_slots_, std::min( c[0], cap ), cap, ovf_entry, ovf16, &active, seq_lo, seq_hi );
     CUDA_CHECK( cudaEventRecord( ev_phase_[2], stream_ ) );
-    CUDA_CHECK( cudaStreamSynchronize( stream_ ) );
+    const unsigned err = read_counts( false )[2];
     serving_ = false;
     if( err )
         fatal( "Internal error in the GPU search (flags 0x%x).", err );
