@@ -35,7 +35,7 @@ CU_SOURCES = ["engine.cu", "emul_kernel.cu", "traceback_kernels.cu", "diag_kerne
               "noalloc.cu", "sw_qpair_kernel.cu",
               "sw_stream_kernel.cu"]
 CPP_SOURCES = ["api.cpp", "replay.cpp", "tuning.cpp"]
-HEADERS = ["device_common.cuh", "wavefront.cuh", "stream_stripes.cuh", "ssa_internal.h", "builtin_matrices.inc"]
+HEADERS = ["device_common.cuh", "stream_stripes.cuh", "ssa_internal.h", "builtin_matrices.inc"]
 
 LIB = os.path.join(OUT, "libssa.so")
 PLUGIN = os.path.join(OUT, "libsdb_b200.so")

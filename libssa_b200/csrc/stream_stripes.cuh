@@ -30,7 +30,6 @@
 #pragma once
 
 #include "device_common.cuh"
-#include "wavefront.cuh"
 
 namespace ssa {
 
@@ -92,6 +91,40 @@ struct StreamStripe {
     unsigned * error_flags;
 };
 
+// The database residues of a stripe on their way through the warp: lane k needs
+// word s - k at step s.  The warp loads 16 words at a time, a chunk of steps
+// ahead, into 64 words of shared memory, and every lane reads its word from
+// there.  (Loads by each lane from global memory, two steps ahead, miss the L1
+// cache most of the time: every acquire of a progress word on the SM empties it.)
+template <class T>
+struct StreamResidues {
+    T * ring;                      // 64 words, the warp's
+    T next;                        // lanes 0 .. 15: the words of the next refill
+
+    // fetch( b ): word b, any value outside the sequence
+    template <class Fetch>
+    __device__ __forceinline__ void start( int lane, const Fetch & fetch ) {
+        __syncwarp();                                   // the last ticket's readers
+        ring[lane] = fetch( lane );
+        ring[32 + lane] = fetch( lane - 32 );
+        next = fetch( 32 + lane );
+        __syncwarp();
+    }
+    // before the steps s0 .. s0 + 15: afterwards words s0 - 32 .. s0 + 31 are there
+    template <class Fetch>
+    __device__ __forceinline__ void refill( uint32_t s0, int lane, const Fetch & fetch ) {
+        if( s0 == 0 )
+            return;
+        __syncwarp();
+        if( lane < 16 ) {
+            ring[(s0 + 16u + (uint32_t) lane) & 63u] = next;
+            next = fetch( (int32_t) s0 + 32 + lane );
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ T at( int32_t b ) const { return ring[b & 63]; }
+};
+
 __device__ __forceinline__ int2 zero_word( const int2 * ) { return make_int2( 0, 0 ); }
 __device__ __forceinline__ int4 zero_word( const int4 * ) { return make_int4( 0, 0, 0, 0 ); }
 
@@ -116,9 +149,14 @@ __device__ __forceinline__ uint32_t stream_columns( const StreamStripe<Word> & s
     uint32_t avail = 0;            // columns of the row above known to be written
     bool have = false;             // pf holds the next chunk of it
     Word pf = zero_word( (const Word *) nullptr );
+    int32_t last = 0;              // the limit as it was a chunk ago, so that its load is not waited for
+    if constexpr( !Limit::NONE )
+        last = limit();
     for( uint32_t s0 = 0;; s0 += CHUNK ) {
-        if constexpr( !Limit::NONE )
-            cols = min( cols, (uint32_t) __shfl_sync( 0xffffffffu, lane == 0 ? limit() : 0, 0 ) + 1u );
+        if constexpr( !Limit::NONE ) {
+            cols = min( cols, (uint32_t) __shfl_sync( 0xffffffffu, last, 0 ) + 1u );
+            last = limit();
+        }
         if( sp.above && s0 < cols ) {
             if( !have ) {
                 const uint32_t need = min( s0 + (uint32_t) CHUNK, cols );
@@ -190,6 +228,14 @@ __device__ __forceinline__ void stream_end( const StreamStripe<Word> & sp, uint3
     __syncwarp();
     if( lane == 0 && !sp.last )
         store_release( sp.mine, STREAM_DONE | cols );
+}
+
+// Tickets are handed out one per warp from a global counter.
+__device__ __forceinline__ uint32_t next_ticket( unsigned long long * counter, int lane ) {
+    unsigned long long v = 0;
+    if( lane == 0 )
+        v = atomicAdd( counter, 1ull );
+    return (uint32_t) __shfl_sync( 0xffffffffu, v, 0 );
 }
 
 // The ticket's stripe and alignment: cum[i] is the first ticket of stripe i,

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
     constexpr int WORDS = R / 4;
     constexpr int ROWS = 32 * R;
     __shared__ StreamStage<int4> stages[STREAM_WARPS];
+    __shared__ uint2 rings[STREAM_WARPS][64];
     __shared__ __align__( 16 ) uint32_t tables[STREAM_WARPS][32 * 32 * WORDS];
     __shared__ int8_t smat[1024];
     const int lane = threadIdx.x & 31;
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
 
     uint64_t loaded_key = ~0ull;
     for( ;; ) {
-        const uint32_t ticket = next_hit( p.counter, lane );
+        const uint32_t ticket = next_ticket( p.counter, lane );
         if( ticket >= p.n_tickets )
             break;
         const uint32_t stripe = ticket_stripe( p.cum, p.levels, ticket );
@@ -156,12 +157,14 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
             out_h[j] = STREAM_BIAS2;
             out_f[j] = STREAM_BIAS2;
         }
-        // the blocks' residues two steps ahead
+        // the blocks' residues, read a step ahead
         auto fetch = [&]( const uint32_t * res, uint32_t nb, int32_t b ) -> uint32_t {
             return (b >= 0 && (uint32_t) b < nb) ? __ldg( res + b ) : STREAM_PAD;
         };
-        uint32_t a0 = fetch( ra, nba, -lane ), a1 = fetch( ra, nba, 1 - lane );
-        uint32_t b0 = fetch( rb, nbb, -lane ), b1 = fetch( rb, nbb, 1 - lane );
+        auto fetch2 = [&]( int32_t b ) -> uint2 { return make_uint2( fetch( ra, nba, b ), fetch( rb, nbb, b ) ); };
+        StreamResidues<uint2> residues{ rings[warp], {} };
+        residues.start( lane, fetch2 );
+        uint2 next = residues.at( -lane );
 
         auto column = [&]( const uint32_t s, const bool edge, const uint32_t cols ) {
             uint32_t up_h[C], up_f[C];
@@ -171,11 +174,8 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
                 up_f[j] = __shfl_up_sync( 0xffffffffu, out_f[j], 1 );
             }
             const int32_t b = (int32_t) s - lane;
-            const uint32_t wa = a0, wb = b0;
-            a0 = a1;
-            b0 = b1;
-            a1 = fetch( ra, nba, b + 2 );
-            b1 = fetch( rb, nbb, b + 2 );
+            const uint32_t wa = next.x, wb = next.y;
+            next = residues.at( b + 1 );
             if( edge && (b < 0 || b >= (int32_t) cols) )
                 return;
             if( lane == 0 ) {
@@ -283,7 +283,8 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
             }
         };
         const CrossLimit<BLOCKS> limit{ cross, two };
-        const uint32_t swept = stream_columns<16>( sp, st, lane, limit, []( uint32_t ) {}, column );
+        const uint32_t swept = stream_columns<16>( sp, st, lane, limit,
+                [&]( uint32_t s0 ) { residues.refill( s0, lane, fetch2 ); }, column );
         if constexpr( NW ) {
             if( owner ) {
                 const uint64_t row = (uint64_t) item.slot * p.sink.score_stride;

@@ -197,6 +197,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
     constexpr bool MAXIMUM = ENDS || PHASE == TB_SCORE;
     constexpr bool REVERSE = PHASE == TB_REVERSE;
     __shared__ StreamStage<int4> stages[TB_WARPS];
+    __shared__ uint32_t rings[TB_WARPS][64];
     __shared__ int32_t smat[1024];
     __shared__ uint32_t tables[P8 ? TB_WARPS : 1][P8 ? 32 * 32 : 1];
     const int lane = threadIdx.x & 31;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
     StreamStage<int4> & st = stages[warp];
 
     for( ;; ) {
-        const uint32_t ticket = next_hit( p.counter, lane );
+        const uint32_t ticket = next_ticket( p.counter, lane );
         if( ticket >= p.n_tickets )
             break;
         const uint32_t stripe = ticket_stripe( p.cum, p.levels, ticket );
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             dir = p.dirs + p.dir_off[h] + (uint64_t) stripe * ((uint64_t) nb + 31) * 32;
         int32_t out_h[C] = {}, out_f[C] = {};
 
-        // Residue words, two steps ahead of use: block b of the forward
+        // Residue words, read a step ahead of use: block b of the forward
         // direction is word b.  The reverse pass reads columns b_end - 4b down
         // to b_end - 4b - 3, which lie in the word of the last of them and the
         // word after it (the previous block's).
@@ -313,7 +314,9 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             const int32_t w = REVERSE ? (rg.b_end - 4 * b - 3) >> 2 : b;
             return (uint32_t) w < nb ? __ldg( res + w ) : 0u;
         };
-        uint32_t before = REVERSE ? fetch( -lane - 1 ) : 0u, w0 = fetch( -lane ), w1 = fetch( 1 - lane );
+        StreamResidues<uint32_t> residues{ rings[warp], 0u };
+        residues.start( lane, fetch );
+        uint32_t before = REVERSE ? residues.at( -lane - 1 ) : 0u, w0 = residues.at( -lane );
         const int32_t last_block = (int32_t) nb - 1, last_chain = (int32_t) (B - 1u) & 3;
 
         auto block = [&]( const uint32_t s, const bool edge, const uint32_t blocks ) {
@@ -329,8 +332,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 word = __byte_perm( __funnelshift_r( w0, before, 8u * ((uint32_t) (rg.b_end - 3) & 3u) ), 0, 0x0123 );
                 before = w0;
             }
-            w0 = w1;
-            w1 = fetch( b + 2 );
+            w0 = residues.at( b + 1 );
             if( edge && (b < 0 || b >= (int32_t) blocks) )
                 return;
             if( lane == 0 ) {
@@ -473,7 +475,8 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             }
         };
         const ColumnLimit<REVERSE> limit{ p.limit + h };
-        const uint32_t swept = stream_columns<16>( sp, st, lane, limit, []( uint32_t ) {}, block );
+        const uint32_t swept = stream_columns<16>( sp, st, lane, limit,
+                [&]( uint32_t s0 ) { residues.refill( s0, lane, fetch ); }, block );
         if constexpr( MAXIMUM || REVERSE ) {
             // this stripe's cell against that of the stripes above (theirs is
             // final once the stripe above has ended)
