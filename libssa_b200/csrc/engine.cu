@@ -59,6 +59,20 @@ struct DevBuf {
         }
         return p;
     }
+    // with an eighth to spare, so that a call on slightly longer sequences does
+    // not allocate again (10 ms for 4 GB); without where that does not fit
+    void * ensure_spare( size_t n ) {
+        if( n > bytes ) {
+            release();
+            if( cudaMalloc( &p, n + n / 8 ) == cudaSuccess ) {
+                bytes = n + n / 8;
+                return p;
+            }
+            (void) cudaGetLastError();
+            p = nullptr;
+        }
+        return ensure( n );
+    }
     void release() {
         if( p )
             cudaFree( p );
@@ -2050,6 +2064,8 @@ static int64_t max_abs_step( const SearchRequest & req ) {
     return m;
 }
 
+// Most direction memory that is kept for later calls.
+constexpr uint64_t TB_KEPT = (uint64_t) 8 << 30;
 // Least direction memory of one traceback wave (automatic budget).
 constexpr uint64_t TB_MIN_BUDGET = (uint64_t) 256 << 20;
 
@@ -2229,8 +2245,10 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         p.result = (int4 *) d_tb_result_.ensure( std::max<size_t>( 16, (size_t) n_tickets * sizeof(int4) ) );
         p.boundary = (int4 *) d_tb_bnd_.ensure( bnd_words * sizeof(int4) + 16 );
         p.limit = (int32_t *) (dsy + s_lim);
-        if( paths )
-            p.dirs = (uint32_t *) d_tb_dirs_.ensure( dir_words * sizeof(uint32_t) + 16 );
+        if( paths ) {
+            const size_t n = dir_words * sizeof(uint32_t) + 16;
+            p.dirs = (uint32_t *) (tb_budget_ || n + n / 8 > TB_KEPT ? d_tb_dirs_.ensure( n ) : d_tb_dirs_.ensure_spare( n ));
+        }
         stage_.send( stream_ );
         CUDA_CHECK( cudaMemcpyAsync( din, hin, in.bytes, cudaMemcpyHostToDevice, stream_ ) );
         CUDA_CHECK( cudaMemsetAsync( dsy, 0, s_zero, stream_ ) );
@@ -2371,7 +2389,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
     run_waves( rows, cols, scores_only ? SCORES : PATHS );
     // a very large direction buffer (long pairs) is not kept for later calls,
     // whose scores, lists and database segments need the device memory
-    if( d_tb_dirs_.bytes > ((uint64_t) 8 << 30) )
+    if( d_tb_dirs_.bytes > TB_KEPT )
         d_tb_dirs_.release();
     if( d_tb_bnd_.bytes > ((uint64_t) 1 << 30) )
         d_tb_bnd_.release();

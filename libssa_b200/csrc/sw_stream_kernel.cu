@@ -68,7 +68,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
     constexpr int C = 4;
     constexpr int WORDS = R / 4;
     constexpr int ROWS = 32 * R;
-    __shared__ StreamStage<int4> stages[STREAM_WARPS];
+    __shared__ StreamStage stages[STREAM_WARPS];
     __shared__ uint2 rings[STREAM_WARPS][64];
     __shared__ __align__( 16 ) uint32_t tables[STREAM_WARPS][32 * 32 * WORDS];
     __shared__ int8_t smat[1024];
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
     for( int i = threadIdx.x; i < 1024; i += STREAM_THREADS )
         smat[i] = (int8_t) p.matrix[i];              // [database code][query code]
     __syncthreads();
-    StreamStage<int4> & st = stages[warp];
+    StreamStage & st = stages[warp];
     uint32_t * table = tables[warp] + lane * WORDS;  // the lane's scores of code d at [d * 32 * WORDS]
     const uint32_t GOE32 = (uint32_t) (p.gap_oe * 65536 + p.gap_oe);
     const uint32_t GE2 = ((uint32_t) (uint16_t) (int16_t) p.gap_e << 16) | (uint16_t) (int16_t) p.gap_e;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
         const uint32_t * ra = reinterpret_cast<const uint32_t *>( p.db.codes + p.db.offsets[item.id_a] );
         const uint32_t * rb = two ? reinterpret_cast<const uint32_t *>( p.db.codes + p.db.offsets[item.id_b] ) : ra;
 
-        StreamStripe<int4> sp;
+        StreamStripe sp;
         sp.cols = max( nba, nbb );
         sp.row = p.boundary + p.bnd_off[it];
         sp.above = stripe ? p.progress + pred : nullptr;
@@ -179,25 +179,15 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
             if( edge && (b < 0 || b >= (int32_t) cols) )
                 return;
             if( lane == 0 ) {
-                if( stripe == 0 ) {
-#pragma unroll
-                    for( int j = 0; j < C; j++ ) {
-                        // H(-1, c) and F entering row 0
-                        up_h[j] = NW ? stream_nw_pack( gO + (4 * b + j + 1) * gE ) : STREAM_BIAS2;
-                        up_f[j] = NW ? stream_nw_pack( 2 * gO + (4 * b + j + 2) * gE ) : STREAM_BIAS2;
-                    }
-                }
-                else {
-                    const int4 x = st.in[2 * (s & 15u)], y = st.in[2 * (s & 15u) + 1];
-                    up_h[0] = (uint32_t) x.x;
-                    up_f[0] = (uint32_t) x.y;
-                    up_h[1] = (uint32_t) x.z;
-                    up_f[1] = (uint32_t) x.w;
-                    up_h[2] = (uint32_t) y.x;
-                    up_f[2] = (uint32_t) y.y;
-                    up_h[3] = (uint32_t) y.z;
-                    up_f[3] = (uint32_t) y.w;
-                }
+                const int4 x = st.in[2 * (s % STREAM_CHUNK)], y = st.in[2 * (s % STREAM_CHUNK) + 1];
+                up_h[0] = (uint32_t) x.x;
+                up_f[0] = (uint32_t) x.y;
+                up_h[1] = (uint32_t) x.z;
+                up_f[1] = (uint32_t) x.w;
+                up_h[2] = (uint32_t) y.x;
+                up_f[2] = (uint32_t) y.y;
+                up_h[3] = (uint32_t) y.z;
+                up_f[3] = (uint32_t) y.w;
             }
             uint32_t pa[C][WORDS], pb[C][WORDS], f[C];
 #pragma unroll
@@ -278,13 +268,25 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
                 }
             }
             if( lane == 31 ) {
-                st.out[2 * (s & 15u)] = make_int4( (int) out_h[0], (int) out_f[0], (int) out_h[1], (int) out_f[1] );
-                st.out[2 * (s & 15u) + 1] = make_int4( (int) out_h[2], (int) out_f[2], (int) out_h[3], (int) out_f[3] );
+                st.out[2 * (s % STREAM_CHUNK)] = make_int4( (int) out_h[0], (int) out_f[0], (int) out_h[1], (int) out_f[1] );
+                st.out[2 * (s % STREAM_CHUNK) + 1] = make_int4( (int) out_h[2], (int) out_f[2], (int) out_h[3], (int) out_f[3] );
             }
         };
+        // the row above the first stripe, columns c and c + 1: H(-1, c) and F entering row 0
+        auto top = [&]( int32_t c ) -> int4 {
+            if constexpr( NW )
+                return make_int4( (int) stream_nw_pack( gO + (c + 1) * gE ), (int) stream_nw_pack( 2 * gO + (c + 2) * gE ),
+                        (int) stream_nw_pack( gO + (c + 2) * gE ), (int) stream_nw_pack( 2 * gO + (c + 3) * gE ) );
+            else
+                return make_int4( (int) STREAM_BIAS2, (int) STREAM_BIAS2, (int) STREAM_BIAS2, (int) STREAM_BIAS2 );
+        };
+        auto refill = [&]( uint32_t s0 ) {
+            if( stripe == 0 && lane < (int) (2 * STREAM_CHUNK) )
+                st.in[lane] = top( 4 * (int32_t) s0 + 2 * lane );
+            residues.refill( s0, lane, fetch2 );
+        };
         const CrossLimit<BLOCKS> limit{ cross, two };
-        const uint32_t swept = stream_columns<16>( sp, st, lane, limit,
-                [&]( uint32_t s0 ) { residues.refill( s0, lane, fetch2 ); }, column );
+        const uint32_t swept = stream_columns( sp, st, lane, limit, refill, column );
         if constexpr( NW ) {
             if( owner ) {
                 const uint64_t row = (uint64_t) item.slot * p.sink.score_stride;

@@ -37,11 +37,17 @@
 // shared-memory word of int8 entries, added to the diagonal by dp4a (off the ALU
 // pipe); tables past int8 are read entry by entry.
 //
+// The flags of a cell are two minimum-of-three and two signs (8 ALU instructions
+// per cell with the recurrence); maxima that also return a predicate, with the
+// predicates combined into flags, took 24 (counters: 647 -> 365 instructions per
+// warp and step of 16 cells).
+//
 // Measured on a B200 (one call each): groups of 1, 2 or 4 warps of one CTA per
 // hit with a group barrier every 32 steps / streamed stripes, one column per
-// step / four columns per step: 48 pairs of 5,000-30,000 residues, SW 780 / 53 /
-// 42 ms and NW 470 / 35 / 24 ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 ms;
-// 320 hits of 30-1,355 rows 4.7 / 1.3 / 1.1 ms.
+// step / four columns per step / signs as flags and three CTAs per SM: 48 pairs
+// of 5,000-30,000 residues, SW 780 / 53 / 42 / 30 ms and NW 470 / 35 / 24 / 18
+// ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 / 4.0 ms; 320 hits of 30-1,355
+// rows 4.7 / 1.3 / 1.1 / 1.0 ms.
 #include "device_common.cuh"
 #include "stream_stripes.cuh"
 
@@ -52,6 +58,13 @@ namespace ssa {
 constexpr int R = TB_ROWS_PER_LANE;                   // query rows per lane
 constexpr int TB_THREADS = 128;
 constexpr int TB_WARPS = TB_THREADS / 32;
+// CTAs per SM.  Five fit, but where many long hits are aligned at once the call
+// takes as long as the stripes of the longest do, one after the other, and those
+// run slower the more other warps share their sub-partition; three keep the ALU as
+// busy.  48 pairs of 5,000-30,000 residues with five / three / two: SW 24.7 /
+// 20.2 / 20.0 ms and the reverse pass 9.0 / 7.3 / 7.2, NW 18.1 / 15.7 / 15.6 ms;
+// 320 hits of 30-1,355 rows 0.60 / 0.60 / 0.60, 1,600 hits 0.58 / 0.58 / 0.62 ms.
+constexpr int TB_BLOCKS = 3;
 
 // What the stripe bodies share: the lane's rows and their scores.
 template <bool P8>
@@ -196,7 +209,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
     constexpr bool MATRIX = ENDS || PHASE == TB_SCORE || PHASE == TB_NW_SCORE;     // every row and column
     constexpr bool MAXIMUM = ENDS || PHASE == TB_SCORE;
     constexpr bool REVERSE = PHASE == TB_REVERSE;
-    __shared__ StreamStage<int4> stages[TB_WARPS];
+    __shared__ StreamStage stages[TB_WARPS];
     __shared__ uint32_t rings[TB_WARPS][64];
     __shared__ int32_t smat[1024];
     __shared__ uint32_t tables[P8 ? TB_WARPS : 1][P8 ? 32 * 32 : 1];
@@ -210,7 +223,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         smat[i] = (int32_t) (PHASE == TB_FORWARD || REVERSE ? p.matrix[(q << 5) + d] : p.matrix[(d << 5) + q]);
     }
     __syncthreads();
-    StreamStage<int4> & st = stages[warp];
+    StreamStage & st = stages[warp];
 
     for( ;; ) {
         const uint32_t ticket = next_ticket( p.counter, lane );
@@ -237,7 +250,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         const uint8_t * a = p.qcodes + p.qoff[hit.qslot];
         const uint32_t nb = (B + 3u) >> 2;              // blocks of four columns
 
-        StreamStripe<int4> sp;
+        StreamStripe sp;
         sp.cols = nb;
         sp.row = p.boundary + p.bnd_off[h];
         sp.above = stripe ? p.progress + pred : nullptr;
@@ -336,42 +349,21 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
             if( edge && (b < 0 || b >= (int32_t) blocks) )
                 return;
             if( lane == 0 ) {
-                if( stripe == 0 ) {
-#pragma unroll
-                    for( int j = 0; j < C; j++ ) {
-                        if constexpr( PHASE == TB_FORWARD ) {
-                            up_h[j] = 0;
-                            up_f[j] = gO + gE;              // f starts at gapO: max(gapO, 0 + gapO) + gapE
-                        }
-                        else if constexpr( REVERSE ) {
-                            up_h[j] = -1;                   // h starts at -1 per row; f = max(-1, h + gapO) + gapE
-                            up_f[j] = max( -1, -1 + gO ) + gE;
-                        }
-                        else {
-                            // H(-1, c) (the next column's diagonal) and F entering row 0
-                            const int32_t c = 4 * b + j;
-                            up_h[j] = NW ? gO + (c + 1) * gE : 0;
-                            up_f[j] = NW ? 2 * gO + (c + 2) * gE : 0;
-                        }
-                    }
-                }
-                else {
-                    const int4 x = st.in[2 * (s & 15u)], y = st.in[2 * (s & 15u) + 1];
-                    up_h[0] = x.x;
-                    up_f[0] = x.y;
-                    up_h[1] = x.z;
-                    up_f[1] = x.w;
-                    up_h[2] = y.x;
-                    up_f[2] = y.y;
-                    up_h[3] = y.z;
-                    up_f[3] = y.w;
-                }
+                const int4 x = st.in[2 * (s % STREAM_CHUNK)], y = st.in[2 * (s % STREAM_CHUNK) + 1];
+                up_h[0] = x.x;
+                up_f[0] = x.y;
+                up_h[1] = x.z;
+                up_f[1] = x.w;
+                up_h[2] = y.x;
+                up_f[2] = y.y;
+                up_h[3] = y.z;
+                up_f[3] = y.w;
             }
             typename TbLane<P8>::Column sc[C];
             int32_t f[C], hv[C][R];
             // 2 bits per cell (bit 1 = insertion, LEFT | EXT_LEFT, takes priority;
-            // bit 0 = deletion, UP | EXT_UP), a byte per column
-            uint32_t flags = 0;
+            // bit 0 = deletion, UP | EXT_UP), a byte per column, the first row in its top bits
+            uint32_t flags[C] = {};
 #pragma unroll
             for( int j = 0; j < C; j++ ) {
                 sc[j] = t.scores( (int) ((word >> (8 * j)) & 0xffu) );
@@ -392,20 +384,19 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                     const int32_t x0 = t.add_score( sc[j], r, hd );
                     int32_t x;
                     if constexpr( DIRS ) {
-                        // flags as in the reference (strict compares in its
-                        // order): each max also yields the negation of one
-                        bool no_up, no_left, no_ext_up, no_ext_left;
-                        const int32_t m1 = __vibmax_s32( x0, f[j], &no_up );       // UP: f > x0
-                        const int32_t xr = __vibmax_s32( m1, e, &no_left );        // LEFT: e > max(x0, f)
-                        x = NW ? xr : max( xr, 0 );
+                        // The reference's flags with its strict compares: UP, f > x0;
+                        // LEFT, e > max(x0, f); EXT_UP, f + gapE > y; EXT_LEFT,
+                        // e + gapE > y, where y = x + gapO + gapE.  So UP or EXT_UP is
+                        // f > min(x0, x + gapO), and LEFT or EXT_LEFT the same with
+                        // e and max(x0, f); each sign goes in from the right.  Rows past
+                        // the query's end get flags too; the walk never reads them.
+                        const int32_t m1 = max( x0, f[j] );
+                        x = NW ? max( m1, e ) : __vimax3_s32( m1, e, 0 );
                         const int32_t y = x + gOE;
-                        f[j] = __vibmax_s32( y, f[j] + gE, &no_ext_up );            // EXT_UP: f + gapE > y
-                        t.E[r] = __vibmax_s32( y, e + gE, &no_ext_left );           // EXT_LEFT: e + gapE > y
-                        // rows past the query's end get flags too; the walk never reads them
-                        if( !(no_left && no_ext_left) )
-                            flags |= 2u << (8 * j + 2 * r);
-                        if( !(no_up && no_ext_up) )
-                            flags |= 1u << (8 * j + 2 * r);
+                        flags[j] = __funnelshift_l( (uint32_t) (__viaddmin_s32( x, gO, m1 ) - e), flags[j], 1 );
+                        flags[j] = __funnelshift_l( (uint32_t) (__viaddmin_s32( x, gO, x0 ) - f[j]), flags[j], 1 );
+                        f[j] = __viaddmax_s32( f[j], gE, y );
+                        t.E[r] = __viaddmax_s32( e, gE, y );
                     }
                     else {
                         x = PHASE == TB_FORWARD || PHASE == TB_SCORE ? __vimax3_s32( max( x0, 0 ), f[j], e )
@@ -423,8 +414,10 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                         t.H[r] = x;
                 }
             }
-            if constexpr( DIRS )
-                dir[(uint64_t) s * 32 + lane] = flags;     // one transaction of 128 bytes per step
+            if constexpr( DIRS ) {
+                const uint32_t lo = __byte_perm( flags[0], flags[1], 0x0040 ), hi = __byte_perm( flags[2], flags[3], 0x0040 );
+                dir[(uint64_t) s * 32 + lane] = __byte_perm( lo, hi, 0x5410 );     // one transaction of 128 bytes per step
+            }
             if constexpr( MAXIMUM || REVERSE ) {
                 // the lane visits its cells in (column, row) order: its first
                 // maximum (its first candidate) counts, and rarely is there one
@@ -470,13 +463,29 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 out_f[j] = f[j];
             }
             if( lane == 31 ) {
-                st.out[2 * (s & 15u)] = make_int4( out_h[0], out_f[0], out_h[1], out_f[1] );
-                st.out[2 * (s & 15u) + 1] = make_int4( out_h[2], out_f[2], out_h[3], out_f[3] );
+                st.out[2 * (s % STREAM_CHUNK)] = make_int4( out_h[0], out_f[0], out_h[1], out_f[1] );
+                st.out[2 * (s % STREAM_CHUNK) + 1] = make_int4( out_h[2], out_f[2], out_h[3], out_f[3] );
             }
         };
+        // the row above the first stripe, columns c and c + 1: H(-1, c) (the next
+        // column's diagonal) and F entering row 0
+        auto top = [&]( int32_t c ) -> int4 {
+            if constexpr( PHASE == TB_FORWARD )         // f starts at gapO: max(gapO, 0 + gapO) + gapE
+                return make_int4( 0, gO + gE, 0, gO + gE );
+            else if constexpr( REVERSE )                // h starts at -1 per row; f = max(-1, h + gapO) + gapE
+                return make_int4( -1, max( -1, -1 + gO ) + gE, -1, max( -1, -1 + gO ) + gE );
+            else if constexpr( NW )
+                return make_int4( gO + (c + 1) * gE, 2 * gO + (c + 2) * gE, gO + (c + 2) * gE, 2 * gO + (c + 3) * gE );
+            else
+                return make_int4( 0, 0, 0, 0 );
+        };
+        auto refill = [&]( uint32_t s0 ) {
+            if( stripe == 0 && lane < (int) (2 * STREAM_CHUNK) )
+                st.in[lane] = top( 4 * (int32_t) s0 + 2 * lane );
+            residues.refill( s0, lane, fetch );
+        };
         const ColumnLimit<REVERSE> limit{ p.limit + h };
-        const uint32_t swept = stream_columns<16>( sp, st, lane, limit,
-                [&]( uint32_t s0 ) { residues.refill( s0, lane, fetch ); }, block );
+        const uint32_t swept = stream_columns( sp, st, lane, limit, refill, block );
         if constexpr( MAXIMUM || REVERSE ) {
             // this stripe's cell against that of the stripes above (theirs is
             // final once the stripe above has ended)
@@ -579,7 +588,7 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
         __syncwarp();
         if( lane == 0 ) {
             for( int m = 0; m < TB_WALK_MOVES && i >= a_begin && j >= b_begin && i >= 0 && j >= 0; m++ ) {
-                const uint32_t op = (win[wib][(i4 - i / 4) * W + (j4 - j / 4)] >> (8 * (j % 4) + 2 * (i % 4))) & 3u;
+                const uint32_t op = (win[wib][(i4 - i / 4) * W + (j4 - j / 4)] >> (8 * (j % 4) + 6 - 2 * (i % 4))) & 3u;
                 char ch;
                 if( op & 2u ) {
                     j--;
@@ -620,7 +629,7 @@ static cudaError_t launch_stripes( const TbParams & p, int sms, cudaStream_t st 
     if( e != cudaSuccess )
         return e;
     const uint32_t want = (p.n_tickets + TB_WARPS - 1) / TB_WARPS;
-    const uint32_t grid = min( want, (uint32_t) (sms * max( 1, shape.blocks )) );
+    const uint32_t grid = min( want, (uint32_t) (sms * min( TB_BLOCKS, max( 1, shape.blocks ) )) );
     if( grid )
         tb_stripes_kernel<PHASE, P8><<<grid, TB_THREADS, 0, st>>>( p );
     return cudaGetLastError();
