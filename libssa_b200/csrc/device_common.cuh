@@ -270,6 +270,7 @@ struct SwStreamParams {
     const SwStreamItem * items;   // most stripes first
     const uint64_t * bnd_off;     // per item offset into boundary
     const uint32_t * cum;         // first ticket of stripe i, i = 0 .. levels
+    int ctas_per_sm;              // at most
     uint32_t levels, n_tickets;
     unsigned long long * counter; // next ticket (0 at the start)
     uint32_t * progress;          // per ticket (0 at the start)

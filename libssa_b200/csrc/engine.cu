@@ -1624,11 +1624,49 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
     std::stable_sort( items.begin(), items.end(), [&]( const SwStreamItem & x, const SwStreamItem & y ) {
         return h_qlen_[x.slot] > h_qlen_[y.slot];
     } );
+    // Rows per lane: 4 while every stripe of 128 rows can be resident (16 warps per
+    // SM), else whichever of 4 .. 6 computes the items' stripes in the fewest
+    // instructions (a step of R rows is 26 R + 20 of the ALU's).  964 items of 300
+    // rows on 2 CTAs per SM: 5.47 ms with 4 (384 rows computed), 3.94 with 5 (320);
+    // 7 and 8 were never the best on batches of 30-1,800 rows (7.3 with 5, 7.4 with
+    // 6, 8.3 and 8.8 ms).  SSA_B200_STREAM_ROWS pins it.
+    auto stripes = [&]( const SwStreamItem & t, int r ) {
+        return (uint64_t) ((h_qlen_[t.slot] + 32u * (uint32_t) r - 1u) / (32u * (uint32_t) r));
+    };
+    auto columns = [&]( const SwStreamItem & t ) { return (uint64_t) db_.len[t.id_a] / 4 + 31; };    // steps of a stripe
     uint64_t stripes128 = 0;
     for( const SwStreamItem & t : items )
-        stripes128 += (h_qlen_[t.slot] + 127u) / 128u;
-    // rows per lane: 4 while every stripe of 128 rows can be resident (24 warps per SM)
-    const int R = nw || stripes128 <= (uint64_t) sms_ * 24 ? 4 : 8;
+        stripes128 += stripes( t, 4 );
+    int R = 4;
+    const char * pinned = getenv( "SSA_B200_STREAM_ROWS" );
+    if( !nw && pinned && atoi( pinned ) >= 4 && atoi( pinned ) <= 6 )
+        R = atoi( pinned );
+    else if( !nw && stripes128 > (uint64_t) sms_ * 16 ) {
+        uint64_t least = UINT64_MAX;
+        for( int r = 4; r <= 6; r++ ) {
+            uint64_t cost = 0;
+            for( const SwStreamItem & t : items )
+                cost += stripes( t, r ) * columns( t );
+            cost *= 26u * (uint64_t) r + 20u;
+            if( cost < least ) {
+                least = cost;
+                R = r;
+            }
+        }
+    }
+    // CTAs per SM: a step takes as long as the warps of the sub-partition (one of
+    // each CTA) share its ALU, so the longest item ends in time where there are
+    // no more of them than its steps go into the sub-partition's share of all
+    // steps; at least 2, which keep the ALU busy, at most the 4 that fit.  On 2 / 3
+    // / 4: 964 items of 300 x 8,000-35,000 (2.0 times) 3.9 / 4.8 / 5.7 ms, 1,031 of
+    // 30-1,800 rows (3.6) 7.4 / 7.1 / 7.1 ms, Needleman-Wunsch of 10,000 (5.6) 1.11
+    // / 1.01 / 0.99 ms; fewer items than warps the same on all.
+    uint64_t steps = 0, longest = 1;
+    for( const SwStreamItem & t : items ) {
+        steps += stripes( t, R ) * columns( t );
+        longest = std::max( longest, columns( t ) + 47 * stripes( t, R ) );
+    }
+    const int ctas = (int) std::min<uint64_t>( 4, std::max<uint64_t>( 2, steps / ((uint64_t) sms_ * 4 * longest) ) );
     const uint32_t rows = 32u * (uint32_t) R;
     const uint32_t ni = (uint32_t) items.size();
     const bool blocks = req.bit_width == 8;       // Smith-Waterman 8-bit entry
@@ -1679,6 +1717,7 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
         p.cum = dev_cum;
         p.levels = (uint32_t) cum.size() - 1;
         p.n_tickets = nt;
+        p.ctas_per_sm = ctas;
         p.counter = (unsigned long long *) sy;
         p.progress = (uint32_t *) (sy + 16);
         p.result = p.progress + nt;

@@ -6,19 +6,21 @@
 // per 80 to 500 query rows, one pass after the other: (a) the longest sequences
 // of a database against long queries, in a call without enough other work to
 // hide them; (b) the pairs that the 8-bit entry re-queued (255 and more), a few
-// per query, often the longest of both.  Here lane k of a warp owns R rows of a stripe of 32 x R rows, and the stripes of a pair follow one
-// another on as many warps as the pair has stripes (stream_stripes.cuh).
+// per query, often the longest of both.  Here lane k of a warp owns R rows of a
+// stripe of 32 x R rows, and the stripes of a pair follow one another on as many
+// warps as the pair has stripes (stream_stripes.cuh).
 //
 // Arithmetic and range are those of sw_fast4_kernel (exact 16x2 scores with a
 // bias of 1024; a sequence whose running maximum reaches the limit goes to
 // sink.redo, for the lane emulation): one 4-column block per step, four
 // skewed dependency chains, 5.5 ALU instructions and one IADD per cell pair.
-// Bound by the ALU pipe when many pairs are re-queued, by the latency of one
-// warp's steps (blocks + 47 x stripes) when few are.  R is 4 while all stripes
-// of 128 rows can be resident, else 8.  Measured on a B200 against the lane
-// emulation (one warp per pair, int32): 102 pairs of 375 rows x 380 columns
-// 0.50 -> 0.16 ms; 1,927 of 300 x 21,000 38.7 -> 6.5 ms; 2,014 of 30-1,803 x
-// 21,000 94 -> 8.4 ms.
+// Bound by the ALU pipe when many pairs are re-queued (78 % of its cycles; what
+// is left is padding of the last stripe and 20 instructions a step besides the
+// cells), by the latency of one warp's steps (blocks + 47 x stripes) when few
+// are.  The host picks R (4 to 6) and the CTAs per SM (2 to 4) for each launch.
+// Measured on a B200 against the lane emulation (one warp per pair, int32): 102
+// pairs of 375 rows x 380 columns 0.50 -> 0.12 ms; 1,927 of 300 x 21,000 38.7 ->
+// 3.9 ms; 2,014 of 30-1,803 x 21,000 94 -> 7.1 ms.
 #include "device_common.cuh"
 #include "stream_stripes.cuh"
 
@@ -28,6 +30,7 @@ constexpr uint32_t STREAM_BIAS = 1024u;
 constexpr uint32_t STREAM_BIAS2 = (STREAM_BIAS << 16) | STREAM_BIAS;
 constexpr int STREAM_THREADS = 128;
 constexpr int STREAM_WARPS = STREAM_THREADS / 32;
+constexpr int STREAM_BLOCKS = 4;                     // most CTAs per SM
 constexpr uint32_t STREAM_PAD = FAST_PAD_CODE * 0x01010101u;   // past a sequence's last block: scores -128
 
 // byte j of a and of b, sign-extended to 16 bits each
@@ -64,9 +67,9 @@ __device__ __forceinline__ uint32_t stream_nw_pack( int32_t v ) {
 }
 
 template <int R, bool BLOCKS, bool NW>
-__global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_kernel( SwStreamParams p ) {
+__global__ void __launch_bounds__( STREAM_THREADS, STREAM_BLOCKS ) sw_stream_kernel( SwStreamParams p ) {
     constexpr int C = 4;
-    constexpr int WORDS = R / 4;
+    constexpr int WORDS = (R + 3) / 4;
     constexpr int ROWS = 32 * R;
     __shared__ StreamStage stages[STREAM_WARPS];
     __shared__ uint2 rings[STREAM_WARPS][64];
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__( STREAM_THREADS, R == 4 ? 6 : 4 ) sw_stream_ke
                     uint32_t v = 0;
 #pragma unroll
                     for( int b = 0; b < 4; b++ ) {
-                        const int c = code[4 * w + b];
+                        const int c = 4 * w + b < R ? code[4 * w + b < R ? 4 * w + b : 0] : -1;
                         const int m = (c >= 0 && d != (int) FAST_PAD_CODE) ? smat[(d << 5) + c] : PAST;
                         v |= ((uint32_t) m & 0xffu) << (8 * b);
                     }
@@ -338,16 +341,25 @@ static cudaError_t launch_stream( const SwStreamParams & p, int sms, cudaStream_
     const cudaError_t e = shape.set( sw_stream_kernel<R, BLOCKS, NW>, STREAM_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
-    const uint32_t grid = min( (p.n_tickets + STREAM_WARPS - 1) / STREAM_WARPS, (uint32_t) (sms * max( 1, shape.blocks )) );
+    const uint32_t grid = min( (p.n_tickets + STREAM_WARPS - 1) / STREAM_WARPS,
+            (uint32_t) (sms * max( 1, min( p.ctas_per_sm, shape.blocks ) )) );
     if( grid )
         sw_stream_kernel<R, BLOCKS, NW><<<grid, STREAM_THREADS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
+template <bool BLOCKS>
+static cudaError_t launch_rows( int R, const SwStreamParams & p, int sms, cudaStream_t st ) {
+    switch( R ) {
+        case 4: return launch_stream<4, BLOCKS, false>( p, sms, st );
+        case 5: return launch_stream<5, BLOCKS, false>( p, sms, st );
+        case 6: return launch_stream<6, BLOCKS, false>( p, sms, st );
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_sw_stream( int R, const SwStreamParams & p, int sms, cudaStream_t st ) {
-    if( p.cross )
-        return R == 4 ? launch_stream<4, true, false>( p, sms, st ) : launch_stream<8, true, false>( p, sms, st );
-    return R == 4 ? launch_stream<4, false, false>( p, sms, st ) : launch_stream<8, false, false>( p, sms, st );
+    return p.cross ? launch_rows<true>( R, p, sms, st ) : launch_rows<false>( R, p, sms, st );
 }
 
 cudaError_t launch_nw_stream( const SwStreamParams & p, int sms, cudaStream_t st ) {

@@ -48,3 +48,22 @@ def test_needleman_wunsch_pairs(built_library, monkeypatch, width, share):
     records += [W.mutate(rng, q, W.AA20, 0.1, 0.03, (1, 5)) for q in queries for _ in range(3)]
     _check(dict(algo="nw", width=width, align=1, hits=14, gap=(-11, -1), chunk=25, simd=2,
                 records=[r.tobytes() for r in records], queries=[q.tobytes() for q in queries]))
+
+
+@pytest.mark.parametrize("rows", [5, 6])
+@pytest.mark.parametrize("width", [8, 64])
+def test_rows_per_lane(built_library, monkeypatch, width, rows):
+    """Stripes of 160 and 192 rows: queries around one and two of them, every
+    pair of the entry and the re-queued ones there."""
+    monkeypatch.setenv("SSA_B200_STREAM_SHARE", "0")
+    monkeypatch.setenv("SSA_B200_STREAM_ROWS", str(rows))
+    rng = np.random.default_rng(51 + rows)
+    s = 32 * rows
+    queries = [W.random_residues(rng, n, W.AA20) for n in (1, rows - 1, rows, rows + 1, s - 1, s, s + 1, 2 * s, 2 * s + 1)]
+    records = [W.random_residues(rng, int(n), W.AA20) for n in rng.integers(1, 400, 40)]
+    records += [W.random_residues(rng, n, W.AA20) for n in (61, 62, 63, 64, 65, 66, 127, 1500)]
+    for q in queries[4:]:
+        for n in (len(q), 1000, 1003):
+            records.append(W.mutate(rng, np.tile(q, n // len(q) + 1)[:n], W.AA20, 0.03, 0.01, (1, 4)))
+    _check(dict(algo="sw", width=width, align=1, hits=16, gap=(-11, -1), chunk=25, simd=2,
+                records=[r.tobytes() for r in records], queries=[q.tobytes() for q in queries]))
