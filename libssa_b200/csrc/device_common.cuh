@@ -144,11 +144,13 @@ struct TbParams {
     int gap_open, gap_extend;
     const TbHit * hits;         // most stripes first
     uint32_t n_hits;
+    int rows_per_lane;          // 4, or 2 (score tables that fit int8)
     TbRegion * regions;
     int32_t * last_h;           // per hit: forward pass last-row H (query-indexed)
     int32_t * last_e;           // per hit: forward pass last-row vertical gap
     const uint64_t * last_off;  // per hit offset into last_h / last_e
-    // per hit direction words, 2 bits per cell: [stripe][wavefront step][lane], a word per 4 rows x 4 columns
+    // per hit direction words, 2 bits per cell: [stripe][wavefront step][lane], a word per
+    // rows_per_lane rows x 4 columns, a byte per column
     uint32_t * dirs;
     const uint64_t * dir_off;   // per hit offset into dirs
     char * ops;                 // per hit reversed op string
@@ -182,7 +184,6 @@ cudaError_t launch_build_profile64( const uint8_t * qcodes, const uint64_t * qof
         const uint32_t * qpad, const uint64_t * prof_off, const int64_t * matrix, int64_t * prof, uint32_t n_slots,
         cudaStream_t st );
 // Traceback passes.  p8: the score table fits int8.
-constexpr int TB_ROWS_PER_LANE = 4;
 cudaError_t launch_tb_forward( const TbParams & p, bool p8, int sms, cudaStream_t st );
 cudaError_t launch_tb_reverse( const TbParams & p, bool p8, int sms, cudaStream_t st );
 cudaError_t launch_tb_directions( const TbParams & p, bool nw, bool p8, int sms, cudaStream_t st );

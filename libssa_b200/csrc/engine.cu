@@ -2146,7 +2146,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         regions[h] = rg;
         last_off[h + 1] = last_off[h] + A;
     }
-    constexpr uint32_t stripe_rows = 32u * TB_ROWS_PER_LANE;
+    uint32_t stripe_rows = 0;                // of the waves: 32 x rows per lane
     bool p8 = true;
     for( int k = 0; k < 1024; k++ )
         p8 = p8 && req.matrix[k] == (int8_t) req.matrix[k];
@@ -2384,17 +2384,38 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         for( uint32_t h = 0; h < nh; h++ )
             order[h] = h;
         auto stripes = [&]( uint32_t h ) { return (rows[h] + stripe_rows - 1) / stripe_rows; };
-        std::stable_sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
-            return stripes( x ) != stripes( y ) ? stripes( x ) > stripes( y ) : cols[x] > cols[y];
-        } );
         auto need = [&]( uint32_t h ) {
             const uint64_t blocks = (cols[h] + 3u) / 4u;
             return (mode == PATHS ? (uint64_t) stripes( h ) * (blocks + 31) * 32 * sizeof(uint32_t) : 0) +
                     (stripes( h ) > 1 ? 2 * blocks * sizeof(int4) : 0);
         };
-        uint64_t total = 0;
-        for( uint32_t h = 0; h < nh; h++ )
+        // Rows per lane: 4, or 2 in the Smith-Waterman sweep of a few long hits.  A
+        // warp alone on its sub-partition takes 352 ns for a step of 4 rows and 274
+        // for one of 2 (Needleman-Wunsch: 270 for both), but 2 make twice the
+        // stripes, each 63 steps behind the one above: it pays from hits five
+        // times as long as high, while each stripe has a sub-partition and the
+        // twice as many direction words are one wave.  10 hits of 300 x 33,000:
+        // 3.8 ms with 4, 2.9 with 2; of 375 x 380 0.12 and 0.16.  SSA_B200_TB_ROWS
+        // pins it.
+        uint64_t total = 0, stripes64 = 0, columns = 0;
+        stripe_rows = 64;
+        for( uint32_t h = 0; h < nh; h++ ) {
             total += need( h );
+            stripes64 += stripes( h );
+            columns += cols[h];
+        }
+        const char * pinned = getenv( "SSA_B200_TB_ROWS" );
+        if( !p8 || !fused || mode != PATHS || (pinned ? atoi( pinned ) != 2 : stripes64 > (uint64_t) sms_ * 4 ||
+                columns < 5 * 64 * stripes64 || total > (tb_budget_ ? tb_budget_ : TB_MIN_BUDGET)) ) {
+            stripe_rows = 128;
+            total = 0;
+            for( uint32_t h = 0; h < nh; h++ )
+                total += need( h );
+        }
+        p.rows_per_lane = (int) stripe_rows / 32;
+        std::stable_sort( order.begin(), order.end(), [&]( uint32_t x, uint32_t y ) {
+            return stripes( x ) != stripes( y ) ? stripes( x ) > stripes( y ) : cols[x] > cols[y];
+        } );
         // matrices within the smallest automatic budget make one wave whatever
         // the free memory is: asking the driver for it costs up to milliseconds
         const uint64_t budget = (!tb_budget_ && total <= TB_MIN_BUDGET) ? TB_MIN_BUDGET : traceback_budget();

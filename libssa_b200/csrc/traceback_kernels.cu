@@ -33,7 +33,8 @@
 // step's fixed work (shuffles, residues, boundary, stores) once per 4 R cells.
 // R is 4: 8 rows per lane measured the same where hits fill the GPU (48 long
 // pairs 32 and 30 ms) and up to 1.7 times longer where they do not (half the
-// warps, twice the work per step).  A lane's scores of a column are one
+// warps, twice the work per step); the host takes 2 for a few Smith-Waterman
+// hits much longer than high (10 of 300 x 33,000: 3.8 -> 2.9 ms).  A lane's scores of a column are one
 // shared-memory word of int8 entries, added to the diagonal by dp4a (off the ALU
 // pipe); tables past int8 are read entry by entry.
 //
@@ -46,8 +47,8 @@
 // hit with a group barrier every 32 steps / streamed stripes, one column per
 // step / four columns per step / signs as flags and three CTAs per SM: 48 pairs
 // of 5,000-30,000 residues, SW 780 / 53 / 42 / 30 ms and NW 470 / 35 / 24 / 18
-// ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 / 4.0 ms; 320 hits of 30-1,355
-// rows 4.7 / 1.3 / 1.1 / 1.0 ms.
+// ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 / 4.0 ms (3.1 with R = 2); 320 hits
+// of 30-1,355 rows 4.7 / 1.3 / 1.1 / 1.0 ms.
 #include "device_common.cuh"
 #include "stream_stripes.cuh"
 
@@ -55,7 +56,6 @@
 
 namespace ssa {
 
-constexpr int R = TB_ROWS_PER_LANE;                   // query rows per lane
 constexpr int TB_THREADS = 128;
 constexpr int TB_WARPS = TB_THREADS / 32;
 // CTAs per SM.  Five fit, but where many long hits are aligned at once the call
@@ -67,7 +67,7 @@ constexpr int TB_WARPS = TB_THREADS / 32;
 constexpr int TB_BLOCKS = 3;
 
 // What the stripe bodies share: the lane's rows and their scores.
-template <bool P8>
+template <int R, bool P8>
 struct TbLane {
     uint32_t * table;              // P8: the warp's scores, a word of four int8 entries per code and lane
     const int32_t * smat;          // the score table, [database code][query code]
@@ -122,6 +122,7 @@ struct TbLane {
 };
 
 // Largest of the lane's new cells.
+template <int R>
 __device__ __forceinline__ int32_t column_max( const int32_t (&x)[R] ) {
     int32_t m = x[0];
 #pragma unroll
@@ -199,7 +200,7 @@ enum TbPhase { TB_FORWARD, TB_REVERSE, TB_DIRECTIONS, TB_FWDDIR, TB_NW_DIRECTION
 //    where (B - 1) x gapE < gapO + gapE, so neither pass's initial term can be
 //    the maximum there.
 // ---------------------------------------------------------------------------
-template <int PHASE, bool P8>
+template <int PHASE, int R, bool P8>
 __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) {
     constexpr int ROWS = 32 * R;
     constexpr int C = 4;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
         sp.last = (stripe + 1u) * (uint32_t) ROWS >= A;
         sp.error_flags = p.error_flags;
 
-        TbLane<P8> t;
+        TbLane<R, P8> t;
         t.table = tables[P8 ? warp : 0];
         t.smat = smat;
         t.lane = lane;
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
                 up_h[3] = y.z;
                 up_f[3] = y.w;
             }
-            typename TbLane<P8>::Column sc[C];
+            typename TbLane<R, P8>::Column sc[C];
             int32_t f[C], hv[C][R];
             // 2 bits per cell (bit 1 = insertion, LEFT | EXT_LEFT, takes priority;
             // bit 0 = deletion, UP | EXT_UP), a byte per column, the first row in its top bits
@@ -544,6 +545,7 @@ constexpr int TB_WALK_WARPS = 4;                 // hits per CTA
 constexpr int TB_WALK_MOVES = 64;
 constexpr int TB_WALK_WORDS = TB_WALK_MOVES / 4 + 1;     // words that a window spans in either direction
 
+template <int R>
 __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams p ) {
     constexpr int ROWS = 32 * R, W = TB_WALK_WORDS;
     __shared__ uint32_t win[TB_WALK_WARPS][W * W];
@@ -576,8 +578,8 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
             v[k] = 0;
             if( t < W * W && row >= 0 && blk >= 0 ) {
                 const int32_t owner = (row % ROWS) / R;        // the rows' lane, at step blk + owner
-                v[k] = dir[(uint64_t) (row / ROWS) * stripe_words +
-                        (uint64_t) (blk + owner) * 32 + owner];
+                const uint32_t * w = dir + (uint64_t) (row / ROWS) * stripe_words + (uint64_t) (blk + owner) * 32 + owner;
+                v[k] = R == 4 ? w[0] : w[0] << 4 | w[33];       // two rows: the next lane has the others a step later
             }
         }
         __syncwarp();
@@ -618,26 +620,30 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
 
 cudaError_t launch_tb_walk( const TbParams & p, cudaStream_t st ) {
     if( p.n_hits )
-        tb_walk_kernel<<<(p.n_hits + TB_WALK_WARPS - 1) / TB_WALK_WARPS, 32 * TB_WALK_WARPS, 0, st>>>( p );
+        (p.rows_per_lane == 2 ? tb_walk_kernel<2> : tb_walk_kernel<4>)<<<(p.n_hits + TB_WALK_WARPS - 1) / TB_WALK_WARPS,
+                32 * TB_WALK_WARPS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
-template <int PHASE, bool P8>
+template <int PHASE, int R, bool P8>
 static cudaError_t launch_stripes( const TbParams & p, int sms, cudaStream_t st ) {
     static LaunchShape shape;
-    const cudaError_t e = shape.set( tb_stripes_kernel<PHASE, P8>, TB_THREADS, 0 );
+    const cudaError_t e = shape.set( tb_stripes_kernel<PHASE, R, P8>, TB_THREADS, 0 );
     if( e != cudaSuccess )
         return e;
     const uint32_t want = (p.n_tickets + TB_WARPS - 1) / TB_WARPS;
     const uint32_t grid = min( want, (uint32_t) (sms * min( TB_BLOCKS, max( 1, shape.blocks ) )) );
     if( grid )
-        tb_stripes_kernel<PHASE, P8><<<grid, TB_THREADS, 0, st>>>( p );
+        tb_stripes_kernel<PHASE, R, P8><<<grid, TB_THREADS, 0, st>>>( p );
     return cudaGetLastError();
 }
 
 template <int PHASE>
 static cudaError_t launch_phase( const TbParams & p, bool p8, int sms, cudaStream_t st ) {
-    return p8 ? launch_stripes<PHASE, true>( p, sms, st ) : launch_stripes<PHASE, false>( p, sms, st );
+    if constexpr( PHASE == TB_FWDDIR || PHASE == TB_REVERSE )
+        if( p8 && p.rows_per_lane == 2 )
+            return launch_stripes<PHASE, 2, true>( p, sms, st );
+    return p8 ? launch_stripes<PHASE, 4, true>( p, sms, st ) : launch_stripes<PHASE, 4, false>( p, sms, st );
 }
 
 cudaError_t launch_tb_forward( const TbParams & p, bool p8, int sms, cudaStream_t st ) {

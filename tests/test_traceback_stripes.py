@@ -69,3 +69,29 @@ def test_pair_scores(built_library, algo):
         res, _ = oracle.search(cfg, oracle.map_codes(q.tobytes().decode(), False, True),
                                [oracle.map_codes(r.tobytes().decode(), False, False)])
         assert [h.score for h in got[i]] == [h.score for h in res], (i, len(q), len(r))
+
+
+@pytest.mark.parametrize("gap", [(-11, -1), (0, -3)])
+def test_two_rows_per_lane(built_library, monkeypatch, gap):
+    """Stripes of 64 rows, which the library takes for a few hits much longer
+    than they are high: queries around one, two and three of them."""
+    monkeypatch.setenv("SSA_B200_TB_ROWS", "2")
+    import libssa_b200 as L
+    rng = np.random.default_rng(12)
+    text = _matrix_text(1, True, rng)
+    table = oracle.parse_matrix(text)
+    queries = [W.random_residues(rng, n, W.AA20) for n in (1, 2, 3, 5, 63, 64, 65, 128, 129, 191, 260)]
+    records = [W.random_residues(rng, n, W.AA20) for n in (61, 64, 65, 68, 129, 700)]
+    records += [W.mutate(rng, np.tile(q, 2), W.AA20, 0.15, 0.05, (1, 9)) for q in queries[4:]]
+    records = [r.tobytes() for r in records]
+    product_setup(1, ("builtin", "blosum62"), gap, 1000, 2, records=records)
+    L.init_score_matrix(L.READ_FROM_STRING, text)
+    queries = [q.tobytes() for q in queries]
+    got, _ = product_search("sw", 64, 1, 12, queries, batch=True)
+    db = [oracle.map_codes(r.decode(), False, False) for r in records]
+    for qi, q in enumerate(queries):
+        cfg = oracle.SearchConfig(algo="sw", bit_width=64, align_type=1, hitcount=12, chunk_size=1000,
+                                  gap_open=gap[0], gap_extend=gap[1], lanes8=32, lanes16=16, matrix=table)
+        res, _ = oracle.search(cfg, oracle.map_codes(q.decode(), False, True), db)
+        exp = [(h.id, h.score, h.cigar, h.q_start, h.q_end, h.d_start, h.d_end) for h in res]
+        assert got[qi] == exp, (qi, len(q))
