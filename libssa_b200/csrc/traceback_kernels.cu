@@ -45,9 +45,9 @@
 //
 // Measured on a B200 (one call each): groups of 1, 2 or 4 warps of one CTA per
 // hit with a group barrier every 32 steps / streamed stripes, one column per
-// step / four columns per step / signs as flags and three CTAs per SM: 48 pairs
-// of 5,000-30,000 residues, SW 780 / 53 / 42 / 30 ms and NW 470 / 35 / 24 / 18
-// ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 / 4.0 ms (3.1 with R = 2); 320 hits
+// step / four columns per step / signs as flags and three CTAs per SM and
+// the walk by runs: 48 pairs of 5,000-30,000 residues, SW 780 / 53 / 42 / 28 ms
+// and NW 470 / 35 / 24 / 16 ms; 10 hits of 300 x 33,000 20.5 / 9.3 / 4.3 / 4.0 ms (3.1 with R = 2); 320 hits
 // of 30-1,355 rows 4.7 / 1.3 / 1.1 / 1.0 ms.
 #include "device_common.cuh"
 #include "stream_stripes.cuh"
@@ -533,27 +533,27 @@ __global__ void __launch_bounds__( TB_THREADS ) tb_stripes_kernel( TbParams p ) 
 // 4. Walk (reference: src/algo/cigar.c:300-334): one warp per hit writes the
 //    moves in traceback order (end to begin); the host run-length encodes.
 //    Each step reads the direction bits of the current cell, which the
-//    previous step chose, so a walk that reads HBM or L2 word by word waits a
-//    memory round trip per move.  In 64 moves the path stays within 64 rows
-//    and 64 columns of its current cell (every move leaves the row or the
-//    column or both by one), so the warp loads that window (at most 17 x 17
-//    words of 4 x 4 cells, ten loads per lane in flight together) into shared
-//    memory, lane 0 walks up to 64 moves from it, and the warp loads the next
-//    window.  Paths of 20,000 moves, 48 hits: 4.6 -> 2.3 ms against windows of 32 moves.
+//    previous step chose.  So that no move waits a memory round trip, the warp
+//    loads a band of words of 4 x 4 cells along the diagonal from its current
+//    cell (33 words down, 8 to either side; 18 loads per lane in flight
+//    together) into shared memory and walks until it leaves the band; and so
+//    that few moves wait for the one before, the lanes read the next 32 cells of
+//    the diagonal, the row or the column, and the moves of one kind up to the
+//    first other one are written together.  Bound by the latency of the loads
+//    and of a shared-memory read and a vote per run.  Paths of 5,500-33,000 moves,
+//    48 hits: lane 0 alone in windows of 32 and of 64 moves 4.6 and 2.3 ms, this
+//    0.64 ms.
 // ---------------------------------------------------------------------------
-constexpr int TB_WALK_WARPS = 4;                 // hits per CTA
-constexpr int TB_WALK_MOVES = 64;
-constexpr int TB_WALK_WORDS = TB_WALK_MOVES / 4 + 1;     // words that a window spans in either direction
+constexpr int TB_WALK_ROWS = 33;                 // words of the band down the diagonal
+constexpr int TB_WALK_SIDE = 8;                  // words to either side of it
+constexpr int TB_WALK_WIDTH = 2 * TB_WALK_SIDE + 1;
 
 template <int R>
-__global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams p ) {
-    constexpr int ROWS = 32 * R, W = TB_WALK_WORDS;
-    __shared__ uint32_t win[TB_WALK_WARPS][W * W];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const uint32_t h = blockIdx.x * TB_WALK_WARPS + (uint32_t) wib;
-    if( h >= p.n_hits )
-        return;                                  // the whole warp
+__global__ void __launch_bounds__( 32 ) tb_walk_kernel( TbParams p ) {
+    constexpr int ROWS = 32 * R, WORDS = TB_WALK_ROWS * TB_WALK_WIDTH, LOADS = (WORDS + 31) / 32;
+    __shared__ uint32_t band[WORDS];
+    const int lane = threadIdx.x;
+    const uint32_t h = blockIdx.x;
     const TbRegion rg = p.regions[h];
     if( rg.status != 0 ) {
         if( lane == 0 )
@@ -563,20 +563,21 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
     const uint32_t * dir = p.dirs + p.dir_off[h];
     char * out = p.ops + p.ops_off[h];
     const uint64_t cap = p.ops_off[h + 1] - p.ops_off[h];
-    const int32_t a_begin = rg.a_begin, b_begin = rg.b_begin;
+    const int32_t a_begin = max( rg.a_begin, 0 ), b_begin = max( rg.b_begin, 0 );
     const uint64_t stripe_words = (uint64_t) rg.dir_steps * 32;
-    int32_t i = rg.a_end, j = rg.b_end;
+    int32_t i = rg.a_end, j = rg.b_end;          // the same in every lane, like n
     uint64_t n = 0;
-    while( i >= a_begin && j >= b_begin && i >= 0 && j >= 0 ) {
-        // the window: word (y, x) holds rows 4 (i / 4 - y) .. + 3 of columns 4 (j / 4 - x) .. + 3
+    while( i >= a_begin && j >= b_begin ) {
+        // word (y, x): rows 4 (i4 - y) .. + 3 of columns 4 (j4 - x) .. + 3, at [y][x - y + SIDE]
         const int32_t i4 = i / 4, j4 = j / 4;
-        uint32_t v[(W * W + 31) / 32];
+        uint32_t v[LOADS];
 #pragma unroll
-        for( int k = 0; k < (W * W + 31) / 32; k++ ) {
+        for( int k = 0; k < LOADS; k++ ) {
             const int t = lane + 32 * k;
-            const int32_t row = 4 * (i4 - t / W), blk = j4 - t % W;
+            const int32_t y = t / TB_WALK_WIDTH, x = y + t % TB_WALK_WIDTH - TB_WALK_SIDE;
+            const int32_t row = 4 * (i4 - y), blk = j4 - x;
             v[k] = 0;
-            if( t < W * W && row >= 0 && blk >= 0 ) {
+            if( t < WORDS && row >= 0 && x >= 0 && blk >= 0 ) {
                 const int32_t owner = (row % ROWS) / R;        // the rows' lane, at step blk + owner
                 const uint32_t * w = dir + (uint64_t) (row / ROWS) * stripe_words + (uint64_t) (blk + owner) * 32 + owner;
                 v[k] = R == 4 ? w[0] : w[0] << 4 | w[33];       // two rows: the next lane has the others a step later
@@ -584,35 +585,42 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
         }
         __syncwarp();
 #pragma unroll
-        for( int k = 0; k < (W * W + 31) / 32; k++ )
-            if( lane + 32 * k < W * W )
-                win[wib][lane + 32 * k] = v[k];
+        for( int k = 0; k < LOADS; k++ )
+            if( lane + 32 * k < WORDS )
+                band[lane + 32 * k] = v[k];
         __syncwarp();
-        if( lane == 0 ) {
-            for( int m = 0; m < TB_WALK_MOVES && i >= a_begin && j >= b_begin && i >= 0 && j >= 0; m++ ) {
-                const uint32_t op = (win[wib][(i4 - i / 4) * W + (j4 - j / 4)] >> (8 * (j % 4) + 6 - 2 * (i % 4))) & 3u;
-                char ch;
-                if( op & 2u ) {
-                    j--;
-                    ch = 'I';
-                }
-                else if( op == 1u ) {
-                    i--;
-                    ch = 'D';
-                }
-                else {
-                    i--;
-                    j--;
-                    ch = 'M';
-                }
-                if( n < cap )
-                    out[n] = ch;
-                n++;
-            }
+        // the move at a cell (2, 3: I; 1: D; 0: M), or 4: not in the band or past the begin cell
+        auto move = [&]( int32_t r, int32_t c ) -> uint32_t {
+            if( r < a_begin || c < b_begin )
+                return 4u;
+            const int32_t y = i4 - r / 4, d = j4 - c / 4 - y + TB_WALK_SIDE;
+            if( y >= TB_WALK_ROWS || d < 0 || d >= TB_WALK_WIDTH )
+                return 4u;
+            return (band[y * TB_WALK_WIDTH + d] >> (8 * (c % 4) + 6 - 2 * (r % 4))) & 3u;
+        };
+        // `all`: which lanes' cells continue the run from lane 0's
+        auto run = [&]( unsigned all, char ch ) -> int32_t {
+            const int32_t len = all == 0xffffffffu ? 32 : __ffs( (int) ~all ) - 1;
+            if( lane < len && n + (uint64_t) lane < cap )
+                out[n + lane] = ch;
+            n += (uint64_t) len;
+            return len;
+        };
+        for( ;; ) {
+            const uint32_t m = move( i - lane, j - lane );
+            const int32_t diagonal = run( __ballot_sync( 0xffffffffu, m == 0u ), 'M' );
+            i -= diagonal;
+            j -= diagonal;
+            if( diagonal == 32 )
+                continue;
+            const uint32_t op = __shfl_sync( 0xffffffffu, m, diagonal );
+            if( op == 4u )
+                break;                           // the end, or the next band
+            if( op & 2u )
+                j -= run( __ballot_sync( 0xffffffffu, (move( i, j - lane ) & 6u) == 2u ), 'I' );
+            else
+                i -= run( __ballot_sync( 0xffffffffu, move( i - lane, j ) == 1u ), 'D' );
         }
-        i = __shfl_sync( 0xffffffffu, i, 0 );
-        j = __shfl_sync( 0xffffffffu, j, 0 );
-        n = __shfl_sync( 0xffffffffu, n, 0 );
     }
     if( lane == 0 )
         p.ops_len[h] = (uint32_t) n;
@@ -620,8 +628,7 @@ __global__ void __launch_bounds__( 32 * TB_WALK_WARPS ) tb_walk_kernel( TbParams
 
 cudaError_t launch_tb_walk( const TbParams & p, cudaStream_t st ) {
     if( p.n_hits )
-        (p.rows_per_lane == 2 ? tb_walk_kernel<2> : tb_walk_kernel<4>)<<<(p.n_hits + TB_WALK_WARPS - 1) / TB_WALK_WARPS,
-                32 * TB_WALK_WARPS, 0, st>>>( p );
+        (p.rows_per_lane == 2 ? tb_walk_kernel<2> : tb_walk_kernel<4>)<<<p.n_hits, 32, 0, st>>>( p );
     return cudaGetLastError();
 }
 
