@@ -1,4 +1,6 @@
-// sw_fast_kernel.cu -- the Smith-Waterman 8-bit-entry search pass.
+// sw_fast_kernel.cu -- the Smith-Waterman entry pass for single queries: the
+// 8-bit entry, described here, and at 16 and 64 bits the same exact scores up
+// to a limit, past which a sequence goes to the lane emulation.
 //
 // The CPU library scores every database sequence first in a lane of a
 // biased, saturating int8 vector kernel (reference:

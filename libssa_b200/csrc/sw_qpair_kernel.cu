@@ -1,10 +1,13 @@
-// sw_qpair_kernel.cu -- the Smith-Waterman 8-bit-entry search pass for
-// batches: two queries per register.
+// sw_qpair_kernel.cu -- the Smith-Waterman entry pass for batches, at every
+// width, and the Needleman-Wunsch passes: two queries per register.
 //
 // Semantics are those of sw_fast_kernel.cu (exact 16-bit scores with a +1024
-// bias per half, the first column at which a running maximum reaches 255
-// gives the reference lane's overflow block; reference:
-// src/algo/simd/search_simd_sw.c:172-182, 369-382, 422-423).  What changes is
+// bias per half; at 8 bits the first column at which a running maximum reaches
+// 255 gives the reference lane's overflow block, at 16 and 64 bits a sequence
+// that reaches the limit goes to the lane emulation; reference:
+// src/algo/simd/search_simd_sw.c:172-182, 369-382, 422-423).  The 2-column
+// kernel below is described here; the 4-column kernels, which run by default,
+// further down.  What changes is
 // what shares a register: here the low half carries query A and the high half
 // query B of a length-sorted query pair, both against the same database
 // sequence.  The profile word of a (residue, row) is then one 16x2 value that
