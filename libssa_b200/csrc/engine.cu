@@ -212,8 +212,11 @@ public:
             CUDA_CHECK( cudaEventCreate( &ev_cls_t_[2 * i] ) );
             CUDA_CHECK( cudaEventCreate( &ev_cls_t_[2 * i + 1] ) );
         }
-        CUDA_CHECK( cudaStreamCreateWithFlags( &long_stream_, cudaStreamNonBlocking ) );
+        int least = 0, greatest = 0;
+        CUDA_CHECK( cudaDeviceGetStreamPriorityRange( &least, &greatest ) );
+        CUDA_CHECK( cudaStreamCreateWithPriority( &long_stream_, cudaStreamNonBlocking, greatest ) );
         CUDA_CHECK( cudaEventCreateWithFlags( &ev_long_, cudaEventDisableTiming ) );
+        CUDA_CHECK( cudaEventCreateWithFlags( &ev_items_, cudaEventDisableTiming ) );
         device_ = dev;
         ready_ = true;
     }
@@ -637,6 +640,7 @@ private:
     cudaEvent_t ev_cls_t_[8] = {};   // per class start / end, timed (SSA_B200_TIMING)
     cudaStream_t long_stream_ = nullptr;      // an entry pass's longest pairs
     cudaEvent_t ev_long_ = nullptr;
+    cudaEvent_t ev_items_ = nullptr;     // the streamed pairs' inputs are there
     cudaEvent_t ev_ready_ = nullptr;
     cudaEvent_t ev_phase_[6] = {};
     cudaEvent_t ev_seg_[2] = {};     // around one segment's entry pass
@@ -946,7 +950,16 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     std::vector<uint32_t> fallback;
     // classes: [columns per step 1 or 4][R = 8, 16, 24, 32]
     std::vector<std::vector<uint32_t>> by_r( 8 );
-    const int bucket = db_bucket( db_.mean_len, db_.order_desc.size() );
+    // The table's costs of a small database include the latency of its longest
+    // pairs, which are streamed here, so those of a large one choose better long
+    // before 50,000 sequences.  Mean length 350, queries of 50-1,500: calls on
+    // 48,000 / 31,000 / 22,000 / 15,000 sequences 1.35 / 1.24 / 1.10 / 1.07 times as
+    // fast, the slowest query 1.00 / 1.01 / 0.81 / 0.89.  Mean lengths 150, 800 and
+    // 1,500 gain as much on average but lose up to 0.83 at 30,000 for one query or
+    // another, and keep the table's line.
+    const size_t n_ne = db_.order_desc.size();
+    const bool middling = db_.mean_len >= 250.0 && db_.mean_len < 500.0;
+    const int bucket = db_bucket( db_.mean_len, middling && n_ne >= 30000 ? std::max<size_t>( n_ne, 50000 ) : n_ne );
     // SSA_B200_FAST_SHAPE=G,R[,C] pins the shape and the kernel (tuning, tests)
     int pin_g = 0, pin_r = 0, pin_c = 1;
     if( const char * pin = getenv( "SSA_B200_FAST_SHAPE" ) ) {
@@ -1103,7 +1116,9 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
         if( const char * cap_env = getenv( "SSA_B200_FAST_CTAS" ) )
             per_sm = std::min( per_sm, std::max( 1, atoi( cap_env ) ) );
         const int grid = sms_ * std::max( 1, per_sm );
-        CUDA_CHECK( cudaStreamWaitEvent( class_stream_[ri], ev_ready_, 0 ) );
+        // after the streamed pairs, which are the longest: a grid that fills the GPU
+        // before they start would have them wait for its end
+        CUDA_CHECK( cudaStreamWaitEvent( class_stream_[ri], pair_skip ? ev_items_ : ev_ready_, 0 ) );
         unsigned long long * unit_counter = d_counts_.as<unsigned long long>() + 8 + ri;   // bytes 64..95
         CUDA_CHECK( cudaMemsetAsync( unit_counter, 0, sizeof(unsigned long long), class_stream_[ri] ) );
         p.pair_res = d_pair_res_.as<uint8_t>();
@@ -1540,7 +1555,9 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         int per_sm = 0;
         CUDA_CHECK( launch( p, 0, &per_sm ) );
         const int grid = sms_ * std::max( 1, per_sm );
-        CUDA_CHECK( cudaStreamWaitEvent( class_stream_[ri], ev_ready_, 0 ) );
+        // after the streamed pairs, which are the longest: a grid that fills the GPU
+        // before they start would have them wait for its end
+        CUDA_CHECK( cudaStreamWaitEvent( class_stream_[ri], !items.empty() ? ev_items_ : ev_ready_, 0 ) );
         unsigned long long * unit_counter = d_counts_.as<unsigned long long>() + 8 + ri;   // bytes 64..95
         CUDA_CHECK( cudaMemsetAsync( unit_counter, 0, sizeof(unsigned long long), class_stream_[ri] ) );
         p.db = db_view();
@@ -1621,22 +1638,36 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
         cudaStream_t st, bool marked ) {
     const bool nw = req.algo == 1;
     // queries with the most rows first: their items have the most stripes
-    std::stable_sort( items.begin(), items.end(), [&]( const SwStreamItem & x, const SwStreamItem & y ) {
-        return h_qlen_[x.slot] > h_qlen_[y.slot];
-    } );
+    auto longer = [&]( const SwStreamItem & x, const SwStreamItem & y ) { return h_qlen_[x.slot] > h_qlen_[y.slot]; };
+    if( !std::is_sorted( items.begin(), items.end(), longer ) )
+        std::stable_sort( items.begin(), items.end(), longer );
+    // the items' lengths, and per run of items of one query their number, steps
+    // of a stripe in all and the most of one
+    struct Run {
+        uint64_t qlen, items, columns, longest;
+    };
+    std::vector<Run> runs;
+    std::vector<uint32_t> len( items.size() );
+    for( size_t k = 0; k < items.size(); k++ ) {
+        if( k == 0 || items[k].slot != items[k - 1].slot )
+            runs.push_back( Run{ h_qlen_[items[k].slot], 0, 0, 0 } );
+        Run & r = runs.back();
+        len[k] = db_.len[items[k].id_a];              // A is the longer
+        const uint64_t c = len[k] / 4 + 31;
+        r.items++;
+        r.columns += c;
+        r.longest = std::max( r.longest, c );
+    }
     // Rows per lane: 4 while every stripe of 128 rows can be resident (16 warps per
     // SM), else whichever of 4 .. 6 computes the items' stripes in the fewest
     // instructions (a step of R rows is 26 R + 20 of the ALU's).  964 items of 300
     // rows on 2 CTAs per SM: 5.47 ms with 4 (384 rows computed), 3.94 with 5 (320);
     // 7 and 8 were never the best on batches of 30-1,800 rows (7.3 with 5, 7.4 with
     // 6, 8.3 and 8.8 ms).  SSA_B200_STREAM_ROWS pins it.
-    auto stripes = [&]( const SwStreamItem & t, int r ) {
-        return (uint64_t) ((h_qlen_[t.slot] + 32u * (uint32_t) r - 1u) / (32u * (uint32_t) r));
-    };
-    auto columns = [&]( const SwStreamItem & t ) { return (uint64_t) db_.len[t.id_a] / 4 + 31; };    // steps of a stripe
+    auto stripes = []( const Run & q, int r ) { return (q.qlen + 32u * (uint64_t) r - 1u) / (32u * (uint64_t) r); };
     uint64_t stripes128 = 0;
-    for( const SwStreamItem & t : items )
-        stripes128 += stripes( t, 4 );
+    for( const Run & q : runs )
+        stripes128 += q.items * stripes( q, 4 );
     int R = 4;
     const char * pinned = getenv( "SSA_B200_STREAM_ROWS" );
     if( !nw && pinned && atoi( pinned ) >= 4 && atoi( pinned ) <= 6 )
@@ -1645,8 +1676,8 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
         uint64_t least = UINT64_MAX;
         for( int r = 4; r <= 6; r++ ) {
             uint64_t cost = 0;
-            for( const SwStreamItem & t : items )
-                cost += stripes( t, r ) * columns( t );
+            for( const Run & q : runs )
+                cost += stripes( q, r ) * q.columns;
             cost *= 26u * (uint64_t) r + 20u;
             if( cost < least ) {
                 least = cost;
@@ -1662,9 +1693,9 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
     // 30-1,800 rows (3.6) 7.4 / 7.1 / 7.1 ms, Needleman-Wunsch of 10,000 (5.6) 1.11
     // / 1.01 / 0.99 ms; fewer items than warps the same on all.
     uint64_t steps = 0, longest = 1;
-    for( const SwStreamItem & t : items ) {
-        steps += stripes( t, R ) * columns( t );
-        longest = std::max( longest, columns( t ) + 47 * stripes( t, R ) );
+    for( const Run & q : runs ) {
+        steps += stripes( q, R ) * q.columns;
+        longest = std::max( longest, q.longest + 47 * stripes( q, R ) );
     }
     const int ctas = (int) std::min<uint64_t>( 4, std::max<uint64_t>( 2, steps / ((uint64_t) sms_ * 4 * longest) ) );
     const uint32_t rows = 32u * (uint32_t) R;
@@ -1673,11 +1704,11 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
     // launches of as many items as 1 GB of boundary rows holds
     for( uint32_t i0 = 0; i0 < ni; ) {
         std::vector<uint64_t> bnd;
+        bnd.reserve( ni - i0 );
         uint64_t words = 0;
         uint32_t i1 = i0;
         for( ; i1 < ni; i1++ ) {
-            const SwStreamItem & t = items[i1];
-            const uint64_t w = h_qlen_[t.slot] > rows ? 2ull * ((db_.len[t.id_a] + 3u) / 4u) : 0;   // A is the longer
+            const uint64_t w = h_qlen_[items[i1].slot] > rows ? 2ull * ((len[i1] + 3u) / 4u) : 0;
             if( i1 > i0 && (words + w) * sizeof(int4) > ((uint64_t) 1 << 30) )
                 break;
             bnd.push_back( words );
@@ -1730,6 +1761,8 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
         p.sink.error_flags = d_counts_.as<unsigned>() + 2;
+        if( i0 == 0 )
+            CUDA_CHECK( cudaEventRecord( ev_items_, st ) );
         CUDA_CHECK( nw ? launch_nw_stream( p, sms_, st ) : launch_sw_stream( R, p, sms_, st ) );
         launches_++;
         i0 = i1;
