@@ -789,15 +789,16 @@ static bool needs_int64( const SearchRequest & req, uint32_t max_qlen, uint32_t 
     return m > (int64_t) INT32_MAX / 2 || steps * (m + 1) * 2 > (int64_t) INT32_MAX;
 }
 
-// The 16x2 pass reproduces the 8-bit Smith-Waterman lanes exactly when the
-// gap extension is not positive and the truncated 8-bit open+extend cost lies
-// in [-128, gapE]; other parameters run the exact lane emulation.
 // Needleman-Wunsch at the 16-bit entry: the query-pair kernel scores exactly
 // the sequences short enough that no value can come near the int16 limits
-// (nw_qpair_kernel); it needs non-positive gap costs.
-// The 64-bit entry takes the same kernel where the score table fits int16.
+// (nw_qpair_kernel); it needs non-positive gap costs, and at 16 bits a cost for
+// a gap of one: the lane's overflow line, -32768 - gapO - gapE - 1 in 16 bits,
+// wraps to 32767 where that is 0, and every sequence then overflows in its first
+// block.  The 64-bit entry takes the same kernel where the score table fits int16.
 static bool nw_fast_eligible( const SearchRequest & req ) {
     if( req.algo != 1 || req.bit_width == 8 || getenv( "SSA_B200_NO_FAST" ) )
+        return false;
+    if( req.bit_width == 16 && req.gap_open + req.gap_extend == 0 )
         return false;
     for( int k = 0; k < 1024 && req.bit_width == 64; k++ )
         if( req.matrix[k] != (int16_t) req.matrix[k] )
@@ -806,7 +807,9 @@ static bool nw_fast_eligible( const SearchRequest & req ) {
 }
 
 // The running maximum at which the 16x2 Smith-Waterman kernels end a
-// sequence, 0 where they do not apply.  8-bit entry: 255, the lane's own
+// sequence, 0 where they do not apply.  They reproduce the 8-bit lanes exactly
+// when the gap extension is not positive and the truncated 8-bit open+extend cost
+// lies in [-128, gapE]; other parameters run the exact lane emulation.  8-bit entry: 255, the lane's own
 // overflow.  At 16 and 64 bits the lane saturates far above (65535) or not at
 // all, and the kernels are exact up to where a 16-bit half could leave its
 // range: a cell below the limit plus one score-table entry stays below 0x7c00
