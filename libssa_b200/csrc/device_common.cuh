@@ -324,7 +324,7 @@ struct QPairParams {
     int gap_open;
     const uint32_t * qlen;        // per slot
     const uint32_t * qp_lmax;     // per query pair: longest sequence the kernel scores exactly
-    // (longer sequences go to sink.redo for the lane emulation)
+    // (longer sequences go to sink.redo for the lane emulation, or nowhere without it)
     bool marked_only;             // score only the pairs that hold SCORE_REQUEUED
 };
 

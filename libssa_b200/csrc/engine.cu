@@ -1391,10 +1391,13 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     const uint32_t * dev_qslots = stage_.add( qp_slots.data(), qp_slots.size(), stream_ );
     const uint32_t * dev_units = stage_.add( units.data(), units.size(), stream_ );
     const uint32_t * dev_lmax = stage_.add( qp_lmax.data(), qp_lmax.size(), stream_ );
-    // pairs outside the kernels' range, for the lane emulation (the 8-bit entry has none)
-    const bool redo = req.bit_width != 8;
+    // Pairs outside the kernels' range, for the lane emulation (the 8-bit entry has
+    // none).  Needleman-Wunsch: the sequences longer than a pair of queries' limit,
+    // which the emulation scores beside the entry pass (`beyond`); of a marked pass
+    // only the device knows which of them it wants.
+    const bool redo = nw ? marked : req.bit_width != 8;
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
-    if( redo )
+    if( req.bit_width != 8 )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
     // work units: ranges of length-sorted sequences (multiples of what a CTA
     // holds side by side) with about equal numbers of columns, the longest
@@ -1506,6 +1509,32 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     const uint2 * dev_skip = stage_.add( qp_skip.data(), qp_skip.size(), stream_ );
     stage_.send( stream_ );
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
+    // The pairs beyond the range, longest first.  A warp of the emulation takes all of
+    // a pair's rows and columns one after the other, so a few long pairs run beside
+    // the entry kernels; more than four per resident warp keep the GPU busy alone and
+    // follow, because the entry kernels' shared memory leaves them little L1 cache.
+    // After the pass / beside it, one query against proteins of mean length 350
+    // (calls on a B200): 64-bit entry 1,300 x 1,000 6.4 / 4.0 ms, 2,000 x 10,000 12.2 /
+    // 7.9; 16-bit entry 2,000 x 10,000 15.4 / 11.6; 15,289 pairs of 2,500 28.0 / 30.6.
+    std::vector<PairTask> beyond;
+    for( uint32_t k = 0; nw && !marked && k < n_seq; k++ ) {
+        const uint32_t id = db_.order_desc[lo + k];
+        bool any = false;
+        for( uint32_t i = 0; i < n_qp; i++ ) {
+            if( db_.len[id] <= qp_lmax[i] )
+                continue;
+            any = true;
+            for( int h = 0; h < 2 && (k < qp_skip[i].x || k >= qp_skip[i].y); h++ )
+                if( qp_slots[2 * i + h] != 0xffffffffu )
+                    beyond.push_back( PairTask{ qp_slots[2 * i + h], id, 0, 0 } );
+        }
+        if( !any )                      // nor is a shorter one
+            break;
+    }
+    const PairTask * beyond_tasks = stage_.add( beyond.data(), beyond.size(), stream_ );
+    const bool beside = beyond.size() <= (size_t) sms_ * 64;
+    if( beside )
+        run_pass( 1, req.bit_width, req, nq, beyond_tasks, beyond.size(), false, next, next_count, cap );
     if( !items.empty() ) {
         PassSink lists{};
         lists.next = next;
@@ -1627,6 +1656,11 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
                     cells / (ms * 1e-3) / 1e9 );
         }
     }
+    if( timing )
+        fprintf( stderr, "[ssa timing] %zu pairs beyond the 16-bit range, %s the entry pass\n", beyond.size(),
+                beside ? "beside" : "after" );
+    if( !beside )
+        run_pass( 1, req.bit_width, req, nq, beyond_tasks, beyond.size(), false, next, next_count, cap );
     if( !fallback.empty() ) {
         const uint32_t * dev_slots = stage_.add( fallback.data(), fallback.size(), stream_ );
         run_pass( req.algo, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_seq, true, next,

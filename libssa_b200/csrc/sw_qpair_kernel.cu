@@ -870,7 +870,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair_kernel( QPairParams 
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const bool exact = valid && L <= lmax;
-            if( valid && !exact && k == 0 ) {
+            if( valid && !exact && k == 0 && p.sink.redo ) {
                 // beyond the guarded range: the lane emulation scores it
                 const uint32_t slots[2] = { slot_a, slot_b };
                 for( int h = 0; h < 2; h++ ) {
@@ -1181,7 +1181,7 @@ __global__ void __launch_bounds__( QP_THREADS, 4 ) nw_qpair4_kernel( QPairParams
             const uint32_t id = valid ? p.order[idx] : 0u;
             const uint32_t L = valid ? p.db.lens[id] : 0u;
             const bool exact = valid && L <= lmax;
-            if( valid && !exact && k == 0 ) {
+            if( valid && !exact && k == 0 && p.sink.redo ) {
                 // beyond the guarded range: the lane emulation scores it
                 const uint32_t slots[2] = { slot_a, slot_b };
                 for( int h = 0; h < 2; h++ ) {
