@@ -648,6 +648,7 @@ private:
     // the current queries and score table: in the stager, or the server's own block
     DevView d_qcodes_, d_qoff_, d_qlen_, d_qpad_, d_prof_off_, d_matrix_;
     DevBuf d_prof_, d_serve_block_;
+    std::vector<uint64_t> blocks_before_;             // of an entry pass
     Stager stage_;
     PinnedBuf h_counts_;
     DevBuf d_score_, d_list_a_, d_list_b_, d_counts_, d_scratch_, d_list_c_, d_sw_sync_, d_sw_bnd_;
@@ -928,18 +929,141 @@ static FastShape choose_shape( uint32_t Q, double mean_len, int bucket ) {
     return best;
 }
 
-// Steps above which an entry pass gives a pair to the streamed stripes: every
-// resident group's share of the pass, at least 64.  Entry pass on a B200 with
-// the line at none / 256 / 64 steps: 4 queries of 200 x 500 proteins 1.51 / 0.62
-// / 0.27 ms, one of 1,000 x 3,000 1.11 / 0.71 / 0.56, one of 128 x 2,000 0.37 /
-// 0.25 / 0.24, 8 of 300 x 3,000 5.0 / 1.5 / 1.6; below the share the streamed
-// kernel loses to the entry kernel (32 x 20,000, share 7,350: 16.7 ms, at 800
-// 19.7).  SSA_B200_STREAM_SHARE pins the line (tests).
-static uint64_t stream_share( uint64_t share ) {
-    if( const char * pin = getenv( "SSA_B200_STREAM_SHARE" ) )
-        return strtoull( pin, nullptr, 10 );
-    return std::max<uint64_t>( share, 64 );
-}
+// Which of an entry pass's pairs go to the streamed stripes (run_stream).  A group
+// of threads of the entry kernel takes the passes x blocks steps of a pair one
+// after the other; the whole pass takes `share` steps of every resident group,
+// and a pair of more steps than that still runs when the rest is done.  On
+// streamed stripes it ends sooner, but costs more instructions (stripes of 128
+// rows and more, 31 steps to fill each) and host time per item.  So the pairs of
+// more steps than the share, and than 64, are streamed where an estimate of the
+// pass's time says that this pays; none where the longest has less than half as
+// many again.  Needleman-Wunsch queries without a partner, for which the entry
+// kernel computes an empty half, may go there whole.
+// Calls on a B200, none streamed / always those above the share (lone
+// Needleman-Wunsch queries whole) / chosen: Smith-Waterman, 30 x 20,000 nucleotide
+// records of 100-1,500 0.56 / 0.83 / 0.56 ms, 300 x 1,500 proteins 0.60 / 0.35 /
+// 0.36, 2 of 30 x 20,000 nucleotide records 0.91 / 1.36 / 0.92; Needleman-Wunsch,
+// 30 x 100,000 reads of 80-150 0.74 / 1.85 / 0.76, 300 x 5,000 proteins 1.65 / 0.49 /
+// 0.50, 32 of 30 x 1,000 nucleotide records 1.65 / 2.18 / 1.63.  Over 1,600 calls of 1 to
+// 32 queries of 30-2,500 against 150-100,000 records, forced both ways, the choice
+// loses 0.4% to the better of the two on average.
+class StreamLine {
+public:
+    // Cycles of an SM sub-partition's ALU: `step` x (26 R + 20) for a warp's step of
+    // R rows over a block of four columns, at least alone0 + alone1 R while it has
+    // the sub-partition to itself; `stream` for a streamed step.  All fitted to the
+    // calls above, each forced both ways, so that the choice between them is right.
+    struct Costs {
+        double step, alone0, alone1, stream;
+    };
+    static constexpr Costs SW_SINGLE{ 2.8, 1430, 30, 450 }, SW_PAIRS{ 2.4, 1500, 25, 225 }, NW_PAIRS{ 1.3, 700, 60, 130 };
+    // A query, or pair of queries, of the entry kernel.
+    struct Query {
+        uint64_t passes;
+        int R;                       // rows per thread
+        bool one_column;             // a step is one column, not a block of four
+        uint32_t rows[2];            // query lengths (0: none)
+        uint32_t from;               // the units before this one are not streamed
+    };
+    // blocks[k]: blocks of four columns of the units (sequences, or pairs of them;
+    // longest first) before unit k; a streamed item holds item_units of them.
+    // lone_whole: queries without a partner may be streamed whole.
+    StreamLine( const Costs & costs, bool lone_whole, int sms, int groups_per_warp, uint32_t item_units,
+            const std::vector<uint64_t> & blocks, const std::vector<Query> & queries )
+        : costs_( costs ), sms_( sms ), groups_( groups_per_warp ), item_units_( item_units ), blocks_( blocks ),
+          queries_( queries ) {
+        uint64_t steps = 0, longest = 0;
+        for( const Query & q : queries_ ) {
+            steps += q.passes * blocks_[units()];
+            longest = std::max( longest, q.passes * unit( first( q ) ) );
+        }
+        const uint64_t share = std::max<uint64_t>( 64, steps / ((uint64_t) sms_ * 16 * (uint64_t) groups_) );
+        // SSA_B200_STREAM_SHARE pins the line (tests)
+        if( const char * pin = getenv( "SSA_B200_STREAM_SHARE" ) ) {
+            line_ = strtoull( pin, nullptr, 10 );
+            return;
+        }
+        double least = cycles( {} );
+        auto consider = [&]( const Choice & c ) {
+            const double t = cycles( c );
+            if( t < least ) {
+                least = t;
+                line_ = c;
+            }
+        };
+        const bool uneven = 2 * longest > 3 * share;
+        if( uneven )
+            consider( { share } );
+        // (the estimate is not fitted to longer passes: 300 x 200,000 proteins, a share
+        // of 2,800 steps, 9.3 ms and whole 14.2)
+        if( lone_whole && share < 2048 )
+            consider( { uneven ? share : UINT64_MAX, true } );
+    }
+    // the first unit that stays with the entry kernel
+    uint32_t end( const Query & q ) const { return end( q, line_ ); }
+
+private:
+    struct Choice {
+        uint64_t line = UINT64_MAX;      // pairs of more steps are streamed
+        bool lone = false;               // queries without a partner whole
+        Choice( uint64_t l = UINT64_MAX, bool w = false ) : line( l ), lone( w ) {}
+    };
+    uint32_t units() const { return (uint32_t) blocks_.size() - 1; }
+    uint64_t unit( uint32_t k ) const { return k < units() ? blocks_[k + 1] - blocks_[k] : 0; }
+    uint32_t first( const Query & q ) const { return std::min( q.from, units() ); }
+    uint32_t end( const Query & q, const Choice & c ) const {
+        const uint64_t line = c.lone && q.rows[1] == 0 ? 0 : c.line;
+        uint32_t a = first( q ), b = units();
+        while( a < b ) {
+            const uint32_t mid = (a + b) / 2;
+            if( q.passes * unit( mid ) <= line )
+                b = mid;
+            else
+                a = mid + 1;
+        }
+        return a;
+    }
+    // The pass's time with the choice's pairs streamed: the work of a
+    // sub-partition, four warps of the entry kernel side by side, and what is then
+    // left of the longest kept pair; at least the longest streamed pair, or the
+    // longest one beyond the kernels' range in the lane emulation.
+    double cycles( const Choice & c ) const {
+        double work = 0, items = 0, last = 0, tail = 0;
+        auto step = [&]( const Query & q ) { return costs_.step * (26.0 * q.R + (q.one_column ? 80.0 : 20.0)); };
+        for( const Query & q : queries_ ) {
+            const uint32_t from = first( q ), to = end( q, c );
+            const double n = to - from, cols = (double) (blocks_[to] - blocks_[from]);
+            work += (double) q.passes * ((double) (blocks_[units()] - blocks_[from]) - cols) * step( q ) /
+                    (groups_ * 4.0 * sms_);
+            if( from )
+                last = std::max( last, (q.rows[0] + 255u) / 256u * 4.0 * (double) unit( 0 ) * EMULATED_COLUMN );
+            for( uint32_t rows : q.rows ) {
+                if( rows == 0 || to == from )
+                    continue;
+                const double stripes = (rows + 127u) / 128u;
+                work += stripes * (cols + 31.0 * n) / item_units_ * costs_.stream / (4.0 * sms_);
+                items += n / item_units_;
+                last = std::max( last, ((double) unit( from ) + 47.0 * stripes) * STREAM_ALONE );
+            }
+        }
+        for( const Query & q : queries_ ) {
+            const double alone = costs_.alone0 + costs_.alone1 * q.R;
+            const double left = (double) (q.passes * unit( end( q, c ) )) - work / std::max( alone, 4.0 * step( q ) );
+            tail = std::max( tail, left * alone );
+        }
+        return ITEM * items + std::max( work + tail, last );
+    }
+    static constexpr double STREAM_ALONE = 200.0;     // a streamed step with the sub-partition to itself
+    static constexpr double EMULATED_COLUMN = 800.0;  // a column of 256 rows in the lane emulation
+    static constexpr double ITEM = 40.0;              // host time
+
+    Costs costs_;
+    int sms_, groups_;
+    uint32_t item_units_;
+    const std::vector<uint64_t> & blocks_;
+    const std::vector<Query> & queries_;
+    Choice line_;
+};
 
 void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * next, unsigned * next_count,
         uint32_t cap ) {
@@ -1012,9 +1136,12 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     // (no idle groups) and, where the columns allow, no more: on a small
     // database the longest pairs then run side by side in separate warps
     // instead of one after another in the same warp.
-    uint64_t total_cols = 0;
-    for( uint32_t c : db_.pair_cols )
-        total_cols += c;
+    std::vector<uint64_t> & blocks = blocks_before_;     // of four columns, of the pairs before each
+    blocks.resize( n_pairs + 1 );
+    blocks[0] = 0;
+    for( uint32_t k = 0; k < n_pairs; k++ )
+        blocks[k + 1] = blocks[k] + db_.pair_cols[k] / 4u;
+    const uint64_t total_cols = 4 * blocks[n_pairs];
     int g_min = 32;
     for( uint32_t s = 0; s < nq; s++ )
         if( shape[s].G )
@@ -1056,20 +1183,18 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
     if( req.bit_width != 8 )
         CUDA_CHECK( cudaMemsetAsync( redo_count, 0, sizeof(unsigned), stream_ ) );
-    // the longest pairs on streamed stripes, as in run_qpair_entry: those that
-    // take more steps than every resident group's share of the pass
+    // the longest pairs on streamed stripes
     uint32_t pair_skip = 0;
     std::vector<SwStreamItem> items;
     if( nq == 1 && n_shaped == 1 && (!pin_g || getenv( "SSA_B200_STREAM_SHARE" )) ) {
-        const uint64_t groups = (uint64_t) sms_ * 16 * (32u / (uint32_t) shape[0].G);
-        const uint64_t P = (uint64_t) shape[0].P;
-        const uint64_t share = stream_share( P * (total_cols / 4u) / groups );
-        if( 2 * P * (db_.pair_cols[0] / 4u) > 3 * share )
-            while( pair_skip < n_pairs && P * (db_.pair_cols[pair_skip] / 4u) > share ) {
-                items.push_back( SwStreamItem{ 0, db_.pair_a[pair_skip], db_.pair_b[pair_skip], 0 } );
-                pair_skip++;
-            }
+        const FastShape & fs = shape[0];
+        const std::vector<StreamLine::Query> queries{ { (uint64_t) fs.P, fs.R, fs.C != 4, { h_qlen_[0], 0 }, 0 } };
+        pair_skip = StreamLine( StreamLine::SW_SINGLE, false, sms_, 32 / fs.G, 1, blocks, queries ).end( queries[0] );
+        for( uint32_t k = 0; k < pair_skip; k++ )
+            items.push_back( SwStreamItem{ 0, db_.pair_a[k], db_.pair_b[k], 0 } );
     }
+    if( getenv( "SSA_B200_TIMING" ) )
+        fprintf( stderr, "[ssa timing] entry pass: %zu items streamed\n", items.size() );
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     if( pair_skip ) {
         PassSink lists{};
@@ -1403,9 +1528,12 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     // holds side by side) with about equal numbers of columns, the longest
     // first; every pair of a class gets every range.  A CTA takes one unit at a
     // time (a warp, in the 2-column kernels).
-    uint64_t total_cols = 0;
-    for( uint32_t i = lo; i < hi; i++ )
-        total_cols += (db_.len[db_.order_desc[i]] + 3u) & ~3u;
+    std::vector<uint64_t> & blocks = blocks_before_;     // of four columns, of the sequences before each
+    blocks.resize( n_seq + 1 );
+    blocks[0] = 0;
+    for( uint32_t k = 0; k < n_seq; k++ )
+        blocks[k + 1] = blocks[k] + (db_.len[db_.order_desc[lo + k]] + 3u) / 4u;
+    const uint64_t total_cols = 4 * blocks[n_seq];
     constexpr uint32_t CTA_SEQS = QP_THREADS_PER_CTA / QP_G;
     const uint64_t want_units = (uint64_t) sms_ * 16 * 24;
     const uint64_t target = std::max<uint64_t>( 1, total_cols * std::max<uint32_t>( 1, n_qp ) / want_units );
@@ -1413,7 +1541,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     {
         uint64_t acc = 0;
         for( uint32_t i = 0; i < n_seq; i++ ) {
-            acc += (db_.len[db_.order_desc[lo + i]] + 3u) & ~3u;
+            acc += 4 * (blocks[i + 1] - blocks[i]);
             if( acc >= target && (i + 1) % CTA_SEQS == 0 ) {
                 bounds.push_back( i + 1 );
                 acc = 0;
@@ -1434,78 +1562,43 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
     const uint32_t scratch_cols = (((db_.max_len + 3u) & ~3u) >> 1) + 2u;
     const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
-    uint64_t seg_residues = 0;
-    for( uint32_t i = lo; i < hi; i++ )
-        seg_residues += db_.len[db_.order_desc[i]];
-    // The longest sequences against the longest queries on streamed stripes.  A
-    // group of 4 threads takes passes x blocks steps for a pair, one after the
-    // other; the whole call takes `share` steps of every resident group.  Pairs
-    // of more steps than that would still run when the rest is done.  Measured on
-    // a B200: a server's 32 requests against 100,000 proteins, whose first wave
-    // holds the longest sequences, 108 -> 96 ms; one query of 300 x 200,000
-    // with 1% of 8,000-35,000 residues (run_fast_entry) entry pass 28.5 -> 5.9
-    // ms, half of it because both sequences of a pair overflow early and end
-    // it.  Where no pair takes half as long again as the
-    // share, the entry kernel keeps them all (it needs fewer instructions per
-    // cell: four chains of 20-28 rows against 4 or 8).  A Needleman-Wunsch query
-    // without a partner goes there whole in calls of less than 2,048 steps per
-    // group: the entry kernel computes an empty half for it, and its longest
-    // pairs take most of such a call (one of 250 x 20,000 proteins, 280 steps,
-    // 1.97 -> 1.00 ms; 500 x 50,000 reads, 2,640 steps, 6.8 and 6.6; 300 x
-    // 200,000, 2,800 steps, 9.3 and 14.2).  Batches: 4 of 200 x 500 1.31 -> 0.31
-    // ms, 8 of 300 x 3,000 7.3 -> 5.0, 64 reads x 20,000 unchanged.
-    constexpr uint64_t NW_STREAM_SHARE = 2048;
+    // the longest sequences against the longest queries on streamed stripes
     const bool table8 = nw ? nw_table8 : fast_single_eligible( req );
     const bool pinned = pin || pin_mb || pin_c || pin_h || pin_g8;      // a pinned shape keeps the entry kernel
     std::vector<uint2> qp_skip( std::max<uint32_t>( 1, n_qp ), make_uint2( 0, 0 ) );
     std::vector<SwStreamItem> items;
-    if( table8 && (!pinned || getenv( "SSA_B200_STREAM_SHARE" )) ) {
-        auto passes_of = [&]( uint32_t i, int R ) { return (uint64_t) qp_rows[i] / (uint64_t) (QP_G * R); };
-        auto len_of = [&]( uint32_t i ) { return db_.len[db_.order_desc[lo + i]]; };
-        // the first sequence from k on that satisfies `past` (monotonic: the lengths descend)
-        auto first = [&]( uint32_t k, auto past ) {
-            uint32_t a = k, b = n_seq;
-            while( a < b ) {
-                const uint32_t mid = (a + b) / 2;
-                if( past( mid ) )
-                    b = mid;
-                else
-                    a = mid + 1;
-            }
-            return a;
-        };
-        uint64_t steps = 0, longest = 0;
+    if( n_qp && table8 && (!pinned || getenv( "SSA_B200_STREAM_SHARE" )) ) {
+        std::vector<StreamLine::Query> queries( n_qp );
         for( int ri = 0; ri < 4; ri++ )
             for( uint32_t i : by_r[ri] ) {
-                steps += passes_of( i, 4 * (ri + 4) ) * (total_cols / 4u);
-                longest = std::max<uint64_t>( longest, passes_of( i, 4 * (ri + 4) ) * ((len_of( 0 ) + 3u) / 4u) );
-            }
-        const uint64_t share = stream_share( steps / ((uint64_t) sms_ * 16 * QP_GPW) );
-        for( int ri = 0; ri < 4; ri++ )
-            for( uint32_t i : by_r[ri] ) {
-                const uint64_t P = passes_of( i, 4 * (ri + 4) );
-                const bool single = qp_slots[2 * i + 1] == 0xffffffffu;
-                const uint32_t Q = h_qlen_[qp_slots[2 * i]];
+                StreamLine::Query & q = queries[i];
+                q = StreamLine::Query{ qp_rows[i] / (uint64_t) (QP_G * 4 * (ri + 4)), 4 * (ri + 4), false, { 0, 0 }, 0 };
+                for( int h = 0; h < 2; h++ )
+                    if( qp_slots[2 * i + h] != 0xffffffffu )
+                        q.rows[h] = h_qlen_[qp_slots[2 * i + h]];
                 // Needleman-Wunsch: within the exact range for stripes of 128
                 // rows (the entry kernel sends the longer ones to the redo list)
-                const int64_t most = nw ? nw_budget / nw_step - (int64_t) ((Q + 127u) & ~127u) - 4 : INT64_MAX;
-                const uint32_t from = first( 0, [&]( uint32_t k ) { return (int64_t) len_of( k ) <= most; } );
-                uint32_t to = from;
-                if( nw && single && share < NW_STREAM_SHARE )
-                    to = n_seq;
-                else if( 2 * longest > 3 * share )
-                    to = first( from, [&]( uint32_t k ) { return P * ((len_of( k ) + 3u) / 4u) <= share; } );
-                if( to < n_seq && ((to - from) & 1u) )
-                    to++;
-                qp_skip[i] = make_uint2( from, to );
-                for( int h = 0; h < 2; h++ ) {
-                    const uint32_t slot = qp_slots[2 * i + h];
-                    for( uint32_t k = from; k < to && slot != 0xffffffffu; k += 2 )
-                        items.push_back( SwStreamItem{ slot, db_.order_desc[lo + k],
-                                k + 1 < to ? db_.order_desc[lo + k + 1] : 0xffffffffu, 0 } );
-                }
+                const int64_t most = nw ? nw_budget / nw_step - (int64_t) ((q.rows[0] + 127u) & ~127u) - 4 : INT64_MAX;
+                while( q.from < n_seq && (int64_t) db_.len[db_.order_desc[lo + q.from]] > most )
+                    q.from++;
             }
+        const StreamLine line( nw ? StreamLine::NW_PAIRS : StreamLine::SW_PAIRS, nw, sms_, QP_GPW, 2, blocks, queries );
+        for( uint32_t i = 0; i < n_qp; i++ ) {
+            const uint32_t from = queries[i].from;
+            uint32_t to = line.end( queries[i] );
+            if( to < n_seq && ((to - from) & 1u) )
+                to++;
+            qp_skip[i] = make_uint2( from, to );
+            for( int h = 0; h < 2; h++ ) {
+                const uint32_t slot = qp_slots[2 * i + h];
+                for( uint32_t k = from; k < to && slot != 0xffffffffu; k += 2 )
+                    items.push_back( SwStreamItem{ slot, db_.order_desc[lo + k],
+                            k + 1 < to ? db_.order_desc[lo + k + 1] : 0xffffffffu, 0 } );
+            }
+        }
     }
+    if( timing )
+        fprintf( stderr, "[ssa timing] entry pass: %zu items streamed\n", items.size() );
     const uint2 * dev_skip = stage_.add( qp_skip.data(), qp_skip.size(), stream_ );
     stage_.send( stream_ );
     CUDA_CHECK( cudaEventRecord( ev_ready_, stream_ ) );
@@ -1648,7 +1741,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
             double cells = 0, padded = 0;
             for( uint32_t i : by_r[ri] ) {
                 const uint32_t a = qp_slots[2 * i], b = qp_slots[2 * i + 1];
-                cells += (double) (h_qlen_[a] + (b == 0xffffffffu ? 0u : h_qlen_[b])) * (double) seg_residues;
+                cells += (double) (h_qlen_[a] + (b == 0xffffffffu ? 0u : h_qlen_[b])) * (double) seq_res;
                 padded += 2.0 * qp_rows[i] * (double) total_cols;
             }
             fprintf( stderr, "[ssa timing] qpair class R=%d: %zu pairs, %.3f ms, %.3e cells (%.1f%% of computed), "
