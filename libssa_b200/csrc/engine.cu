@@ -1078,15 +1078,27 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     // classes: [columns per step 1 or 4][R = 8, 16, 24, 32]
     std::vector<std::vector<uint32_t>> by_r( 8 );
     // The table's costs of a small database include the latency of its longest
-    // pairs, which are streamed here, so those of a large one choose better long
-    // before 50,000 sequences.  Mean length 350, queries of 50-1,500: calls on
-    // 48,000 / 31,000 / 22,000 / 15,000 sequences 1.35 / 1.24 / 1.10 / 1.07 times as
-    // fast, the slowest query 1.00 / 1.01 / 0.81 / 0.89.  Mean lengths 150, 800 and
-    // 1,500 gain as much on average but lose up to 0.83 at 30,000 for one query or
-    // another, and keep the table's line.
+    // pairs, which are streamed here, so those of a large one choose better before
+    // 50,000 sequences, as long as that shape's groups each have work: at least five
+    // pairs and passes for four groups.  Where it has fewer, its more rows per thread
+    // only make every pair slower (80 x 30,000 proteins: 18,944 groups of 4 threads
+    // and 24 rows for 15,000 pairs, 0.68 ms; the small database's shape 0.60).
+    // Mean lengths 250-500, queries of 30-2,000: calls on 30,000 / 38,000 / 49,999
+    // sequences 1.22 / 1.28 / 1.33 times as fast, none slower than 0.98.  From 30,000
+    // on, and for these mean lengths: at 20,000 a call gains 1.11 on average and the
+    // slowest is 0.98; mean length 60 loses up to 0.54, 150 0.82, 800 0.90 and 1,500
+    // 0.85 for one query or another, and keep the table's line.
     const size_t n_ne = db_.order_desc.size();
-    const bool middling = db_.mean_len >= 250.0 && db_.mean_len < 500.0;
-    const int bucket = db_bucket( db_.mean_len, middling && n_ne >= 30000 ? std::max<size_t>( n_ne, 50000 ) : n_ne );
+    const int bucket = db_bucket( db_.mean_len, n_ne );
+    const bool middling = db_.mean_len >= 250.0 && db_.mean_len < 500.0 && n_ne >= 30000;
+    const int crowded = middling ? db_bucket( db_.mean_len, std::max<size_t>( n_ne, 50000 ) ) : bucket;
+    auto shape_of = [&]( uint32_t Q ) {
+        const FastShape f = choose_shape( Q, db_.mean_len, crowded );
+        if( crowded == bucket || !f.G ||
+                4ull * n_pairs * (uint64_t) f.P >= 5ull * (uint64_t) sms_ * 16 * (uint64_t) (32 / f.G) )
+            return f;
+        return choose_shape( Q, db_.mean_len, bucket );
+    };
     // SSA_B200_FAST_SHAPE=G,R[,C] pins the shape and the kernel (tuning, tests)
     int pin_g = 0, pin_r = 0, pin_c = 1;
     if( const char * pin = getenv( "SSA_B200_FAST_SHAPE" ) ) {
@@ -1098,7 +1110,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
             pin_g = pin_r = 0;
     }
     for( uint32_t s = 0; s < nq; s++ ) {
-        shape[s] = choose_shape( h_qlen_[s], db_.mean_len, bucket );
+        shape[s] = shape_of( h_qlen_[s] );
         if( pin_g && shape[s].G ) {
             const uint32_t per = (uint32_t) (pin_g * pin_r);
             const uint32_t P = (h_qlen_[s] + per - 1) / per;
