@@ -956,7 +956,7 @@ public:
     struct Costs {
         double step, alone0, alone1, stream;
     };
-    static constexpr Costs SW_SINGLE{ 2.8, 1430, 30, 450 }, SW_PAIRS{ 2.4, 1500, 25, 225 }, NW_PAIRS{ 1.3, 700, 60, 130 };
+    static constexpr Costs SW_SINGLE{ 2.8, 1430, 30, 520 }, SW_PAIRS{ 2.4, 1500, 25, 225 }, NW_PAIRS{ 1.3, 700, 60, 130 };
     // A query, or pair of queries, of the entry kernel.
     struct Query {
         uint64_t passes;
