@@ -1843,19 +1843,41 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
     const uint32_t rows = 32u * (uint32_t) R;
     const uint32_t ni = (uint32_t) items.size();
     const bool blocks = req.bit_width == 8;       // Smith-Waterman 8-bit entry
-    // launches of as many items as 1 GB of boundary rows holds
-    for( uint32_t i0 = 0; i0 < ni; ) {
-        std::vector<uint64_t> bnd;
-        bnd.reserve( ni - i0 );
-        uint64_t words = 0;
-        uint32_t i1 = i0;
-        for( ; i1 < ni; i1++ ) {
-            const uint64_t w = h_qlen_[items[i1].slot] > rows ? 2ull * ((len[i1] + 3u) / 4u) : 0;
-            if( i1 > i0 && (words + w) * sizeof(int4) > ((uint64_t) 1 << 30) )
-                break;
-            bnd.push_back( words );
+    // Launches of as many items as 1 GB of boundary rows and ticket words holds
+    // (SSA_B200_STREAM_MEMORY: another limit, for tests).  The buffers are those of the
+    // largest: growing one would free it behind the launch before.
+    uint64_t most = (uint64_t) 1 << 30;
+    if( const char * m = getenv( "SSA_B200_STREAM_MEMORY" ) )
+        most = strtoull( m, nullptr, 10 );
+    std::vector<uint64_t> bnd( ni );             // per item, from the start of its launch's rows
+    std::vector<uint32_t> part_end;
+    uint64_t most_words = 0, most_sync = 0;
+    {
+        uint64_t words = 0, sync = 16;
+        for( uint32_t i = 0; i < ni; i++ ) {
+            const uint32_t q = h_qlen_[items[i].slot];
+            const uint64_t w = q > rows ? 2ull * ((len[i] + 3u) / 4u) : 0;
+            // progress and result of every stripe, and the first crossings
+            const uint64_t t = (uint64_t) ((q + rows - 1u) / rows) * 2 * sizeof(uint32_t) + (blocks ? 2 * sizeof(int32_t) : 0);
+            if( i > (part_end.empty() ? 0 : part_end.back()) && (words + w) * sizeof(int4) + sync + t > most ) {
+                part_end.push_back( i );
+                words = 0;
+                sync = 16;
+            }
+            bnd[i] = words;
             words += w;
+            sync += t;
+            most_words = std::max( most_words, words );
+            most_sync = std::max( most_sync, sync );
         }
+        part_end.push_back( ni );
+    }
+    uint8_t * sy = (uint8_t *) d_sw_sync_.ensure( most_sync );
+    int4 * boundary = (int4 *) d_sw_bnd_.ensure( most_words * sizeof(int4) + 16 );
+    if( getenv( "SSA_B200_TIMING" ) )
+        fprintf( stderr, "[ssa timing] %u items on streamed stripes in %zu launches\n", ni, part_end.size() );
+    uint32_t i0 = 0;
+    for( const uint32_t i1 : part_end ) {
         const uint32_t n = i1 - i0;
         std::vector<uint32_t> cum{ 0 };
         for( uint32_t left = n, i = 0;; i++ ) {
@@ -1866,13 +1888,12 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
             cum.push_back( cum.back() + left );
         }
         const SwStreamItem * dev_items = stage_.add( items.data() + i0, n, st );
-        const uint64_t * dev_bnd = stage_.add( bnd.data(), n, st );
+        const uint64_t * dev_bnd = stage_.add( bnd.data() + i0, n, st );
         const uint32_t * dev_cum = stage_.add( cum.data(), cum.size(), st );
         stage_.send( st );
         const uint32_t nt = cum.back();
         // ticket counter, progress, results, and per sequence its first crossing
         const size_t b_zero = 16 + (size_t) nt * sizeof(uint32_t), b_cross = blocks ? n * 2 * sizeof(int32_t) : 0;
-        uint8_t * sy = (uint8_t *) d_sw_sync_.ensure( b_zero + (size_t) nt * sizeof(uint32_t) + b_cross );
         CUDA_CHECK( cudaMemsetAsync( sy, 0, b_zero, st ) );
         SwStreamParams p{};
         p.db = db_view();
@@ -1898,7 +1919,7 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
             p.cross = (int32_t *) (p.result + nt);
             CUDA_CHECK( cudaMemsetAsync( p.cross, 0x7f, b_cross, st ) );
         }
-        p.boundary = (int4 *) d_sw_bnd_.ensure( words * sizeof(int4) + 16 );
+        p.boundary = boundary;
         p.sink = lists;
         p.sink.score = score_sink();
         p.sink.score_stride = db_.n_ids;
