@@ -386,11 +386,13 @@ public:
         db.pair_cols.resize( n_pairs );
         db.pair_a.resize( n_pairs );
         db.pair_b.resize( n_pairs );
+        db.pair_blocks.assign( n_pairs + 1, 0 );
         std::vector<uint64_t> pair_off( n_pairs + 1, 0 );
         for( size_t pi = 0; pi < n_pairs; pi++ ) {
             db.pair_a[pi] = db.order_desc[2 * pi];
             db.pair_b[pi] = (2 * pi + 1 < db.order_desc.size()) ? db.order_desc[2 * pi + 1] : 0xffffffffu;
             db.pair_cols[pi] = (db.len[db.pair_a[pi]] + 7u) & ~7u;
+            db.pair_blocks[pi + 1] = db.pair_blocks[pi] + db.pair_cols[pi] / 4u;
             pair_off[pi + 1] = pair_off[pi] + 2ull * db.pair_cols[pi];
         }
         std::vector<uint8_t> pair_res( pair_off[n_pairs] + 16, (uint8_t) FAST_PAD_CODE );
@@ -1148,12 +1150,7 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     // (no idle groups) and, where the columns allow, no more: on a small
     // database the longest pairs then run side by side in separate warps
     // instead of one after another in the same warp.
-    std::vector<uint64_t> & blocks = blocks_before_;     // of four columns, of the pairs before each
-    blocks.resize( n_pairs + 1 );
-    blocks[0] = 0;
-    for( uint32_t k = 0; k < n_pairs; k++ )
-        blocks[k + 1] = blocks[k] + db_.pair_cols[k] / 4u;
-    const uint64_t total_cols = 4 * blocks[n_pairs];
+    const uint64_t total_cols = 4 * db_.pair_blocks[n_pairs];
     int g_min = 32;
     for( uint32_t s = 0; s < nq; s++ )
         if( shape[s].G )
@@ -1201,7 +1198,8 @@ void Engine::run_fast_entry( const SearchRequest & req, uint32_t nq, PairTask * 
     if( nq == 1 && n_shaped == 1 && (!pin_g || getenv( "SSA_B200_STREAM_SHARE" )) ) {
         const FastShape & fs = shape[0];
         const std::vector<StreamLine::Query> queries{ { (uint64_t) fs.P, fs.R, fs.C != 4, { h_qlen_[0], 0 }, 0 } };
-        pair_skip = StreamLine( StreamLine::SW_SINGLE, false, sms_, 32 / fs.G, 1, blocks, queries ).end( queries[0] );
+        pair_skip = StreamLine( StreamLine::SW_SINGLE, false, sms_, 32 / fs.G, 1, db_.pair_blocks, queries )
+                .end( queries[0] );
         for( uint32_t k = 0; k < pair_skip; k++ )
             items.push_back( SwStreamItem{ 0, db_.pair_a[k], db_.pair_b[k], 0 } );
     }

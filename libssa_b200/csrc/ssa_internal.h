@@ -65,6 +65,7 @@ struct HostDb {
     // column counts (the interleaved residues live only in HBM)
     std::vector<uint32_t> pair_cols;
     std::vector<uint32_t> pair_a, pair_b;   // pair_b = 0xffffffff when absent
+    std::vector<uint64_t> pair_blocks;      // blocks of four columns of the pairs before each, and of all
     double mean_len = 0;
     uint64_t residues = 0;
     uint32_t max_len = 0;
