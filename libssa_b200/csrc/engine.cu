@@ -116,6 +116,14 @@ struct DevView {
     }
 };
 
+// Most pinned memory that one buffer keeps for later calls, where its size follows
+// from a call's work and not from the database (SSA_B200_PINNED_KEPT: another bound,
+// for tests).
+static size_t pinned_kept() {
+    const char * e = getenv( "SSA_B200_PINNED_KEPT" );
+    return e ? strtoull( e, nullptr, 10 ) : (size_t) 64 << 20;
+}
+
 // The small arrays of one call on their way to the device: gathered in pinned
 // memory and sent in one copy.  (A copy from pageable memory costs the host
 // several microseconds, and a call has a dozen of them.)
@@ -124,6 +132,10 @@ public:
     // A new call: the device has finished the one before.
     void begin() {
         used_ = sent_ = 0;
+        if( h_.bytes > pinned_kept() ) {         // a call with very many pairs
+            h_.release();
+            d_.release();
+        }
         for( auto & o : old_ ) {
             o.first.release();
             o.second.release();
@@ -2453,7 +2465,9 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
                 r_len = res.add( nw * sizeof(uint32_t) ), r_ops = res.add( paths ? ops_bytes : 0 );
         uint8_t * din = (uint8_t *) d_tb_io_.ensure( in.bytes + res.bytes );
         uint8_t * dout = din + o_reg;            // the regions and flags of the inputs are the first results
-        uint8_t * hout = (uint8_t *) h_tb_out_.ensure( res.bytes );
+        // (the moves of a wave of chromosome-sized hits: pageable, and given back)
+        std::vector<uint8_t> large( res.bytes > pinned_kept() ? res.bytes : 0 );
+        uint8_t * hout = large.empty() ? (uint8_t *) h_tb_out_.ensure( res.bytes ) : large.data();
         p.error_flags = (unsigned *) (dout + r_err);
         // progress of both sweeps, ticket counters and column limits: cleared
         // by one memset (the limits to a large positive number)
