@@ -285,7 +285,7 @@ struct SwStreamParams {
     bool marked_only;             // as in QPairParams
 };
 
-// R: query rows per lane (4 or 8; Needleman-Wunsch: 4)
+// R: query rows per lane (4 to 6; Needleman-Wunsch: 4)
 cudaError_t launch_sw_stream( int R, const SwStreamParams & p, int sms, cudaStream_t st );
 cudaError_t launch_nw_stream( const SwStreamParams & p, int sms, cudaStream_t st );
 

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__( 256 ) emul_kernel( EmulParams p ) {
             prof = p.qv.prof32 + p.qv.prof32_off[slot];
         const uint32_t passes = (Q + EMUL_ROWS - 1) / EMUL_ROWS;
 
-        V s_run = SW ? SW_ZERO : (V) 0;              // last lane, final pass
+        V s_run = SW ? SW_ZERO : (V) 0;              // last lane: the rows so far
         V blk_min = 0, blk_max = 0;
         int first_ovf = -1;
         V nw_score = 0;

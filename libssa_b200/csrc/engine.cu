@@ -18,6 +18,7 @@
 //      (replay.cpp) to get the exact CPU hit list;
 //   5. for COMPUTE_ALIGNMENT the hits go through the traceback kernels.
 #include "device_common.cuh"
+#include "stream_stripes.cuh"
 #include "ssa_internal.h"
 #include "libssa_extern_db.h"
 
@@ -1057,7 +1058,7 @@ private:
                 const double stripes = (rows + 127u) / 128u;
                 work += stripes * (cols + 31.0 * n) / item_units_ * costs_.stream / (4.0 * sms_);
                 items += n / item_units_;
-                last = std::max( last, ((double) unit( from ) + 47.0 * stripes) * STREAM_ALONE );
+                last = std::max( last, ((double) unit( from ) + STREAM_LAG * stripes) * STREAM_ALONE );
             }
         }
         for( const Query & q : queries_ ) {
@@ -1847,7 +1848,7 @@ void Engine::run_stream( const SearchRequest & req, std::vector<SwStreamItem> & 
     uint64_t steps = 0, longest = 1;
     for( const Run & q : runs ) {
         steps += stripes( q, R ) * q.columns;
-        longest = std::max( longest, q.longest + 47 * stripes( q, R ) );
+        longest = std::max( longest, q.longest + STREAM_LAG * stripes( q, R ) );
     }
     const int ctas = (int) std::min<uint64_t>( 4, std::max<uint64_t>( 2, steps / ((uint64_t) sms_ * 4 * longest) ) );
     const uint32_t rows = 32u * (uint32_t) R;
@@ -2600,7 +2601,7 @@ void Engine::traceback( const SearchRequest & req, std::vector<std::vector<Hit>>
         // Rows per lane: 4, or 2 in the Smith-Waterman sweep of a few long hits.  A
         // warp alone on its sub-partition takes 352 ns for a step of 4 rows and 274
         // for one of 2 (Needleman-Wunsch: 270 for both), but 2 make twice the
-        // stripes, each 63 steps behind the one above: it pays from hits five
+        // stripes, each 48 steps behind the one above: it pays from hits five
         // times as long as high, while each stripe has a sub-partition and the
         // twice as many direction words are one wave.  10 hits of 300 x 33,000:
         // 3.8 ms with 4, 2.9 with 2; of 375 x 380 0.12 and 0.16.  SSA_B200_TB_ROWS
@@ -2713,8 +2714,7 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
     if( units.size() != n )
         fatal( "Internal error: pairs without a database sequence." );
     const int64_t mabs = max_abs_step( req );
-    std::vector<uint32_t> work;     // pairs with a non-empty sequence, largest first
-    uint32_t max_b = 0, max_a = 0;
+    bool any = false;               // pairs with a non-empty sequence
     for( uint32_t i = 0; i < n; i++ ) {
         if( units[i] >= db.n_ids )
             fatal( "Internal error: database unit %u out of range.", units[i] );
@@ -2724,21 +2724,18 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
         stats.cells += (uint64_t) A * B;
         if( B == 0 )
             continue;       // the reference never searches an empty sequence
-        work.push_back( i );
-        max_b = std::max( max_b, B );
-        max_a = std::max( max_a, A );
+        any = true;
+        Hit h;
+        h.unit = units[i];
+        h.id = units[i] / db.upi;
+        out[i].push_back( h );
     }
-    std::stable_sort( work.begin(), work.end(), [&]( uint32_t x, uint32_t y ) {
-        return (uint64_t) queries[x].len * db.len[units[x]] > (uint64_t) queries[y].len * db.len[units[y]];
-    } );
-    const bool timing = getenv( "SSA_B200_TIMING" ) != nullptr;
     CUDA_CHECK( cudaEventRecord( ev0_, stream_ ) );
     stage_.begin();
     upload_queries( req, queries.data(), n, false, stats );
     stage_.send( stream_ );
     d_counts_.ensure( 32 * sizeof(unsigned long long) );
     CUDA_CHECK( cudaMemsetAsync( d_counts_.p, 0, 32 * sizeof(unsigned long long), stream_ ) );
-    const uint32_t nw = (uint32_t) work.size();
     // With alignments the traceback passes compute the score themselves: the
     // direction pass ends on cell (A - 1, B - 1) of the same recurrence
     // (Needleman-Wunsch), the forward region pass finds the same maximum when
@@ -2748,14 +2745,7 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
         for( int q = 0; q < 32; q++ )
             symmetric = symmetric && req.matrix[(d << 5) + q] == req.matrix[(q << 5) + d];
     const bool scores_in_traceback = req.align_type == COMPUTE_ALIGNMENT && (req.algo == 1 || symmetric);
-    for( uint32_t k = 0; k < nw; k++ ) {
-        const uint32_t i = work[k];
-        Hit h;
-        h.unit = units[i];
-        h.id = units[i] / db.upi;
-        out[i].push_back( h );
-    }
-    if( nw && !scores_in_traceback ) {
+    if( any && !scores_in_traceback ) {
         std::vector<std::pair<uint32_t, uint32_t>> lists;
         for( uint32_t i = 0; i < n; i++ )
             if( !out[i].empty() )
@@ -2766,7 +2756,7 @@ void Engine::align_pairs( const SearchRequest & req, const std::vector<QueryCode
         stats.entry_seconds += seconds;
         stats.kernel_seconds += seconds;
     }
-    if( req.align_type == COMPUTE_ALIGNMENT && nw ) {
+    if( req.align_type == COMPUTE_ALIGNMENT && any ) {
         std::vector<std::pair<uint32_t, uint32_t>> lists;
         for( uint32_t i = 0; i < n; i++ )
             if( !out[i].empty() )

@@ -37,6 +37,9 @@ namespace ssa {
 // stripe but cost a fence every 8 steps (10 hits of 300 x 33,000: 3.8 ms against
 // 4.2, 48 long pairs 20.2 against 21.1).
 constexpr uint32_t STREAM_CHUNK = 16;
+// Steps from a stripe to the next at the same speed: a chunk starts when the chunk
+// above that holds its last block, 31 steps further on, has ended.
+constexpr uint32_t STREAM_LAG = 48;
 constexpr uint32_t STREAM_DONE = 0x80000000u;         // progress word: the stripe has ended
 constexpr uint32_t STREAM_WAIT_LIMIT = 1u << 24;      // polls of 100 ns and more each
 
@@ -133,12 +136,6 @@ struct StreamStripe {
     uint32_t * mine;               // this stripe's progress
     bool last;                     // no stripe below
     unsigned * error_flags;
-};
-
-// No column limit.
-struct StreamAll {
-    static constexpr bool NONE = true;
-    __device__ int32_t operator()() const { return 0; }
 };
 
 // Sweeps one stripe, 16 steps (a chunk) at a time.  limit() reads the last block

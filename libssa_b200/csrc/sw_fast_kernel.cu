@@ -315,7 +315,7 @@ cudaError_t launch_sw_fast( int R, const FastParams & p, int grid, cudaStream_t 
 // profile word and half a 3-way max for the running maximum, 5.5 ALU
 // instructions and one IADD per cell pair (the one-column kernel above needs
 // 7 and 2 to keep its row-to-row chain at one instruction).  Each thread
-// records the first block in which its own running maximum reached 255; the
+// records the first block in which its own running maximum reached the limit (255 at 8 bits); the
 // group's minimum over threads and passes is the reference lane's overflow
 // block.  A block's residues are one 8-byte load (4 columns x 2 sequences),
 // read with the streaming cache operator; the boundary row of a multi-pass
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__( 128, 4 ) sw_fast4_kernel( FastParams p ) {
                         out_h[j] = hv[j][R - 1];
                         out_f[j] = f[j];
                     }
-                    // first block at which this thread's maximum reached 255
+                    // first block at which this thread's maximum reached the limit
                     const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )

@@ -26,7 +26,7 @@
 //   * H and F of the bottom rows of both columns go to thread k + 1 by
 //     shuffle; the running maximum is kept per thread and combined over the
 //     group only at the end of the sequence, together with the first column
-//     pair at which each thread's maximum reached 255;
+//     pair at which each thread's maximum reached the limit (255 at 8 bits);
 //   * queries longer than QP_G x R rows take several passes over a sequence;
 //     the bottom row's H and F go through a per-group scratch row in global
 //     memory, read back by thread 0 two steps ahead;
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
             const uint8_t * res = p.db.codes + (valid ? p.db.offsets[id] : 0ull);
 
             // per thread over all passes: running maximum and the first column
-            // pair at which it reached 255 (per half)
+            // pair at which it reached the limit (per half)
             uint32_t best = QP_BIAS2;
             int cross_a = INT_MAX, cross_b = INT_MAX;
 
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
                     out_f0 = fa;
                     out_h1 = H[R - 1];
                     out_f1 = fb;
-                    // first column pair at which this thread's maximum reached 255
+                    // first column pair at which this thread's maximum reached the limit
                     const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )
@@ -268,11 +268,11 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
 // ---------------------------------------------------------------------------
 // The same pass, one 4-column block per step: a thread interleaves four
 // columns (cell (r, c + j) in row iteration r + j, j = 0..3), four independent
-// dependency chains instead of two.  The semantics, the group layout, the
-// profile slices and the scheduling are those of sw_qpair_kernel; a step reads
+// dependency chains instead of two.  The semantics and the group layout are those
+// of sw_qpair_kernel, profile slices and work units the CTA's (below); a step reads
 // one 32-bit word of residues (the block) and crosses the pass boundary as two
 // int4 per block (H and F of the bottom row, four columns).  The running
-// maximum's first crossing of 255 is recorded per block directly.
+// maximum's first crossing of the limit is recorded per block directly.
 //
 // H[r] holds column c - 1 (the previous step's last column) until chain 3
 // overwrites it with column c + 3 (iteration r + 3); chain j reads the
@@ -282,12 +282,14 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair_kernel( QPairParams
 // The running maximum of H as fp16x2: every H is at least the bias (1024, the
 // fp16 bit pattern of a positive normal number), and positive fp16 values
 // order like their bit patterns, so a half-precision max of the bit patterns
-// is the integer max.  Patterns past 0x7c00 (infinity, NaN) -- scores more
-// than 30,000 above the bias -- are ignored or taken as the largest; a cell
-// only gets there through cells that crossed 255 earlier on its path, whose
-// own crossing is recorded, so the first crossing and every reported score
-// (below 255) are unchanged.  This max issues to another pipe than the
-// integer ALU, which the rest of the recurrence saturates.
+// is the integer max.  Patterns from 0x7c00 (infinity, NaN) on are ignored or
+// taken as the largest.  Biased, the limit is 0x7c00 less the largest score-table
+// entry (sw_fast_limit in engine.cu), or 1024 + 255 at 8 bits: a cell gets to 0x7c00
+// only along a path whose cells rise by at most one entry each, so one of them is a
+// finite value at or above the limit, and that one is recorded.  So the first
+// crossing and every reported score (below the limit) are those of the integer
+// maximum.  This max issues to another pipe than the integer ALU, which the rest of
+// the recurrence saturates.
 __device__ __forceinline__ uint32_t hmax_bits( uint32_t a, uint32_t b ) {
     uint32_t r;
     asm( "max.f16x2 %0, %1, %2;" : "=r"( r ) : "r"( a ), "r"( b ) );
@@ -614,7 +616,7 @@ __global__ void __launch_bounds__( QP_THREADS, MB ) sw_qpair4_kernel( QPairParam
                         out_h[j] = hv[j][R - 1];
                         out_f[j] = f[j];
                     }
-                    // first block at which this thread's maximum reached 255
+                    // first block at which this thread's maximum reached the limit
                     const uint32_t ge = (smax + CROSS_ADD) & 0x80008000u;
                     if( ge != seen ) {
                         if( (ge & 0x8000u) && !(seen & 0x8000u) )

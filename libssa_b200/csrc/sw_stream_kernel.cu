@@ -16,7 +16,7 @@
 // skewed dependency chains, 5.5 ALU instructions and one IADD per cell pair.
 // Bound by the ALU pipe when many pairs are re-queued (78 % of its cycles; what
 // is left is padding of the last stripe and 20 instructions a step besides the
-// cells), by the latency of one warp's steps (blocks + 47 x stripes) when few
+// cells), by the latency of one warp's steps (blocks + STREAM_LAG x stripes) when few
 // are.  The host picks R (4 to 6) and the CTAs per SM (2 to 4) for each launch.
 // Measured on a B200 against the lane emulation (one warp per pair, int32): 102
 // pairs of 375 rows x 380 columns 0.50 -> 0.12 ms; 1,927 of 300 x 21,000 38.7 ->

@@ -27,7 +27,7 @@
 //
 // What bounds it: the integer ALU pipe (16 lanes per clock per SM
 // sub-partition) when many hits fill the GPU, the latency of one warp's steps
-// (blocks + 48 x stripes of them per hit) when few do.  A step interleaves the
+// (blocks + STREAM_LAG x stripes of them per hit) when few do.  A step interleaves the
 // four columns of a block row by row (cell (it - j, j) in iteration `it`): four
 // independent dependency chains where one column at a time has one, and the
 // step's fixed work (shuffles, residues, boundary, stores) once per 4 R cells.
