@@ -1541,7 +1541,7 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     const uint32_t * dev_lmax = stage_.add( qp_lmax.data(), qp_lmax.size(), stream_ );
     // Pairs outside the kernels' range, for the lane emulation (the 8-bit entry has
     // none).  Needleman-Wunsch: the sequences longer than a pair of queries' limit,
-    // which the emulation scores beside the entry pass (`beyond`); of a marked pass
+    // which the emulation scores beside the entry pass (run_beyond); of a marked pass
     // only the device knows which of them it wants.
     const bool redo = nw ? marked : req.bit_width != 8;
     unsigned * redo_count = d_counts_.as<unsigned>() + 5;
@@ -1632,25 +1632,48 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
     // After the pass / beside it, one query against proteins of mean length 350
     // (calls on a B200): 64-bit entry 1,300 x 1,000 6.4 / 4.0 ms, 2,000 x 10,000 12.2 /
     // 7.9; 16-bit entry 2,000 x 10,000 15.4 / 11.6; 15,289 pairs of 2,500 28.0 / 30.6.
-    std::vector<PairTask> beyond;
-    for( uint32_t k = 0; nw && !marked && k < n_seq; k++ ) {
-        const uint32_t id = db_.order_desc[lo + k];
-        bool any = false;
-        for( uint32_t i = 0; i < n_qp; i++ ) {
-            if( db_.len[id] <= qp_lmax[i] )
-                continue;
-            any = true;
-            for( int h = 0; h < 2 && (k < qp_skip[i].x || k >= qp_skip[i].y); h++ )
-                if( qp_slots[2 * i + h] != 0xffffffffu )
-                    beyond.push_back( PairTask{ qp_slots[2 * i + h], id, 0, 0 } );
-        }
-        if( !any )                      // nor is a shorter one
-            break;
+    uint64_t n_beyond = 0;
+    std::vector<uint32_t> beyond_end( n_qp, 0 );     // the first sequence within each pair's range
+    for( uint32_t i = 0; i < n_qp && nw && !marked; i++ ) {
+        beyond_end[i] = (uint32_t) (std::partition_point( db_.order_desc.begin() + lo, db_.order_desc.begin() + hi,
+                [&]( uint32_t id ) { return db_.len[id] > qp_lmax[i]; } ) - (db_.order_desc.begin() + lo));
+        n_beyond += (uint64_t) beyond_end[i] * (qp_slots[2 * i + 1] == 0xffffffffu ? 1 : 2);
     }
-    const PairTask * beyond_tasks = stage_.add( beyond.data(), beyond.size(), stream_ );
-    const bool beside = beyond.size() <= (size_t) sms_ * 64;
+    const bool beside = n_beyond <= (uint64_t) sms_ * 64;
+    // in lists of at most this many, so that a query longer than the range itself,
+    // whose pairs are all beyond, takes no memory of the database's size
+    const size_t beyond_cap = std::min<size_t>( cap, (size_t) 1 << 20 );
+    auto run_beyond = [&]() {
+        std::vector<PairTask> tasks;
+        auto flush = [&]() {
+            if( tasks.empty() )
+                return;
+            const PairTask * dev;
+            if( beside ) {
+                dev = stage_.add( tasks.data(), tasks.size(), stream_ );
+            }
+            else {
+                dev = (const PairTask *) d_list_c_.ensure( beyond_cap * sizeof(PairTask) );
+                CUDA_CHECK( cudaMemcpyAsync( d_list_c_.p, tasks.data(), tasks.size() * sizeof(PairTask),
+                        cudaMemcpyHostToDevice, stream_ ) );
+            }
+            run_pass( 1, req.bit_width, req, nq, dev, tasks.size(), false, next, next_count, cap );
+            tasks.clear();
+        };
+        const uint32_t last = n_qp ? *std::max_element( beyond_end.begin(), beyond_end.end() ) : 0;
+        for( uint32_t k = 0; k < last; k++ )
+            for( uint32_t i = 0; i < n_qp; i++ )
+                for( int h = 0; h < 2 && k < beyond_end[i] && (k < qp_skip[i].x || k >= qp_skip[i].y); h++ ) {
+                    if( qp_slots[2 * i + h] == 0xffffffffu )
+                        continue;
+                    tasks.push_back( PairTask{ qp_slots[2 * i + h], db_.order_desc[lo + k], 0, 0 } );
+                    if( tasks.size() == beyond_cap )
+                        flush();
+                }
+        flush();
+    };
     if( beside )
-        run_pass( 1, req.bit_width, req, nq, beyond_tasks, beyond.size(), false, next, next_count, cap );
+        run_beyond();
     if( !items.empty() ) {
         PassSink lists{};
         lists.next = next;
@@ -1773,10 +1796,10 @@ void Engine::run_qpair_entry( const SearchRequest & req, uint32_t nq, PairTask *
         }
     }
     if( timing )
-        fprintf( stderr, "[ssa timing] %zu pairs beyond the 16-bit range, %s the entry pass\n", beyond.size(),
-                beside ? "beside" : "after" );
+        fprintf( stderr, "[ssa timing] %llu pairs beyond the 16-bit range, %s the entry pass\n",
+                (unsigned long long) n_beyond, beside ? "beside" : "after" );
     if( !beside )
-        run_pass( 1, req.bit_width, req, nq, beyond_tasks, beyond.size(), false, next, next_count, cap );
+        run_beyond();
     if( !fallback.empty() ) {
         const uint32_t * dev_slots = stage_.add( fallback.data(), fallback.size(), stream_ );
         run_pass( req.algo, req.bit_width, req, nq, nullptr, (uint64_t) fallback.size() * n_seq, true, next,

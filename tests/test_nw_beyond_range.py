@@ -42,9 +42,12 @@ def test_records_around_the_limit(built_library, monkeypatch, capfd, width, shar
     assert max(int(n) for n, _ in found) > 20 and all(where == "beside" for _, where in found)
 
 
-def test_many(built_library, monkeypatch, capfd):
+@pytest.mark.parametrize("cap", [None, "700"])
+def test_many(built_library, monkeypatch, capfd, cap):
     """16 x BLOSUM62, a step of 176 at most: a limit of 170 columns less the
-    query's rows, which 10,500 pairs exceed."""
+    query's rows, which 10,500 pairs exceed; in one list, and in lists of 700."""
+    if cap is not None:
+        monkeypatch.setenv("SSA_B200_REQUEUE_CAP", cap)
     rng = np.random.default_rng(72)
     queries = [W.random_residues(rng, n, W.AA20) for n in (41, 45, 50, 55, 60)]
     records = [W.random_residues(rng, int(n), W.AA20) for n in rng.integers(140, 160, 2100)]
